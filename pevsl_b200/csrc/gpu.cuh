@@ -75,6 +75,7 @@ enum Ws {
   WS_GEN,       /* generalized problem: filter / KPM vectors  */
   WS_IL,        /* interleaved filter: three n x S blocks     */
   WS_ILMU,      /* interleaved filter: per-degree coefficients */
+  WS_CLMU,      /* cluster filter: one polynomial's coefficients */
   WS_COUNT
 };
 
@@ -290,6 +291,26 @@ int cheb_filter_persistent(int ne, const FiltDev *entries, int maxdeg);
 int persistent_filter_error();
 void set_barrier_spins(unsigned spins);
 int seed_barrier_arrivals(unsigned count);
+
+/* One filter application y = p(A) x of a small problem by one thread-block
+ * cluster, all degrees in one launch (gpu_cluster.cu).  With B set each
+ * degree is preceded by the B-solve sum_j lmu[j] T_j((B - ccB)/ddB), j <=
+ * degB.  mu, lmu: device; deg, degB >= 1; y may alias x. */
+struct ClusterJob {
+  const pevsl_devcsr *A, *B;
+  const double *x;
+  double *y;
+  const double *mu, *lmu;
+  double cc, dd, ccB, ddB;
+  int deg, degB;
+};
+/* largest matrix of a cluster launch; pEVSL_ParcsrSetup finds the bandwidths
+ * of the matrices up to here */
+constexpr int kClusterMaxRows = 32768;
+/* whether the matrices fit the shared memory of a cluster */
+bool cluster_filter_ok(const pevsl_devcsr *A, const pevsl_devcsr *B, bool fp32);
+/* the applications of ne jobs, all with B or all without */
+int cluster_filter(int ne, const ClusterJob *jobs, bool fp32);
 
 /* ---------------------------------------------------------------- FP32 (mixed) */
 int csr_make_fp32(pevsl_devcsr *A); /* FP32 copy of the values, once */

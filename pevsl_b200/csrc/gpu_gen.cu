@@ -42,6 +42,7 @@ struct pevsl_lspol {
   int max_deg, deg;
   double intv[2], cc, dd, tol;
   double *mu;          /* host, max_deg */
+  double *dmu;         /* its deg + 1 coefficients on the device */
   pevsl_devcsr *B;
   double *wk;          /* device: 3 n doubles */
   MPI_Comm comm;
@@ -65,10 +66,14 @@ namespace {
 
 /* y = sum_k mu[k] T_k((M - cc)/dd) v on a device CSR: the filter
  * recurrence (pnav, SRC/lspolapprox.c:235-283).  w holds 3 n doubles; y
- * may alias v. */
-int cheb_series(const pevsl_devcsr *M, const double *mu, int m, double cc, double dd,
-                const double *v, double *y, double *w) {
+ * may alias v.  dmu: mu on the device. */
+int cheb_series(const pevsl_devcsr *M, const double *mu, const double *dmu, int m, double cc,
+                double dd, const double *v, double *y, double *w) {
   const long n = M->nrows;
+  if (m > 0 && cluster_filter_ok(M, nullptr, false)) {
+    const ClusterJob J{M, nullptr, v, y, dmu, nullptr, cc, dd, 0.0, 0.0, m, 0};
+    return cluster_filter(1, &J, false);
+  }
   if (y == v) {
     if (vcopy(v, w + 2 * n, n)) return PEVSL_ERR_CUDA;
     v = w + 2 * n;
@@ -91,7 +96,7 @@ int cheb_series(const pevsl_devcsr *M, const double *mu, int m, double cc, doubl
 
 int lspol_apply(pevsl_lspol *L, const double *b, double *x) {
   if (!L || !L->B) return PEVSL_ERR_ARG;
-  return cheb_series(L->B, L->mu, L->deg, L->cc, L->dd, b, x, L->wk);
+  return cheb_series(L->B, L->mu, L->dmu, L->deg, L->cc, L->dd, b, x, L->wk);
 }
 
 /* Chebyshev iteration, first kind (EXTERNAL/ITERSOL/chebiter.c:121-197),
@@ -317,6 +322,20 @@ double solve_bytes(pevsl_Data *pevsl) {
   return 0.0;
 }
 
+/* the least-squares B-solver of a problem whose filter applications run as
+ * one cluster launch (A and B resident in shared memory), or NULL */
+const pevsl_lspol *gen_cluster(pevsl_Data *pevsl) {
+  pevsl_devcsr *A = pevsl_builtin_A(pevsl);
+  if (!A || !pevsl->Bsol || pevsl->Bsol->func != pEVSL_LSPolSol) return nullptr;
+  const pevsl_lspol *L = (const pevsl_lspol *)pevsl->Bsol->data;
+  return L && L->B && L->deg >= 1 && cluster_filter_ok(A, L->B, false) ? L : nullptr;
+}
+
+ClusterJob gen_cluster_job(const pevsl_devcsr *A, const pevsl_lspol *L, const pevsl_Polparams *pol,
+                           const double *dmu, const double *x, double *y) {
+  return ClusterJob{A, L->B, x, y, dmu, L->dmu, pol->cc, pol->dd, L->cc, L->dd, pol->deg, L->deg};
+}
+
 /* The generalized filter (pEVSL_ChebAv with ifGenEv, SRC/chebpol.c:509-574):
  * y = p(A B^{-1}) v, each degree a B-solve then the fused degree kernel
  * whose SpMV reads B^{-1} v_k.  w holds 4 n doubles. */
@@ -338,6 +357,15 @@ int gen_filter(pevsl_Data *pevsl, const pevsl_Polparams *pol, const double *v, d
   }
   g_gen_degrees += (uint64_t)m;
   g_gen_filters++;
+  if (const pevsl_lspol *L = gen_cluster(pevsl)) {
+    double *dmu = (double *)ws(WS_CLMU, sizeof(double) * (size_t)(m + 1));
+    if (!dmu) return PEVSL_ERR_NOMEM;
+    if (memcpy_async(dmu, mu, sizeof(double) * (size_t)(m + 1))) return PEVSL_ERR_CUDA;
+    pevsl->stats->n_mvA += (size_t)m;
+    pevsl->stats->n_svB += (size_t)m;
+    const ClusterJob J = gen_cluster_job(A, L, pol, dmu, v, y);
+    return cluster_filter(1, &J, false);
+  }
   double *buf[2] = {w, w + n}, *w2 = w + 2 * n, *tmp = w + 3 * n;
   const double *vk = v, *vkm1 = nullptr;
   int st = 0;
@@ -1004,10 +1032,26 @@ struct GenIl {
   double cc = 0, dd = 0, ccB = 0, ddB = 0;
   double *blk = nullptr; /* X0, B0, B1, Y, W, L0, L1: n x S each */
   double *smu = nullptr, *lmu = nullptr; /* coefficient tables on the device */
+  /* cluster form: each slice one job of a launch, no interleaving */
+  const pevsl_lspol *cl = nullptr;
+  const pevsl_Polparams *pol[kMaxBatch] = {};
+  const double *dmu[kMaxBatch] = {};
   GenGraph graph;
   bool use_graph = false;
   double *X(int i) const { return blk + (size_t)i * (size_t)n * (size_t)S; }
 };
+
+/* statistics of one application up to degree deg */
+void genil_count(pevsl_Data *pevsl, const GenIl &G, int deg) {
+  pevsl->stats->n_mvA += (size_t)deg * G.S;
+  pevsl->stats->n_svB += (size_t)deg * G.S;
+  g_gen_filters++;
+  g_gen_degrees += (uint64_t)deg;
+  const double n = (double)G.n;
+  g_gen_bytes += (double)deg *
+                 (G.degB * (il_entry_bytes(G.B) * G.B->nnz + 4.0 * (n + 1) + 40.0 * n * G.S) +
+                  il_entry_bytes(G.A) * G.A->nnz + 4.0 * (n + 1) + 48.0 * n * G.S);
+}
 
 int genil_degrees(pevsl_Data *pevsl, GenIl &G) {
   const double *vk = G.X(0), *vkm1 = nullptr;
@@ -1029,20 +1073,28 @@ int genil_degrees(pevsl_Data *pevsl, GenIl &G) {
     vkm1 = vk;
     vk = vkp1;
   }
-  pevsl->stats->n_mvA += (size_t)G.maxdeg * G.S;
-  pevsl->stats->n_svB += (size_t)G.maxdeg * G.S;
-  g_gen_filters++;
-  g_gen_degrees += (uint64_t)G.maxdeg;
-  const double n = (double)G.n;
-  g_gen_bytes += (double)G.maxdeg *
-                 (G.degB * (il_entry_bytes(G.B) * G.B->nnz + 4.0 * (n + 1) + 40.0 * n * G.S) +
-                  il_entry_bytes(G.A) * G.A->nnz + 4.0 * (n + 1) + 48.0 * n * G.S);
+  genil_count(pevsl, G, G.maxdeg);
   return st;
 }
 
-/* one lockstep filter application: column c filters xs[c] into ys[c] */
-int genil_apply(pevsl_Data *pevsl, GenIl &G, const double *const *xs, double *const *ys) {
+/* one lockstep filter application: column c filters xs[c] into ys[c]; on
+ * marks the columns whose result is wanted */
+int genil_apply(pevsl_Data *pevsl, GenIl &G, const double *const *xs, double *const *ys,
+                const bool *on) {
   g_gen_ev.begin();
+  if (G.cl) {
+    ClusterJob jobs[kMaxBatch];
+    int nj = 0, dmax = 0;
+    for (int c = 0; c < G.S; c++)
+      if (on[c]) {
+        jobs[nj++] = gen_cluster_job(G.A, G.cl, G.pol[c], G.dmu[c], xs[c], ys[c]);
+        dmax = PEVSL_MAX(dmax, G.pol[c]->deg);
+      }
+    const int st = cluster_filter(nj, jobs, false);
+    genil_count(pevsl, G, dmax);
+    g_gen_ev.end();
+    return st;
+  }
   int st = il_pack(G.n, G.S, xs, G.X(0));
   if (!st) {
     if (G.use_graph)
@@ -1079,7 +1131,7 @@ int pevsl_gen_cheblannr(pevsl_Data *pevsl, double *intv, int maxit, double tol, 
   S.V = V;
   S.Z = Z;
   double *vrand = wf + 4 * ld, *xs = wf + 5 * ld, *ys = wf + 6 * ld;
-  const bool use_graph = graphable(pevsl);
+  const bool use_graph = !gen_cluster(pevsl) && graphable(pevsl);
   if (use_graph) pretune(pevsl);
   GenGraph fg;
   auto filter = [&](const double *in, double *out) -> int {
@@ -1159,12 +1211,22 @@ int pevsl_gen_cheblannr_lockstep(pevsl_Data *pevsl, int ns, const double *intvs,
   /* four filter work vectors, a random vector, one scratch output per
    * padding or finished column */
   double *wf = (double *)ws(WS_GEN, sizeof(double) * (5 + kMaxBatch) * (size_t)ld);
-  G.blk = (double *)ws(WS_IL, sizeof(double) * 7 * (size_t)n * (size_t)G.S);
+  G.cl = gen_cluster(pevsl);
+  if (!G.cl) G.blk = (double *)ws(WS_IL, sizeof(double) * 7 * (size_t)n * (size_t)G.S);
   double *mu = (double *)ws(WS_ILMU, sizeof(double) * (size_t)(G.maxdeg + 1 + G.degB + 1) * G.S);
-  if (!V || !Z || !wf || !G.blk || !mu) return PEVSL_ERR_NOMEM;
+  if (!V || !Z || !wf || (!G.blk && !G.cl) || !mu) return PEVSL_ERR_NOMEM;
   G.smu = mu;
   G.lmu = mu + (size_t)(G.maxdeg + 1) * G.S;
-  {
+  if (G.cl) {
+    /* one row of coefficients per slice */
+    for (int s = 0; s < ns; s++) {
+      G.pol[s] = &pols[s];
+      G.dmu[s] = mu + (size_t)s * (G.maxdeg + 1);
+      if (memcpy_async(mu + (size_t)s * (G.maxdeg + 1), pols[s].mu,
+                       sizeof(double) * (size_t)(pols[s].deg + 1)))
+        return PEVSL_ERR_CUDA;
+    }
+  } else {
     std::vector<double> tab((size_t)(G.maxdeg + 1 + G.degB + 1) * G.S, 0.0);
     for (int s = 0; s < ns; s++)
       for (int k = 0; k <= pols[s].deg; k++) tab[(size_t)k * G.S + s] = pols[s].mu[k];
@@ -1183,7 +1245,7 @@ int pevsl_gen_cheblannr_lockstep(pevsl_Data *pevsl, int ns, const double *intvs,
     }
   double *vrand = wf + 4 * ld;
   auto dummy = [&](int c) { return wf + (5 + (size_t)c) * ld; };
-  G.use_graph = graphable(pevsl);
+  G.use_graph = !G.cl && graphable(pevsl);
   if (G.use_graph) pretune(pevsl);
   auto filter1 = [&](const pevsl_Polparams *pol, const double *in, double *out) -> int {
     return gen_filter(pevsl, pol, in, out, wf, n);
@@ -1191,24 +1253,26 @@ int pevsl_gen_cheblannr_lockstep(pevsl_Data *pevsl, int ns, const double *intvs,
   /* filtered initial vectors of every slice in one application */
   const double *xs[kMaxBatch];
   double *ys[kMaxBatch];
+  bool live[kMaxBatch];
   for (int c = 0; c < G.S; c++) {
+    live[c] = c < ns && SL[c].active;
     xs[c] = vinit->data;
-    ys[c] = c < ns && SL[c].active ? SL[c].V : dummy(c);
+    ys[c] = live[c] ? SL[c].V : dummy(c);
   }
-  int st = genil_apply(pevsl, G, xs, ys);
+  int st = genil_apply(pevsl, G, xs, ys, live);
   for (int s = 0; s < ns && !st; s++)
     if (SL[s].active) st = gs_normalize0(pevsl, SL[s], n);
   for (;;) {
     if (st) break;
     bool any = false;
     for (int c = 0; c < G.S; c++) {
-      const bool on = c < ns && SL[c].active;
+      const bool on = live[c] = c < ns && SL[c].active;
       any = any || on;
       xs[c] = on ? SL[c].Z + (size_t)SL[c].k * ld : vinit->data;
       ys[c] = on ? SL[c].Z + (size_t)(SL[c].k + 1) * ld : dummy(c);
     }
     if (!any) break;
-    st = genil_apply(pevsl, G, xs, ys);
+    st = genil_apply(pevsl, G, xs, ys, live);
     for (int s = 0; s < ns && !st; s++) {
       if (!SL[s].active) continue;
       const pevsl_Polparams *pol = SL[s].pol;
@@ -1271,6 +1335,15 @@ void pEVSL_SetupLSPol(int max_deg, double tol, double lmin, double lmax, pevsl_P
     free(L);
     return;
   }
+  const size_t mub = sizeof(double) * (size_t)(L->deg + 1);
+  if (fail(cudaMalloc(&L->dmu, mub), "cudaMalloc lspol") || memcpy_async(L->dmu, L->mu, mub) ||
+      sync()) {
+    cudaFree(L->dmu);
+    cudaFree(L->wk);
+    free(L->mu);
+    free(L);
+    return;
+  }
   *vdata = L;
 }
 
@@ -1294,6 +1367,7 @@ void pEVSL_LSPolFree(void *vdata) {
   if (L->wk) {
     cudaStreamSynchronize(ctx().stream);
     cudaFree(L->wk);
+    cudaFree(L->dmu);
   }
   free(L->mu);
   free(L);

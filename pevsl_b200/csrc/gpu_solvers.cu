@@ -118,6 +118,17 @@ int cheb_apply(pevsl_Data *pevsl, const pevsl_Polparams *pol, const double *v, d
     return vscal(y, n, mu[0]);
   }
   if (!A && (!pevsl->Amv || !pevsl->Amv->func)) return PEVSL_ERR_NOMATVEC;
+  if (A && cluster_filter_ok(A, nullptr, false)) {
+    /* a small problem: every degree in one launch, the same bits */
+    double *dmu = (double *)ws(WS_CLMU, sizeof(double) * (size_t)(m + 1));
+    if (!dmu) return PEVSL_ERR_NOMEM;
+    if (memcpy_async(dmu, mu, sizeof(double) * (size_t)(m + 1))) return PEVSL_ERR_CUDA;
+    const ClusterJob J{A, nullptr, v, y, dmu, nullptr, cc, dd, 0.0, 0.0, m, 0};
+    for (int k = 1; k <= m; k++) g_filter_bytes += cheb_step_bytes(A, k == 1);
+    g_filter_launches += (uint64_t)m;
+    pevsl->stats->n_mvA += (size_t)m;
+    return cluster_filter(1, &J, false);
+  }
   double *buf[2] = {w3, w3 + n};
   double *ax = A ? nullptr : (double *)ws(WS_VEC, sizeof(double) * (size_t)n);
   if (!A && !ax) return PEVSL_ERR_NOMEM;
@@ -362,7 +373,9 @@ static int cheb_filter_batch(int ne, const FilterJob *jobs, bool fp32) {
       continue;
     }
     maxdeg = PEVSL_MAX(maxdeg, pol->deg);
-    if (fp32) st = cvt_f64_f32(n, J.x, (float *)J.work);
+    /* the cluster form converts its input itself */
+    if (fp32 && (filter_form() == 1 || !cluster_filter_ok(J.A, nullptr, true)))
+      st = cvt_f64_f32(n, J.x, (float *)J.work);
     live[nlive++] = e;
   }
   if (st || !nlive) return st;
@@ -440,10 +453,31 @@ static int cheb_filter_batch(int ne, const FilterJob *jobs, bool fp32) {
   }
   /* one launch per degree for all live entries; a matrix is read once per
    * launch for all entries on it.  Entries taken by interleaved groups run
-   * as one interleaved launch per group and degree instead. */
+   * as one interleaved launch per group and degree instead, small problems
+   * as one cluster launch for all their degrees. */
   std::vector<IlGroup> ig;
   std::vector<char> taken;
   il_partition(ne, jobs, fp32, ig, taken);
+  std::vector<ClusterJob> cj;
+  for (int i = 0; i < nlive; i++) {
+    const FilterJob &J = jobs[live[i]];
+    if (taken[(size_t)live[i]] || !cluster_filter_ok(J.A, nullptr, fp32)) continue;
+    taken[(size_t)live[i]] = 1;
+    cj.push_back(ClusterJob{J.A, nullptr, J.x, J.y, J.dmu, nullptr, J.pol->cc, J.pol->dd, 0.0, 0.0,
+                            J.pol->deg, 0});
+  }
+  if (!cj.empty()) {
+    if ((st = cluster_filter((int)cj.size(), cj.data(), fp32))) return st;
+    int dmax = 0;
+    for (size_t i = 0; i < cj.size(); i++) {
+      const pevsl_devcsr *A = cj[i].A;
+      dmax = PEVSL_MAX(dmax, cj[i].deg);
+      for (int k = 1; k <= cj[i].deg; k++)
+        g_filter_bytes += filter_bytes_degree(A, k, fp32, fp32 && k == cj[i].deg) +
+                          entry_bytes(A, fp32) * (double)A->nnz + 4.0 * (A->nrows + 1.0);
+    }
+    g_filter_launches += (uint64_t)dmax;
+  }
   std::vector<std::array<const double *, 3>> ilv(ig.size()); /* vk, vkm1 per group */
   std::vector<int> ilw(ig.size(), 0);                          /* last degree added to y */
   const int defer = il_defer_setting();
@@ -512,7 +546,12 @@ static int cheb_filter_batch(int ne, const FilterJob *jobs, bool fp32) {
     }
   }
   bool others = false;
-  for (int i = 0; i < nlive && !others; i++) others = !taken[(size_t)live[i]];
+  maxdeg = 0;
+  for (int i = 0; i < nlive; i++)
+    if (!taken[(size_t)live[i]]) {
+      others = true;
+      maxdeg = PEVSL_MAX(maxdeg, jobs[live[i]].pol->deg);
+    }
   std::vector<ChebEntry> en(nlive);
   for (int k = 1; k <= maxdeg && !st && others; k++) {
     int nb = 0;
@@ -572,6 +611,13 @@ static int cheb_filter_batch(int ne, const FilterJob *jobs, bool fp32) {
  * FP32 conversion included) and replayed, with one copy in and one copy out
  * per slice around it.  A new set of live slices is captured anew. */
 static bool filter_graph_enabled() { return filter_form_setting() == 2; }
+
+/* whether every job runs as a cluster launch (or is a copy) */
+static bool all_cluster(const std::vector<FilterJob> &jobs, bool fp32) {
+  for (const FilterJob &J : jobs)
+    if (J.pol->deg > 0 && !cluster_filter_ok(J.A, nullptr, fp32)) return false;
+  return true;
+}
 
 struct FilterGraph {
   cudaGraphExec_t exec = nullptr;
@@ -1745,7 +1791,8 @@ static int cheblannr_group(SliceState *SL, int ns, double tol, FILE *fstats,
                                    xin ? SL[s].vinit->data : SL[s].V + (size_t)kin * SL[s].ld,
                                    SL[s].V + (size_t)kout * SL[s].ld, SL[s].pol, dmu[s], work[s],
                                    SL[s].ld});
-      if (graph_form)
+      /* with every application one cluster launch there is nothing to capture */
+      if (graph_form && !all_cluster(jobs, mixed))
         r = filter_graphed(fg, sel, jobs);
       else
         r = cheb_filter_batch((int)jobs.size(), jobs.data(), mixed);

@@ -1866,6 +1866,11 @@ int pEVSL_ParcsrSetup(pevsl_Csr *Ai, pevsl_Parcsr *A) {
   for (int i = 0; i < nr; i++) {
     const int r = Ai->ia[i + 1] - Ai->ia[i];
     if (r > maxr) maxr = r;
+    for (int k = Ai->ia[i]; k < Ai->ia[i + 1] && nr <= kClusterMaxRows; k++) {
+      const int off = Ai->ja[k] - i;
+      if (off > d->band_hi) d->band_hi = off;
+      if (-off > d->band_lo) d->band_lo = -off;
+    }
   }
   d->max_row_nnz = maxr;
   d->avg_row_nnz = nr ? (double)nnz / nr : 0.0;

@@ -46,6 +46,8 @@ typedef struct pevsl_devcsr {
   double *a;  /* device, nnz     */
   float *a32; /* device fp32 copy, made on first use */
   int max_row_nnz;
+  int band_lo, band_hi; /* largest row - column and column - row (>= 0) of any
+                           * entry; found only for the matrices of cluster launches */
   double avg_row_nnz;
   int lanes; /* threads per row in the row-group SpMV kernels */
   int stream_r; /* rows per lane of the CSR-stream kernels, 0 until tuned */
