@@ -158,6 +158,24 @@ int spmv(const pevsl_devcsr *A, const double *x, double *y);
  *   vkp1 = w;  y = first ? mu0 * vk + muk * w : y + muk * w            */
 int cheb_step(const pevsl_devcsr *A, const double *vk, const double *vkm1, double *vkp1,
               double *y, double cc, double t, double mu0, double muk, int first);
+/* cheb_step with a deferred sum, for matrices where cheb_defers: degree k
+ * adds the terms of the last ny degrees (0..3) to y as cheb_step_il_y does;
+ * mu on the host */
+bool cheb_defers(const pevsl_devcsr *A);
+int cheb_step_y(const pevsl_devcsr *A, const double *vk, const double *vkm1, double *vkp1, double *y,
+                double cc, double t, const double *mu, int k, int ny, int fresh);
+/* terms that degree k of a sum up to degree maxdeg adds to y when the last
+ * update was at degree lastw (0: none yet) and D degrees share an update:
+ * the first update at degree min(D, 2), the last at maxdeg */
+inline int deferred_terms(int k, int lastw, int maxdeg, int D) {
+  const int span = lastw == 0 ? (D < 2 ? D : 2) : D;
+  return (k == maxdeg || k - lastw == span) ? k - lastw : 0;
+}
+/* y = sum_{k <= m} mu[k] T_k((A - cc)/dd) v, m >= 1: the degrees of one
+ * vector, the sum deferred where cheb_defers; b0, b1: n doubles each.
+ * *bytes (if given) receives the algorithmic bytes. */
+int cheb_degrees(const pevsl_devcsr *A, const double *mu, int m, double cc, double dd,
+                 const double *v, double *y, double *b0, double *b1, double *bytes);
 /* The degree of the generalized filter (SRC/chebpol.c:543-546): the SpMV
  * reads x = B^{-1} vk, the recurrence uses vk; tmp (n doubles) is used
  * only by the row-group kernels. */
@@ -250,12 +268,12 @@ int cheb_step_il_y(const pevsl_devcsr *A, int S, const double *Xg, const double 
  * the first cols columns */
 int il_pack(long n, int S, const double *const *xs, double *X);
 int il_unpack(long n, int S, int cols, const double *X, double *const *ys);
-/* bytes per stored entry that the CSR-stream kernels read for A: 3 for the
- * packed form (int16 column offset + uint8 value index), else 12 (int32
- * column + FP64 value) or 8 (FP32 value) */
-double entry_bytes(const pevsl_devcsr *A, bool fp32, bool batch = false);
-/* bytes per entry the interleaved kernel reads for A (3 packed, 12 plain) */
-double il_entry_bytes(const pevsl_devcsr *A);
+/* bytes a pass over A reads for the matrix: a row's mask in the stencil
+ * form, else per entry 3 (packed: int16 column offset + uint8 value index), 12
+ * (int32 column + FP64 value) or 8 (FP32 value), and the row pointers */
+double matrix_bytes(const pevsl_devcsr *A, bool fp32, bool batch = false);
+/* the same of the interleaved kernels */
+double il_matrix_bytes(const pevsl_devcsr *A);
 /* L2 persistence window over the part of A the kernels read (if enabled) */
 void matrix_window(const pevsl_devcsr *A);
 /* choose the CSR-stream rows per lane of a matrix by timing (once) */

@@ -22,9 +22,10 @@
  * cycles (0.24 us) with 16 blocks, a row's chain (gather, seven multiply-adds
  * of 8 cycles each, the recurrence) about 200, and the stores into the
  * neighbours' windows about 0.7 cycles per value.  Measured per degree, one
- * vector, against a launch per degree: 729 rows 0.60 / 2.5 us, 7980 rows
- * (19 x 20 x 21) 1.00 / 3.2 us, 15600 rows 1.17 / 3.2 us, 26970 rows 2.58 /
- * 3.36 us, 32399 rows in 2D 2.11 / 3.13 us; a degree of the generalized
+ * vector, against a launch per degree (of the CSR kernels, and of the
+ * stencil form where a matrix has it): 729 rows 0.60 / 2.5 / 2.1 us, 7980
+ * rows (19 x 20 x 21) 1.00 / 3.2 / 2.2 us, 15600 rows 1.17 / 3.2 / 2.2 us,
+ * 26970 rows 2.58 / 3.36 / 2.2 us; a degree of the generalized
  * filter of two slices at 7980 rows with a 16-term B-solve 17 / 53 us.  Past
  * 32768 rows (four rows per thread) the entries no longer fit beside the
  * windows; a build with them packed to 3 bytes took 5.3 us at 63960 rows
@@ -472,7 +473,10 @@ bool cluster_filter_ok(const pevsl_devcsr *A, const pevsl_devcsr *B, bool fp32) 
   J.A = A;
   J.B = B;
   ClShape s;
-  return cl_choose(1, &J, fp32, &s);
+  if (!cl_choose(1, &J, fp32, &s)) return false;
+  /* a matrix in the stencil form takes 2.1 us per launched degree, less than
+   * a cluster with more than two rows per thread (2.6 us at 26970 rows) */
+  return B || fp32 || !A->smask || s.rpt <= 2;
 }
 
 int cluster_filter(int ne, const ClusterJob *jobs, bool fp32) {

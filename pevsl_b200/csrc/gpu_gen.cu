@@ -82,16 +82,7 @@ int cheb_series(const pevsl_devcsr *M, const double *mu, const double *dmu, int 
     if (vcopy(v, y, n)) return PEVSL_ERR_CUDA;
     return vscal(y, n, mu[0]);
   }
-  double *buf[2] = {w, w + n};
-  const double *vk = v, *vkm1 = nullptr;
-  for (int k = 1; k <= m; k++) {
-    double *vkp1 = k <= 2 ? buf[k - 1] : const_cast<double *>(vkm1);
-    const double t = (k == 1 ? 1.0 : 2.0) / dd;
-    if (cheb_step(M, vk, vkm1, vkp1, y, cc, t, mu[0], mu[k], k == 1)) return PEVSL_ERR_CUDA;
-    vkm1 = vk;
-    vk = vkp1;
-  }
-  return 0;
+  return cheb_degrees(M, mu, m, cc, dd, v, y, w, w + n, nullptr);
 }
 
 int lspol_apply(pevsl_lspol *L, const double *b, double *x) {
@@ -296,13 +287,12 @@ struct EvPool {
 };
 EvPool g_gen_ev;
 
-/* algorithmic bytes: a matrix pass is entry_bytes (3 packed, 12 plain) per
- * entry + 4 (n + 1); a fused
+/* algorithmic bytes: a matrix pass is matrix_bytes; a fused
  * Chebyshev degree adds v_k, v_{k-1}, y read and v_{k+1}, y written (the
  * first degree reads neither v_{k-1} nor y); a second-kind Chebyshev-
  * iteration step gathers d and reads/writes x and r, writes d_new */
 double mat_bytes(const pevsl_devcsr *M) {
-  return entry_bytes(M, false) * (double)M->nnz + 4.0 * (M->nrows + 1.0);
+  return matrix_bytes(M, false);
 }
 
 double solve_bytes(pevsl_Data *pevsl) {
@@ -1049,8 +1039,8 @@ void genil_count(pevsl_Data *pevsl, const GenIl &G, int deg) {
   g_gen_degrees += (uint64_t)deg;
   const double n = (double)G.n;
   g_gen_bytes += (double)deg *
-                 (G.degB * (il_entry_bytes(G.B) * G.B->nnz + 4.0 * (n + 1) + 40.0 * n * G.S) +
-                  il_entry_bytes(G.A) * G.A->nnz + 4.0 * (n + 1) + 48.0 * n * G.S);
+                 (G.degB * (il_matrix_bytes(G.B) + 40.0 * n * G.S) + il_matrix_bytes(G.A) +
+                  48.0 * n * G.S);
 }
 
 int genil_degrees(pevsl_Data *pevsl, GenIl &G) {

@@ -90,7 +90,7 @@ double g_filter_ms = 0.0;
  * written) */
 double cheb_step_bytes(const pevsl_devcsr *A, int first) {
   const double n = A->nrows;
-  return entry_bytes(A, false) * (double)A->nnz + 4.0 * (n + 1) + (first ? 24.0 : 40.0) * n;
+  return matrix_bytes(A, false) + (first ? 24.0 : 40.0) * n;
 }
 
 /* matvec through the installed operator: fused kernels use the device CSR
@@ -110,7 +110,7 @@ int cheb_apply(pevsl_Data *pevsl, const pevsl_Polparams *pol, const double *v, d
                double *w3, long n) {
   pevsl_devcsr *A = pevsl_builtin_A(pevsl);
   const int m = pol->deg;
-  const double cc = pol->cc, dd = pol->dd, t1 = 1.0 / dd, t2 = 2.0 / dd;
+  const double cc = pol->cc, dd = pol->dd;
   const double *mu = pol->mu;
   pevsl->stats->n_polAv++;
   if (m <= 0) {
@@ -130,23 +130,21 @@ int cheb_apply(pevsl_Data *pevsl, const pevsl_Polparams *pol, const double *v, d
     return cluster_filter(1, &J, false);
   }
   double *buf[2] = {w3, w3 + n};
-  double *ax = A ? nullptr : (double *)ws(WS_VEC, sizeof(double) * (size_t)n);
-  if (!A && !ax) return PEVSL_ERR_NOMEM;
+  if (A) {
+    g_filter_launches += (uint64_t)m;
+    pevsl->stats->n_mvA += (size_t)m;
+    return cheb_degrees(A, mu, m, cc, dd, v, y, buf[0], buf[1], &g_filter_bytes);
+  }
+  double *ax = (double *)ws(WS_VEC, sizeof(double) * (size_t)n);
+  if (!ax) return PEVSL_ERR_NOMEM;
   const double *vk = v, *vkm1 = nullptr;
   for (int k = 1; k <= m; k++) {
-    /* two work vectors: from degree 3 on, v_{k+1} replaces v_{k-1} in place */
     double *vkp1 = k <= 2 ? buf[k - 1] : const_cast<double *>(vkm1);
-    const double t = k == 1 ? t1 : t2;
-    int st;
-    if (A) {
-      st = cheb_step(A, vk, vkm1, vkp1, y, cc, t, mu[0], mu[k], k == 1);
-      g_filter_launches++;
-      g_filter_bytes += cheb_step_bytes(A, k == 1);
-    } else {
-      st = apply_A(pevsl, vk, ax);
-      if (!st) st = cheb_combine(n, ax, vk, vkm1, vkp1, y, cc, t, mu[0], mu[k], k == 1);
-      pevsl->stats->n_mvA--; /* counted below */
-    }
+    int st = apply_A(pevsl, vk, ax);
+    if (!st)
+      st = cheb_combine(n, ax, vk, vkm1, vkp1, y, cc, (k == 1 ? 1.0 : 2.0) / dd, mu[0], mu[k],
+                        k == 1);
+    pevsl->stats->n_mvA--; /* counted below */
     if (st) return st;
     vkm1 = vk;
     vk = vkp1;
@@ -194,8 +192,7 @@ static int filter_form() { return filter_form_setting() == 1 ? 1 : 0; }
  * their vectors row-interleaved, so one gather serves every slice
  * (cheb_step_il); the input is packed once and the result unpacked once per
  * filter application.  Applies to 2..16 FP64 slices on a short-row matrix
- * of at least 2^16 rows whose polynomials share the spectrum bounds
- * (cc, dd).  Measured per
+ * whose polynomials share the spectrum bounds (cc, dd) (il_partition).  Measured per
  * degree against the grid-interleaved batch kernel: 100^3, 4 slices 52.6
  * vs 80.1 us (2 slices 34.0 vs 44.6, 16 slices 182 vs 310); random sparse
  * n = 2e6 with ~17 entries per row, 16 slices 758 vs 2160 us. */
@@ -246,13 +243,6 @@ static int il_defer_setting() {
   return v;
 }
 
-/* terms that degree k of a group of top degree maxdeg adds to y when the
- * last update was at degree lastw (0: none yet), under deferral D */
-static int il_terms(int k, int lastw, int maxdeg, int D) {
-  const int span = lastw == 0 ? PEVSL_MIN(D, 2) : D;
-  return (k == maxdeg || k - lastw == span) ? k - lastw : 0;
-}
-
 /* a set of slices the interleaved form serves together */
 struct IlGroup {
   const pevsl_devcsr *A;
@@ -263,11 +253,12 @@ struct IlGroup {
 };
 
 /* The entries the interleaved form takes: groups of 2..16 live FP64
- * entries on one short-row matrix of at least 2^16 rows with the same
- * spectrum bounds (cc, dd), in job order; the other entries stay with the
- * grid-interleaved batch kernel.  Below 2^16 rows the problem sits in L2
- * and the launch is latency-bound, where the batch kernel is faster (20^3,
- * 5 slices: the whole run 0.115 vs 0.125 s). */
+ * entries on one short-row matrix with the same spectrum bounds (cc, dd), in
+ * job order, that is in the stencil form or has at least 2^16 rows, and is
+ * too large for a cluster; the other entries stay with the grid-interleaved
+ * batch kernel.  Below 2^16 rows the plain kernel is latency-bound, where
+ * the batch kernel is faster (20^3, 5 slices: the whole run 0.115 vs 0.125
+ * s). */
 static void il_partition(int ne, const FilterJob *jobs, bool fp32, std::vector<IlGroup> &g,
                          std::vector<char> &taken) {
   g.clear();
@@ -279,7 +270,8 @@ static void il_partition(int ne, const FilterJob *jobs, bool fp32, std::vector<I
     const FilterJob &J = jobs[e];
     if (seen[e] || J.pol->deg <= 0) continue;
     const pevsl_devcsr *A = J.A;
-    if (A->lanes != 0 || A->nrows < 65536) continue;
+    if (A->lanes != 0 || (A->nrows < 65536 && !A->smask) || cluster_filter_ok(A, nullptr, false))
+      continue;
     std::vector<int> L;
     for (int f = e; f < ne; f++)
       if (!seen[f] && jobs[f].pol->deg > 0 && jobs[f].A == A && jobs[f].pol->cc == J.pol->cc &&
@@ -474,7 +466,7 @@ static int cheb_filter_batch(int ne, const FilterJob *jobs, bool fp32) {
       dmax = PEVSL_MAX(dmax, cj[i].deg);
       for (int k = 1; k <= cj[i].deg; k++)
         g_filter_bytes += filter_bytes_degree(A, k, fp32, fp32 && k == cj[i].deg) +
-                          entry_bytes(A, fp32) * (double)A->nnz + 4.0 * (A->nrows + 1.0);
+                          matrix_bytes(A, fp32);
     }
     g_filter_launches += (uint64_t)dmax;
   }
@@ -531,27 +523,36 @@ static int cheb_filter_batch(int ne, const FilterJob *jobs, bool fp32) {
     for (int k = 1; k <= G.maxdeg && !st; k++) {
       const double *gk = ilv[gi][0], *gkm1 = ilv[gi][1];
       double *gkp1 = k == 1 ? B0 : k == 2 ? B1 : const_cast<double *>(gkm1);
-      const int ny = il_terms(k, ilw[gi], G.maxdeg, defer), fresh = ny > 0 && ilw[gi] == 0;
+      const int ny = deferred_terms(k, ilw[gi], G.maxdeg, defer), fresh = ny > 0 && ilw[gi] == 0;
       st = cheb_step_il_y(G.A, G.S, gk, gk, gkm1, gkp1, Y, G.cc, (k == 1 ? 1.0 : 2.0) / G.dd, dmu,
                           dmu + (size_t)k * G.S, ny, fresh);
       if (ny > 0) ilw[gi] = k;
       /* read v_k, v_{k-1} (from degree 2), write v_{k+1}; y read unless
        * fresh and written when updated */
       const double vec = (k == 1 ? 16.0 : 24.0) + (ny > 0 ? (fresh ? 8.0 : 16.0) : 0.0);
-      g_filter_bytes += il_entry_bytes(G.A) * (double)G.A->nnz + 4.0 * (G.A->nrows + 1.0) +
-                        vec * (double)G.A->nrows * G.S;
+      g_filter_bytes += il_matrix_bytes(G.A) + vec * (double)G.A->nrows * G.S;
       g_filter_launches++;
       ilv[gi][1] = gk;
       ilv[gi][0] = gkp1;
     }
   }
-  bool others = false;
+  int nother = 0, other = -1;
   maxdeg = 0;
   for (int i = 0; i < nlive; i++)
     if (!taken[(size_t)live[i]]) {
-      others = true;
+      nother++;
+      other = i;
       maxdeg = PEVSL_MAX(maxdeg, jobs[live[i]].pol->deg);
     }
+  bool others = nother > 0;
+  if (!st && nother == 1 && !fp32 && jobs[live[other]].A->lanes == 0) {
+    /* one slice outside the groups: all its degrees */
+    const FilterJob &J = jobs[live[other]];
+    st = cheb_degrees(J.A, J.pol->mu, maxdeg, J.pol->cc, J.pol->dd, J.x, J.y, (double *)b0[other],
+                      (double *)b1[other], &g_filter_bytes);
+    g_filter_launches += (uint64_t)maxdeg;
+    others = false;
+  }
   std::vector<ChebEntry> en(nlive);
   for (int k = 1; k <= maxdeg && !st && others; k++) {
     int nb = 0;
@@ -576,8 +577,7 @@ static int cheb_filter_batch(int ne, const FilterJob *jobs, bool fp32) {
       bool seen = false;
       for (int t = 0; t < i && !seen; t++) seen = en[t].A == en[i].A;
       if (!seen)
-        bytes += entry_bytes(en[i].A, fp32, nb > 1) * (double)en[i].A->nnz +
-                 4.0 * (en[i].A->nrows + 1.0);
+        bytes += matrix_bytes(en[i].A, fp32, nb > 1);
     }
     if (nb == 0) {
       /* every live entry of this degree is in an interleaved group */

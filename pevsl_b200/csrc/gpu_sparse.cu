@@ -186,10 +186,13 @@ __device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, 
 
 /* An epilogue loads what it needs of its row (pre) before the row's
  * products are formed, so those loads overlap the matrix and gather loads,
- * and then combines (operator()). */
+ * and then combines (operator()).  kOwn: pre holds the row's element of the
+ * vector that the SpMV reads (own). */
 struct EpiStore {
   double *y;
+  static constexpr bool kOwn = false;
   struct Pre {};
+  __device__ __forceinline__ static double own(const Pre &) { return 0.0; }
   __device__ __forceinline__ Pre pre(int) const { return Pre{}; }
   __device__ __forceinline__ void operator()(int row, double r, const Pre &) const { y[row] = r; }
 };
@@ -200,9 +203,11 @@ struct EpiCheb {
   double *vkp1, *y;
   double cc, t, mu0, muk;
   int first;
+  static constexpr bool kOwn = false; /* the SpMV may read another vector */
   struct Pre {
     double x, xm1, y;
   };
+  __device__ __forceinline__ static double own(const Pre &) { return 0.0; }
   __device__ __forceinline__ Pre pre(int row) const {
     return Pre{vk[row], vkm1 ? vkm1[row] : 0.0, first ? 0.0 : y[row]};
   }
@@ -248,9 +253,11 @@ struct EpiChebIter1 {
   const double *b, *x;
   double *p, *xnew;
   double bet, alp;
+  static constexpr bool kOwn = true;
   struct Pre {
     double b, p, x;
   };
+  __device__ __forceinline__ static double own(const Pre &q) { return q.x; }
   __device__ __forceinline__ Pre pre(int row) const { return Pre{b[row], p[row], x[row]}; }
   __device__ __forceinline__ void operator()(int row, double w, const Pre &q) const {
     const double r = __dsub_rn(q.b, w);
@@ -267,9 +274,11 @@ struct EpiChebIter2 {
   const double *d;
   double *x, *r, *dnew;
   double c1, c2;
+  static constexpr bool kOwn = true;
   struct Pre {
     double d, x, r;
   };
+  __device__ __forceinline__ static double own(const Pre &q) { return q.d; }
   __device__ __forceinline__ Pre pre(int row) const { return Pre{d[row], x[row], r[row]}; }
   __device__ __forceinline__ void operator()(int row, double w, const Pre &q) const {
     x[row] = __dadd_rn(q.x, q.d);
@@ -462,6 +471,119 @@ __global__ void __launch_bounds__(kThreads, 4)
   stream_rows_e<1, T, Epi, true>(n0, ia0, EntriesPacked<T>{dj, vi, vt}, (const T *)b.epi[e].vk,
                                  b.epi[e], (long)(blockIdx.x / (unsigned)b.nb), prod);
 }
+
+/* ---------------------------------------------------------------- stencil form
+ * Matrices whose entries are few (column offset, value) pairs -- a stencil
+ * with constant coefficients has one per neighbour.  The pairs come as a
+ * kernel parameter, so offsets and values are constant-bank operands; a row
+ * reads its mask of pairs (1 byte for up to eight, against 21 bytes packed)
+ * and no load precedes the gathers but that one.  One thread per row; the
+ * products are formed unfused and added in entry order: the bits of the
+ * CSR-stream kernels.
+ *
+ * What bounds it: up to about 10^6 rows the vectors sit in L2 and a degree is
+ * three to four waves of blocks, each the length of the chain mask, gather,
+ * sum, store; larger ones stream from HBM.  Per degree of one vector with the
+ * sum deferred, against the ELL and packed kernels: 41 x 40 x 42 2.2 / 2.5
+ * us, 64 x 65 x 63 3.1 / 4.1 us, 99 x 100 x 101 7.4 / 10.6 us (30 MB: 4.1
+ * TB/s), 159 x 160 x 161 24.7 / 54 us.  (The same rows described by a table
+ * of row patterns in shared memory took 8.1 us at 99 x 100 x 101, with the
+ * value and the offset in one 16-byte entry 11.6 us: the table's broadcast
+ * loads use as many L1 cycles as the gathers, which ran at 78%.) */
+struct Stencil {
+  const void *mask;
+  int k;
+  int off[32];
+  double val[32];
+};
+
+static Stencil stencil_of(const pevsl_devcsr *A) {
+  Stencil S;
+  S.mask = A->smask;
+  S.k = A->sk;
+  memcpy(S.off, A->soff, sizeof S.off);
+  memcpy(S.val, A->sval, sizeof S.val);
+  return S;
+}
+
+template <class M>
+__device__ __forceinline__ unsigned stencil_mask(const Stencil &S, int row) {
+  return (unsigned)__ldg((const M *)S.mask + row);
+}
+
+/* sum over the row's pairs.  K: their number fixed at compile time, with the
+ * diagonal in the middle (every gather of a row in flight at once), 0: any
+ * number, eight at a time.  OWN: x0 is the row's element, so the diagonal
+ * needs no load. */
+template <int K, bool OWN>
+__device__ __forceinline__ double stencil_dot(const Stencil &S, unsigned m,
+                                              const double *__restrict__ x, double x0) {
+  constexpr int B = K > 0 ? K : 8;
+  double r = 0.0;
+  for (int j0 = 0; j0 < (K > 0 ? 1 : S.k); j0 += B) {
+    double xv[B];
+#pragma unroll
+    for (int u = 0; u < B; u++) {
+      xv[u] = 0.0;
+      if (K > 0 && OWN && u == K / 2)
+        xv[u] = x0;
+      else if ((m >> (j0 + u)) & 1u)
+        xv[u] = __ldg(x + S.off[j0 + u]);
+    }
+#pragma unroll
+    for (int u = 0; u < B; u++)
+      if ((m >> (j0 + u)) & 1u) r = add_rn(r, mul_rn(S.val[j0 + u], xv[u]));
+  }
+  return r;
+}
+
+/* RPT rows per thread, kThreads apart */
+template <int RPT, int K, class M, class Epi>
+__global__ void __launch_bounds__(kThreads)
+    k_rows_stencil(int n, const __grid_constant__ Stencil S, const double *__restrict__ x, Epi epi) {
+  const int r0 = (int)(blockIdx.x * (unsigned)(kThreads * RPT) + threadIdx.x);
+  unsigned m[RPT];
+#pragma unroll
+  for (int q = 0; q < RPT; q++) m[q] = r0 + q * kThreads < n ? stencil_mask<M>(S, r0 + q * kThreads) : 0u;
+  pdl_wait_then_release();
+  typename Epi::Pre pre[RPT];
+#pragma unroll
+  for (int q = 0; q < RPT; q++)
+    if (r0 + q * kThreads < n) pre[q] = epi.pre(r0 + q * kThreads);
+#pragma unroll
+  for (int q = 0; q < RPT; q++) {
+    const int row = r0 + q * kThreads;
+    if (row < n)
+      epi(row, stencil_dot<K, Epi::kOwn>(S, m[q], x + row, Epi::own(pre[q])), pre[q]);
+  }
+}
+
+/* a filter degree with the sum's update deferred (cheb_step_y) */
+struct EpiChebY {
+  const double *vk, *vkm1;
+  double *vkp1, *y;
+  double cc, t, mu0, mua, mub, muk; /* mua, mub: two degrees and one degree back */
+  int ny, fresh;
+  static constexpr bool kOwn = true;
+  struct Pre {
+    double x, xm1, y;
+  };
+  __device__ __forceinline__ static double own(const Pre &q) { return q.x; }
+  __device__ __forceinline__ Pre pre(int row) const {
+    return Pre{vk[row], vkm1 ? vkm1[row] : 0.0, ny > 0 && !fresh ? y[row] : 0.0};
+  }
+  __device__ __forceinline__ void operator()(int row, double r, const Pre &p) const {
+    double w = __dmul_rn(__fma_rn(-cc, p.x, r), t);
+    if (vkm1) w = __dsub_rn(w, p.xm1);
+    vkp1[row] = w;
+    if (ny > 0) {
+      double s = fresh ? __dmul_rn(mu0, ny == 1 ? p.x : p.xm1) : p.y;
+      if (ny >= 3) s = __fma_rn(mua, p.xm1, s);
+      if (ny >= 2) s = __fma_rn(mub, p.x, s);
+      y[row] = __fma_rn(muk, w, s);
+    }
+  }
+};
 
 /* ---------------------------------------------------------------- persistent filter */
 
@@ -842,7 +964,7 @@ int stream_tune(pevsl_devcsr *A) {
   }
   A->stream_r = 1;
   const long n = A->nrows;
-  if (n < 4096) return 0;
+  if (n < 4096 || A->smask) return 0; /* the stencil form: other kernels */
   double *buf = nullptr;
   if (cudaMalloc(&buf, sizeof(double) * 4 * (size_t)n) != cudaSuccess) {
     cudaGetLastError();
@@ -918,8 +1040,10 @@ void matrix_window(const pevsl_devcsr *A) {
     l2_window(A->a, A->bytes);
 }
 
-double entry_bytes(const pevsl_devcsr *A, bool fp32, bool batch) {
-  return (batch ? use_packed_batch(A) : use_packed(A)) ? 3.0 : (fp32 ? 8.0 : 12.0);
+double matrix_bytes(const pevsl_devcsr *A, bool fp32, bool batch) {
+  if (A->smask && !fp32 && !batch) return (double)A->sbytes * A->nrows;
+  const double e = (batch ? use_packed_batch(A) : use_packed(A)) ? 3.0 : (fp32 ? 8.0 : 12.0);
+  return e * (double)A->nnz + 4.0 * (A->nrows + 1.0);
 }
 
 template <class T>
@@ -927,8 +1051,40 @@ static const T *packed_table(const pevsl_devcsr *A) {
   return sizeof(T) == 4 ? (const T *)(const void *)A->pvtab32 : (const T *)(const void *)A->pvtab;
 }
 
+/* the width the kernels are built for (5 and 7, the diagonal in the middle)
+ * or 0 */
+static int stencil_width(const pevsl_devcsr *A) {
+  return (A->sk == 5 || A->sk == 7) && A->sdiag == A->sk / 2 ? A->sk : 0;
+}
+
+template <class Epi>
+static void launch_rows_stencil(const pevsl_devcsr *A, const double *x, const Epi &epi) {
+  /* two rows per thread where one would be more than three waves of blocks
+   * and the row is wide: 160^3 29.8 -> 24.7 us per degree, 126^3 13.4 ->
+   * 12.4, 100^3 7.49 -> 7.32; 90^3 5.96 -> 6.23, and 1200 x 1201 with five
+   * entries 7.80 -> 8.12 */
+  const int rpt = A->sk > 5 && (long)A->nrows > 3L * 8 * kThreads * ctx().sms ? 2 : 1;
+  const unsigned g = (unsigned)((A->nrows + kThreads * rpt - 1) / (kThreads * rpt));
+  const int w = stencil_width(A);
+#define PV_RS(R)                                                                                \
+  launch_pdl(w == 7               ? k_rows_stencil<R, 7, unsigned char, Epi>                    \
+             : w == 5             ? k_rows_stencil<R, 5, unsigned char, Epi>                    \
+             : A->sbytes == 1     ? k_rows_stencil<R, 0, unsigned char, Epi>                    \
+             : A->sbytes == 2     ? k_rows_stencil<R, 0, unsigned short, Epi>                   \
+                                  : k_rows_stencil<R, 0, unsigned, Epi>,                        \
+             g, ctx().stream, A->nrows, stencil_of(A), x, epi)
+  if (rpt == 1) PV_RS(1); else PV_RS(2);
+#undef PV_RS
+}
+
 template <class T, class Epi>
 static void launch_stream(const pevsl_devcsr *A, const T *a, const T *x, const Epi &epi) {
+  if constexpr (sizeof(T) == 8) {
+    if (A->smask) {
+      launch_rows_stencil(A, x, epi);
+      return;
+    }
+  }
   if (use_packed(A)) {
     launch_pdl(k_csr_stream_packed<T, Epi>, stream_grid(A->nrows, 1), ctx().stream, A->nrows,
                A->ia, A->pdj, A->pvi, packed_table<T>(A), A->pnv, x, epi);
@@ -1037,6 +1193,40 @@ int cheb_step(const pevsl_devcsr *A, const double *vk, const double *vkm1, doubl
   PV_LANE_SWITCH(k_cheb_step, A->lanes, A->nrows, A->nrows, A->ia, A->ja, A->a, vk, vkm1, vkp1, y,
                  cc, t, mu0, muk, first);
   return launched("cheb_step");
+}
+
+bool cheb_defers(const pevsl_devcsr *A) { return A->lanes == 0 && A->smask != nullptr; }
+
+int cheb_step_y(const pevsl_devcsr *A, const double *vk, const double *vkm1, double *vkp1, double *y,
+                double cc, double t, const double *mu, int k, int ny, int fresh) {
+  if (A->nrows <= 0) return 0;
+  if (!cheb_defers(A) || ny < 0 || ny > 3 || ny > k || (ny > 1 && !vkm1)) return PEVSL_ERR_ARG;
+  launch_rows_stencil(A, vk, EpiChebY{vk, vkm1, vkp1, y, cc, t, mu[0], ny > 2 ? mu[k - 2] : 0.0,
+                                  ny > 1 ? mu[k - 1] : 0.0, mu[k], ny, fresh});
+  return launched("cheb_step_y");
+}
+
+int cheb_degrees(const pevsl_devcsr *A, const double *mu, int m, double cc, double dd,
+                 const double *v, double *y, double *b0, double *b1, double *bytes) {
+  const bool defer = cheb_defers(A);
+  const double n = A->nrows, mat = matrix_bytes(A, false);
+  const double *vk = v, *vkm1 = nullptr;
+  double moved = 0.0;
+  for (int k = 1, lastw = 0; k <= m; k++) {
+    /* two work vectors: from degree 3 on, v_{k+1} replaces v_{k-1} in place */
+    double *vkp1 = k == 1 ? b0 : k == 2 ? b1 : const_cast<double *>(vkm1);
+    const double t = (k == 1 ? 1.0 : 2.0) / dd;
+    const int ny = defer ? deferred_terms(k, lastw, m, 3) : 1, fresh = ny > 0 && lastw == 0;
+    const int st = defer ? cheb_step_y(A, vk, vkm1, vkp1, y, cc, t, mu, k, ny, fresh)
+                         : cheb_step(A, vk, vkm1, vkp1, y, cc, t, mu[0], mu[k], k == 1);
+    if (st) return st;
+    moved += mat + ((k == 1 ? 16.0 : 24.0) + (ny > 0 ? (fresh ? 8.0 : 16.0) : 0.0)) * n;
+    if (ny > 0) lastw = k;
+    vkm1 = vk;
+    vk = vkp1;
+  }
+  if (bytes) *bytes += moved;
+  return 0;
 }
 
 int cheb_step_x(const pevsl_devcsr *A, const double *x, const double *vk, const double *vkm1,
@@ -1352,6 +1542,85 @@ __global__ void __launch_bounds__(kThreads, 5)
                           il_accumulate<2>(ny, fresh, yold.y, w1, x.y, xm1.y, mu0, muk, 1));
 }
 
+/* S = 2 L interleaved vectors on the stencil form: L lanes per row, each two
+ * vectors (16-byte gathers, half a row's in flight: 32 registers),
+ * k_cheb_il's arithmetic.  The SpMV reads Xg, which is Xk except in the
+ * generalized filter (GEN).  Per degree, against the ELL and packed kernels:
+ * 100^3 with two slices 9.3 / 15.7 us (60 MB, 6.4 TB/s out of L2), 64 x 65 x
+ * 63 with three 6.0 / 11.5 and with eight 10.2 / 19.9 us, 50^3 with sixteen
+ * 9.9 / 19.3 us. */
+template <int L, int K, class M, bool GEN>
+__global__ void __launch_bounds__(kThreads)
+    k_cheb_il_stencil(int n, const __grid_constant__ Stencil S, const double2 *__restrict__ Xg,
+                      const double2 *__restrict__ Xk, const double2 *Xkm1, double2 *Xkp1,
+                      double2 *Y, double cc, double t, const double *__restrict__ mu0,
+                      const double *__restrict__ muk, int ny, int fresh) {
+  const unsigned me = blockIdx.x * (unsigned)kThreads + threadIdx.x;
+  const int row = (int)(me / L), l = (int)(me % L);
+  const unsigned m = row < n ? stencil_mask<M>(S, row) : 0u;
+  pdl_wait_then_release();
+  if (row >= n) return;
+  const double2 x = Xk[me];
+  const double2 xm1 = Xkm1 ? Xkm1[me] : make_double2(0.0, 0.0);
+  const double2 yold = (ny > 0 && !fresh) ? Y[me] : make_double2(0.0, 0.0);
+  const double2 *xr = Xg + me;
+  double r0 = 0.0, r1 = 0.0;
+  constexpr int B = K > 0 ? (K + 1) / 2 : 4;
+  auto batch = [&](int j0) {
+    double2 xv[B];
+#pragma unroll
+    for (int u = 0; u < B; u++) {
+      xv[u] = make_double2(0.0, 0.0);
+      if (K > 0 && !GEN && j0 + u == K / 2)
+        xv[u] = x;
+      else if ((m >> (j0 + u)) & 1u)
+        xv[u] = __ldg(xr + (long)S.off[j0 + u] * L);
+    }
+#pragma unroll
+    for (int u = 0; u < B; u++)
+      if ((m >> (j0 + u)) & 1u) {
+        r0 = __dadd_rn(r0, __dmul_rn(S.val[j0 + u], xv[u].x));
+        r1 = __dadd_rn(r1, __dmul_rn(S.val[j0 + u], xv[u].y));
+      }
+  };
+  if constexpr (K > 0) {
+    batch(0);
+    batch(B);
+  } else {
+    for (int j0 = 0; j0 < S.k; j0 += B) batch(j0);
+  }
+  double w0 = __dmul_rn(__fma_rn(-cc, x.x, r0), t);
+  double w1 = __dmul_rn(__fma_rn(-cc, x.y, r1), t);
+  if (Xkm1) {
+    w0 = __dsub_rn(w0, xm1.x);
+    w1 = __dsub_rn(w1, xm1.y);
+  }
+  Xkp1[me] = make_double2(w0, w1);
+  if (ny > 0)
+    Y[me] = make_double2(
+        il_accumulate<2 * L>(ny, fresh, yold.x, w0, x.x, xm1.x, mu0, muk, 2 * l),
+        il_accumulate<2 * L>(ny, fresh, yold.y, w1, x.y, xm1.y, mu0, muk, 2 * l + 1));
+}
+
+template <int L>
+static int launch_il_stencil(const pevsl_devcsr *A, const double *Xg, const double *Xk,
+                             const double *Xkm1, double *Xkp1, double *Y, double cc, double t,
+                             const double *mu0, const double *muk, int ny, int fresh) {
+  const unsigned g = (unsigned)(((long)A->nrows * L + kThreads - 1) / kThreads);
+  const int w = Xg == Xk ? stencil_width(A) : 0;
+  auto go = [&](auto k) {
+    launch_pdl(k, g, ctx().stream, A->nrows, stencil_of(A), (const double2 *)Xg,
+               (const double2 *)Xk, (const double2 *)Xkm1, (double2 *)Xkp1, (double2 *)Y, cc, t,
+               mu0, muk, ny, fresh);
+  };
+  if (w == 7) go(k_cheb_il_stencil<L, 7, unsigned char, false>);
+  else if (w == 5) go(k_cheb_il_stencil<L, 5, unsigned char, false>);
+  else if (A->sbytes == 1) go(k_cheb_il_stencil<L, 0, unsigned char, true>);
+  else if (A->sbytes == 2) go(k_cheb_il_stencil<L, 0, unsigned short, true>);
+  else go(k_cheb_il_stencil<L, 0, unsigned, true>);
+  return launched("cheb_step_il_stencil");
+}
+
 /* PEVSL_B200_ELL_W: 1 (default) the ELL kernels compiled for the matrix's
  * width where it is a common stencil width (5 or 7), 0 the any-width
  * kernels.  Same results either way. */
@@ -1554,7 +1823,10 @@ static bool il_packed(const pevsl_devcsr *A) {
   return v && A->pdj != nullptr && packed_mode() >= 1 && A->nrows >= 65536;
 }
 
-double il_entry_bytes(const pevsl_devcsr *A) { return il_packed(A) ? 3.0 : 12.0; }
+double il_matrix_bytes(const pevsl_devcsr *A) {
+  if (A->smask) return (double)A->sbytes * A->nrows;
+  return (il_packed(A) ? 3.0 : 12.0) * (double)A->nnz + 4.0 * (A->nrows + 1.0);
+}
 
 int cheb_step_il_x(const pevsl_devcsr *A, int S, const double *Xg, const double *Xk,
                    const double *Xkm1, double *Xkp1, double *Y, double cc, double t,
@@ -1571,6 +1843,15 @@ int cheb_step_il_y(const pevsl_devcsr *A, int S, const double *Xg, const double 
   if (ny == 3 && !Xkm1) return PEVSL_ERR_ARG;
   if (fresh && (ny < 1 || ny > 2 || (ny == 2 && !Xkm1) || muk != mu0 + (size_t)ny * S))
     return PEVSL_ERR_ARG;
+  if (A->smask) {
+    switch (S) {
+      case 2: return launch_il_stencil<1>(A, Xg, Xk, Xkm1, Xkp1, Y, cc, t, mu0, muk, ny, fresh);
+      case 4: return launch_il_stencil<2>(A, Xg, Xk, Xkm1, Xkp1, Y, cc, t, mu0, muk, ny, fresh);
+      case 8: return launch_il_stencil<4>(A, Xg, Xk, Xkm1, Xkp1, Y, cc, t, mu0, muk, ny, fresh);
+      case 16: return launch_il_stencil<8>(A, Xg, Xk, Xkm1, Xkp1, Y, cc, t, mu0, muk, ny, fresh);
+      default: return PEVSL_ERR_ARG;
+    }
+  }
   const long rows_per_block = (kThreads / 32) * (32 / S);
   const unsigned g = (unsigned)((A->nrows + rows_per_block - 1) / rows_per_block);
   cudaStream_t st = ctx().stream;
@@ -1851,6 +2132,87 @@ static int pack_entries(pevsl_devcsr *d, const pevsl_Csr *Ai) {
   return st;
 }
 
+/* The stencil form of a matrix: at most 32 (offset, value) pairs in all,
+ * values compared bit for bit, and every row's entries in ascending column
+ * order.  *done is set when the matrix has it. */
+static int build_stencil(pevsl_devcsr *d, const pevsl_Csr *Ai, bool *done) {
+  *done = false;
+  const int nr = d->nrows;
+  if (nr <= 0 || d->nnz <= 0 || d->max_row_nnz > 32 || d->lanes != 0) return 0;
+  struct Pair {
+    int off;
+    uint64_t val;
+  };
+  Pair pair[32];
+  int np = 0; /* in order of first appearance */
+  std::vector<unsigned> mask((size_t)nr);
+  for (int i = 0; i < nr; i++) {
+    /* most rows repeat the one before, one column further */
+    const int s = Ai->ia[i], len = Ai->ia[i + 1] - s;
+    if (i > 0 && len == s - Ai->ia[i - 1]) {
+      const int *c = Ai->ja + s, *cp = c - len;
+      bool same = memcmp(Ai->a + s, Ai->a + s - len, sizeof(double) * (size_t)len) == 0;
+      for (int j = 0; j < len && same; j++) same = c[j] == cp[j] + 1;
+      if (same) {
+        mask[(size_t)i] = mask[(size_t)i - 1];
+        continue;
+      }
+    }
+    unsigned m = 0;
+    for (int k = Ai->ia[i], j = 0; k < Ai->ia[i + 1]; k++, j++) {
+      if (k > Ai->ia[i] && Ai->ja[k] <= Ai->ja[k - 1]) return 0;
+      const int off = Ai->ja[k] - i;
+      uint64_t v;
+      memcpy(&v, Ai->a + k, sizeof v);
+      while (j < np && (pair[j].off != off || pair[j].val != v)) j++;
+      if (j >= np) { /* not after the last pair: from the start */
+        for (j = 0; j < np && (pair[j].off != off || pair[j].val != v); j++) {
+        }
+        if (j == np) {
+          if (np == 32) return 0;
+          pair[np++] = Pair{off, v};
+        }
+      }
+      m |= 1u << j;
+    }
+    mask[(size_t)i] = m;
+  }
+  /* the pairs by offset, and the masks in that order */
+  int at[32];
+  for (int j = 0; j < np; j++) {
+    at[j] = 0;
+    for (int q = 0; q < np; q++)
+      at[j] += pair[q].off < pair[j].off || (pair[q].off == pair[j].off && q < j);
+  }
+  d->sdiag = -1;
+  for (int j = 0; j < np; j++) {
+    d->soff[at[j]] = pair[j].off;
+    memcpy(&d->sval[at[j]], &pair[j].val, sizeof(double));
+    if (pair[j].off == 0) d->sdiag = at[j];
+  }
+  d->sk = np;
+  d->sbytes = np <= 8 ? 1 : np <= 16 ? 2 : 4;
+  std::vector<unsigned char> out((size_t)nr * (size_t)d->sbytes);
+  unsigned last_in = 0, last_out = 0; /* masks repeat along a grid line */
+  for (int i = 0; i < nr; i++) {
+    const unsigned m = mask[(size_t)i];
+    if (m != last_in) {
+      last_in = m;
+      last_out = 0;
+      for (int j = 0; j < np; j++)
+        if ((m >> j) & 1u) last_out |= 1u << at[j];
+    }
+    memcpy(out.data() + (size_t)i * d->sbytes, &last_out, (size_t)d->sbytes); /* little endian */
+  }
+  void *p = alloc_dev(out.size());
+  if (!p) return PEVSL_ERR_NOMEM;
+  d->smask = p;
+  int st = memcpy_async(p, out.data(), out.size());
+  if (!st) st = sync();
+  *done = st == 0;
+  return st;
+}
+
 int pEVSL_ParcsrSetup(pevsl_Csr *Ai, pevsl_Parcsr *A) {
   if (ensure()) return PEVSL_ERR_CUDA;
   const int nr = A->nrow_local;
@@ -1866,11 +2228,6 @@ int pEVSL_ParcsrSetup(pevsl_Csr *Ai, pevsl_Parcsr *A) {
   for (int i = 0; i < nr; i++) {
     const int r = Ai->ia[i + 1] - Ai->ia[i];
     if (r > maxr) maxr = r;
-    for (int k = Ai->ia[i]; k < Ai->ia[i + 1] && nr <= kClusterMaxRows; k++) {
-      const int off = Ai->ja[k] - i;
-      if (off > d->band_hi) d->band_hi = off;
-      if (-off > d->band_lo) d->band_lo = -off;
-    }
   }
   d->max_row_nnz = maxr;
   d->avg_row_nnz = nr ? (double)nnz / nr : 0.0;
@@ -1899,7 +2256,18 @@ int pEVSL_ParcsrSetup(pevsl_Csr *Ai, pevsl_Parcsr *A) {
   if (!st) st = memcpy_async(d->a, Ai->a, sizeof(double) * (size_t)nnz);
   if (!st) st = sync();
   if (st) return st;
-  st = pack_entries(d, Ai);
+  bool stencil = false;
+  st = build_stencil(d, Ai, &stencil);
+  for (int j = 0; j < d->sk; j++) {
+    d->band_hi = std::max(d->band_hi, d->soff[j]);
+    d->band_lo = std::max(d->band_lo, -d->soff[j]);
+  }
+  for (int i = 0; i < nr && !stencil && nr <= kClusterMaxRows; i++)
+    for (int k = Ai->ia[i]; k < Ai->ia[i + 1]; k++) {
+      d->band_hi = std::max(d->band_hi, Ai->ja[k] - i);
+      d->band_lo = std::max(d->band_lo, i - Ai->ja[k]);
+    }
+  if (!st && !stencil) st = pack_entries(d, Ai);
   if (st) return st;
   A->comm_handle = (commHandle *)d;
   A->diag = (pevsl_Csr *)calloc(1, sizeof(pevsl_Csr));
@@ -1920,6 +2288,7 @@ void pEVSL_ParcsrFree(pevsl_Parcsr *A) {
     cudaStreamSynchronize(ctx().stream);
     cudaFree(d->a); /* the whole [values | indices | pointers] block */
     if (d->a32) cudaFree(d->a32);
+    if (d->smask) cudaFree(d->smask);
     if (d->pdj) cudaFree(d->pdj); /* the packed block */
     d->magic = 0;
     free(d);

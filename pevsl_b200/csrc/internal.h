@@ -52,6 +52,15 @@ typedef struct pevsl_devcsr {
   int lanes; /* threads per row in the row-group SpMV kernels */
   int stream_r; /* rows per lane of the CSR-stream kernels, 0 until tuned */
   size_t bytes; /* size of the one device block holding a, ja, ia */
+  /* stencil form (smask NULL when the matrix does not qualify): at most 32
+   * (column offset, value) pairs in all, soff ascending; bit j of row r's
+   * mask (sbytes = 1, 2 or 4 bytes) says that the row has the entry of
+   * column r + soff[j] with value sval[j].  A matrix in this form has no
+   * packed copy. */
+  void *smask;
+  int sk, sbytes, sdiag; /* pairs; the pair of offset 0, or -1 */
+  int soff[32];
+  double sval[32];
   /* packed copy of the entries (NULL when the matrix does not qualify):
    * pdj = column - 32 * (row / 32) as int16, pvi = index of the value in
    * pvtab (at most 256 distinct values, exact doubles; pvtab32 their FP32
