@@ -192,10 +192,19 @@ int chebiter2_step(const pevsl_devcsr *B, const double *d, double *x, double *r,
 /* Same recurrence when A x is computed by a user callback: ax = A vk. */
 int cheb_combine(long n, const double *ax, const double *vk, const double *vkm1, double *vkp1,
                  double *y, double cc, double t, double mu0, double muk, int first);
-/* One KPM degree for s interleaved vectors (row-major n x ld blocks):
- *   Xkp1 = (A Xk - ctr Xk) sc - Xkm1;   mom[c] = <Xkp1[:,c], V0[:,c]>   */
-int kpm_step(const pevsl_devcsr *A, int s, int ld, const double *Xk, const double *Xkm1,
-             double *Xkp1, const double *V0, double ctr, double sc, double *mom);
+/* KPM: one degree for s <= 64 vectors, row-interleaved with ld = s rounded
+ * up to even, Xkp1 = (A Xk - ctr Xk) sc - Xkm1 (Xkm1 may be NULL, and Xkp1
+ * may be Xkm1), and per
+ * block the sums of <x_{k+1}, x_{k+1}> and <x_{k+1}, x_k> of every column
+ * into part (kpm_blocks x 2 ld doubles).  kpm_reduce adds them over the
+ * blocks for all steps: out[step][c][0..1] and [2..3], high and low part of
+ * each (4 ld doubles per step). */
+int kpm_blocks(const pevsl_devcsr *A, int s);
+int kpm_step(const pevsl_devcsr *A, int s, const double *Xk, const double *Xkm1, double *Xkp1,
+             double ctr, double sc, double *part);
+int kpm_reduce(const pevsl_devcsr *A, int s, int steps, const double *part, double *out);
+/* vectors that share a group (at most 64) */
+int kpm_group(const pevsl_devcsr *A, int nvec);
 /* out[c] = sum_b partials[b*s + c] over nb blocks, fixed order */
 int col_reduce(const double *partials, int nb, int s, double *out);
 /* Column sums of squares of an interleaved block: out[c] = sum_i X[i*ld+c]^2 */

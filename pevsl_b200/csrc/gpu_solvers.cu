@@ -828,46 +828,59 @@ int pEVSL_Kpmdos(pevsl_Data *pevsl, int Mdeg, int damping, int nvec, double *int
       free(hmom);
     }
   } else if (A && !st) {
-    /* blocks of up to 64 vectors, row-interleaved; one launch per degree */
-    const int smax = 64;
+    /* groups of vectors, row-interleaved; one launch per degree.  With
+     * c_k = <v_k, v_0>, T_{2k} = 2 T_k^2 - 1 and T_{2k+1} = 2 T_{k+1} T_k -
+     * T_1 give c_{2k} = 2 <v_k, v_k> - c_0 and c_{2k+1} = 2 <v_{k+1}, v_k> -
+     * c_1, so half the degrees do. */
+    const int smax = kpm_group(A, vec_end - vec_start), steps = (Mdeg + 1) / 2;
+    std::vector<double> hmom;
+    double hn[64];
     for (int m0 = vec_start; m0 < vec_end && !st; m0 += smax) {
-      const int s = vec_end - m0 < smax ? vec_end - m0 : smax;
-      const int ld = s;
-      const size_t blk = (size_t)n * (size_t)ld;
-      double *X = (double *)ws(WS_KPM, sizeof(double) * 4 * blk);
-      double *mom = (double *)ws(WS_MOM, sizeof(double) * (size_t)(Mdeg + 1) * (size_t)s);
+      const int s = PEVSL_MIN(smax, vec_end - m0), ld = (s + 1) / 2 * 2;
+      const size_t blk = (size_t)n * (size_t)ld, np = (size_t)kpm_blocks(A, s) * 2 * (size_t)ld;
+      double *X = (double *)ws(WS_KPM, sizeof(double) * 2 * blk);
+      double *part = (double *)ws(WS_PART, sizeof(double) * np * (size_t)PEVSL_MAX(steps, 1));
+      double *mom = (double *)ws(WS_MOM, sizeof(double) * 4 * (size_t)ld * (size_t)PEVSL_MAX(steps, 1));
       double *nrm2 = (double *)ws(WS_SMALL, sizeof(double) * 64);
-      double *hmom = (double *)malloc(sizeof(double) * (size_t)(Mdeg + 1) * (size_t)s);
-      if (!X || !mom || !nrm2 || !hmom) {
-        free(hmom);
+      if (!X || !part || !mom || !nrm2) {
         st = PEVSL_ERR_NOMEM;
         break;
       }
-      double *V0 = X, *B[3] = {X + blk, X + 2 * blk, X + 3 * blk};
-      st = pevsl_rand_block_dev(V0, (int)n, s, ld);
-      if (!st) st = block_colnorm2(n, s, ld, V0, nrm2);
-      if (!st) st = block_normalize(n, s, ld, V0, nrm2);
-      for (int k = 0; k < Mdeg && !st; k++) {
-        const double sc = (k == 0 ? 1.0 : 2.0) / wid;
-        const double *Xk = k == 0 ? V0 : B[(k - 1) % 3];
-        const double *Xkm1 = k == 0 ? nullptr : (k == 1 ? V0 : B[(k - 2) % 3]);
-        st = kpm_step(A, s, ld, Xk, Xkm1, B[k % 3], V0, ctr, sc, mom + (size_t)k * s);
-      }
-      if (!st) st = memcpy_async(hmom, mom, sizeof(double) * (size_t)Mdeg * (size_t)s);
+      hmom.resize(4 * (size_t)ld * (size_t)steps);
+      double *B[2] = {X, X + blk};
+      if (s < ld)
+        st = fail(cudaMemset2DAsync(X + s, sizeof(double) * (size_t)ld, 0, sizeof(double), (size_t)n,
+                                    ctx().stream),
+                  "cudaMemset2DAsync");
+      if (!st) st = pevsl_rand_block_dev(X, (int)n, s, ld);
+      if (!st) st = block_colnorm2(n, s, ld, X, nrm2);
+      if (!st) st = block_normalize(n, s, ld, X, nrm2);
+      for (int k = 0; k < steps && !st; k++)
+        st = kpm_step(A, s, B[k % 2], k > 0 ? B[(k + 1) % 2] : nullptr, B[(k + 1) % 2], ctr,
+                      (k == 0 ? 1.0 : 2.0) / wid, part + np * (size_t)k);
+      if (!st) st = kpm_reduce(A, s, steps, part, mom);
+      if (!st) st = memcpy_async(hmom.data(), mom, sizeof(double) * hmom.size());
+      if (!st) st = memcpy_async(hn, nrm2, sizeof(double) * (size_t)s);
       if (!st) st = sync();
-      pevsl->stats->n_mvA += (size_t)Mdeg * (size_t)s;
+      pevsl->stats->n_mvA += (size_t)steps * (size_t)s;
       /* accumulate exactly as the reference: vector by vector, degree by degree */
       for (int c = 0; c < s && !st; c++) {
         mu[0] += jac[0];
         tcnt -= jac[0] * (beta2 - beta1);
+        /* c_0 of the start vector as block_normalize left it: one up to rounding */
+        const long double q = 1.0 / sqrt(hn[c]), c0 = (long double)hn[c] * q * q;
+        const long double c1 = steps > 0 ? (long double)hmom[4 * (size_t)c + 2] + hmom[4 * (size_t)c + 3] : 0;
         for (int k = 0; k < Mdeg; k++) {
           const int k1 = k + 1;
-          const double t = hmom[(size_t)k * s + c] * 2.0 * jac[k1];
+          const double *d = &hmom[4 * ((size_t)(k / 2) * ld + c)];
+          const double ck = (double)(k == 0       ? c1
+                                     : k1 % 2 ? 2.0L * ((long double)d[2] + d[3]) - c1
+                                              : 2.0L * ((long double)d[0] + d[1]) - c0);
+          const double t = ck * 2.0 * jac[k1];
           mu[k1] += t;
           tcnt -= t * (sin(k1 * beta2) - sin(k1 * beta1)) / k1;
         }
       }
-      free(hmom);
     }
   } else if (!st) {
     /* user matvec: one vector at a time, as the reference */

@@ -7,9 +7,8 @@
  *    pEVSL_ChebAv (SRC/chebpol.c:538-568) with the SpMV fused in, so that a
  *    degree reads A, v_k, v_{k-1}, y and writes v_{k+1}, y once;
  *  - kpm_step: one degree of the KPM recurrence of pEVSL_Kpmdos
- *    (SRC/kpmdos.c:129-156) for a block of s random vectors at once, with the
- *    moment dot products fused in, so that A is read once per degree for all
- *    vectors.
+ *    (SRC/kpmdos.c:129-156) for a group of random vectors at once, with the
+ *    dot products of two moments fused in.
  *
  * Layout: CSR with int32 row pointers / column indices and fp64 values; a
  * row is handled by a group of L lanes (L = 1..32, a power of two picked from
@@ -829,74 +828,179 @@ static unsigned stream_grid(int n, int R) {
 }
 
 
-/* KPM degree for s <= 32*CPL interleaved vectors; one warp per row (grid
- * stride), lane c handles columns c, c+32, ...  Moments: per-block partial
- * sums in partials[block*s + c], the last block adds them in block order. */
-template <int CPL>
-__global__ void __launch_bounds__(kThreads)
-    k_kpm_step(int n, int s, int ld, const int *__restrict__ ia, const int *__restrict__ ja,
-               const double *__restrict__ a, const double *__restrict__ Xk,
-               const double *__restrict__ Xkm1, double *__restrict__ Xkp1,
-               const double *__restrict__ V0, double ctr, double sc, double *partials,
-               unsigned *counter, double *mom) {
-  __shared__ double acc_sh[kThreads / 32][32 * CPL];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int wpb = blockDim.x >> 5;
-  double acc[CPL];
+/* ---------------------------------------------------------------- KPM
+ * One degree for 2 L row-interleaved vectors: L lanes per row, each two
+ * vectors (16-byte accesses), RB = kThreads / L rows per block at a time,
+ *   X_{k+1} = (A X_k - ctr X_k) sc - X_{k-1},
+ * and the two inner products from which the doubled moments follow,
+ *   d0 = <x_{k+1}, x_{k+1}> (moment 2k + 2),  d1 = <x_{k+1}, x_k> (2k + 1).
+ * A degree thus gives two moments and does not read the start vectors: half
+ * the degrees and three block transfers instead of four in each.  Each
+ * thread keeps its columns over all its rows; per block the sums go to
+ * part[block][4 L] = (d0, d1 of column 0, of column 1, ...), added over the
+ * blocks in order by k_kpm_reduce for all degrees at the end.
+ *
+ * Bound by L2 and HBM bandwidth (48 bytes per row and pair of vectors, 16 of
+ * them written).  With more blocks than are resident, each wave of blocks
+ * sweeps every other stripe of rows and reads its neighbours again: 985
+ * instead of 720 MB of DRAM traffic per degree of 30 vectors at 101 x 100 x
+ * 99.  Five or six blocks per SM with four gathers in flight: 23.1 and 25.2
+ * against 22.0 ms for the 300 moments. */
+constexpr int kKpmPerSm = 4; /* 64 registers, every gather of a row in flight */
+constexpr int kKpmBlocks = kKpmPerSm * 148; /* all resident: the blocks sweep the rows together */
+
+struct KpmAcc {
+  double a0, a1, b0, b1; /* d0, d1 of the first column, of the second */
+};
+
+__device__ __forceinline__ void kpm_row(double2 r, double2 x, double2 xm1, double2 *Xkp1, size_t me,
+                                        double ctr, double sc, KpmAcc &t) {
+  const double2 w = make_double2((r.x - ctr * x.x) * sc - xm1.x, (r.y - ctr * x.y) * sc - xm1.y);
+  Xkp1[me] = w;
+  t.a0 = fma(w.x, w.x, t.a0);
+  t.a1 = fma(w.x, x.x, t.a1);
+  t.b0 = fma(w.y, w.y, t.b0);
+  t.b1 = fma(w.y, x.y, t.b1);
+}
+
+/* the block's sums per column, a fixed tree over the rows of a pass: in the
+ * warps where their rows line up (L a power of two up to 16), else in shared
+ * memory */
+__device__ __forceinline__ void kpm_finish(KpmAcc t, int L, int RB, double *part) {
+  __shared__ KpmAcc sh[kThreads];
+  const bool warps = 32 % L == 0 && L < 32;
+  if (warps)
+    for (int o = 16; o >= L; o >>= 1) {
+      t.a0 += __shfl_xor_sync(0xffffffffu, t.a0, o);
+      t.a1 += __shfl_xor_sync(0xffffffffu, t.a1, o);
+      t.b0 += __shfl_xor_sync(0xffffffffu, t.b0, o);
+      t.b1 += __shfl_xor_sync(0xffffffffu, t.b1, o);
+    }
+  sh[threadIdx.x] = t;
+  __syncthreads();
+  /* rows left, and the threads from one to the next */
+  const int rows = warps ? kThreads / 32 : RB, step = warps ? 32 : L;
+  const int row = (int)threadIdx.x / step, col = (int)threadIdx.x % step;
+  int h = 1;
+  while (h < rows) h <<= 1;
+  for (h >>= 1; h > 0; h >>= 1) {
+    if (row < h && row + h < rows && col < L) {
+      KpmAcc &s = sh[threadIdx.x];
+      const KpmAcc v = sh[threadIdx.x + h * step];
+      s.a0 += v.a0;
+      s.a1 += v.a1;
+      s.b0 += v.b0;
+      s.b1 += v.b1;
+    }
+    __syncthreads();
+  }
+  if ((int)threadIdx.x < L) *(KpmAcc *)(part + ((size_t)blockIdx.x * L + threadIdx.x) * 4) = sh[threadIdx.x];
+}
+
+template <int K, class M>
+__global__ void __launch_bounds__(kThreads, kKpmPerSm)
+    k_kpm_stencil(int n, int L, const __grid_constant__ Stencil S, const double2 *__restrict__ Xk,
+                  const double2 *Xkm1, double2 *Xkp1, double ctr, double sc, double *part) {
+  pdl_wait_then_release();
+  const int RB = kThreads / L, rl = (int)threadIdx.x / L, l = (int)threadIdx.x % L;
+  const bool on = rl < RB;
+  KpmAcc t{0.0, 0.0, 0.0, 0.0};
+  for (int row = on ? (int)blockIdx.x * RB + rl : n; row < n; row += (int)gridDim.x * RB) {
+    const size_t me = (size_t)row * L + l;
+    const unsigned m = stencil_mask<M>(S, row);
+    const double2 x = __ldg(Xk + me);
+    const double2 xm1 = Xkm1 ? Xkm1[me] : make_double2(0.0, 0.0);
+    double2 r = make_double2(0.0, 0.0);
+    constexpr int B = K > 0 ? K : 4;
 #pragma unroll
-  for (int q = 0; q < CPL; q++) acc[q] = 0.0;
-  for (int row = blockIdx.x * wpb + wib; row < n; row += gridDim.x * wpb) {
-    double r[CPL];
+    for (int j0 = 0; j0 < (K > 0 ? K : S.k); j0 += B) {
+      double2 xv[B];
 #pragma unroll
-    for (int q = 0; q < CPL; q++) r[q] = 0.0;
-    const int e = ia[row + 1];
-    int j = ia[row];
-    /* four entries per iteration: their loads are independent and in flight
-     * together; each column still accumulates in entry order */
-    for (; j + 3 < e; j += 4) {
-      const double a0 = a[j], a1 = a[j + 1], a2 = a[j + 2], a3 = a[j + 3];
-      const double *x0 = Xk + (size_t)ja[j] * ld, *x1 = Xk + (size_t)ja[j + 1] * ld;
-      const double *x2 = Xk + (size_t)ja[j + 2] * ld, *x3 = Xk + (size_t)ja[j + 3] * ld;
+      for (int u = 0; u < B; u++) {
+        xv[u] = x;
+        if (!(K > 0 && j0 + u == K / 2) && ((m >> (j0 + u)) & 1u))
+          xv[u] = __ldg(Xk + me + (long)S.off[j0 + u] * L);
+      }
 #pragma unroll
-      for (int q = 0; q < CPL; q++) {
-        const int c = lane + 32 * q;
-        if (c < s) {
-          const double v0 = x0[c], v1 = x1[c], v2 = x2[c], v3 = x3[c];
-          r[q] = fma(a3, v3, fma(a2, v2, fma(a1, v1, fma(a0, v0, r[q]))));
+      for (int u = 0; u < B; u++)
+        if ((m >> (j0 + u)) & 1u) {
+          r.x = fma(S.val[j0 + u], xv[u].x, r.x);
+          r.y = fma(S.val[j0 + u], xv[u].y, r.y);
+        }
+    }
+    kpm_row(r, x, xm1, Xkp1, me, ctr, sc, t);
+  }
+  kpm_finish(t, L, RB, part);
+}
+
+__global__ void __launch_bounds__(kThreads, kKpmPerSm)
+    k_kpm_csr(int n, int L, const int *__restrict__ ia, const int *__restrict__ ja,
+              const double *__restrict__ a, const double2 *__restrict__ Xk,
+              const double2 *Xkm1, double2 *Xkp1, double ctr, double sc, double *part) {
+  pdl_wait_then_release();
+  const int RB = kThreads / L, rl = (int)threadIdx.x / L, l = (int)threadIdx.x % L;
+  const bool on = rl < RB;
+  KpmAcc t{0.0, 0.0, 0.0, 0.0};
+  for (int row = on ? (int)blockIdx.x * RB + rl : n; row < n; row += (int)gridDim.x * RB) {
+    const size_t me = (size_t)row * L + l;
+    const int e = __ldg(ia + row + 1);
+    int j = __ldg(ia + row);
+    const double2 x = __ldg(Xk + me);
+    const double2 xm1 = Xkm1 ? Xkm1[me] : make_double2(0.0, 0.0);
+    double2 r = make_double2(0.0, 0.0);
+    for (; j < e; j += 4) {
+      double2 xv[4];
+      double av[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        av[u] = 0.0;
+        xv[u] = x;
+        if (j + u < e) {
+          av[u] = __ldg(a + j + u);
+          xv[u] = __ldg(Xk + (size_t)__ldg(ja + j + u) * L + l);
         }
       }
-    }
-    for (; j < e; j++) {
-      const double aj = a[j];
-      const double *xr = Xk + (size_t)ja[j] * ld;
 #pragma unroll
-      for (int q = 0; q < CPL; q++) {
-        const int c = lane + 32 * q;
-        if (c < s) r[q] = fma(aj, xr[c], r[q]);
-      }
+      for (int u = 0; u < 4; u++)
+        if (j + u < e) {
+          r.x = fma(av[u], xv[u].x, r.x);
+          r.y = fma(av[u], xv[u].y, r.y);
+        }
     }
-    const size_t base = (size_t)row * ld;
-#pragma unroll
-    for (int q = 0; q < CPL; q++) {
-      const int c = lane + 32 * q;
-      if (c < s) {
-        double w = (r[q] - ctr * Xk[base + c]) * sc;
-        if (Xkm1) w -= Xkm1[base + c];
-        Xkp1[base + c] = w;
-        acc[q] = fma(w, V0[base + c], acc[q]);
-      }
-    }
+    kpm_row(r, x, xm1, Xkp1, me, ctr, sc, t);
   }
-#pragma unroll
-  for (int q = 0; q < CPL; q++) acc_sh[wib][lane + 32 * q] = acc[q];
+  kpm_finish(t, L, RB, part);
+}
+
+/* hi + lo += v, the rounding errors of hi collected in lo (Knuth's two-sum) */
+__device__ __forceinline__ void two_sum_add(double &hi, double &lo, double v) {
+  const double s = __dadd_rn(hi, v), z = __dsub_rn(s, hi);
+  lo = __dadd_rn(lo, __dadd_rn(__dsub_rn(hi, __dsub_rn(s, z)), __dsub_rn(v, z)));
+  hi = s;
+}
+
+/* out[step][c] = sum over nb blocks of part[step][block][c], c < w <=
+ * kThreads, as high and low parts out[..][2 c], [2 c + 1]: one block per
+ * step, fixed order.  The doubled moments subtract sums near one, so these
+ * are kept past the rounding of a double. */
+__global__ void k_kpm_reduce(const double *__restrict__ part, int nb, int w, double *out) {
+  __shared__ double sh[2][kThreads];
+  const int ns = kThreads / w, seg = (int)threadIdx.x / w, c = (int)threadIdx.x % w;
+  const double *p = part + (size_t)blockIdx.x * nb * w;
+  double hi = 0.0, lo = 0.0;
+  if (seg < ns)
+    for (int b = seg; b < nb; b += ns) two_sum_add(hi, lo, p[(size_t)b * w + c]);
+  sh[0][threadIdx.x] = hi;
+  sh[1][threadIdx.x] = lo;
   __syncthreads();
-  for (int c = threadIdx.x; c < s; c += blockDim.x) {
-    double t = 0.0;
-    for (int w = 0; w < wpb; w++) t += acc_sh[w][c];
-    partials[(size_t)blockIdx.x * s + c] = t;
+  if ((int)threadIdx.x < w) {
+    for (int q = 1; q < ns; q++) {
+      two_sum_add(hi, lo, sh[0][q * w + threadIdx.x]);
+      lo += sh[1][q * w + threadIdx.x];
+    }
+    out[((size_t)blockIdx.x * w + threadIdx.x) * 2] = hi;
+    out[((size_t)blockIdx.x * w + threadIdx.x) * 2 + 1] = lo;
   }
-  /* the columns are added across blocks by k_col_reduce */
-  (void)counter;
 }
 
 /* out[c] = sum_i X[i*ld + c]^2: per-block partials, last block adds them */
@@ -1958,19 +2062,52 @@ static unsigned warp_row_grid(long n) {
   return (unsigned)(g < 1 ? 1 : g);
 }
 
-int kpm_step(const pevsl_devcsr *A, int s, int ld, const double *Xk, const double *Xkm1,
-             double *Xkp1, const double *V0, double ctr, double sc, double *mom) {
+int kpm_blocks(const pevsl_devcsr *A, int s) {
+  const int RB = kThreads / ((s + 1) / 2);
+  return (int)std::min<long>(((long)A->nrows + RB - 1) / RB, kKpmBlocks);
+}
+
+int kpm_step(const pevsl_devcsr *A, int s, const double *Xk, const double *Xkm1, double *Xkp1,
+             double ctr, double sc, double *part) {
   if (s < 1 || s > 64) return PEVSL_ERR_ARG;
-  const unsigned g = warp_row_grid(A->nrows);
-  if (s <= 32) {
-    k_kpm_step<1><<<g, kThreads, 0, ctx().stream>>>(A->nrows, s, ld, A->ia, A->ja, A->a, Xk, Xkm1,
-                                                    Xkp1, V0, ctr, sc, ctx().red, ctx().cnt, mom);
-  } else {
-    k_kpm_step<2><<<g, kThreads, 0, ctx().stream>>>(A->nrows, s, ld, A->ia, A->ja, A->a, Xk, Xkm1,
-                                                    Xkp1, V0, ctr, sc, ctx().red, ctx().cnt, mom);
+  const int L = (s + 1) / 2;
+  const unsigned g = (unsigned)kpm_blocks(A, s);
+  cudaStream_t st = ctx().stream;
+  const double2 *xk = (const double2 *)Xk, *xm = (const double2 *)Xkm1;
+  double2 *xp = (double2 *)Xkp1;
+  if (A->smask) {
+    const int w = stencil_width(A);
+    auto go = [&](auto k) { launch_pdl(k, g, st, A->nrows, L, stencil_of(A), xk, xm, xp, ctr, sc, part); };
+    if (w == 7) go(k_kpm_stencil<7, unsigned char>);
+    else if (w == 5) go(k_kpm_stencil<5, unsigned char>);
+    else if (A->sbytes == 1) go(k_kpm_stencil<0, unsigned char>);
+    else if (A->sbytes == 2) go(k_kpm_stencil<0, unsigned short>);
+    else go(k_kpm_stencil<0, unsigned>);
+    return launched("kpm_stencil");
   }
-  if (launched("kpm_step")) return PEVSL_ERR_CUDA;
-  return col_reduce(ctx().red, (int)g, s, mom);
+  launch_pdl(k_kpm_csr, g, st, A->nrows, L, A->ia, A->ja, A->a, xk, xm, xp, ctr, sc, part);
+  return launched("kpm_csr");
+}
+
+int kpm_reduce(const pevsl_devcsr *A, int s, int steps, const double *part, double *out) {
+  if (steps <= 0) return 0;
+  k_kpm_reduce<<<(unsigned)steps, kThreads, 0, ctx().stream>>>(part, kpm_blocks(A, s),
+                                                               4 * ((s + 1) / 2), out);
+  return launched("kpm_reduce");
+}
+
+/* Vectors per group.  A degree reads X_k and X_{k-1} and writes over X_{k-1}:
+ * 16 bytes per row and vector.  In the stencil form the matrix costs nothing,
+ * so a group holds what stays in L2 from one degree to the next (72 MB of
+ * 126), the groups about equal: 101 x 100 x 99, 300 moments of 30 vectors, in
+ * groups of 4 22.0 ms, of 8 27.8, of 2 29.6, all 30 25.4; 64 x 65 x 63 of 16
+ * 5.5, all 30 7.2.  Where not even two fit, and for a matrix whose entries
+ * each group would read again, as many as a launch takes (64). */
+int kpm_group(const pevsl_devcsr *A, int nvec) {
+  long g = A->smask ? (long)(72e6 / (16.0 * std::max(A->nrows, 1))) / 2 * 2 : 0;
+  g = g < 2 ? 64 : std::min(g, 64L);
+  const long groups = std::max(1L, (nvec + g - 1) / g);
+  return (int)std::min(g, ((nvec + groups - 1) / groups + 1) / 2 * 2);
 }
 
 int block_colnorm2(long n, int s, int ld, const double *X, double *out) {
