@@ -27,7 +27,10 @@ namespace pv {
 
 #define PV_ACTIVE(mask, s) (((mask) >> (s)) & 1u)
 
-/* per-entry decomposition of one launch */
+/* per-entry decomposition of one launch.  The kernels take this and the
+ * pointer tables as __grid_constant__ parameters: indexed by the entry, a
+ * plain by-value parameter is copied to local memory by every thread, which
+ * cost a skipped pass over 10^6 rows 12-14 us and a dot product 17. */
 struct BGeom {
   long n[kMaxBatch];
   long ld[kMaxBatch];
@@ -59,7 +62,7 @@ __device__ __forceinline__ double grid_sum_n(double part, double *partials, unsi
 
 /* ---------------------------------------------------------------- level 1 */
 
-__global__ void k_b_axpy(BGeom g, CPtrs x, VPtrs y, BScal a, unsigned mask) {
+__global__ void k_b_axpy(const __grid_constant__ BGeom g, const __grid_constant__ CPtrs x, const __grid_constant__ VPtrs y, const __grid_constant__ BScal a, unsigned mask) {
   const int s = blockIdx.y;
   if (!PV_ACTIVE(mask, s) || blockIdx.x >= g.nb[s]) return;
   const long n = g.n[s];
@@ -70,7 +73,31 @@ __global__ void k_b_axpy(BGeom g, CPtrs x, VPtrs y, BScal a, unsigned mask) {
     ys[i] += c * xs[i];
 }
 
-__global__ void k_b_scal(BGeom g, VPtrs x, BScal a, unsigned mask) {
+/* y += sign coef[s] x, and x *= 1 / nrm[s], the scalars on the device */
+__global__ void k_b_axpy_dev(const __grid_constant__ BGeom g, const __grid_constant__ CPtrs x,
+                             const __grid_constant__ VPtrs y, const double *coef, double sign) {
+  const int s = blockIdx.y;
+  if (blockIdx.x >= g.nb[s]) return;
+  const long n = g.n[s];
+  const double c = sign * coef[s];
+  const double *xs = x.p[s];
+  double *ys = y.p[s];
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)g.nb[s] * blockDim.x)
+    ys[i] += c * xs[i];
+}
+
+__global__ void k_b_scal_inv_dev(const __grid_constant__ BGeom g, const __grid_constant__ VPtrs x,
+                                 const double *nrm) {
+  const int s = blockIdx.y;
+  if (blockIdx.x >= g.nb[s]) return;
+  const long n = g.n[s];
+  const double c = 1.0 / nrm[s];
+  double *xs = x.p[s];
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)g.nb[s] * blockDim.x)
+    xs[i] *= c;
+}
+
+__global__ void k_b_scal(const __grid_constant__ BGeom g, const __grid_constant__ VPtrs x, const __grid_constant__ BScal a, unsigned mask) {
   const int s = blockIdx.y;
   if (!PV_ACTIVE(mask, s) || blockIdx.x >= g.nb[s]) return;
   const long n = g.n[s];
@@ -80,7 +107,7 @@ __global__ void k_b_scal(BGeom g, VPtrs x, BScal a, unsigned mask) {
     xs[i] *= c;
 }
 
-__global__ void k_b_dot(BGeom g, CPtrs x, CPtrs y, double *partials, unsigned *counters, double *out,
+__global__ void k_b_dot(const __grid_constant__ BGeom g, const __grid_constant__ CPtrs x, const __grid_constant__ CPtrs y, double *partials, unsigned *counters, double *out,
                         int fin, unsigned mask) {
   const int s = blockIdx.y;
   if (!PV_ACTIVE(mask, s) || blockIdx.x >= g.nb[s]) return;
@@ -96,7 +123,7 @@ __global__ void k_b_dot(BGeom g, CPtrs x, CPtrs y, double *partials, unsigned *c
 }
 
 /* y -= coef[s] x, then ||y|| */
-__global__ void k_b_axpy_dev_nrm2(BGeom g, const double *coef, CPtrs x, VPtrs y, double *partials,
+__global__ void k_b_axpy_dev_nrm2(const __grid_constant__ BGeom g, const double *coef, const __grid_constant__ CPtrs x, const __grid_constant__ VPtrs y, double *partials,
                                   unsigned *counters, double *nrm, unsigned mask) {
   const int s = blockIdx.y;
   if (!PV_ACTIVE(mask, s) || blockIdx.x >= g.nb[s]) return;
@@ -125,7 +152,7 @@ static int gemvt_rows(long n) { return n < (1L << 16) ? 256 : 1024; }
 /* partial[s][rb][j] = sum_{i in row block rb} V_s[i + j ld_s] v_s[i] (nb[s]
  * row blocks of rows[s] rows; the partials of entry s start at s*pstride) */
 __global__ void __launch_bounds__(kThreads)
-    k_b_gemvt_partial(BGeom g, int k, CPtrs V, CPtrs v, double *__restrict__ partial,
+    k_b_gemvt_partial(const __grid_constant__ BGeom g, int k, const __grid_constant__ CPtrs V, const __grid_constant__ CPtrs v, double *__restrict__ partial,
                       size_t pstride, const int *run, unsigned mask) {
   const int s = blockIdx.z;
   if (!PV_ACTIVE(mask, s) || (run && run[s] == 0) || blockIdx.x >= g.nb[s]) return;
@@ -146,31 +173,72 @@ __global__ void __launch_bounds__(kThreads)
     if (j >= k) break;
     const double *col = V.p[s] + (size_t)j * ldv + r0;
     double acc = 0.0;
-#pragma unroll 4
+#pragma unroll 8
     for (int i = lane; i < nr; i += 32) acc = fma(col[i], vsh[i], acc);
     acc = warp_sum(acc);
     if (lane == 0) ps[(size_t)blockIdx.x * k + j] = acc;
   }
 }
 
-/* w[s*ldw + j] = sum_rb partial[s][rb][j], in row-block order */
-__global__ void k_b_gemvt_reduce(BGeom g, int k, const double *__restrict__ partial, size_t pstride,
-                                 double *__restrict__ w, long ldw, const int *run, unsigned mask) {
+/* w[s*ldw + j] = sum_rb partial[s][rb][j], in row-block order: a block sums
+ * 32 columns, all its warps loading tiles of 64 row blocks ahead (registers,
+ * then two shared-memory buffers) and warp 0 adding them in order, so that
+ * the time is that of the additions (8 cycles each) and not one load latency
+ * per few row blocks: 977 row blocks 136 -> 6 us. */
+constexpr int kRedTile = 64;
+__global__ void __launch_bounds__(kThreads)
+    k_b_gemvt_reduce(const __grid_constant__ BGeom g, int k, const double *__restrict__ partial,
+                     size_t pstride, double *__restrict__ w, long ldw, const int *run,
+                     unsigned mask) {
   const int s = blockIdx.y;
   if (!PV_ACTIVE(mask, s) || (run && run[s] == 0)) return;
-  const double *ps = partial + (size_t)s * pstride;
-  const unsigned nrb = g.nb[s];
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < k; j += gridDim.x * blockDim.x) {
-    double acc = 0.0;
-    for (unsigned b = 0; b < nrb; b++) acc += ps[(size_t)b * k + j];
-    w[(size_t)s * ldw + j] = acc;
+  __shared__ double sh[2][kRedTile][32];
+  constexpr int NW = kThreads / 32, PER = kRedTile / NW;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int j = blockIdx.x * 32 + lane;
+  const double *ps = partial + (size_t)s * pstride + (j < k ? j : 0);
+  const int nrb = (int)g.nb[s];
+  double next[PER], acc = 0.0;
+  auto fetch = [&](int t) {
+#pragma unroll
+    for (int q = 0; q < PER; q++) {
+      const int b = t + wib * PER + q;
+      next[q] = b < nrb ? ps[(size_t)b * k] : 0.0;
+    }
+  };
+  fetch(0);
+  for (int t = 0, buf = 0; t < nrb; t += kRedTile, buf ^= 1) {
+#pragma unroll
+    for (int q = 0; q < PER; q++) sh[buf][wib * PER + q][lane] = next[q];
+    __syncthreads();
+    fetch(t + kRedTile);
+    if (wib == 0) {
+      const int m = nrb - t < kRedTile ? nrb - t : kRedTile;
+#pragma unroll 16
+      for (int r = 0; r < m; r++) acc += sh[buf][r][lane];
+    }
   }
+  if (wib == 0 && j < k) w[(size_t)s * ldw + j] = acc;
 }
 
+/* row . w over k columns: four sums, column j in sum j % 4 (the k % 4 last
+ * ones in the first) */
+struct RowSums {
+  double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
+  __device__ __forceinline__ double total() const { return (a0 + a1) + (a2 + a3); }
+};
+
 /* v_s -= V_s w_s (thread per row, w_s in shared memory), ||v_s||, and the
- * DGKS flag for the next pass: flag[s] = ||v_s|| <= eta * nrm_old[s]. */
-__global__ void __launch_bounds__(kThreads)
-    k_b_gemv_sub_nrm(BGeom g, int k, CPtrs V, const double *__restrict__ w, long ldw, VPtrs v,
+ * DGKS flag for the next pass: flag[s] = ||v_s|| <= eta * nrm_old[s].  Bound
+ * by the basis' bytes; two rows of a thread run together with eight columns
+ * in flight each (64 registers, four blocks per SM): at 10^6 rows, 25 columns
+ * on average, 44 us (4.9 TB/s) against 46 for one row with four in flight;
+ * 69960 rows (fewer blocks than SMs) 4.1 / 5.7 us; three blocks per SM 46,
+ * five (spills) 59 us. */
+constexpr int kSubRows = 2;
+__global__ void __launch_bounds__(kThreads, 4)
+    k_b_gemv_sub_nrm(const __grid_constant__ BGeom g, int k, const __grid_constant__ CPtrs V,
+                     const double *__restrict__ w, long ldw, const __grid_constant__ VPtrs v,
                      double *partials, unsigned *counters, double *nrm, const int *run,
                      int *flag_out, double *nrm_old, double eta, unsigned mask) {
   const int s = blockIdx.y;
@@ -178,24 +246,60 @@ __global__ void __launch_bounds__(kThreads)
   extern __shared__ double wsh[];
   for (int j = threadIdx.x; j < k; j += blockDim.x) wsh[j] = w[(size_t)s * ldw + j];
   __syncthreads();
-  const long n = g.n[s], ldv = g.ld[s];
-  const double *Vs = V.p[s];
+  const long n = g.n[s], ldv = g.ld[s], stride = (long)g.nb[s] * blockDim.x;
+  const double *__restrict__ Vs = V.p[s];
   double *vs = v.p[s];
   double ss = 0.0;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)g.nb[s] * blockDim.x) {
-    const double *row = Vs + i;
-    double acc0 = 0.0, acc1 = 0.0, acc2 = 0.0, acc3 = 0.0;
-    int j = 0;
-    for (; j + 3 < k; j += 4) {
-      acc0 = fma(row[(size_t)j * ldv], wsh[j], acc0);
-      acc1 = fma(row[(size_t)(j + 1) * ldv], wsh[j + 1], acc1);
-      acc2 = fma(row[(size_t)(j + 2) * ldv], wsh[j + 2], acc2);
-      acc3 = fma(row[(size_t)(j + 3) * ldv], wsh[j + 3], acc3);
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += kSubRows * stride) {
+    RowSums acc[kSubRows];
+    const double *p[kSubRows];
+    double old[kSubRows];
+#pragma unroll
+    for (int q = 0; q < kSubRows; q++) {
+      const long r = i + q * stride;
+      p[q] = Vs + (r < n ? r : i); /* a row past the end repeats the first, unused */
+      old[q] = vs[r < n ? r : i];
     }
-    for (; j < k; j++) acc0 = fma(row[(size_t)j * ldv], wsh[j], acc0);
-    const double nv = vs[i] - ((acc0 + acc1) + (acc2 + acc3));
-    vs[i] = nv;
-    ss = fma(nv, nv, ss);
+    int j = 0;
+    for (; j + 7 < k; j += 8) {
+      double x[kSubRows][8];
+#pragma unroll
+      for (int q = 0; q < kSubRows; q++)
+#pragma unroll
+        for (int u = 0; u < 8; u++) x[q][u] = __ldg(p[q] + (size_t)(j + u) * ldv);
+#pragma unroll
+      for (int q = 0; q < kSubRows; q++)
+#pragma unroll
+        for (int u = 0; u < 8; u += 4) {
+          acc[q].a0 = fma(x[q][u], wsh[j + u], acc[q].a0);
+          acc[q].a1 = fma(x[q][u + 1], wsh[j + u + 1], acc[q].a1);
+          acc[q].a2 = fma(x[q][u + 2], wsh[j + u + 2], acc[q].a2);
+          acc[q].a3 = fma(x[q][u + 3], wsh[j + u + 3], acc[q].a3);
+        }
+    }
+    for (; j + 3 < k; j += 4) {
+#pragma unroll
+      for (int q = 0; q < kSubRows; q++) {
+        const double x0 = __ldg(p[q] + (size_t)j * ldv), x1 = __ldg(p[q] + (size_t)(j + 1) * ldv);
+        const double x2 = __ldg(p[q] + (size_t)(j + 2) * ldv), x3 = __ldg(p[q] + (size_t)(j + 3) * ldv);
+        acc[q].a0 = fma(x0, wsh[j], acc[q].a0);
+        acc[q].a1 = fma(x1, wsh[j + 1], acc[q].a1);
+        acc[q].a2 = fma(x2, wsh[j + 2], acc[q].a2);
+        acc[q].a3 = fma(x3, wsh[j + 3], acc[q].a3);
+      }
+    }
+    for (; j < k; j++)
+#pragma unroll
+      for (int q = 0; q < kSubRows; q++) acc[q].a0 = fma(__ldg(p[q] + (size_t)j * ldv), wsh[j], acc[q].a0);
+#pragma unroll
+    for (int q = 0; q < kSubRows; q++) {
+      const long r = i + q * stride;
+      if (r < n) {
+        const double nv = old[q] - acc[q].total();
+        vs[r] = nv;
+        ss = fma(nv, nv, ss);
+      }
+    }
   }
   bool last;
   const double t = grid_sum_n(ss, partials + (size_t)s * kMaxRedBlocks, counters + s, FIN_SQRT,
@@ -238,6 +342,22 @@ int b_axpy(const BLen &len, int S, CPtrs x, VPtrs y, BScal a, unsigned mask) {
   if (!gx) return 0;
   k_b_axpy<<<dim3(gx, S), kThreads, 0, ctx().stream>>>(g, x, y, a, mask);
   return launched("b_axpy");
+}
+
+int b_axpy_dev(const BLen &len, int S, const double *coef, double sign, CPtrs x, VPtrs y) {
+  BGeom g;
+  const unsigned gx = geom(len, S, (1u << S) - 1u, 4, &g);
+  if (!gx) return 0;
+  k_b_axpy_dev<<<dim3(gx, S), kThreads, 0, ctx().stream>>>(g, x, y, coef, sign);
+  return launched("b_axpy_dev");
+}
+
+int b_scal_inv_dev(const BLen &len, int S, const double *nrm, VPtrs x) {
+  BGeom g;
+  const unsigned gx = geom(len, S, (1u << S) - 1u, 4, &g);
+  if (!gx) return 0;
+  k_b_scal_inv_dev<<<dim3(gx, S), kThreads, 0, ctx().stream>>>(g, x, nrm);
+  return launched("b_scal_inv_dev");
 }
 
 int b_scal(const BLen &len, int S, VPtrs x, BScal a, unsigned mask) {
@@ -297,7 +417,7 @@ int b_gemvT(const BLen &len, int S, int k, CPtrs V, CPtrs v, double *w, long ldw
   k_b_gemvt_partial<<<g1, kThreads, sizeof(double) * maxrows, ctx().stream>>>(g, k, V, v, part,
                                                                               pstride, run, mask);
   if (launched("b_gemvT_partial")) return PEVSL_ERR_CUDA;
-  dim3 g2((unsigned)((k + kThreads - 1) / kThreads), S);
+  dim3 g2((unsigned)((k + 31) / 32), S);
   k_b_gemvt_reduce<<<g2, kThreads, 0, ctx().stream>>>(g, k, part, pstride, w, ldw, run, mask);
   return launched("b_gemvT_reduce");
 }
