@@ -76,6 +76,8 @@ enum Ws {
   WS_IL,        /* interleaved filter: three n x S blocks     */
   WS_ILMU,      /* interleaved filter: per-degree coefficients */
   WS_CLMU,      /* cluster filter: one polynomial's coefficients */
+  WS_LAN,       /* Lanczos runs: alpha and beta of every step, CGS coefficients */
+  WS_LANV,      /* Lanczos DOS: the start vectors of a group */
   WS_COUNT
 };
 
@@ -153,6 +155,8 @@ int rand_gauss(double *X, long n, int nv, long rs, long cs, uint64_t seed, uint6
 
 /* ---------------------------------------------------------------- sparse */
 int spmv(const pevsl_devcsr *A, const double *x, double *y);
+/* y_s = A x_s for S <= kMaxBatch vectors, each as spmv gives it */
+int spmv_batch(const pevsl_devcsr *A, int S, CPtrs x, VPtrs y);
 /* One degree of the Chebyshev filter recurrence (fused SpMV):
  *   w = ((A vk - cc vk) * t) - vkm1   (vkm1 may be NULL)
  *   vkp1 = w;  y = first ? mu0 * vk + muk * w : y + muk * w            */
@@ -231,6 +235,10 @@ struct BLen {
 BLen blen_uniform(long n, long ld, int S);
 int b_axpy(const BLen &len, int S, CPtrs x, VPtrs y, BScal a, unsigned mask);
 int b_scal(const BLen &len, int S, VPtrs x, BScal a, unsigned mask);
+/* y_s += sign coef[s] x_s and x_s *= 1 / nrm[s] for all S entries, the
+ * scalars in device memory */
+int b_axpy_dev(const BLen &len, int S, const double *coef, double sign, CPtrs x, VPtrs y);
+int b_scal_inv_dev(const BLen &len, int S, const double *nrm, VPtrs x);
 int b_dot(const BLen &len, int S, CPtrs x, CPtrs y, double *out, int fin, unsigned mask);
 int b_axpy_dev_nrm2(const BLen &len, int S, const double *coef, CPtrs x, VPtrs y, double *nrm,
                     unsigned mask);

@@ -968,11 +968,127 @@ int pEVSL_Kpmdos(pevsl_Data *pevsl, int Mdeg, int damping, int nvec, double *int
 
 /* ================================================================ Lanczos DOS */
 
+/* Host threads for the per-slice host work of a lockstep group (the
+ * tridiagonal eigenproblems of the convergence tests and the Ritz
+ * extraction): PEVSL_B200_HOST_THREADS caps them (1: the calling thread
+ * only; default: every hardware thread). */
+static unsigned host_threads() {
+  static unsigned v = 0;
+  if (!v) {
+    const char *e = getenv("PEVSL_B200_HOST_THREADS");
+    const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
+    const int r = e ? atoi(e) : 0;
+    v = r >= 1 ? std::min((unsigned)r, hw) : hw;
+  }
+  return v;
+}
+
+/* f(0), ..., f(m-1) on up to host_threads() threads, this one included,
+ * when worth is set; else in order on this thread.  f must be host-only
+ * code (no CUDA call) that writes nothing another index reads. */
+extern "C++" {
+template <class F>
+static void host_parallel(size_t m, bool worth, F f) {
+  const size_t nt = std::min<size_t>(m, host_threads());
+  if (!worth || nt <= 1) {
+    for (size_t i = 0; i < m; i++) f(i);
+    return;
+  }
+  std::atomic<size_t> next{0};
+  auto work = [&]() {
+    for (size_t i = next.fetch_add(1); i < m; i = next.fetch_add(1)) f(i);
+  };
+  std::vector<std::thread> th;
+  for (size_t t = 1; t < nt; t++) {
+    try {
+      th.emplace_back(work);
+    } catch (...) {
+      break; /* no more threads: this one does the rest */
+    }
+  }
+  work();
+  for (auto &x : th) x.join();
+}
+}  // extern "C++"
+
+/* Lanczos steps of S <= kMaxBatch independent runs in lockstep, queued
+ * without a host synchronisation: alpha and beta stay on the device, where
+ * the next step reads them, and the host reads all steps at once.  (A
+ * breakdown therefore shows only then; what was queued past it is dropped.)
+ * Run s has its basis at V[s] (leading dimension ld).  Per run the kernels
+ * and their decompositions are those of a single run, so each run's values
+ * are the bits it has alone. */
+struct LanRuns {
+  pevsl_Data *pevsl;
+  int S;
+  long n, ld;
+  int maxk;                /* columns of a basis */
+  double *V[kMaxBatch];
+  double *hist, *nrm0, *w; /* [step][alpha, beta][S]; norms; CGS coefficients */
+  double *alpha(int step) const { return hist + 2 * (size_t)step * S; }
+  double *beta(int step) const { return alpha(step) + S; }
+};
+
+static int lan_init(LanRuns &R, pevsl_Data *pevsl, int S, double *V, long stride, long n, long ld,
+                    int maxk) {
+  R.pevsl = pevsl;
+  R.S = S;
+  R.n = n;
+  R.ld = ld;
+  R.maxk = maxk;
+  for (int s = 0; s < S; s++) R.V[s] = V + (size_t)s * (size_t)stride;
+  const size_t h = 2 * (size_t)maxk * S;
+  R.hist = (double *)ws(WS_LAN, sizeof(double) * (h + S + (size_t)S * (size_t)(maxk + 1)));
+  if (!R.hist) return PEVSL_ERR_NOMEM;
+  R.nrm0 = R.hist + h;
+  R.w = R.nrm0 + S;
+  return 0;
+}
+
+/* step k: V(:, k+1) from V(:, k) and V(:, k-1); prev: subtract beta(k-1)
+ * V(:, k-1) */
+static int lan_step(LanRuns &R, int k, bool prev) {
+  const int S = R.S;
+  const unsigned all = (1u << S) - 1u;
+  const BLen len = blen_uniform(R.n, R.ld, S);
+  CPtrs v{}, vm{}, vc{}, base{};
+  VPtrs vn{};
+  for (int s = 0; s < S; s++) {
+    base.p[s] = R.V[s];
+    v.p[s] = R.V[s] + (size_t)k * R.ld;
+    vm.p[s] = prev ? v.p[s] - R.ld : nullptr;
+    vn.p[s] = R.V[s] + (size_t)(k + 1) * R.ld;
+    vc.p[s] = vn.p[s];
+  }
+  int *flag = ctx().gflag;
+  int st = 0;
+  if (pevsl_devcsr *A = pevsl_builtin_A(R.pevsl)) {
+    R.pevsl->stats->n_mvA += (size_t)S;
+    st = spmv_batch(A, S, v, vn);
+  } else {
+    for (int s = 0; s < S && !st; s++) st = apply_A(R.pevsl, v.p[s], vn.p[s]);
+  }
+  if (!st && prev) st = b_axpy_dev(len, S, R.beta(k - 1), -1.0, vm, vn);
+  if (!st) st = b_dot(len, S, v, vc, R.alpha(k), FIN_ID, all);
+  if (!st) st = b_axpy_dev_nrm2(len, S, R.alpha(k), v, vn, R.nrm0, all);
+  const long ldw = R.maxk + 1;
+  if (!st) st = b_gemvT(len, S, k + 1, base, vc, R.w, ldw, nullptr, all);
+  if (!st)
+    st = b_gemv_sub_nrm(len, S, k + 1, base, R.w, ldw, vn, R.beta(k), nullptr, flag, R.nrm0, kEta, all);
+  if (!st) st = b_gemvT(len, S, k + 1, base, vc, R.w, ldw, flag, all);
+  if (!st)
+    st = b_gemv_sub_nrm(len, S, k + 1, base, R.w, ldw, vn, R.beta(k), flag, nullptr, nullptr, kEta, all);
+  if (!st) st = b_scal_inv_dev(len, S, R.beta(k), vn);
+  return st;
+}
+
 /* one Lanczos run of pEVSL_LanDosG (SRC/landos.c:134-262): v_0 = vinit
  * normalised, maxit steps with full reorthogonalisation; the tridiagonal
  * matrix into dT, eT */
+extern "C++" {
+template <class Draw>
 static int landos_lanczos(pevsl_Data *pevsl, int maxit, double *V, long ld, const double *vinit,
-                          long n, double *dT, double *eT) {
+                          long n, double *dT, double *eT, Draw draw) {
   Ctx &c = ctx();
   int st = vnrm2(n, vinit, c.dscal + S_TMP0);
   const double *h = st ? nullptr : fetch_scalars(S_TMP0, 1);
@@ -998,7 +1114,7 @@ static int landos_lanczos(pevsl_Data *pevsl, int maxit, double *V, long ld, cons
     wn += fabs(alpha) + 2.0 * beta;
     nwn += 3;
     if (beta * nwn < orthTol * wn) {
-      st = pevsl_rand_vector_dev(vnew, (int)n);
+      st = draw(vnew);
       if (!st) st = vnrm2(n, vnew, c.dscal + S_NRM0);
       if (!st) st = cgs_dgks(V, ld, k + 1, vnew, n);
       const double *hb = st ? nullptr : fetch_scalars(S_NRM, 1);
@@ -1013,6 +1129,44 @@ static int landos_lanczos(pevsl_Data *pevsl, int maxit, double *V, long ld, cons
   return st;
 }
 
+}  // extern "C++"
+
+/* the S runs of a group in lockstep from the start vectors vinit(:, 0:S)
+ * (unchanged); *broke: a run broke down, the group is to be run one by one */
+static int landos_lockstep(pevsl_Data *pevsl, int S, int maxit, double *V, long ld,
+                           const double *vinit, long n, double *dT, double *eT, bool *broke) {
+  *broke = false;
+  LanRuns R;
+  int st = lan_init(R, pevsl, S, V, ld * (maxit + 1), n, ld, maxit + 1);
+  CPtrs x{};
+  VPtrs v0{};
+  for (int s = 0; s < S && !st; s++) {
+    st = vcopy(vinit + (size_t)s * ld, R.V[s], n);
+    x.p[s] = R.V[s];
+    v0.p[s] = R.V[s];
+  }
+  const BLen len = blen_uniform(n, ld, S);
+  if (!st) st = b_dot(len, S, x, x, R.nrm0, FIN_SQRT, (1u << S) - 1u);
+  if (!st) st = b_scal_inv_dev(len, S, R.nrm0, v0);
+  for (int k = 0; k < maxit && !st; k++) st = lan_step(R, k, k > 0);
+  std::vector<double> h(2 * (size_t)maxit * S);
+  if (!st) st = memcpy_async(h.data(), R.hist, sizeof(double) * h.size());
+  if (!st) st = sync();
+  for (int s = 0; s < S && !st; s++) {
+    double wn = 0.0;
+    int nwn = 0;
+    for (int k = 0; k < maxit; k++) {
+      const double alpha = h[2 * (size_t)k * S + s], beta = h[(2 * (size_t)k + 1) * S + s];
+      dT[(size_t)s * maxit + k] = alpha;
+      eT[(size_t)s * maxit + k] = beta;
+      wn += fabs(alpha) + 2.0 * beta;
+      nwn += 3;
+      if (beta * nwn < orthTol * wn) *broke = true;
+    }
+  }
+  return st;
+}
+
 int pEVSL_LanDosG(pevsl_Data *pevsl, const int nvec, int msteps, int npts, double *xdos,
                   double *ydos, double *neig, double *intv, int ngroups, int groupid,
                   MPI_Comm gl_comm) {
@@ -1020,14 +1174,23 @@ int pEVSL_LanDosG(pevsl_Data *pevsl, const int nvec, int msteps, int npts, doubl
   const double t0 = pevsl_now();
   const long n = pevsl->n, ld = round_ld(n);
   const int maxit = msteps < pevsl->N ? msteps : pevsl->N;
-  double *V = (double *)ws(WS_BASIS, sizeof(double) * (size_t)ld * (size_t)(maxit + 1));
-  double *vinit = (double *)ws(WS_VEC, sizeof(double) * (size_t)n);
+  int vec_start = 0, vec_end = nvec;
+  if (ngroups > 1) pEVSL_Part1d(nvec, ngroups, &groupid, &vec_start, &vec_end, 1);
+  /* runs in lockstep: up to kMaxBatch, their bases within 4 GB, the groups
+   * about equal; one at a time with B-solves */
+  const double basis = 8.0 * (double)ld * (maxit + 1);
+  const int nrun = PEVSL_MAX(vec_end - vec_start, 0);
+  int lock = pevsl->ifGenEv ? 1 : (int)PEVSL_MIN((double)kMaxBatch, PEVSL_MAX(1.0, 4e9 / basis));
+  const int ngr = PEVSL_MAX(1, (nrun + lock - 1) / lock);
+  lock = PEVSL_MAX(1, (nrun + ngr - 1) / ngr);
+  double *V = (double *)ws(WS_BASIS, sizeof(double) * (size_t)ld * (size_t)(maxit + 1) * (size_t)lock);
+  double *vinit = (double *)ws(WS_LANV, sizeof(double) * (size_t)ld * (size_t)(lock + 1));
   double *y = (double *)calloc((size_t)npts, sizeof(double));
   int *ind = (int *)malloc(sizeof(int) * (size_t)npts);
-  double *dT = (double *)malloc(sizeof(double) * (size_t)maxit);
-  double *eT = (double *)malloc(sizeof(double) * (size_t)maxit);
-  double *EvalT = (double *)malloc(sizeof(double) * (size_t)maxit);
-  double *EvecT = (double *)malloc(sizeof(double) * (size_t)maxit * (size_t)maxit);
+  double *dT = (double *)malloc(sizeof(double) * (size_t)maxit * (size_t)lock);
+  double *eT = (double *)malloc(sizeof(double) * (size_t)maxit * (size_t)lock);
+  double *EvalT = (double *)malloc(sizeof(double) * (size_t)maxit * (size_t)lock);
+  double *EvecT = (double *)malloc(sizeof(double) * (size_t)maxit * (size_t)maxit * (size_t)lock);
   int st = (!V || !vinit || !y || !ind || !dT || !eT || !EvalT || !EvecT) ? PEVSL_ERR_NOMEM : 0;
   const double lm = intv[2], lM = intv[3];
   const double aa = PEVSL_MAX(intv[0], intv[2]), bb = PEVSL_MIN(intv[1], intv[3]);
@@ -1037,25 +1200,47 @@ int pEVSL_LanDosG(pevsl_Data *pevsl, const int nvec, int msteps, int npts, doubl
   const double sigma2 = 2 * sigma * sigma;
   const double width = sigma * sqrt(-2.0 * log(1e-08));
   if (!st) linspace(aa, bb, npts, xdos);
-  int vec_start = 0, vec_end = nvec;
-  if (ngroups > 1) pEVSL_Part1d(nvec, ngroups, &groupid, &vec_start, &vec_end, 1);
-  for (int m = vec_start; m < vec_end && !st; m++) {
-    st = pevsl_rand_vector_dev(vinit, (int)n);
-    if (!st) st = pevsl->ifGenEv ? pevsl_gen_landos_lanczos(pevsl, maxit, vinit, dT, eT)
-                                 : landos_lanczos(pevsl, maxit, V, ld, vinit, n, dT, eT);
-    if (st) break;
-    if (pevsl_tridiag_eig(maxit, dT, eT, EvalT, EvecT)) {
-      st = PEVSL_ERR_EIG;
-      break;
+  for (int m0 = vec_start; m0 < vec_end && !st; m0 += lock) {
+    const int S = PEVSL_MIN(lock, vec_end - m0);
+    /* the group's start vectors in draw order; a breakdown restart takes the
+     * next one, as in runs one after the other */
+    int drawn = 0, next = 0;
+    for (; drawn < S && !st; drawn++) st = pevsl_rand_vector_dev(vinit + (size_t)drawn * ld, (int)n);
+    auto draw = [&](double *v) -> int {
+      return next < drawn ? vcopy(vinit + (size_t)next++ * ld, v, n) : pevsl_rand_vector_dev(v, (int)n);
+    };
+    bool broke = true;
+    if (!st && !pevsl->ifGenEv) st = landos_lockstep(pevsl, S, maxit, V, ld, vinit, n, dT, eT, &broke);
+    double *one = vinit + (size_t)lock * ld;
+    for (int s = 0; s < S && broke && !st; s++) {
+      st = draw(one);
+      if (!st)
+        st = pevsl->ifGenEv
+                 ? pevsl_gen_landos_lanczos(pevsl, maxit, one, dT + (size_t)s * maxit, eT + (size_t)s * maxit)
+                 : landos_lanczos(pevsl, maxit, V, ld, one, n, dT + (size_t)s * maxit,
+                                  eT + (size_t)s * maxit, draw);
     }
-    for (int i = 0; i < maxit; i++) {
-      const double g2 = EvecT[(size_t)i * maxit] * EvecT[(size_t)i * maxit];
-      const double th = EvalT[i];
-      int np = 0;
-      for (int j = 0; j < npts; j++)
-        if (fabs(xdos[j] - th) < width) ind[np++] = j;
-      for (int j = 0; j < np; j++)
-        y[ind[j]] += g2 * exp(-((xdos[ind[j]] - th) * (xdos[ind[j]] - th)) / sigma2);
+    if (st) break;
+    std::vector<int> es((size_t)S, 0);
+    host_parallel((size_t)S, maxit >= 30, [&](size_t s) {
+      es[s] = pevsl_tridiag_eig(maxit, dT + s * maxit, eT + s * maxit, EvalT + s * maxit,
+                                EvecT + s * (size_t)maxit * maxit);
+    });
+    for (int s = 0; s < S && !st; s++) {
+      if (es[(size_t)s]) {
+        st = PEVSL_ERR_EIG;
+        break;
+      }
+      const double *ev = EvecT + (size_t)s * maxit * maxit;
+      for (int i = 0; i < maxit; i++) {
+        const double g2 = ev[(size_t)i * maxit] * ev[(size_t)i * maxit];
+        const double th = EvalT[(size_t)s * maxit + i];
+        int np = 0;
+        for (int j = 0; j < npts; j++)
+          if (fabs(xdos[j] - th) < width) ind[np++] = j;
+        for (int j = 0; j < np; j++)
+          y[ind[j]] += g2 * exp(-((xdos[ind[j]] - th) * (xdos[ind[j]] - th)) / sigma2);
+      }
     }
   }
   if (!st && ngroups > 1) {
@@ -1117,9 +1302,12 @@ int pEVSL_LanTrbounds(pevsl_Data *pevsl, int lanm, int maxit, double tol, pevsl_
   double *dS = dY + 2 * L; /* coefficients s of the restart step */
   Ctx &c = ctx();
   int st = 0, it = 0, trlen = 0;
+  LanRuns R;
+  st = lan_init(R, pevsl, 1, V, 0, n, ld, lanm1);
+  std::vector<double> hist(2 * L);
   double lmin = 0.0, lmax = 0.0, s[3] = {0, 0, 0};
   if (fstats) fprintf(fstats, " LanTR for bounds: dim %d, maxits %d\n", lanm, maxit);
-  st = vcopy(vinit->data, V, n);
+  if (!st) st = vcopy(vinit->data, V, n);
   if (!st) st = vnrm2(n, V, c.dscal + S_TMP0);
   const double *h0 = st ? nullptr : fetch_scalars(S_TMP0, 1);
   if (!h0) st = st ? st : PEVSL_ERR_CUDA;
@@ -1185,42 +1373,45 @@ int pEVSL_LanTrbounds(pevsl_Data *pevsl, int lanm, int maxit, double tol, pevsl_
       T[k1 * L + k] = beta;
       T[k * L + k1] = beta;
     }
-    const double *zold = k > 0 ? VC(k - 1) : nullptr;
-    while (k < lanm && it < maxit && !st) {
-      k++;
-      double *v = VC(k - 1), *vnew = VC(k);
-      st = apply_A(pevsl, v, vnew);
-      it++;
-      if (!st && zold) st = vaxpy(n, -beta, zold, vnew);
-      if (!st) st = vdot(n, v, vnew, c.dscal + S_ALPHA);
-      if (!st) st = vaxpy_dev_nrm2(n, c.dscal + S_ALPHA, v, vnew, c.dscal + S_NRM0);
-      if (!st) st = cgs_dgks(V, ld, k, vnew, n);
-      if (!st) st = memcpy_async(c.hscal + S_ALPHA, c.dscal + S_ALPHA, sizeof(double) * 4);
+    /* the steps of this cycle, queued at once; then their alpha and beta are
+     * read, and after a breakdown the steps past it are queued again */
+    bool prev = k > 0;
+    const int kend = PEVSL_MIN(lanm, k + maxit - it);
+    while (k < kend && !st) {
+      const int k0 = k;
+      if (prev) st = memcpy_async(R.beta(k0 - 1), &beta, sizeof(double));
+      for (int j = k0; j < kend && !st; j++) st = lan_step(R, j, j > k0 || prev);
+      const int m = kend - k0;
+      if (!st) st = memcpy_async(hist.data(), R.alpha(k0), sizeof(double) * 2 * (size_t)m);
       if (!st) st = sync();
-      if (st) break;
-      const double alpha = c.hscal[S_ALPHA];
-      beta = c.hscal[S_NRM];
-      T[(k - 1) * L + (k - 1)] = alpha;
-      wn += fabs(alpha) + 2.0 * beta;
-      nwn += 3;
-      zold = v;
-      if (beta * nwn < orthTol * wn) {
-        if (fstats) fprintf(fstats, "it %4d: Lucky breakdown, beta = %.15e\n", it, beta);
-        st = pevsl_rand_vector_dev(vnew, (int)n);
-        if (!st) st = vnrm2(n, vnew, c.dscal + S_NRM0);
-        if (!st) st = cgs_dgks(V, ld, k, vnew, n);
-        const double *hb = st ? nullptr : fetch_scalars(S_NRM, 1);
-        if (!hb) {
-          st = st ? st : PEVSL_ERR_CUDA;
-          break;
+      bool broke = false;
+      for (int j = 0; j < m && !st && !broke; j++) {
+        const double alpha = hist[2 * (size_t)j];
+        beta = hist[2 * (size_t)j + 1];
+        k++;
+        it++;
+        T[(k - 1) * L + (k - 1)] = alpha;
+        wn += fabs(alpha) + 2.0 * beta;
+        nwn += 3;
+        if (beta * nwn < orthTol * wn) {
+          if (fstats) fprintf(fstats, "it %4d: Lucky breakdown, beta = %.15e\n", it, beta);
+          double *vnew = VC(k);
+          st = pevsl_rand_vector_dev(vnew, (int)n);
+          if (!st) st = vnrm2(n, vnew, c.dscal + S_NRM0);
+          if (!st) st = cgs_dgks(V, ld, k, vnew, n);
+          const double *hb = st ? nullptr : fetch_scalars(S_NRM, 1);
+          if (!hb) {
+            st = st ? st : PEVSL_ERR_CUDA;
+            break;
+          }
+          st = vscal(vnew, n, 1.0 / hb[0]);
+          beta = 0.0;
+          broke = true;
         }
-        st = vscal(vnew, n, 1.0 / hb[0]);
-        beta = 0.0;
-      } else {
-        st = vscal(vnew, n, 1.0 / beta);
+        T[k * L + (k - 1)] = beta;
+        T[(k - 1) * L + k] = beta;
       }
-      T[k * L + (k - 1)] = beta;
-      T[(k - 1) * L + k] = beta;
+      prev = true;
     }
     if (st) break;
     if (pevsl_dense_symeig(k, T, lanm1, EvecT, lanm1, Rval)) {
@@ -1298,49 +1489,6 @@ struct SliceState {
   double *Lam, *res;
   pevsl_Parvecs *Rvec;
 };
-
-/* Host threads for the per-slice host work of a lockstep group (the
- * tridiagonal eigenproblems of the convergence tests and the Ritz
- * extraction): PEVSL_B200_HOST_THREADS caps them (1: the calling thread
- * only; default: every hardware thread). */
-static unsigned host_threads() {
-  static unsigned v = 0;
-  if (!v) {
-    const char *e = getenv("PEVSL_B200_HOST_THREADS");
-    const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-    const int r = e ? atoi(e) : 0;
-    v = r >= 1 ? std::min((unsigned)r, hw) : hw;
-  }
-  return v;
-}
-
-/* f(0), ..., f(m-1) on up to host_threads() threads, this one included,
- * when worth is set; else in order on this thread.  f must be host-only
- * code (no CUDA call) that writes nothing another index reads. */
-extern "C++" {
-template <class F>
-static void host_parallel(size_t m, bool worth, F f) {
-  const size_t nt = std::min<size_t>(m, host_threads());
-  if (!worth || nt <= 1) {
-    for (size_t i = 0; i < m; i++) f(i);
-    return;
-  }
-  std::atomic<size_t> next{0};
-  auto work = [&]() {
-    for (size_t i = next.fetch_add(1); i < m; i = next.fetch_add(1)) f(i);
-  };
-  std::vector<std::thread> th;
-  for (size_t t = 1; t < nt; t++) {
-    try {
-      th.emplace_back(work);
-    } catch (...) {
-      break; /* no more threads: this one does the rest */
-    }
-  }
-  work();
-  for (auto &x : th) x.join();
-}
-}  // extern "C++"
 
 /* The host part of a slice's Ritz extraction: the eigenvalues of T again
  * and the eigenvectors of those >= bar.  Host arithmetic only, so the

@@ -557,6 +557,17 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
+/* y_s = A x_s, vector s = blockIdx.y */
+template <int K, class M>
+__global__ void __launch_bounds__(kThreads)
+    k_spmv_stencil_batch(int n, const __grid_constant__ Stencil S, const __grid_constant__ CPtrs x,
+                         const __grid_constant__ VPtrs y) {
+  const int row = (int)(blockIdx.x * (unsigned)kThreads + threadIdx.x);
+  if (row >= n) return;
+  const unsigned m = stencil_mask<M>(S, row);
+  y.p[blockIdx.y][row] = stencil_dot<K, false>(S, m, x.p[blockIdx.y] + row, 0.0);
+}
+
 /* a filter degree with the sum's update deferred (cheb_step_y) */
 struct EpiChebY {
   const double *vk, *vkm1;
@@ -1267,6 +1278,25 @@ int spmv(const pevsl_devcsr *A, const double *x, double *y) {
   return launched("spmv");
 }
 
+int spmv_batch(const pevsl_devcsr *A, int S, CPtrs x, VPtrs y) {
+  if (A->nrows <= 0 || S <= 0) return 0;
+  if (S > kMaxBatch) return PEVSL_ERR_ARG;
+  if (!A->smask || S == 1) {
+    for (int s = 0; s < S; s++)
+      if (spmv(A, x.p[s], y.p[s])) return PEVSL_ERR_CUDA;
+    return 0;
+  }
+  const int w = stencil_width(A);
+  const dim3 g((unsigned)((A->nrows + kThreads - 1) / kThreads), (unsigned)S);
+  auto k = w == 7           ? k_spmv_stencil_batch<7, unsigned char>
+           : w == 5         ? k_spmv_stencil_batch<5, unsigned char>
+           : A->sbytes == 1 ? k_spmv_stencil_batch<0, unsigned char>
+           : A->sbytes == 2 ? k_spmv_stencil_batch<0, unsigned short>
+                            : k_spmv_stencil_batch<0, unsigned>;
+  k<<<g, kThreads, 0, ctx().stream>>>(A->nrows, stencil_of(A), x, y);
+  return launched("spmv_stencil_batch");
+}
+
 /* the ELL kernel and its switch (defined with the interleaved kernels) */
 template <int S, int EW = 0>
 __global__ void k_cheb_il_e(int n, const short *__restrict__ edj,
@@ -1877,13 +1907,13 @@ int filter_tune(pevsl_devcsr *A) {
 }
 
 /* X[i*S + s] = x_s[i] and back */
-__global__ void k_il_pack(long n, int S, CPtrs xs, double *X) {
+__global__ void k_il_pack(long n, int S, const __grid_constant__ CPtrs xs, double *X) {
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n * S;
        i += (long)gridDim.x * blockDim.x)
     X[i] = xs.p[i % S][i / S];
 }
 
-__global__ void k_il_unpack(long n, int S, int cols, const double *X, VPtrs ys) {
+__global__ void k_il_unpack(long n, int S, int cols, const double *X, const __grid_constant__ VPtrs ys) {
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n * S;
        i += (long)gridDim.x * blockDim.x)
     if ((int)(i % S) < cols) ys.p[i % S][i / S] = X[i];
