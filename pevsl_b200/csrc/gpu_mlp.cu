@@ -5,15 +5,14 @@
  * inference run on this file's kernels:
  *
  *   k_gemm_bf16   C = op(A) op(B) on the tensor cores (warp-level
- *                 mma.sync m16n8k16, BF16 inputs, FP32 accumulators), 64x64
+ *                 mma.sync m16n8k16, BF16 inputs, FP32 accumulators), 32x32
  *                 tiles, operands staged in shared memory (either operand
- *                 may be transposed while staging), with fused epilogues:
+ *                 may be transposed), with fused epilogues:
  *                 bias + GELU (forward), bias (output layer), GELU'
  *                 (backward through an activation), plain store (weight
- *                 gradients);
+ *                 gradients, with the bias gradients' column sums);
  *   k_mse         dY = 2 (Y - T) / (B * nout) on the real outputs, and the
  *                 loss (deterministic block-ordered sum);
- *   k_colsum      bias gradients (column sums in row order);
  *   k_adam        Adam on the FP32 master weights, then the BF16 copies.
  *
  * Layer l maps K_l inputs to N_l outputs (dimensions padded to multiples of
@@ -28,14 +27,14 @@
 #include <string.h>
 
 #include "gpu.cuh"
+#include "gpu_device.cuh"
 
 namespace pv {
 
 typedef __nv_bfloat16 bf16;
 
-constexpr int kGT = 64;    /* block tile (M and N) */
-constexpr int kGK = 16;    /* K step = mma k */
-constexpr int kGPad = 24;  /* shared row stride in bf16 (48 bytes): conflict-light, 4-byte aligned */
+constexpr int kGT = 32;    /* block tile (M and N) */
+constexpr int kGKC = 320;  /* k staged at once (a multiple of 16) */
 
 enum { EPI_STORE = 0, EPI_BIAS = 1, EPI_BIAS_GELU = 2, EPI_DGELU = 3 };
 
@@ -54,84 +53,169 @@ __device__ __forceinline__ void mma_bf16_16816(float c[4], const uint32_t a[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
+__device__ __forceinline__ uint32_t smem_addr(const void *p) {
+  return (uint32_t)__cvta_generic_to_shared(p);
+}
+
+/* 16 bytes to shared memory, zeros when !ok */
+__device__ __forceinline__ void cp16(void *dst, const void *src, bool ok) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_addr(dst)), "l"(src),
+               "r"(ok ? 16 : 0)
+               : "memory");
+}
+
+__device__ __forceinline__ void ldm4(uint32_t r[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
+}
+__device__ __forceinline__ void ldm4t(uint32_t r[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
+}
+
+/* db[n] = sum_m dZ[m][n], rows in order, for the 32 columns from n0 on: the
+ * block's warps stage 64 rows at a time and warp 0 adds them */
+__device__ __forceinline__ void colsum(int Bn, int N, int n0, const float *__restrict__ dZ, int ld,
+                                       float *__restrict__ db, float *sh) {
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, n = n0 + lane;
+  float s = 0.f, next[16];
+  auto fetch = [&](int t) {
+#pragma unroll
+    for (int q = 0; q < 16; q++) {
+      const int m = t + wib * 16 + q;
+      next[q] = m < Bn && n < N ? __ldg(dZ + (size_t)m * ld + n) : 0.f;
+    }
+  };
+  fetch(0);
+  for (int t = 0, buf = 0; t < Bn; t += 64, buf ^= 1) {
+#pragma unroll
+    for (int q = 0; q < 16; q++) sh[(buf * 64 + wib * 16 + q) * 32 + lane] = next[q];
+    __syncthreads();
+    fetch(t + 64);
+    if (wib == 0) {
+      const int m = Bn - t < 64 ? Bn - t : 64;
+#pragma unroll 16
+      for (int r = 0; r < m; r++) s += sh[(buf * 64 + r) * 32 + lane];
+    }
+  }
+  if (wib == 0 && n < N) db[n] = s;
+}
+
 /* C[m][n] = sum_k A'(m,k) B'(k,n) for m < M, n < N, with
  * A'(m,k) = TA ? A[k*lda + m] : A[m*lda + k] and
  * B'(k,n) = TB ? B[n*ldb + k] : B[k*ldb + n]; out-of-range elements are 0.
- * 128 threads: warp w owns rows 32*(w/2) .. +32 and columns 32*(w%2) .. +32
- * of the 64x64 tile, as 2 x 4 tiles of 16x8.  Epilogue (row m, column n):
- *   EPI_STORE      C = acc
+ * Every extent along a row of A or B is a multiple of 16 (padded layer
+ * sizes), so rows are staged in 16-byte copies; the batch, which is not,
+ * runs along the rows' index.  128 threads: warp w owns the 16 x 16 piece
+ * (w / 2, w % 2) of a 32 x 32 tile.  Epilogue (row m, column n):
+ *   EPI_STORE      C = acc; one more block per row of tiles forms the column
+ *                  sums db of the FP32 dZ (zp, the K rows of C's m columns)
  *   EPI_BIAS       C = acc + bias[n]
  *   EPI_BIAS_GELU  C = z = acc + bias[n];  act = bf16(gelu(z))
- *   EPI_DGELU      C = g = acc * gelu'(zp[m][n]);  act = bf16(g) */
+ *   EPI_DGELU      C = g = acc * gelu'(zp[m][n]);  act = bf16(g)
+ * What bounds it is latency: a layer of 128 x 256 x 304 is 20 MFLOP on a few
+ * dozen blocks.  So all of K (up to kGKC) is staged at once, in one round
+ * trip, and the k steps run without a barrier: a forward layer 26.7 -> 5.5 us
+ * against 64 x 64 tiles staged 16 deep element by element (ten blocks, a
+ * round trip per k step).  The k steps come in the same order: the same bits. */
 template <bool TA, bool TB, int EPI>
 __global__ void __launch_bounds__(128)
     k_gemm_bf16(int M, int N, int K, const bf16 *__restrict__ A, int lda,
                 const bf16 *__restrict__ B, int ldb, float *__restrict__ C, int ldc,
                 const float *__restrict__ bias, bf16 *__restrict__ act, int ldact,
-                const float *__restrict__ zp, int ldzp) {
-  __shared__ __align__(16) bf16 As[kGT][kGPad];
-  __shared__ __align__(16) bf16 Bs[kGT][kGPad]; /* [n][k] */
+                const float *__restrict__ zp, int ldzp, float *__restrict__ db) {
+  /* a tile's rows: k along them (32 rows of kGKC + 8) or across (kGKC rows of
+   * 32 + 8); the padding makes the eight rows of an ldmatrix hit eight banks */
+  constexpr int LDK = kGKC + 8, LDT = kGT + 8;
+  constexpr int SZ = kGT * LDK > kGKC * LDT ? kGT * LDK : kGKC * LDT;
+  extern __shared__ __align__(16) bf16 gsm[];
+  bf16 *As = gsm, *Bs = gsm + SZ;
+  if (EPI == EPI_STORE && (int)blockIdx.x * kGT >= N) {
+    pdl_wait_then_release();
+    colsum(K, M, (int)blockIdx.y * kGT, zp, ldzp, db, (float *)gsm);
+    return;
+  }
   const int m0 = blockIdx.y * kGT, n0 = blockIdx.x * kGT;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gid = lane >> 2, tig = lane & 3;
-  const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
-  float acc[2][4][4];
+  const int wm = (warp >> 1) * 16, wn = (warp & 1) * 16;
+  float acc[2][4], pre[2][4] = {}; /* pre: what the epilogue multiplies by */
 #pragma unroll
-  for (int i = 0; i < 2; i++)
+  for (int j = 0; j < 2; j++)
 #pragma unroll
-    for (int j = 0; j < 4; j++)
+    for (int q = 0; q < 4; q++) acc[j][q] = 0.f;
+  for (int k0 = 0; k0 < K; k0 += kGKC) {
+    const int kc = K - k0 < kGKC ? K - k0 : kGKC, kr = (kc + 15) / 16 * 16;
+    if (k0) __syncthreads();
+    auto stage = [&](bf16 *S, const bf16 *G, int ld, bool across, int o, int lim) {
+      if (across) { /* row = k, 32 elements from column o on */
+        for (int t = threadIdx.x; t < kr * (kGT / 8); t += 128) {
+          const int r = t / (kGT / 8), c = t % (kGT / 8) * 8;
+          const bool ok = r < kc && o + c < lim;
+          cp16(S + r * LDT + c, ok ? G + (size_t)(k0 + r) * ld + o + c : G, ok);
+        }
+      } else { /* row = m or n, kr elements from k0 on */
+        const int per = kr / 8;
+        for (int t = threadIdx.x; t < kGT * per; t += 128) {
+          const int r = t / per, c = t % per * 8;
+          const bool ok = o + r < lim && c < kc;
+          cp16(S + r * LDK + c, ok ? G + (size_t)(o + r) * ld + k0 + c : G, ok);
+        }
+      }
+    };
+    /* B (weights, or a layer's stored input) is never what the launch before
+     * this one wrote, A may be */
+    stage(Bs, B, ldb, !TB, n0, N);
+    if (k0 == 0) {
+      pdl_wait_then_release();
+      if (EPI == EPI_DGELU) {
 #pragma unroll
-      for (int q = 0; q < 4; q++) acc[i][j][q] = 0.f;
-  const bf16 zero = __float2bfloat16(0.f);
-  for (int k0 = 0; k0 < K; k0 += kGK) {
-    /* stage 64 x 16 of A' and of B' (as [n][k]): 8 elements per thread each */
-    for (int t = threadIdx.x; t < kGT * kGK; t += 128) {
-      const int r = t / kGK, kk = t % kGK;
-      const int m = m0 + r, n = n0 + r, k = k0 + kk;
-      bf16 av = zero, bv = zero;
-      if (m < M && k < K) av = TA ? A[(size_t)k * lda + m] : A[(size_t)m * lda + k];
-      if (n < N && k < K) bv = TB ? B[(size_t)n * ldb + k] : B[(size_t)k * ldb + n];
-      As[r][kk] = av;
-      Bs[r][kk] = bv;
+        for (int j = 0; j < 2; j++)
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            const int m = m0 + wm + gid + (q >= 2 ? 8 : 0), n = n0 + wn + 8 * j + 2 * tig + (q & 1);
+            pre[j][q] = m < M && n < N ? zp[(size_t)m * ldzp + n] : 0.f;
+          }
+      }
     }
+    stage(As, A, lda, TA, m0, M);
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
-    uint32_t af[2][4], bfr[4][2];
-#pragma unroll
-    for (int i = 0; i < 2; i++) {
-      const int r = wm + 16 * i + gid;
-      af[i][0] = *reinterpret_cast<const uint32_t *>(&As[r][2 * tig]);
-      af[i][1] = *reinterpret_cast<const uint32_t *>(&As[r + 8][2 * tig]);
-      af[i][2] = *reinterpret_cast<const uint32_t *>(&As[r][2 * tig + 8]);
-      af[i][3] = *reinterpret_cast<const uint32_t *>(&As[r + 8][2 * tig + 8]);
+    /* matrix q of an ldmatrix.x4 is addressed by lanes 8 q .. 8 q + 7.  A: rows
+     * +0, +8, +0, +8 at k +0, +0, +8, +8.  B: columns +0, +0, +8, +8 at k +0,
+     * +8, +0, +8 (two 8-column tiles). */
+    const int q = lane >> 3, r8 = lane & 7;
+    const int am = wm + (q & 1) * 8, ak = (q >> 1) * 8, bn = wn + (q >> 1) * 8, bk = (q & 1) * 8;
+    for (int kk = 0; kk < kr; kk += 16) {
+      uint32_t af[4], bf[4];
+      if constexpr (TA)
+        ldm4t(af, smem_addr(As + (kk + ak + r8) * LDT + am));
+      else
+        ldm4(af, smem_addr(As + (am + r8) * LDK + kk + ak));
+      if constexpr (TB)
+        ldm4(bf, smem_addr(Bs + (bn + r8) * LDK + kk + bk));
+      else
+        ldm4t(bf, smem_addr(Bs + (kk + bk + r8) * LDT + bn));
+      mma_bf16_16816(acc[0], af, bf);
+      mma_bf16_16816(acc[1], af, bf + 2);
     }
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int c = wn + 8 * j + gid;
-      bfr[j][0] = *reinterpret_cast<const uint32_t *>(&Bs[c][2 * tig]);
-      bfr[j][1] = *reinterpret_cast<const uint32_t *>(&Bs[c][2 * tig + 8]);
-    }
-#pragma unroll
-    for (int i = 0; i < 2; i++)
-#pragma unroll
-      for (int j = 0; j < 4; j++) mma_bf16_16816(acc[i][j], af[i], bfr[j]);
-    __syncthreads();
   }
 #pragma unroll
-  for (int i = 0; i < 2; i++)
+  for (int j = 0; j < 2; j++)
 #pragma unroll
-    for (int j = 0; j < 4; j++)
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const int m = m0 + wm + 16 * i + gid + (q >= 2 ? 8 : 0);
-        const int n = n0 + wn + 8 * j + 2 * tig + (q & 1);
-        if (m >= M || n >= N) continue;
-        float v = acc[i][j][q];
-        if (EPI == EPI_BIAS || EPI == EPI_BIAS_GELU) v += bias[n];
-        if (EPI == EPI_DGELU) v *= gelu_grad(zp[(size_t)m * ldzp + n]);
-        C[(size_t)m * ldc + n] = v;
-        if (EPI == EPI_BIAS_GELU) act[(size_t)m * ldact + n] = __float2bfloat16(gelu(v));
-        if (EPI == EPI_DGELU) act[(size_t)m * ldact + n] = __float2bfloat16(v);
-      }
+    for (int q = 0; q < 4; q++) {
+      const int m = m0 + wm + gid + (q >= 2 ? 8 : 0);
+      const int n = n0 + wn + 8 * j + 2 * tig + (q & 1);
+      if (m >= M || n >= N) continue;
+      float v = acc[j][q];
+      if (EPI == EPI_BIAS || EPI == EPI_BIAS_GELU) v += bias[n];
+      if (EPI == EPI_DGELU) v *= gelu_grad(pre[j][q]);
+      C[(size_t)m * ldc + n] = v;
+      if (EPI == EPI_BIAS_GELU) act[(size_t)m * ldact + n] = __float2bfloat16(gelu(v));
+      if (EPI == EPI_DGELU) act[(size_t)m * ldact + n] = __float2bfloat16(v);
+    }
 }
 
 /* dY = 2 (Y - T) / (B * nout) on columns < nout (0 elsewhere), bf16 copy,
@@ -142,6 +226,7 @@ __global__ void k_mse(int Bn, int ld, int nout, const float *__restrict__ Y,
                       bf16 *__restrict__ dYh, double *partials, unsigned *counter, float *loss) {
   __shared__ double sh[256];
   __shared__ bool am_last;
+  pdl_wait_then_release();
   const double scale = 2.0 / ((double)Bn * nout);
   double s = 0.0;
   const long tot = (long)Bn * ld;
@@ -177,21 +262,13 @@ __global__ void k_mse(int Bn, int ld, int nout, const float *__restrict__ Y,
   }
 }
 
-/* db[n] = sum_m dZ[m][n], rows in order */
-__global__ void k_colsum(int Bn, int N, const float *__restrict__ dZ, int ld, float *__restrict__ db) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
-  float s = 0.f;
-  for (int m = 0; m < Bn; m++) s += dZ[(size_t)m * ld + n];
-  db[n] = s;
-}
-
 /* Adam (Kingma & Ba, 2015) with bias correction on FP32 master weights;
  * entries with mask 0 (padding) stay 0 */
 __global__ void k_adam(long np, float *__restrict__ p, const float *__restrict__ g,
                        float *__restrict__ m1, float *__restrict__ m2, const uint8_t *__restrict__ mask,
                        bf16 *__restrict__ ph, float lr, float b1, float b2, float eps, float c1,
                        float c2) {
+  pdl_wait_then_release();
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < np; i += (long)gridDim.x * blockDim.x) {
     if (!mask[i]) {
       p[i] = 0.f;
@@ -216,6 +293,7 @@ __global__ void k_to_bf16(long n, const float *__restrict__ x, bf16 *__restrict_
 
 /* X [B][ld] (bf16, zero padding) from a row-major FP32 block [B][nin] */
 __global__ void k_pack_input(int Bn, int nin, int ld, const float *__restrict__ x, bf16 *__restrict__ xh) {
+  pdl_wait_then_release();
   const long tot = (long)Bn * ld;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < tot; i += (long)gridDim.x * blockDim.x) {
     const int m = (int)(i / ld), n = (int)(i % ld);
@@ -225,11 +303,18 @@ __global__ void k_pack_input(int Bn, int nin, int ld, const float *__restrict__ 
 
 template <bool TA, bool TB, int EPI>
 static int gemm(int M, int N, int K, const bf16 *A, int lda, const bf16 *B, int ldb, float *C, int ldc,
-                const float *bias, bf16 *act, int ldact, const float *zp, int ldzp) {
+                const float *bias, bf16 *act, int ldact, const float *zp, int ldzp,
+                float *db = nullptr) {
   if (M <= 0 || N <= 0) return 0;
-  dim3 g((unsigned)((N + kGT - 1) / kGT), (unsigned)((M + kGT - 1) / kGT));
-  k_gemm_bf16<TA, TB, EPI><<<g, 128, 0, ctx().stream>>>(M, N, K, A, lda, B, ldb, C, ldc, bias, act,
-                                                        ldact, zp, ldzp);
+  dim3 g((unsigned)((N + kGT - 1) / kGT + (EPI == EPI_STORE)), (unsigned)((M + kGT - 1) / kGT));
+  /* two operands of at most kGKC x (kGT + 8) or kGT x (kGKC + 8) elements */
+  constexpr size_t sm = 2 * sizeof(bf16) * (kGT * (kGKC + 8) > kGKC * (kGT + 8) ? kGT * (kGKC + 8) : kGKC * (kGT + 8));
+  static_assert(sm >= 2 * 64 * 32 * sizeof(float), "the column sums stage two tiles");
+  static const cudaError_t attr = cudaFuncSetAttribute(
+      k_gemm_bf16<TA, TB, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (fail(attr, "cudaFuncSetAttribute")) return PEVSL_ERR_CUDA;
+  launch_pdl_block(k_gemm_bf16<TA, TB, EPI>, g, 128, sm, ctx().stream, M, N, K, A, lda, B, ldb, C, ldc,
+                   bias, act, ldact, zp, ldzp, db);
   return launched("gemm_bf16");
 }
 
@@ -319,12 +404,12 @@ static int mlp_forward(pevsl_mlp *net, int B) {
 static int mlp_backward(pevsl_mlp *net, int B, const float *T, int ldt) {
   Ctx &c = ctx();
   const int L = net->layers;
-  int st = fail(cudaMemsetAsync(net->g, 0, sizeof(float) * (size_t)net->np, c.stream), "memset g");
+  int st = 0; /* every entry of g is written below */
   const int NL = net->ndim[L - 1];
   const unsigned gb = grid_for((long)B * NL, 4) > 256 ? 256 : grid_for((long)B * NL, 4);
   if (!st) {
-    k_mse<<<gb, 256, 0, c.stream>>>(B, NL, net->nout, net->z[L - 1], T, ldt, net->dz, net->dzh[0],
-                                    net->partials, net->counter, net->loss);
+    launch_pdl_block(k_mse, dim3(gb), 256, 0, c.stream, B, NL, net->nout, net->z[L - 1], T, ldt, net->dz,
+                     net->dzh[0], net->partials, net->counter, net->loss);
     st = launched("mse");
   }
   int cur = 0;
@@ -332,11 +417,7 @@ static int mlp_backward(pevsl_mlp *net, int B, const float *T, int ldt) {
     const int K = net->kdim[l], N = net->ndim[l];
     /* dW_l = dZ_l^T a_l (N x K), db_l = column sums of dZ_l */
     st = gemm<true, false, EPI_STORE>(N, K, B, net->dzh[cur], N, net->a[l], K, net->g + net->woff[l],
-                                      K, nullptr, nullptr, 0, nullptr, 0);
-    if (!st) {
-      k_colsum<<<(N + 127) / 128, 128, 0, c.stream>>>(B, N, net->dz, N, net->g + net->boff[l]);
-      st = launched("colsum");
-    }
+                                      K, nullptr, nullptr, 0, net->dz, N, net->g + net->boff[l]);
     if (l == 0 || st) break;
     /* dZ_{l-1} = (dZ_l W_l) * gelu'(z_{l-1}) */
     st = gemm<false, false, EPI_DGELU>(B, K, N, net->dzh[cur], N, net->ph + net->woff[l], K, net->dz,
@@ -462,7 +543,7 @@ int pEVSL_B200_MlpForward(pevsl_mlp *net, const float *X, float *Y, int B) {
   if (B == 0) return 0;
   if (mlp_reserve(net, B)) return PEVSL_ERR_NOMEM;
   const int K0 = net->kdim[0];
-  k_pack_input<<<grid_for((long)B * K0, 4), kThreads, 0, ctx().stream>>>(B, net->nin, K0, X, net->a[0]);
+  launch_pdl(k_pack_input, grid_for((long)B * K0, 4), ctx().stream, B, net->nin, K0, X, net->a[0]);
   if (launched("pack_input")) return PEVSL_ERR_CUDA;
   if (mlp_forward(net, B)) return PEVSL_ERR_CUDA;
   const int L = net->layers, NL = net->ndim[L - 1];
@@ -480,7 +561,7 @@ int pEVSL_B200_MlpGradients(pevsl_mlp *net, const float *X, const float *T, int 
   if (!net || B <= 0) return PEVSL_ERR_ARG;
   if (mlp_reserve(net, B)) return PEVSL_ERR_NOMEM;
   const int K0 = net->kdim[0];
-  k_pack_input<<<grid_for((long)B * K0, 4), kThreads, 0, ctx().stream>>>(B, net->nin, K0, X, net->a[0]);
+  launch_pdl(k_pack_input, grid_for((long)B * K0, 4), ctx().stream, B, net->nin, K0, X, net->a[0]);
   if (launched("pack_input")) return PEVSL_ERR_CUDA;
   if (mlp_forward(net, B) || mlp_backward(net, B, T, net->nout)) return PEVSL_ERR_CUDA;
   if (sync()) return PEVSL_ERR_CUDA;
@@ -500,19 +581,18 @@ int pEVSL_B200_MlpTrainStep(pevsl_mlp *net, const float *X, const float *T, int 
   if (mlp_reserve(net, B)) return PEVSL_ERR_NOMEM;
   Ctx &c = ctx();
   const int K0 = net->kdim[0];
-  k_pack_input<<<grid_for((long)B * K0, 4), kThreads, 0, c.stream>>>(B, net->nin, K0, X, net->a[0]);
+  launch_pdl(k_pack_input, grid_for((long)B * K0, 4), c.stream, B, net->nin, K0, X, net->a[0]);
   if (launched("pack_input")) return PEVSL_ERR_CUDA;
   if (mlp_forward(net, B) || mlp_backward(net, B, T, net->nout)) return PEVSL_ERR_CUDA;
   net->step++;
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.f - powf(b1, (float)net->step), c2 = 1.f - powf(b2, (float)net->step);
-  k_adam<<<grid_for(net->np, 4), kThreads, 0, c.stream>>>(net->np, net->p, net->g, net->m1, net->m2,
-                                                         net->mask, net->ph, lr, b1, b2, 1e-8f, c1, c2);
+  launch_pdl(k_adam, grid_for(net->np, 4), c.stream, net->np, net->p, net->g, net->m1, net->m2, net->mask,
+             net->ph, lr, b1, b2, 1e-8f, c1, c2);
   if (launched("adam")) return PEVSL_ERR_CUDA;
   if (loss) {
-    if (sync()) return PEVSL_ERR_CUDA;
-    if (cudaMemcpy(loss, net->loss, sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess)
-      return PEVSL_ERR_CUDA;
+    if (memcpy_async(c.hscal + S_TMP0, net->loss, sizeof(float)) || sync()) return PEVSL_ERR_CUDA;
+    memcpy(loss, c.hscal + S_TMP0, sizeof(float));
   }
   return 0;
 }

@@ -29,50 +29,6 @@
 
 namespace pv {
 
-/* Programmatic dependent launch of the ELL filter-degree kernels.  A degree
- * launched with the stream-serialisation attribute may be scheduled while
- * the previous degree's last blocks still run: its blocks stage the value
- * table in shared memory, then wait (griddepcontrol.wait) until the
- * previous grid has completed and its writes are visible, and only then
- * read a vector.  A block lets the next degree be scheduled
- * (griddepcontrol.launch_dependents) only after its own wait, so the early
- * part of degree k+1 overlaps degree k and nothing older.  What the early
- * part reads, the value table, is written at set-up, followed by a device
- * synchronisation, and never again while the matrix lives.  Without the
- * attribute the wait returns at once.  (Loading the first entries of a row
- * before the wait as well took the one-vector kernel from 32 to 48
- * registers and measured slower.) */
-__device__ __forceinline__ void pdl_wait_then_release() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
-/* PEVSL_B200_PDL: 1 (default) launches the ELL filter degrees with the
- * attribute, 0 as plain stream-ordered launches */
-static int pdl_mode() {
-  static int v = -1;
-  if (v < 0) {
-    const char *e = getenv("PEVSL_B200_PDL");
-    v = e ? atoi(e) != 0 : 1;
-  }
-  return v;
-}
-
-template <class... KA, class... AA>
-static void launch_pdl(void (*k)(KA...), unsigned grid, cudaStream_t st, AA &&...args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = pdl_mode();
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, k, std::forward<AA>(args)...);
-}
-
 template <int L>
 __device__ __forceinline__ unsigned group_mask() {
   if constexpr (L == 32) {
