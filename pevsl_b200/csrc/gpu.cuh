@@ -77,6 +77,8 @@ enum Ws {
   WS_ILMU,      /* interleaved filter: per-degree coefficients */
   WS_CLMU,      /* cluster filter: one polynomial's coefficients */
   WS_LAN,       /* Lanczos runs: alpha and beta of every step, CGS coefficients */
+  WS_TUNE,      /* scratch vectors of the autotuner (its own: a tuning may come
+                   between other uses)                        */
   WS_LANV,      /* Lanczos DOS: the start vectors of a group */
   WS_COUNT
 };
@@ -293,7 +295,7 @@ double matrix_bytes(const pevsl_devcsr *A, bool fp32, bool batch = false);
 double il_matrix_bytes(const pevsl_devcsr *A);
 /* L2 persistence window over the part of A the kernels read (if enabled) */
 void matrix_window(const pevsl_devcsr *A);
-/* choose the CSR-stream rows per lane of a matrix by timing (once) */
+/* choose the CSR-stream form of a matrix by timing (once) */
 int stream_tune(pevsl_devcsr *A);
 /* choose the CSR or ELL form of the one- and two-vector filter degrees of a
  * packed matrix with an ELL copy by timing both (at set-up) */
@@ -339,8 +341,7 @@ struct ClusterJob {
   double cc, dd, ccB, ddB;
   int deg, degB;
 };
-/* largest matrix of a cluster launch; pEVSL_ParcsrSetup finds the bandwidths
- * of the matrices up to here */
+/* largest matrix of a cluster launch */
 constexpr int kClusterMaxRows = 32768;
 /* whether the matrices fit the shared memory of a cluster */
 bool cluster_filter_ok(const pevsl_devcsr *A, const pevsl_devcsr *B, bool fp32);

@@ -367,6 +367,147 @@ __global__ void __launch_bounds__(kThreads, R == 1 ? 5 : 1)
   stream_rows<R>(n, ia, ja, a, x, epi, blockIdx.x, prod);
 }
 
+/* ---------------------------------------------------------------- windowed CSR
+ * Scattered columns within a band: a gather that touches 32 lines takes 32
+ * cycles of the L1 pipeline (the CSR-stream kernel ran at 90% of it on a
+ * matrix of 17 entries per row within +-5000), where shared memory serves 32
+ * scattered doubles in about six.  So one block per SM owns consecutive rows,
+ * copies the part of x that its rows touch into shared memory, and its warps
+ * then stream their rows' entries as the CSR-stream kernel does: 2-byte column
+ * offsets (from the 32-row group) and values in batches, the products staged
+ * in entry order, each lane adding its own row's.  The same bits.  Chosen per
+ * matrix by timing (stream_tune).  Now bound by the shared-memory pipeline
+ * (about 15 cycles per 32 entries: the gather, the staging, the rows' sums)
+ * and HBM in about equal parts.  Per degree with 17 entries per row against
+ * the CSR-stream kernel: 10^6 rows within +-5000 63 / 84 us (214 MB, 3.4
+ * TB/s), within +-9000 (two blocks per SM in turn) 70 / 85, within +-500 55 /
+ * 66; 5 10^5 rows 30 / 45, 10^5 8.4 / 12.7, 4 10^4 5.6 / 7.8. */
+constexpr int kWinThreads = 1024;
+constexpr size_t kWinSmem = 232000; /* dynamic shared memory of a block, of 232448 bytes */
+
+/* CH entries per warp and pass, loaded ahead: while a warp adds up one pass
+ * the next one's loads (the next 32 rows' where these are done) are under way */
+template <int CH, class Epi>
+__global__ void __launch_bounds__(kWinThreads, 1)
+    k_csr_window(int n, int kl, int ku, const int *__restrict__ split, const int *__restrict__ ia,
+                 const short *__restrict__ dj, const double *__restrict__ a,
+                 const double *__restrict__ x, Epi epi) {
+  constexpr int PL = CH / 32;
+  extern __shared__ __align__(16) double wsm[];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double *pw = wsm + w * CH;
+  const int r0 = __ldg(split + blockIdx.x), r1 = __ldg(split + blockIdx.x + 1);
+  const int lo = r0 > kl ? r0 - kl : 0, hi = n - r1 > ku ? r1 + ku : n;
+  /* element i of the window at win[i]; win + i and x + lo + i share their
+   * 16-byte alignment */
+  const int odd = (int)((((uintptr_t)x >> 3) + (unsigned)lo) & 1u);
+  double *win = wsm + (kWinThreads / 32) * CH + odd;
+  pdl_wait_then_release();
+  if (r0 >= r1) return;
+  if (threadIdx.x == 0 && odd) win[0] = __ldg(x + lo);
+  for (int i = odd + 2 * (int)threadIdx.x; i < hi - lo; i += 2 * kWinThreads) {
+    if (i + 1 < hi - lo)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
+                       (unsigned)__cvta_generic_to_shared(win + i)),
+                   "l"(x + lo + i)
+                   : "memory");
+    else
+      win[i] = __ldg(x + lo + i);
+  }
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+  int col[PL];
+  double val[PL];
+  auto fetch = [&](int base, int len, int c0) {
+#pragma unroll
+    for (int q = 0; q < PL; q++) {
+      const int t = c0 + q * 32 + lane;
+      col[q] = t < len ? (int)__ldg(dj + base + t) : 0;
+      val[q] = t < len ? __ldg(a + base + t) : 0.0;
+    }
+  };
+  /* a group's first entry and its count, and the lane's row in it */
+  auto rows = [&](int g, int &rs, int &re) {
+    rs = re = 0;
+    if (g + lane < r1) {
+      rs = __ldg(ia + g + lane);
+      re = __ldg(ia + g + lane + 1);
+    }
+  };
+  auto extent = [&](int g, int rs, int re, int &base, int &len) {
+    const int last = (r1 - g < 32 ? r1 - g : 32) - 1;
+    base = __shfl_sync(0xffffffffu, rs, 0);
+    len = __shfl_sync(0xffffffffu, re, last) - base;
+  };
+  int g = r0 + 32 * w, rs, re, base = 0, len = 0;
+  rows(g, rs, re);
+  if (g < r1) {
+    extent(g, rs, re, base, len);
+    fetch(base, len, 0);
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
+  while (g < r1) {
+    const int row = g + lane, gn = g + kWinThreads;
+    int rsn, ren, basen = 0, lenn = 0;
+    rows(gn, rsn, ren);
+    typename Epi::Pre pre;
+    if (row < r1) pre = epi.pre(row);
+    const double *wg = win + (g - lo);
+    const int b0 = rs - base, e0 = re - base;
+    double acc = 0.0;
+    int c0 = 0;
+    do {
+#pragma unroll
+      for (int q = 0; q < PL; q++) pw[q * 32 + lane] = mul_rn(val[q], wg[col[q]]);
+      if (c0 + CH < len) {
+        fetch(base, len, c0 + CH);
+      } else if (gn < r1) {
+        extent(gn, rsn, ren, basen, lenn);
+        fetch(basen, lenn, 0);
+      }
+      __syncwarp();
+      const int b = b0 > c0 ? b0 : c0, e = e0 < c0 + CH ? e0 : c0 + CH;
+      for (int t = b; t < e; t++) acc = add_rn(acc, pw[t - c0]);
+      __syncwarp();
+      c0 += CH;
+    } while (c0 < len);
+    if (row < r1) epi(row, acc, pre);
+    g = gn;
+    rs = rsn;
+    re = ren;
+    base = basen;
+    len = lenn;
+  }
+}
+
+/* band[0] = the largest row - column, band[1] = the largest column - row
+ * (both start at 0); a warp per 32 rows, lane l row l */
+__global__ void k_csr_band(int n, const int *__restrict__ ia, const int *__restrict__ ja, int *band) {
+  const int row = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  int lo = 0, hi = 0;
+  if (row < n)
+    for (int t = __ldg(ia + row); t < __ldg(ia + row + 1); t++) {
+      const int o = __ldg(ja + t) - row;
+      lo = max(lo, -o);
+      hi = max(hi, o);
+    }
+  lo = __reduce_max_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(band, lo);
+    atomicMax(band + 1, hi);
+  }
+}
+
+__global__ void k_window_offsets(int n, const int *__restrict__ ia, const int *__restrict__ ja,
+                                 short *__restrict__ dj) {
+  const int g = (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  const int g0 = g * 32;
+  if (g0 >= n) return;
+  const int e = __ldg(ia + (n - g0 < 32 ? n : g0 + 32));
+  for (int t = __ldg(ia + g0) + lane; t < e; t += 32) dj[t] = (short)(__ldg(ja + t) - g0);
+}
+
 /* Up to CAP independent products y_e = A_e x_e (x_e = epi[e].vk), each with
  * its own matrix and epilogue, in one launch.  With `shared` (all entries
  * on one matrix) block b serves entry b % nb on row block b / nb: the nb
@@ -789,6 +930,9 @@ int persistent_filter_error() {
 /* Rows per lane of the CSR-stream kernels, per matrix: 1 until tuned */
 static int stream_r(const pevsl_devcsr *A) { return A && A->stream_r == 2 ? 2 : 1; }
 
+/* whether products run in the windowed form */
+static bool use_window(const pevsl_devcsr *A) { return A->stream_r == 3 && A->wdj; }
+
 static unsigned stream_grid(int n, int R) {
   const long rows_per_block = (kThreads / 32) * 32L * R;
   return (unsigned)((n + rows_per_block - 1) / rows_per_block);
@@ -1020,39 +1164,120 @@ __global__ void k_block_normalize(long n, int s, int ld, double *X, const double
   } while (0)
 
 /* Autotuner of the CSR-stream kernels: on a matrix's first use, time one
- * Chebyshev degree with one and with two rows per lane (1 warm-up + 5 timed
- * launches each, CUDA events, scratch vectors of the matrix's size) and keep
- * the faster; two rows per lane must win by 3%.  Both give the same bits
- * (the per-row summation order is the same), so the choice never changes a
- * result.  PEVSL_B200_STREAM_R=1|2 fixes it; matrices under 4096 rows keep
- * one.  Must not run while the stream is being captured. */
-int stream_tune(pevsl_devcsr *A) {
-  if (!A || A->stream_r) return 0;
-  const char *e = getenv("PEVSL_B200_STREAM_R");
-  if (e && (atoi(e) == 1 || atoi(e) == 2)) {
-    A->stream_r = atoi(e);
-    return 0;
-  }
-  A->stream_r = 1;
+ * Chebyshev degree with one and with two rows per lane and, where the windows
+ * fit, the windowed form (1 warm-up + 5 timed launches each, CUDA events,
+ * scratch vectors of the matrix's size) and keep the fastest; a later one must
+ * win by 3%.  All give the same bits (the per-row summation order is the
+ * same), so the choice never changes a result.  PEVSL_B200_STREAM_R=1|2|3
+ * fixes it; matrices under 4096 rows keep one.  Must not run while the stream is being captured. */
+/* 256 entries per pass where the staging leaves room for the window */
+static int window_chunk(const pevsl_devcsr *A) {
+  const size_t win = sizeof(double) * (size_t)(A->wlen + 2);
+  return win + sizeof(double) * kWinThreads * 8 <= kWinSmem ? 256 : 128;
+}
+static size_t window_smem(const pevsl_devcsr *A) {
+  return sizeof(double) * ((size_t)(kWinThreads / 32) * window_chunk(A) + (size_t)A->wlen + 2);
+}
+
+template <int CH, class Epi>
+static int launch_window_ch(const pevsl_devcsr *A, const double *x, const Epi &epi) {
+  static const cudaError_t attr = cudaFuncSetAttribute(
+      k_csr_window<CH, Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWinSmem);
+  if (attr != cudaSuccess) return fail(attr, "cudaFuncSetAttribute");
+  launch_pdl_block(k_csr_window<CH, Epi>, dim3((unsigned)A->wblocks), kWinThreads, window_smem(A),
+                   ctx().stream, A->nrows, A->band_lo, A->band_hi, A->wsplit, A->ia, A->wdj,
+                   (const double *)A->a, x, epi);
+  return 0;
+}
+
+template <class Epi>
+static int launch_window(const pevsl_devcsr *A, const double *x, const Epi &epi) {
+  return window_chunk(A) == 256 ? launch_window_ch<256>(A, x, epi) : launch_window_ch<128>(A, x, epi);
+}
+
+/* The windowed form's offsets and row split, when the windows fit: one, two
+ * or three blocks per SM one after the other, rows in multiples of 32, about
+ * equal entries.  Leaves wdj NULL otherwise. */
+static int window_prepare(pevsl_devcsr *A) {
   const long n = A->nrows;
-  if (n < 4096 || A->smask) return 0; /* the stencil form: other kernels */
-  double *buf = nullptr;
-  if (cudaMalloc(&buf, sizeof(double) * 4 * (size_t)n) != cudaSuccess) {
+  const int sms = ctx().sms;
+  if (A->lanes != 0 || A->smask || A->ncols != n || A->nnz <= 0 || n < 64L * sms) return 0;
+  const long ng = (n - 1) / 32 + 1;
+  const unsigned gg = (unsigned)((ng * 32 + kThreads - 1) / kThreads); /* a warp per 32 rows */
+  std::vector<int> ia((size_t)ng), split;
+  int *dband = (int *)ws(WS_TUNE, 2 * sizeof(int)), band[2];
+  if (!dband) return PEVSL_ERR_NOMEM;
+  if (fail(cudaMemsetAsync(dband, 0, 2 * sizeof(int), ctx().stream), "cudaMemsetAsync")) return PEVSL_ERR_CUDA;
+  k_csr_band<<<gg, kThreads, 0, ctx().stream>>>(A->nrows, A->ia, A->ja, dband);
+  if (launched("csr_band") || memcpy_async(band, dband, sizeof band) || fail(cudaMemcpy2DAsync(ia.data(), sizeof(int), A->ia, 32 * sizeof(int), sizeof(int), (size_t)ng,
+                             cudaMemcpyDeviceToHost, ctx().stream),
+           "cudaMemcpy2DAsync") ||
+      sync())
+    return PEVSL_ERR_CUDA;
+  A->band_lo = band[0];
+  A->band_hi = band[1];
+  if (band[0] > 32000 || band[1] > 32000) return 0;
+  int nb = 0;
+  for (int m = 1; m <= 3; m++) {
+    nb = m * sms;
+    split.assign((size_t)nb + 1, (int)n);
+    split[0] = 0;
+    int rows = 0;
+    for (int b = 1; b < nb; b++) {
+      const int want = (int)((double)A->nnz * b / nb);
+      split[(size_t)b] = (int)std::min<long>(n, 32 * (std::lower_bound(ia.begin(), ia.end(), want) - ia.begin()));
+    }
+    for (int b = 0; b < nb; b++) rows = std::max(rows, split[(size_t)b + 1] - split[(size_t)b]);
+    A->wlen = (int)std::min<long>(n, (long)rows + A->band_lo + A->band_hi);
+    if (window_smem(A) <= kWinSmem) break;
+    nb = 0;
+  }
+  if (!nb) return 0;
+  const size_t bo = (sizeof(short) * (size_t)A->nnz + 255) / 256 * 256;
+  char *p = nullptr;
+  if (cudaMalloc(&p, bo + sizeof(int) * (size_t)(nb + 1)) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
+  A->wdj = (short *)p;
+  A->wsplit = (int *)(p + bo);
+  A->wblocks = nb;
+  if (memcpy_async(A->wsplit, split.data(), sizeof(int) * (size_t)(nb + 1))) return PEVSL_ERR_CUDA;
+  k_window_offsets<<<gg, kThreads, 0, ctx().stream>>>(A->nrows, A->ia, A->ja, A->wdj);
+  return launched("window_offsets");
+}
+
+int stream_tune(pevsl_devcsr *A) {
+  if (!A || A->stream_r) return 0;
+  const char *e = getenv("PEVSL_B200_STREAM_R");
+  const int force = e && atoi(e) >= 1 && atoi(e) <= 3 ? atoi(e) : 0;
+  A->stream_r = force == 2 ? 2 : 1;
+  const long n = A->nrows;
+  if (force == 1 || force == 2 || n < 4096 || A->smask) return 0; /* the stencil form: other kernels */
+  if (window_prepare(A)) return PEVSL_ERR_CUDA;
+  if (force == 3) {
+    if (A->wdj) A->stream_r = 3;
+    return 0;
+  }
+  /* scratch vectors, kept in a workspace: no allocation per matrix */
+  const long ld = (n + 31) / 32 * 32;
+  double *buf = (double *)ws(WS_TUNE, sizeof(double) * 4 * (size_t)ld);
+  if (!buf) return 0;
   cudaStream_t st = ctx().stream;
-  cudaMemsetAsync(buf, 0, sizeof(double) * 4 * (size_t)n, st);
-  double *x = buf, *xm1 = buf + n, *xp1 = buf + 2 * n, *y = buf + 3 * n;
+  cudaMemsetAsync(buf, 0, sizeof(double) * 4 * (size_t)ld, st);
+  double *x = buf, *xm1 = buf + ld, *xp1 = buf + 2 * ld, *y = buf + 3 * ld;
   const EpiCheb epi{x, xm1, xp1, y, 0.5, 0.5, 0.0, 0.5, 0};
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
-  float ms[3] = {0.f, 0.f, 0.f};
-  for (int R = 1; R <= 2; R++) {
+  float ms[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int R = 1; R <= 3; R++) {
+    if (R == 3 && !A->wdj) break;
     for (int it = 0; it < 6; it++) {
       if (it == 1) cudaEventRecord(e0, st);
-      if (R == 2)
+      if (R == 3)
+        launch_window(A, x, epi);
+      else if (R == 2)
         launch_pdl(k_csr_stream<2, double, EpiCheb>, stream_grid(n, 2), st, A->nrows, A->ia, A->ja,
                    (const double *)A->a, x, epi);
       else
@@ -1062,17 +1287,20 @@ int stream_tune(pevsl_devcsr *A) {
     cudaEventRecord(e1, st);
     cudaEventSynchronize(e1);
     cudaEventElapsedTime(&ms[R], e0, e1);
+    ctx().launches += 6;
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  cudaStreamSynchronize(st);
-  cudaFree(buf);
   if (fail(cudaGetLastError(), "stream_tune")) return PEVSL_ERR_CUDA;
-  ctx().launches += 12;
   if (ms[2] > 0.f && ms[2] < 0.97f * ms[1]) A->stream_r = 2;
+  if (ms[3] > 0.f && ms[3] < 0.97f * ms[A->stream_r]) A->stream_r = 3;
+  if (A->wdj && A->stream_r != 3) {
+    cudaFree(A->wdj);
+    A->wdj = nullptr;
+  }
   if (getenv("PEVSL_B200_VERBOSE"))
-    fprintf(stderr, "stream_tune n=%ld: 1 row/lane %.2f us, 2 rows/lane %.2f us -> %d\n", n,
-            ms[1] * 200.f, ms[2] * 200.f, A->stream_r);
+    fprintf(stderr, "stream_tune n=%ld: 1 row/lane %.2f us, 2 rows/lane %.2f us, window %.2f us -> %d\n", n,
+            ms[1] * 200.f, ms[2] * 200.f, ms[3] * 200.f, A->stream_r);
   return 0;
 }
 
@@ -1165,6 +1393,12 @@ static void launch_stream(const pevsl_devcsr *A, const T *a, const T *x, const E
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(ctx().stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone)
       stream_tune(const_cast<pevsl_devcsr *>(A));
+  }
+  if constexpr (sizeof(T) == 8) {
+    if (use_window(A)) {
+      launch_window(A, x, epi);
+      return;
+    }
   }
   if (stream_r(A) == 2)
     launch_pdl(k_csr_stream<2, T, Epi>, stream_grid(A->nrows, 2), ctx().stream, A->nrows, A->ia,
@@ -2412,6 +2646,7 @@ void pEVSL_ParcsrFree(pevsl_Parcsr *A) {
     cudaFree(d->a); /* the whole [values | indices | pointers] block */
     if (d->a32) cudaFree(d->a32);
     if (d->smask) cudaFree(d->smask);
+    if (d->wdj) cudaFree(d->wdj); /* and wsplit */
     if (d->pdj) cudaFree(d->pdj); /* the packed block */
     d->magic = 0;
     free(d);

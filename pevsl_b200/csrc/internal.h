@@ -47,10 +47,18 @@ typedef struct pevsl_devcsr {
   float *a32; /* device fp32 copy, made on first use */
   int max_row_nnz;
   int band_lo, band_hi; /* largest row - column and column - row (>= 0) of any
-                           * entry; found only for the matrices of cluster launches */
+                           * entry: set up for the matrices of cluster launches,
+                           * else with the windowed form */
   double avg_row_nnz;
   int lanes; /* threads per row in the row-group SpMV kernels */
-  int stream_r; /* rows per lane of the CSR-stream kernels, 0 until tuned */
+  /* form of the CSR-stream kernels, 0 until tuned: 1 or 2 rows per lane, or
+   * 3, the gathered vector's window in shared memory (with wdj = column -
+   * 32 * (row / 32) as int16 and the rows of each block, wsplit[0..wblocks],
+   * on the device; wlen: the largest window) */
+  int stream_r;
+  short *wdj;
+  int *wsplit;
+  int wblocks, wlen;
   size_t bytes; /* size of the one device block holding a, ja, ia */
   /* stencil form (smask NULL when the matrix does not qualify): at most 32
    * (column offset, value) pairs in all, soff ascending; bit j of row r's
