@@ -101,6 +101,7 @@ struct Ctx {
   cudaEvent_t tab_ev[4] = {};  /* copy of slot i done             */
   int tab_next = 0;
   unsigned *bar = nullptr;     /* grid barrier: count, generation, error   */
+  unsigned *cl_err = nullptr;  /* pinned: a wait of a cluster launch ran out */
   void *ws[WS_COUNT] = {};
   size_t wsz[WS_COUNT] = {};
   uint64_t launches = 0;

@@ -11,25 +11,31 @@
  * they touch.  A thread keeps v_k, v_{k-1} and the filter sum of its rows in
  * registers.  Per degree it gathers from the window (shared memory, no
  * global load but the coefficient), forms its rows' v_{k+1}, stores them
- * into the other of two windows and, through distributed shared memory, into
- * the windows of the blocks that gather them; one cluster barrier ends the
- * degree.  The cluster barrier is the hardware's; nothing spins on memory.
+ * into the next window and, through distributed shared memory, into the
+ * windows of the blocks that gather them.
  *
  * The generalized filter (each degree a least-squares B-solve, then the A
  * step) runs the same way with the entries of A and B resident.
  *
- * What bounds it is latency: the release / acquire barrier takes about 450
- * cycles (0.24 us) with 16 blocks, a row's chain (gather, seven multiply-adds
- * of 8 cycles each, the recurrence) about 200, and the stores into the
- * neighbours' windows about 0.7 cycles per value.  Measured per degree, one
- * vector, against a launch per degree (of the CSR kernels, and of the
- * stencil form where a matrix has it): 729 rows 0.60 / 2.5 / 2.1 us, 7980
- * rows (19 x 20 x 21) 1.00 / 3.2 / 2.2 us, 15600 rows 1.17 / 3.2 / 2.2 us,
- * 26970 rows 2.58 / 3.36 / 2.2 us; a degree of the generalized
- * filter of two slices at 7980 rows with a 16-term B-solve 17 / 53 us.  Past
- * 32768 rows (four rows per thread) the entries no longer fit beside the
- * windows; a build with them packed to 3 bytes took 5.3 us at 63960 rows
- * against 3.5 us for the launches, which spread over the whole chip.
+ * What bounds it is latency.  A cluster barrier with release and acquire
+ * takes about 450 cycles, and a value stored for a neighbour about 0.7 more,
+ * so the degrees do not meet there: the values are sent with st.async, which
+ * counts their bytes on the receiving block's mbarrier, and a block goes on
+ * when its own have arrived (three windows instead of two keep a faster
+ * neighbour from overwriting what is still read).  The waits are bounded; one
+ * that runs out makes the call return PEVSL_ERR_CUDA.  Where some block would
+ * send to one that it does not hear from (windows of a matrix without
+ * symmetric structure), the cluster barrier ends each degree.
+ *
+ * Measured per degree, one vector, against a launch per degree (of the CSR
+ * kernels, and of the stencil form where a matrix has it): 60 rows 0.38 us,
+ * 720 0.57 / 2.5 / 2.1, 7980 rows (19 x 20 x 21) 0.77 / 3.2 / 2.2, 15600 rows
+ * 1.03 / 3.2 / 2.2, 2000 rows with 17 scattered entries 1.53 / 4.9; with the
+ * barrier 7980 rows 1.0 and 15600 rows 1.17 us.  The generalized filter of two
+ * slices at 7980 rows with a 16-term B-solve TGEN us per degree against 53.
+ * Past 16384 rows a launch per degree of the stencil form is as fast (26970
+ * rows: 2.6 us with the entries in shared memory against 2.2); other matrices
+ * run here up to 32768 rows where their entries fit beside the windows.
  *
  * A row's products are formed and added in entry order, unfused, and the
  * recurrence is cheb_update_v's: the results are the bits of the
@@ -92,6 +98,33 @@ __device__ __forceinline__ void cl_store(unsigned addr, double v) {
 }
 __device__ __forceinline__ void cl_store(unsigned addr, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+/* the same, counted by the receiving block's mbarrier when it arrives */
+__device__ __forceinline__ void cl_send(unsigned addr, double v, unsigned mbar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr),
+               "l"(__double_as_longlong(v)), "r"(mbar)
+               : "memory");
+}
+__device__ __forceinline__ void cl_send(unsigned addr, float v, unsigned mbar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr),
+               "r"(__float_as_uint(v)), "r"(mbar)
+               : "memory");
+}
+
+/* wait for the phase of this parity, at most kClPolls polls */
+constexpr int kClPolls = 1 << 22;
+__device__ __forceinline__ bool cl_wait(unsigned mbar, unsigned parity) {
+  for (int i = 0; i < kClPolls; i++) {
+    unsigned ok;
+    asm volatile(
+        "{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(mbar), "r"(parity)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
 }
 
 /* one matrix of a job, as the kernel reads it */
@@ -183,18 +216,19 @@ __device__ __forceinline__ void cl_load(ClRow<T, CW> &row, const ClEnt<T> &e, co
  * slot; Rp: at least R, a multiple of 32. */
 template <class T, int RPT, int CW, bool GEN>
 __global__ void __launch_bounds__(kClThreads, 1)
-    k_filter_cluster(const __grid_constant__ ClTable tab, int Z, int Rp) {
+    k_filter_cluster(const __grid_constant__ ClTable tab, int Z, int Rp, int nwin, unsigned *err) {
   extern __shared__ __align__(16) unsigned char cl_smem[];
-  __shared__ int s_lo, s_hi, s_tlo[kClMaxBlocks], s_thi[kClMaxBlocks];
+  __shared__ int s_lo, s_hi, s_tlo[kClMaxBlocks], s_thi[kClMaxBlocks], s_async;
+  __shared__ __align__(8) unsigned long long s_mbar[3];
   const unsigned nc = cl_size(), rank = cl_rank();
   const ClJob &J = tab.job[blockIdx.x / nc];
   const int n = J.n, R = (n + (int)nc - 1) / (int)nc, r0 = (int)rank * R;
   const int nloc = n - r0 < 0 ? 0 : (n - r0 < R ? n - r0 : R);
-  T *win = (T *)cl_smem; /* two windows of Z + 1 slots, rounded up to 16 bytes */
+  T *win = (T *)cl_smem; /* nwin windows of Z + 1 slots, rounded up to 16 bytes */
   const int ws1 = (Z + 4) / 4 * 4;
   ClEnt<T> eA{}, eB{};
   {
-    unsigned char *p = cl_smem + 2 * (size_t)ws1 * sizeof(T);
+    unsigned char *p = cl_smem + (size_t)nwin * ws1 * sizeof(T);
     auto take = [&](ClEnt<T> &e, const ClMat &M) {
       e.Rp = Rp;
       if constexpr (CW == 0) {
@@ -211,7 +245,15 @@ __global__ void __launch_bounds__(kClThreads, 1)
     s_lo = nloc > 0 ? r0 : 0;
     s_hi = nloc > 0 ? r0 + nloc : 0;
   }
-  if (threadIdx.x == 0) win[Z] = win[ws1 + Z] = T(0);
+  if ((int)threadIdx.x < nwin) win[(int)threadIdx.x * ws1 + Z] = T(0);
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 3; i++)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(
+                       (unsigned)__cvta_generic_to_shared(&s_mbar[i]))
+                   : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    s_async = nwin == 3;
+  }
   __syncthreads();
   /* the window: every column the block's rows touch, and the rows */
   {
@@ -243,7 +285,19 @@ __global__ void __launch_bounds__(kClThreads, 1)
     s_tlo[threadIdx.x] = lo;
     s_thi[threadIdx.x] = hi < lo + Z ? hi : lo + Z;
   }
-  cl_barrier(); /* a block that has no further barrier may end after this one */
+  __syncthreads();
+  /* the blocks may run without the cluster barrier when every block that
+   * sends to another also receives from it: the same answer in every block */
+  if (nwin == 3 && threadIdx.x < nc * nc) {
+    auto sends = [&](int from, int to) {
+      const int f0 = from * R < n ? from * R : n, f1 = f0 + R < n ? f0 + R : n;
+      return f0 < s_thi[to] && f1 > s_tlo[to] && f0 < f1;
+    };
+    const int a = (int)threadIdx.x / (int)nc, b = (int)threadIdx.x % (int)nc;
+    if (a != b && sends(a, b) != sends(b, a)) s_async = 0;
+  }
+  cl_barrier(); /* also: a block that has no further barrier may end after this one */
+  const bool async = s_async != 0;
   const int lo = s_lo, hi = s_hi < lo + Z ? s_hi : lo + Z;
   for (int i = threadIdx.x; i < hi - lo; i += kClThreads) win[i] = (T)J.x[lo + i];
   ClRow<T, CW> rowA[RPT], rowB[GEN ? RPT : 1];
@@ -264,26 +318,63 @@ __global__ void __launch_bounds__(kClThreads, 1)
     }
   }
   __syncthreads();
-  /* the value of row q into window `to` here and where it is gathered */
-  auto publish = [&](int q, T v, int to) {
-    const int r = r0 + q * kClThreads + (int)threadIdx.x;
-    T *w = win + (to ? ws1 : 0);
+  int cur = 0; /* the window read */
+  auto next = [&]() { return cur + 1 == nwin ? 0 : cur + 1; };
+  /* the value of row q into the next window, here and where it is gathered */
+  auto publish = [&](int q, T v) {
+    const int r = r0 + q * kClThreads + (int)threadIdx.x, to = next();
+    T *w = win + to * ws1;
     w[r - lo] = v;
     unsigned m = push[q];
     const unsigned base = (unsigned)__cvta_generic_to_shared(w);
+    const unsigned mb = (unsigned)__cvta_generic_to_shared(&s_mbar[to]);
     while (m) {
       const int b = __ffs((int)m) - 1;
       m &= m - 1;
-      cl_store(cl_map(base + (unsigned)(r - s_tlo[b]) * (unsigned)sizeof(T), (unsigned)b), v);
+      const unsigned at = cl_map(base + (unsigned)(r - s_tlo[b]) * (unsigned)sizeof(T), (unsigned)b);
+      if (async)
+        cl_send(at, v, cl_map(mb, (unsigned)b));
+      else
+        cl_store(at, v);
     }
   };
+  /* The end of a step: the next window is complete and becomes the one read.
+   * With the barrier, every block's.  Without: this block's rows (the block
+   * barrier) and the values sent to it (its mbarrier counts their bytes).  A
+   * block that is a step ahead writes the window after that one, which the
+   * slower block read two steps ago: its own values for the step before, which
+   * the faster one waited for, were sent past the barrier that ended those
+   * reads.  False when a wait ran out. */
+  const unsigned rx = (unsigned)(hi - lo - nloc) * (unsigned)sizeof(T);
+  unsigned parity = 0; /* bit i: of window i's mbarrier */
+  auto arm = [&]() {
+    if (async && rx && threadIdx.x == 0)
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
+                       (unsigned)__cvta_generic_to_shared(&s_mbar[next()])),
+                   "r"(rx)
+                   : "memory");
+  };
+  auto advance = [&]() -> bool {
+    cur = next();
+    if (!async) {
+      cl_barrier();
+      return true;
+    }
+    bool ok = true;
+    if (rx) {
+      ok = cl_wait((unsigned)__cvta_generic_to_shared(&s_mbar[cur]), (parity >> cur) & 1u);
+      parity ^= 1u << cur;
+    }
+    return !__syncthreads_or(!ok);
+  };
+  bool ok = true;
   const T cc = (T)J.cc, t1 = (T)(1.0 / J.dd), t2 = (T)(2.0 / J.dd), mu0 = (T)__ldg(J.mu);
-  int cur = 0;
   if constexpr (!GEN) {
     T muk = (T)__ldg(J.mu + 1);
-    for (int k = 1; k <= J.deg; k++) {
+    for (int k = 1; k <= J.deg && ok; k++) {
+      if (k < J.deg) arm();
       const T mnext = k < J.deg ? (T)__ldg(J.mu + k + 1) : T(0);
-      const T *w = win + (cur ? ws1 : 0);
+      const T *w = win + cur * ws1;
 #pragma unroll
       for (int q = 0; q < RPT; q++) {
         const int i = q * kClThreads + (int)threadIdx.x;
@@ -294,23 +385,23 @@ __global__ void __launch_bounds__(kClThreads, 1)
         y[q] = k == 1 ? cl_fma(muk, v, cl_mul(mu0, x[q])) : cl_fma(muk, v, y[q]);
         xm1[q] = x[q];
         x[q] = v;
-        if (k < J.deg) publish(q, v, cur ^ 1);
+        if (k < J.deg) publish(q, v);
       }
       muk = mnext;
-      cur ^= 1;
-      if (k < J.deg) cl_barrier();
+      if (k < J.deg) ok = advance();
     }
-    if (J.deg == 1) cl_barrier(); /* y may be x: every block has read it */
+    if (J.deg == 1 && !async) cl_barrier(); /* y may be x: every block has read it */
   } else {
     const T ccB = (T)J.ccB, b1 = (T)(1.0 / J.ddB), b2 = (T)(2.0 / J.ddB), lmu0 = (T)__ldg(J.lmu);
     T l[RPT], lm1[RPT], s[RPT];
-    for (int k = 1; k <= J.deg; k++) {
+    for (int k = 1; k <= J.deg && ok; k++) {
       const T muk = (T)__ldg(J.mu + k);
       /* s = the least-squares B^{-1} of v_k (in the window) */
       T lk = (T)__ldg(J.lmu + 1);
-      for (int j = 1; j <= J.degB; j++) {
+      for (int j = 1; j <= J.degB && ok; j++) {
+        arm();
         const T lnext = j < J.degB ? (T)__ldg(J.lmu + j + 1) : T(0);
-        const T *w = win + (cur ? ws1 : 0);
+        const T *w = win + cur * ws1;
 #pragma unroll
         for (int q = 0; q < RPT; q++) {
           const int i = q * kClThreads + (int)threadIdx.x;
@@ -322,13 +413,14 @@ __global__ void __launch_bounds__(kClThreads, 1)
           s[q] = j == 1 ? cl_fma(lk, v, cl_mul(lmu0, l[q])) : cl_fma(lk, v, s[q]);
           lm1[q] = l[q];
           l[q] = v;
-          publish(q, j < J.degB ? v : s[q], cur ^ 1);
+          publish(q, j < J.degB ? v : s[q]);
         }
         lk = lnext;
-        cur ^= 1;
-        cl_barrier();
+        ok = advance();
       }
-      const T *w = win + (cur ? ws1 : 0);
+      if (!ok) break;
+      if (k < J.deg) arm();
+      const T *w = win + cur * ws1;
 #pragma unroll
       for (int q = 0; q < RPT; q++) {
         const int i = q * kClThreads + (int)threadIdx.x;
@@ -339,16 +431,24 @@ __global__ void __launch_bounds__(kClThreads, 1)
         y[q] = k == 1 ? cl_fma(muk, v, cl_mul(mu0, x[q])) : cl_fma(muk, v, y[q]);
         xm1[q] = x[q];
         x[q] = v;
-        if (k < J.deg) publish(q, v, cur ^ 1);
+        if (k < J.deg) publish(q, v);
       }
-      cur ^= 1;
-      if (k < J.deg) cl_barrier();
+      if (k < J.deg) ok = advance();
     }
+  }
+  if (async) {
+    /* no block ends while another may still write its windows, nor writes a
+     * result over an input that another has yet to read */
+    if (!ok) {
+      if (threadIdx.x == 0) atomicExch_system(err, 1u);
+      __nanosleep(200000); /* stores still under way */
+    }
+    cl_barrier();
   }
 #pragma unroll
   for (int q = 0; q < RPT; q++) {
     const int i = q * kClThreads + (int)threadIdx.x;
-    if (i < nloc) J.y[r0 + i] = (double)y[q];
+    if (i < nloc) J.y[r0 + i] = ok ? (double)y[q] : nan("");
   }
 }
 
@@ -357,7 +457,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
 /* shape of a launch: blocks per cluster, rows per thread, row entries in
  * registers (0: shared memory), window slots, rows and shared memory */
 struct ClShape {
-  int nc, rpt, cw, Z, Rp;
+  int nc, rpt, cw, Z, Rp, nwin;
   size_t smem;
 };
 
@@ -385,9 +485,15 @@ static bool cl_shape(int ne, const ClusterJob *jobs, bool fp32, int nc, ClShape 
   s->rpt = 1;
   while (s->rpt * kClThreads < rmax) s->rpt *= 2;
   if (s->rpt > 4 || zmax > 65535) return false;
-  s->smem = 2 * T * (size_t)(zmax + 4);
+  const size_t win = T * (size_t)(zmax + 4);
+  s->nwin = 2;
+  s->smem = 2 * win;
   s->cw = ew <= kClRegs && s->rpt <= (jobs[0].B ? 1 : 2) ? kClRegs : 0;
   if (!s->cw) s->smem += (T + 2) * (size_t)s->Rp * (size_t)ewsum;
+  if (s->smem + win <= kClSmem) {
+    s->nwin = 3;
+    s->smem += win;
+  }
   return s->smem <= kClSmem;
 }
 
@@ -430,7 +536,7 @@ static int cl_attributes(const void *k, const ClShape &s) {
 static int cl_resident(int nc) {
   static int have[kClMaxBlocks + 1] = {0}; /* 0: not asked yet, -1: none */
   if (!have[nc]) {
-    ClShape s{nc, 1, kClRegs, 0, 0, kClSmem};
+    ClShape s{nc, 1, kClRegs, 0, 0, 2, kClSmem};
     const void *k = cl_kernel<double, false>(s);
     cudaLaunchAttribute at;
     cudaLaunchConfig_t cfg;
@@ -446,9 +552,10 @@ static int cl_resident(int nc) {
 }
 
 /* The shape for ne jobs in one launch: the one whose waves of clusters take
- * the least time by the measured cost of a degree, 0.6 us (the barrier and
- * the chain of dependent operations) + 8 ns per block of the cluster + 0.5
- * ns per row of a block (1.1 ns with the entries in shared memory). */
+ * the least time by the measured cost of a step (us): the chain of dependent
+ * operations and the wait for the other blocks, 0.4 ns per row of a block
+ * (1.8 ns with the entries in shared memory) and 60 ns per value that a row
+ * sends (the window beyond a block's own rows, over these). */
 static bool cl_choose(int ne, const ClusterJob *jobs, bool fp32, ClShape *best) {
   double tbest = 0.0;
   for (int nc = 1; nc <= kClMaxBlocks; nc *= 2) {
@@ -456,7 +563,9 @@ static bool cl_choose(int ne, const ClusterJob *jobs, bool fp32, ClShape *best) 
     if (!cl_shape(ne, jobs, fp32, nc, &s)) continue;
     const int m = cl_resident(nc);
     if (m <= 0) continue;
-    const double t = ((ne + m - 1) / m) * (0.6 + 0.008 * nc + (s.cw ? 0.0005 : 0.0011) * s.Rp);
+    const double step = (nc > 1 ? 0.43 : 0.3) + (s.cw ? 0.0 : 0.6) + (s.cw ? 0.0004 : 0.0018) * s.Rp +
+                        0.06 * (s.Z - s.Rp > 0 ? (double)(s.Z - s.Rp) / s.Rp : 0.0);
+    const double t = ((ne + m - 1) / m) * step;
     if (tbest == 0.0 || t < tbest) {
       tbest = t;
       *best = s;
@@ -475,7 +584,7 @@ bool cluster_filter_ok(const pevsl_devcsr *A, const pevsl_devcsr *B, bool fp32) 
   ClShape s;
   if (!cl_choose(1, &J, fp32, &s)) return false;
   /* a matrix in the stencil form takes 2.1 us per launched degree, less than
-   * a cluster with more than two rows per thread (2.6 us at 26970 rows) */
+   * a cluster with more than two rows per thread */
   return B || fp32 || !A->smask || s.rpt <= 2;
 }
 
@@ -508,7 +617,8 @@ int cluster_filter(int ne, const ClusterJob *jobs, bool fp32) {
     cudaLaunchAttribute at;
     cudaLaunchConfig_t cfg;
     cl_config(s, nb, &cfg, &at);
-    void *args[] = {(void *)&tab, (void *)&s.Z, (void *)&s.Rp};
+    unsigned *err = ctx().cl_err;
+    void *args[] = {(void *)&tab, (void *)&s.Z, (void *)&s.Rp, (void *)&s.nwin, (void *)&err};
     if (fail(cudaLaunchKernelExC(&cfg, k, args), "filter_cluster")) return PEVSL_ERR_CUDA;
     if (launched("filter_cluster")) return PEVSL_ERR_CUDA;
   }

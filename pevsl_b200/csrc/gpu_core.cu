@@ -80,6 +80,8 @@ int ensure() {
       return PEVSL_ERR_CUDA;
   if (fail(cudaMalloc(&g_ctx.bar, sizeof(unsigned) * 4), "cudaMalloc bar")) return PEVSL_ERR_CUDA;
   if (fail(cudaMemset(g_ctx.bar, 0, sizeof(unsigned) * 4), "cudaMemset bar")) return PEVSL_ERR_CUDA;
+  if (fail(cudaMallocHost(&g_ctx.cl_err, sizeof(unsigned)), "cudaMallocHost")) return PEVSL_ERR_CUDA;
+  *g_ctx.cl_err = 0;
   g_ctx.ready = true;
   return 0;
 }
@@ -124,7 +126,17 @@ int launched(const char *what) {
   return fail(cudaGetLastError(), what);
 }
 
-int sync() { return fail(cudaStreamSynchronize(g_ctx.stream), "cudaStreamSynchronize"); }
+int sync() {
+  if (fail(cudaStreamSynchronize(g_ctx.stream), "cudaStreamSynchronize")) return PEVSL_ERR_CUDA;
+  volatile unsigned *e = g_ctx.cl_err;
+  if (e && *e) {
+    *e = 0;
+    fprintf(stderr, "pevsl-b200: a wait between the blocks of a filter launch ran out\n");
+    g_ctx.sticky_error = PEVSL_ERR_CUDA;
+    return PEVSL_ERR_CUDA;
+  }
+  return 0;
+}
 
 void *ws(int slot, size_t bytes) {
   if (ensure()) return nullptr;
