@@ -101,6 +101,7 @@ struct Ctx {
   cudaEvent_t tab_ev[4] = {};  /* copy of slot i done             */
   int tab_next = 0;
   unsigned *bar = nullptr;     /* grid barrier: count, generation, error   */
+  cudaMemPool_t pool = nullptr; /* matrices (pool_alloc)          */
   unsigned *cl_err = nullptr;  /* pinned: a wait of a cluster launch ran out */
   void *ws[WS_COUNT] = {};
   size_t wsz[WS_COUNT] = {};
@@ -116,6 +117,11 @@ int launched(const char *what); /* count a launch and check for errors */
 void l2_window(const void *base, size_t bytes);
 int sync();
 void *ws(int slot, size_t bytes);
+/* device memory of matrices, in order on the context stream, from a pool that
+ * keeps up to 64 MB of freed memory (pEVSL_B200_ReleaseWorkspace gives it
+ * back); NULL when there is none */
+void *pool_alloc(size_t bytes);
+void pool_free(void *p);
 int memcpy_async(void *dst, const void *src, size_t bytes);
 /* scalar slots: copy device slots [first, first+count) to the pinned mirror
  * and wait; returns pointer into the mirror or NULL */

@@ -32,6 +32,8 @@ int fail(cudaError_t e, const char *what) {
 }
 
 static int g_req_device = -1;
+/* freed memory that the matrices' pool keeps (pool_alloc) */
+static constexpr uint64_t kPoolKeep = (uint64_t)64 << 20;
 
 int ensure() {
   if (g_ctx.ready) return 0;
@@ -82,6 +84,17 @@ int ensure() {
   if (fail(cudaMemset(g_ctx.bar, 0, sizeof(unsigned) * 4), "cudaMemset bar")) return PEVSL_ERR_CUDA;
   if (fail(cudaMallocHost(&g_ctx.cl_err, sizeof(unsigned)), "cudaMallocHost")) return PEVSL_ERR_CUDA;
   *g_ctx.cl_err = 0;
+  cudaMemPoolProps pp;
+  memset(&pp, 0, sizeof pp);
+  pp.allocType = cudaMemAllocationTypePinned;
+  pp.location.type = cudaMemLocationTypeDevice;
+  pp.location.id = dev;
+  uint64_t keep = kPoolKeep;
+  if (cudaMemPoolCreate(&g_ctx.pool, &pp) != cudaSuccess ||
+      cudaMemPoolSetAttribute(g_ctx.pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+    cudaGetLastError();
+    g_ctx.pool = nullptr;
+  }
   g_ctx.ready = true;
   return 0;
 }
@@ -149,10 +162,43 @@ void *ws(int slot, size_t bytes) {
     g_ctx.wsz[slot] = 0;
   }
   void *p = nullptr;
-  if (fail(cudaMalloc(&p, bytes), "cudaMalloc workspace")) return nullptr;
+  if (cudaMalloc(&p, bytes) != cudaSuccess) {
+    /* once more without the memory that the pool keeps */
+    cudaGetLastError();
+    cudaStreamSynchronize(g_ctx.stream);
+    if (g_ctx.pool) cudaMemPoolTrimTo(g_ctx.pool, 0);
+    if (fail(cudaMalloc(&p, bytes), "cudaMalloc workspace")) return nullptr;
+  }
   g_ctx.ws[slot] = p;
   g_ctx.wsz[slot] = bytes;
   return p;
+}
+
+/* The blocks of a matrix.  cudaMalloc and cudaFree of the 660 KB of an 8000-row
+ * stencil open or close one of the driver's 2 MB chunks in every third call or
+ * so, 400 us and up to 4 ms each, against 180 us for the rest of the set-up:
+ * pEVSL_ParcsrSetup with other matrices alive 0.6-0.8 ms from cudaMalloc, 0.19
+ * ms from the pool.  Larger matrices (100^3: 19 ms) do not gain, and the pool
+ * returns what it holds above kPoolKeep at the next synchronisation.
+ * Allocation and release are in order on the context stream, the only one
+ * that kernels of this library run on; both are safe from any thread. */
+void *pool_alloc(size_t bytes) {
+  if (ensure()) return nullptr;
+  void *p = nullptr;
+  if (bytes == 0) bytes = 16;
+  const cudaError_t e = g_ctx.pool ? cudaMallocFromPoolAsync(&p, bytes, g_ctx.pool, g_ctx.stream)
+                                   : cudaMalloc(&p, bytes);
+  if (e == cudaSuccess) return p;
+  cudaGetLastError();
+  return nullptr;
+}
+
+void pool_free(void *p) {
+  if (!p) return;
+  if (g_ctx.pool)
+    cudaFreeAsync(p, g_ctx.stream);
+  else
+    cudaFree(p);
 }
 
 int memcpy_async(void *dst, const void *src, size_t bytes) {
@@ -556,6 +602,7 @@ void pEVSL_B200_ReleaseWorkspace(void) {
     g_ctx.ws[i] = nullptr;
     g_ctx.wsz[i] = 0;
   }
+  if (g_ctx.pool) cudaMemPoolTrimTo(g_ctx.pool, 0);
 }
 
 int pEVSL_B200_Info(char *buf, int len) {

@@ -1234,11 +1234,8 @@ static int window_prepare(pevsl_devcsr *A) {
   }
   if (!nb) return 0;
   const size_t bo = (sizeof(short) * (size_t)A->nnz + 255) / 256 * 256;
-  char *p = nullptr;
-  if (cudaMalloc(&p, bo + sizeof(int) * (size_t)(nb + 1)) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
+  char *p = (char *)pool_alloc(bo + sizeof(int) * (size_t)(nb + 1));
+  if (!p) return 0;
   A->wdj = (short *)p;
   A->wsplit = (int *)(p + bo);
   A->wblocks = nb;
@@ -1295,7 +1292,7 @@ int stream_tune(pevsl_devcsr *A) {
   if (ms[2] > 0.f && ms[2] < 0.97f * ms[1]) A->stream_r = 2;
   if (ms[3] > 0.f && ms[3] < 0.97f * ms[A->stream_r]) A->stream_r = 3;
   if (A->wdj && A->stream_r != 3) {
-    cudaFree(A->wdj);
+    pool_free(A->wdj);
     A->wdj = nullptr;
   }
   if (getenv("PEVSL_B200_VERBOSE"))
@@ -2358,8 +2355,8 @@ static int choose_lanes(double avg) {
 }
 
 static void *alloc_dev(size_t bytes) {
-  void *p = nullptr;
-  if (fail(cudaMalloc(&p, bytes ? bytes : 16), "cudaMalloc matrix")) return nullptr;
+  void *p = pool_alloc(bytes);
+  if (!p) fail(cudaErrorMemoryAllocation, "matrix allocation");
   return p;
 }
 
@@ -2491,11 +2488,10 @@ static int pack_entries(pevsl_devcsr *d, const pevsl_Csr *Ai) {
 
 /* The stencil form of a matrix: at most 32 (offset, value) pairs in all,
  * values compared bit for bit, and every row's entries in ascending column
- * order.  *done is set when the matrix has it. */
-static int build_stencil(pevsl_devcsr *d, const pevsl_Csr *Ai, bool *done) {
-  *done = false;
+ * order.  True, with the rows' masks in out, when the matrix has it. */
+static bool build_stencil(pevsl_devcsr *d, const pevsl_Csr *Ai, std::vector<unsigned char> &out) {
   const int nr = d->nrows;
-  if (nr <= 0 || d->nnz <= 0 || d->max_row_nnz > 32 || d->lanes != 0) return 0;
+  if (nr <= 0 || d->nnz <= 0 || d->max_row_nnz > 32 || d->lanes != 0) return false;
   struct Pair {
     int off;
     uint64_t val;
@@ -2517,7 +2513,7 @@ static int build_stencil(pevsl_devcsr *d, const pevsl_Csr *Ai, bool *done) {
     }
     unsigned m = 0;
     for (int k = Ai->ia[i], j = 0; k < Ai->ia[i + 1]; k++, j++) {
-      if (k > Ai->ia[i] && Ai->ja[k] <= Ai->ja[k - 1]) return 0;
+      if (k > Ai->ia[i] && Ai->ja[k] <= Ai->ja[k - 1]) return false;
       const int off = Ai->ja[k] - i;
       uint64_t v;
       memcpy(&v, Ai->a + k, sizeof v);
@@ -2526,7 +2522,7 @@ static int build_stencil(pevsl_devcsr *d, const pevsl_Csr *Ai, bool *done) {
         for (j = 0; j < np && (pair[j].off != off || pair[j].val != v); j++) {
         }
         if (j == np) {
-          if (np == 32) return 0;
+          if (np == 32) return false;
           pair[np++] = Pair{off, v};
         }
       }
@@ -2549,7 +2545,7 @@ static int build_stencil(pevsl_devcsr *d, const pevsl_Csr *Ai, bool *done) {
   }
   d->sk = np;
   d->sbytes = np <= 8 ? 1 : np <= 16 ? 2 : 4;
-  std::vector<unsigned char> out((size_t)nr * (size_t)d->sbytes);
+  out.resize((size_t)nr * (size_t)d->sbytes);
   unsigned last_in = 0, last_out = 0; /* masks repeat along a grid line */
   for (int i = 0; i < nr; i++) {
     const unsigned m = mask[(size_t)i];
@@ -2561,13 +2557,7 @@ static int build_stencil(pevsl_devcsr *d, const pevsl_Csr *Ai, bool *done) {
     }
     memcpy(out.data() + (size_t)i * d->sbytes, &last_out, (size_t)d->sbytes); /* little endian */
   }
-  void *p = alloc_dev(out.size());
-  if (!p) return PEVSL_ERR_NOMEM;
-  d->smask = p;
-  int st = memcpy_async(p, out.data(), out.size());
-  if (!st) st = sync();
-  *done = st == 0;
-  return st;
+  return true;
 }
 
 int pEVSL_ParcsrSetup(pevsl_Csr *Ai, pevsl_Parcsr *A) {
@@ -2594,12 +2584,16 @@ int pEVSL_ParcsrSetup(pevsl_Csr *Ai, pevsl_Parcsr *A) {
     const int L = atoi(lenv);
     if (L == 0 || L == 1 || L == 2 || L == 4 || L == 8 || L == 16 || L == 32) d->lanes = L;
   }
-  /* one allocation [values | column indices | row pointers], 256-byte
-   * aligned parts, so that a single L2 access-policy window can cover it */
+  /* one allocation [values | column indices | row pointers | stencil masks],
+   * 256-byte aligned parts, so that a single L2 access-policy window can
+   * cover it */
   const size_t bytes_a = ((sizeof(double) * (size_t)nnz + 255) / 256) * 256;
   const size_t bytes_ja = ((sizeof(int) * (size_t)nnz + 255) / 256) * 256;
   const size_t bytes_ia = sizeof(int) * (size_t)(nr + 1);
-  char *base = (char *)alloc_dev(bytes_a + bytes_ja + bytes_ia);
+  std::vector<unsigned char> smask;
+  const bool stencil = build_stencil(d, Ai, smask);
+  const size_t off_mask = (bytes_a + bytes_ja + bytes_ia + 255) / 256 * 256;
+  char *base = (char *)alloc_dev(off_mask + smask.size());
   if (!base) {
     free(d);
     return PEVSL_ERR_NOMEM;
@@ -2611,10 +2605,12 @@ int pEVSL_ParcsrSetup(pevsl_Csr *Ai, pevsl_Parcsr *A) {
   int st = memcpy_async(d->ia, Ai->ia, sizeof(int) * (size_t)(nr + 1));
   if (!st) st = memcpy_async(d->ja, Ai->ja, sizeof(int) * (size_t)nnz);
   if (!st) st = memcpy_async(d->a, Ai->a, sizeof(double) * (size_t)nnz);
+  if (stencil) {
+    d->smask = base + off_mask;
+    if (!st) st = memcpy_async(d->smask, smask.data(), smask.size());
+  }
   if (!st) st = sync();
   if (st) return st;
-  bool stencil = false;
-  st = build_stencil(d, Ai, &stencil);
   for (int j = 0; j < d->sk; j++) {
     d->band_hi = std::max(d->band_hi, d->soff[j]);
     d->band_lo = std::max(d->band_lo, -d->soff[j]);
@@ -2643,11 +2639,10 @@ void pEVSL_ParcsrFree(pevsl_Parcsr *A) {
   pevsl_devcsr *d = pevsl_devcsr_of(A);
   if (d) {
     cudaStreamSynchronize(ctx().stream);
-    cudaFree(d->a); /* the whole [values | indices | pointers] block */
+    pool_free(d->a); /* the whole [values | indices | pointers | masks] block */
     if (d->a32) cudaFree(d->a32);
-    if (d->smask) cudaFree(d->smask);
-    if (d->wdj) cudaFree(d->wdj); /* and wsplit */
-    if (d->pdj) cudaFree(d->pdj); /* the packed block */
+    if (d->wdj) pool_free(d->wdj); /* and wsplit */
+    if (d->pdj) pool_free(d->pdj); /* the packed block */
     d->magic = 0;
     free(d);
   }
