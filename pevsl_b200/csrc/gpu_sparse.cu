@@ -581,8 +581,8 @@ __global__ void __launch_bounds__(kThreads, 4)
  * three to four waves of blocks, each the length of the chain mask, gather,
  * sum, store; larger ones stream from HBM.  Per degree of one vector with the
  * sum deferred, against the ELL and packed kernels: 41 x 40 x 42 2.2 / 2.5
- * us, 64 x 65 x 63 3.1 / 4.1 us, 99 x 100 x 101 7.4 / 10.6 us (30 MB: 4.1
- * TB/s), 159 x 160 x 161 24.7 / 54 us.  (The same rows described by a table
+ * us, 64 x 65 x 63 2.7 / 4.1 us, 99 x 100 x 101 6.6 / 10.6 us (30 MB: 4.6
+ * TB/s), 159 x 160 x 161 24.4 / 54 us.  (The same rows described by a table
  * of row patterns in shared memory took 8.1 us at 99 x 100 x 101, with the
  * value and the offset in one 16-byte entry 11.6 us: the table's broadcast
  * loads use as many L1 cycles as the gathers, which ran at 78%.) */
@@ -691,6 +691,67 @@ struct EpiChebY {
     }
   }
 };
+
+/* The degrees between the first and the last update of the sum (EpiChebY with
+ * v_{k-1} there, and no terms or three of them): nearly all of them, in a
+ * kernel of their own without the cases that do not occur.  The branches of
+ * the general one keep loads apart that can be in flight together.  Per
+ * degree, general / this one: 45 x 44 x 43 1.67 / 1.63 us, 64 x 65 x 63 2.71 /
+ * 2.48, 80 x 81 x 79 4.2 / 3.85, 99 x 100 x 101 6.75 / 6.25 (4.8 TB/s out of
+ * L2), 1000 x 1001 5.56 / 5.30.  One row per thread, which leaves after the
+ * wait where there is no row: the guarded form needs 37 registers and took
+ * 2.88 us at 64 x 65 x 63. */
+template <int K>
+__global__ void __launch_bounds__(kThreads)
+    k_cheb_stencil(int n, const __grid_constant__ Stencil S, const double *__restrict__ vk,
+                   const double *vkm1, double *vkp1, double *y, double cc, double t, double mua,
+                   double mub, double muk, int upd) {
+  const int row = (int)(blockIdx.x * (unsigned)kThreads + threadIdx.x);
+  const unsigned m = row < n ? stencil_mask<unsigned char>(S, row) : 0u;
+  pdl_wait_then_release();
+  if (row >= n) return;
+  const double x = vk[row], xm1 = vkm1[row], yold = upd ? y[row] : 0.0;
+  const double r = stencil_dot<K, true>(S, m, vk + row, x);
+  const double w = __dsub_rn(__dmul_rn(__fma_rn(-cc, x, r), t), xm1);
+  vkp1[row] = w;
+  if (upd) y[row] = __fma_rn(muk, w, __fma_rn(mub, x, __fma_rn(mua, xm1, yold)));
+}
+
+/* two rows per thread, 32 registers: 126 x 125 x 127 10.7 us against 11.3
+ * with one, 160 x 161 x 159 23 against 25-26, 1500 x 1501 9.9 against 10.4;
+ * 99 x 100 x 101 6.3 against 6.25 */
+template <int K>
+__global__ void __launch_bounds__(kThreads, 8)
+    k_cheb_stencil2(int n, const __grid_constant__ Stencil S, const double *__restrict__ vk,
+                    const double *vkm1, double *vkp1, double *y, double cc, double t, double mua,
+                    double mub, double muk, int upd) {
+  const int r0 = (int)(blockIdx.x * (unsigned)(2 * kThreads) + threadIdx.x);
+  unsigned m[2];
+  double x[2], xm1[2], yold[2];
+#pragma unroll
+  for (int q = 0; q < 2; q++)
+    m[q] = r0 + q * kThreads < n ? stencil_mask<unsigned char>(S, r0 + q * kThreads) : 0u;
+  pdl_wait_then_release();
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    const int row = r0 + q * kThreads;
+    if (row < n) {
+      x[q] = vk[row];
+      xm1[q] = vkm1[row];
+      yold[q] = upd ? y[row] : 0.0;
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    const int row = r0 + q * kThreads;
+    if (row < n) {
+      const double r = stencil_dot<K, true>(S, m[q], vk + row, x[q]);
+      const double w = __dsub_rn(__dmul_rn(__fma_rn(-cc, x[q], r), t), xm1[q]);
+      vkp1[row] = w;
+      if (upd) y[row] = __fma_rn(muk, w, __fma_rn(mub, x[q], __fma_rn(mua, xm1[q], yold[q])));
+    }
+  }
+}
 
 /* ---------------------------------------------------------------- persistent filter */
 
@@ -1356,9 +1417,9 @@ static int stencil_width(const pevsl_devcsr *A) {
 template <class Epi>
 static void launch_rows_stencil(const pevsl_devcsr *A, const double *x, const Epi &epi) {
   /* two rows per thread where one would be more than three waves of blocks
-   * and the row is wide: 160^3 29.8 -> 24.7 us per degree, 126^3 13.4 ->
-   * 12.4, 100^3 7.49 -> 7.32; 90^3 5.96 -> 6.23, and 1200 x 1201 with five
-   * entries 7.80 -> 8.12 */
+   * and the row is wide: 160^3 29.8 -> 24.7 us per filter degree of this
+   * kernel, 126^3 13.4 -> 12.4, 100^3 7.49 -> 7.32; 90^3 5.96 -> 6.23, and
+   * 1200 x 1201 with five entries 7.80 -> 8.12 */
   const int rpt = A->sk > 5 && (long)A->nrows > 3L * 8 * kThreads * ctx().sms ? 2 : 1;
   const unsigned g = (unsigned)((A->nrows + kThreads * rpt - 1) / (kThreads * rpt));
   const int w = stencil_width(A);
@@ -1522,6 +1583,17 @@ int cheb_step_y(const pevsl_devcsr *A, const double *vk, const double *vkm1, dou
                 double cc, double t, const double *mu, int k, int ny, int fresh) {
   if (A->nrows <= 0) return 0;
   if (!cheb_defers(A) || ny < 0 || ny > 3 || ny > k || (ny > 1 && !vkm1)) return PEVSL_ERR_ARG;
+  const int w = stencil_width(A);
+  if (w && vkm1 && (ny == 0 || (ny == 3 && !fresh))) {
+    /* two rows per thread from four waves of blocks on */
+    const int rpt = (long)A->nrows > 4L * 8 * kThreads * ctx().sms ? 2 : 1;
+    const unsigned g = (unsigned)((A->nrows + kThreads * rpt - 1) / (kThreads * rpt));
+    launch_pdl(rpt == 1 ? (w == 7 ? k_cheb_stencil<7> : k_cheb_stencil<5>)
+                        : (w == 7 ? k_cheb_stencil2<7> : k_cheb_stencil2<5>),
+               g, ctx().stream, A->nrows, stencil_of(A), vk, vkm1, vkp1, y, cc, t,
+               ny ? mu[k - 2] : 0.0, ny ? mu[k - 1] : 0.0, mu[k], ny);
+    return launched("cheb_step_y");
+  }
   launch_rows_stencil(A, vk, EpiChebY{vk, vkm1, vkp1, y, cc, t, mu[0], ny > 2 ? mu[k - 2] : 0.0,
                                   ny > 1 ? mu[k - 1] : 0.0, mu[k], ny, fresh});
   return launched("cheb_step_y");
@@ -1867,9 +1939,9 @@ __global__ void __launch_bounds__(kThreads, 5)
  * vectors (16-byte gathers, half a row's in flight: 32 registers),
  * k_cheb_il's arithmetic.  The SpMV reads Xg, which is Xk except in the
  * generalized filter (GEN).  Per degree, against the ELL and packed kernels:
- * 100^3 with two slices 9.3 / 15.7 us (60 MB, 6.4 TB/s out of L2), 64 x 65 x
- * 63 with three 6.0 / 11.5 and with eight 10.2 / 19.9 us, 50^3 with sixteen
- * 9.9 / 19.3 us. */
+ * 100^3 with two slices 9.3 / 15.7 us, 64 x 65 x 63 with three 6.0 / 11.5 and
+ * with eight 10.2 / 19.9 us, 50^3 with sixteen 9.9 / 19.3 us; most degrees run
+ * k_cheb_il_mid. */
 template <int L, int K, class M, bool GEN>
 __global__ void __launch_bounds__(kThreads)
     k_cheb_il_stencil(int n, const __grid_constant__ Stencil S, const double2 *__restrict__ Xg,
@@ -1923,12 +1995,75 @@ __global__ void __launch_bounds__(kThreads)
         il_accumulate<2 * L>(ny, fresh, yold.y, w1, x.y, xm1.y, mu0, muk, 2 * l + 1));
 }
 
+/* The same for the degrees between the first and the last update of the sum
+ * (v_{k-1} there; no terms or three of them), without the other cases.  B:
+ * gathers in flight; MB: blocks per SM.  What bounds it beyond one wave of
+ * blocks is the number of loads in flight on an SM, and eight blocks of 32
+ * registers keep more of them there than four of 54.  Per degree, general /
+ * this one: two vectors at 64 x 65 x 63 3.6 / 3.3 us, 99 x 100 x 101 10.2 /
+ * 8.5, 126 x 125 x 127 24.7 / 19.5; four at 64 x 65 x 63 5.95 / 5.13, 99 x
+ * 100 x 101 25.6 / 19.0 (past L2); eight at 64 x 65 x 63 10.6 / 8.65.  Below
+ * one wave the registers are free with one or two lanes per row: 45 x 44 x 43
+ * with four 2.94 against 3.31 at MB = 8, five-point rows there gain nothing
+ * from more than three gathers in flight (400 x 401 with two 2.37 against
+ * 2.61); with more lanes they are not (181 x 179 with eight 2.1 at MB = 8
+ * against 2.5). */
+template <int L, int K, int B, int MB>
+__global__ void __launch_bounds__(kThreads, MB)
+    k_cheb_il_mid(int n, const __grid_constant__ Stencil S, const double2 *__restrict__ Xk,
+                  const double2 *Xkm1, double2 *Xkp1, double2 *Y, double cc, double t,
+                  const double *__restrict__ muk, int upd) {
+  const unsigned me = blockIdx.x * (unsigned)kThreads + threadIdx.x;
+  const int row = (int)(me / L), l = (int)(me % L);
+  const unsigned m = row < n ? stencil_mask<unsigned char>(S, row) : 0u;
+  pdl_wait_then_release();
+  if (row >= n) return;
+  const double2 x = Xk[me];
+  const double2 xm1 = Xkm1[me];
+  const double2 yold = upd ? Y[me] : make_double2(0.0, 0.0);
+  const double2 *xr = Xk + me;
+  double r0 = 0.0, r1 = 0.0;
+#pragma unroll
+  for (int j0 = 0; j0 < K; j0 += B) {
+    double2 xv[B];
+#pragma unroll
+    for (int u = 0; u < B; u++) {
+      xv[u] = make_double2(0.0, 0.0);
+      if (j0 + u == K / 2)
+        xv[u] = x;
+      else if (j0 + u < K && ((m >> (j0 + u)) & 1u))
+        xv[u] = __ldg(xr + (long)S.off[j0 + u] * L);
+    }
+#pragma unroll
+    for (int u = 0; u < B; u++)
+      if (j0 + u < K && ((m >> (j0 + u)) & 1u)) {
+        r0 = __dadd_rn(r0, __dmul_rn(S.val[j0 + u], xv[u].x));
+        r1 = __dadd_rn(r1, __dmul_rn(S.val[j0 + u], xv[u].y));
+      }
+  }
+  const double w0 = __dsub_rn(__dmul_rn(__fma_rn(-cc, x.x, r0), t), xm1.x);
+  const double w1 = __dsub_rn(__dmul_rn(__fma_rn(-cc, x.y, r1), t), xm1.y);
+  Xkp1[me] = make_double2(w0, w1);
+  if (upd)
+    Y[me] = make_double2(
+        il_accumulate<2 * L>(3, 0, yold.x, w0, x.x, xm1.x, nullptr, muk, 2 * l),
+        il_accumulate<2 * L>(3, 0, yold.y, w1, x.y, xm1.y, nullptr, muk, 2 * l + 1));
+}
+
 template <int L>
 static int launch_il_stencil(const pevsl_devcsr *A, const double *Xg, const double *Xk,
                              const double *Xkm1, double *Xkp1, double *Y, double cc, double t,
                              const double *mu0, const double *muk, int ny, int fresh) {
   const unsigned g = (unsigned)(((long)A->nrows * L + kThreads - 1) / kThreads);
   const int w = Xg == Xk ? stencil_width(A) : 0;
+  if (w && Xkm1 && (ny == 0 || (ny == 3 && !fresh))) {
+    const bool one = L < 4 && (long)g <= 8L * ctx().sms;
+    launch_pdl(w == 7 ? (one ? k_cheb_il_mid<L, 7, 7, 1> : k_cheb_il_mid<L, 7, 7, 8>)
+                      : (one ? k_cheb_il_mid<L, 5, 3, 1> : k_cheb_il_mid<L, 5, 5, 8>),
+               g, ctx().stream, A->nrows, stencil_of(A), (const double2 *)Xk,
+               (const double2 *)Xkm1, (double2 *)Xkp1, (double2 *)Y, cc, t, muk, ny);
+    return launched("cheb_step_il_stencil");
+  }
   auto go = [&](auto k) {
     launch_pdl(k, g, ctx().stream, A->nrows, stencil_of(A), (const double2 *)Xg,
                (const double2 *)Xk, (const double2 *)Xkm1, (double2 *)Xkp1, (double2 *)Y, cc, t,

@@ -101,3 +101,35 @@ def test_generalized_lockstep_equals_one_by_one(gpu):
             assert one["nev"] == outs[s]["nev"] and np.array_equal(one["lam"], outs[s]["lam"])
     for x in (S, B, M):
         x.free()
+
+
+@pytest.mark.parametrize("grid", [(107, 108, 106), (1103, 1101, 1)])
+def test_two_rows_per_thread(gpu, grid):
+    """Past four waves of blocks the degrees between the sum's first and last update take two rows per thread."""
+    n, ia, ja, a = laplacian(*grid)
+    M, G = pv.Matrix.from_csr(n, ia, ja, a), pv.Matrix.from_csr(*with_extra_rows(n, ia, ja, a))
+    v = np.random.default_rng(9).standard_normal(n + 40)
+    with pv.Instance(M) as e, pv.Instance(G) as f:
+        for deg in (4, 23):
+            k = np.arange(deg + 1)
+            p = pv.Filter(1, deg, 0.0, 0.5, 6.0, 7.5, np.cos(0.7 * k) / (1.0 + 0.1 * k))
+            assert np.array_equal(e.chebav(p, v[:n]), f.chebav(p, v)[:n])
+    M.free()
+    G.free()
+
+
+@pytest.mark.parametrize("grid", [(68, 67, 69), (561, 563, 1)])
+@pytest.mark.parametrize("slices", [2, 3])
+def test_lockstep_past_one_wave(gpu, grid, slices):
+    M = pv.Matrix.from_csr(*laplacian(*grid))
+    edges = np.linspace(1.0, 3.0, slices + 1)
+    ivs = [[edges[i], edges[i + 1], 0.0, 12.0] for i in range(slices)]
+    fl = [pv.findpol(iv, deg_in=20 + i)[1] for i, iv in enumerate(ivs)]
+    v = np.cos(0.3 * np.arange(M.n))
+    with pv.Instance(M) as ev:
+        st, outs = pv.cheblannr_batch(ev, ivs, [30] * slices, 1e3, v, fl)
+        assert st == 0
+        for s in range(slices):
+            one = ev.cheblannr(ivs[s], 30, 1e3, v, fl[s])
+            assert one["nev"] == outs[s]["nev"] and np.array_equal(one["lam"], outs[s]["lam"])
+    M.free()
