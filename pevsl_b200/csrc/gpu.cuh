@@ -83,6 +83,7 @@ enum Ws {
   WS_COUNT
 };
 
+constexpr int kSideStreams = 3;
 struct Ctx {
   bool ready = false;
   int device = 0;
@@ -102,6 +103,8 @@ struct Ctx {
   int tab_next = 0;
   unsigned *bar = nullptr;     /* grid barrier: count, generation, error   */
   cudaMemPool_t pool = nullptr; /* matrices (pool_alloc)          */
+  cudaStream_t side[kSideStreams] = {}; /* branches of captured graphs */
+  cudaEvent_t side_ev[kSideStreams + 1] = {};
   unsigned *cl_err = nullptr;  /* pinned: a wait of a cluster launch ran out */
   void *ws[WS_COUNT] = {};
   size_t wsz[WS_COUNT] = {};

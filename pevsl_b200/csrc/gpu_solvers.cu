@@ -220,10 +220,11 @@ static int il_group_cap(const pevsl_devcsr *A) {
   const char *e = getenv("PEVSL_B200_IL_MAXS"); /* read per call: tests change it */
   const int env = e ? atoi(e) : 0;
   if (env >= 2) return PEVSL_MIN(env, kMaxBatch);
-  const double mat = 3.0 * (double)A->nnz + 4.0 * (A->nrows + 1.0);
+  const double mat = A->smask ? il_matrix_bytes(A) : 3.0 * (double)A->nnz + 4.0 * (A->nrows + 1.0);
+  const double most = (A->smask ? 70.0 : 64.0) * 1024 * 1024;
   int cap = 2;
   for (int S = 4; S <= kMaxBatch; S *= 2)
-    if (24.0 * (double)A->nrows * S + mat <= 64.0 * 1024 * 1024) cap = S;
+    if (24.0 * (double)A->nrows * S + mat <= most) cap = S;
   return cap;
 }
 
@@ -242,6 +243,8 @@ static int il_defer_setting() {
   }
   return v;
 }
+
+static constexpr double kBranchBytes = 64.0 * 1024 * 1024;
 
 /* a set of slices the interleaved form serves together */
 struct IlGroup {
@@ -347,7 +350,105 @@ static double filter_bytes_degree(const pevsl_devcsr *A, int deg_k, bool fp32, b
   return (deg_k == 1 ? 3.0 : 5.0) * vb * n + (last ? 4.0 * n : 0.0);
 }
 
-static int cheb_filter_batch(int ne, const FilterJob *jobs, bool fp32) {
+/* the group's inputs from the jobs' x, and its results to their y */
+static int il_pack_group(const IlGroup &G, const FilterJob *jobs) {
+  const double *xs[kMaxBatch];
+  for (int c = 0; c < G.S; c++) xs[c] = jobs[G.idx[c < G.cnt ? c : 0]].x; /* padding: mu 0 */
+  double *X0, *B0, *B1, *Y;
+  il_buffers(G, &X0, &B0, &B1, &Y);
+  return il_pack(G.A->nrows, G.S, xs, X0);
+}
+static int il_unpack_group(const IlGroup &G, const FilterJob *jobs) {
+  double *ys[kMaxBatch];
+  for (int c = 0; c < G.cnt; c++) ys[c] = jobs[G.idx[c]].y;
+  double *X0, *B0, *B1, *Y;
+  il_buffers(G, &X0, &B0, &B1, &Y);
+  return il_unpack(G.A->nrows, G.S, G.cnt, Y, ys);
+}
+
+/* Branches of a captured application: the groups over up to kSideStreams + 1
+ * branches, the longest first to the branch with the least time.  A group
+ * alone is bound by the latency of its degrees, so several at a time gain as
+ * long as they stay in L2 together: the largest working sets of the branches
+ * must sum to at most kBranchBytes, else there is one branch less.  Returns
+ * their number.  Whole runs, one after another / as branches: three grids of
+ * 216000, 32399 and 21924 rows with three slices each 391 / 275 ms, two of
+ * 216000 with three 513 / 372, four of 85000 with three 415 / 242, 40 slices
+ * at 26970 rows (three groups) 864 / 550; with a limit of 110 MB two groups of
+ * two at 10^6 rows 2.51 -> 2.71 s.  (The cluster launch of small problems
+ * stays ahead of them: beside the groups its blocks and theirs share SMs, and
+ * 7980 rows with 216000 gained 4%.) */
+static int filter_branches(const std::vector<IlGroup> &g, std::vector<int> *branch) {
+  const size_t ng = g.size();
+  std::vector<double> us(ng), bytes(ng);
+  std::vector<size_t> ord(ng);
+  for (size_t i = 0; i < ng; i++) {
+    const double v = 24.0 * (double)g[i].A->nrows * g[i].S;
+    ord[i] = i;
+    bytes[i] = v + il_matrix_bytes(g[i].A);
+    us[i] = g[i].maxdeg * (1.5 + v / 5e6); /* latency, and 5 TB/s */
+  }
+  std::sort(ord.begin(), ord.end(), [&](size_t a, size_t b) { return us[a] > us[b]; });
+  for (int nb = (int)PEVSL_MIN((size_t)kSideStreams + 1, ng); nb > 1; nb--) {
+    std::vector<double> load((size_t)nb, 0.0), most((size_t)nb, 0.0);
+    for (size_t i : ord) {
+      const size_t b = (size_t)(std::min_element(load.begin(), load.end()) - load.begin());
+      (*branch)[i] = (int)b;
+      load[b] += us[i];
+      most[b] = PEVSL_MAX(most[b], bytes[i]);
+    }
+    double sum = 0.0;
+    for (double m : most) sum += m;
+    if (sum <= kBranchBytes) return nb;
+  }
+  std::fill(branch->begin(), branch->end(), 0);
+  return 1;
+}
+
+/* The side streams only ever carry work inside a capture of the context
+ * stream, as branches of its graph: what runs, runs in the graph's launch on
+ * the context stream. */
+static int fork_branches(int nb) {
+  Ctx &c = ctx();
+  if (fail(cudaEventRecord(c.side_ev[0], c.stream), "cudaEventRecord")) return PEVSL_ERR_CUDA;
+  for (int b = 1; b < nb; b++)
+    if (fail(cudaStreamWaitEvent(c.side[b - 1], c.side_ev[0], 0), "cudaStreamWaitEvent"))
+      return PEVSL_ERR_CUDA;
+  return 0;
+}
+static int join_branches(int nb) {
+  Ctx &c = ctx();
+  int st = 0;
+  for (int b = 1; b < nb; b++)
+    if (fail(cudaEventRecord(c.side_ev[b], c.side[b - 1]), "cudaEventRecord") ||
+        fail(cudaStreamWaitEvent(c.stream, c.side_ev[b], 0), "cudaStreamWaitEvent"))
+      st = PEVSL_ERR_CUDA;
+  return st;
+}
+/* launches go to branch b's stream while one of these is alive */
+struct BranchScope {
+  cudaStream_t main;
+  explicit BranchScope(int b) : main(ctx().stream) {
+    if (b > 0) ctx().stream = ctx().side[b - 1];
+  }
+  ~BranchScope() { ctx().stream = main; }
+};
+static int branch_streams() {
+  Ctx &c = ctx();
+  for (int b = 0; b <= kSideStreams; b++) {
+    if (!c.side_ev[b] &&
+        fail(cudaEventCreateWithFlags(&c.side_ev[b], cudaEventDisableTiming), "cudaEventCreate"))
+      return PEVSL_ERR_CUDA;
+    if (b < kSideStreams && !c.side[b] &&
+        fail(cudaStreamCreateWithFlags(&c.side[b], cudaStreamNonBlocking), "cudaStreamCreate"))
+      return PEVSL_ERR_CUDA;
+  }
+  return 0;
+}
+
+/* packed: the interleaved groups' inputs are in their buffers and the results
+ * stay there */
+static int cheb_filter_batch(int ne, const FilterJob *jobs, bool fp32, bool packed = false) {
   if (ne <= 0) return 0;
   if (ne > kMaxEntries) return PEVSL_ERR_ARG;
   int st = 0, maxdeg = 0, nlive = 0;
@@ -458,8 +559,22 @@ static int cheb_filter_batch(int ne, const FilterJob *jobs, bool fp32) {
     cj.push_back(ClusterJob{J.A, nullptr, J.x, J.y, J.dmu, nullptr, J.pol->cc, J.pol->dd, 0.0, 0.0,
                             J.pol->deg, 0});
   }
-  if (!cj.empty()) {
-    if ((st = cluster_filter((int)cj.size(), cj.data(), fp32))) return st;
+  const int defer = il_defer_setting();
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(ctx().stream, &cs);
+  const bool capturing = cs != cudaStreamCaptureStatusNone;
+  if (!ig.empty()) {
+    /* inside a capture the caller prepared the workspace and coefficients */
+    if (!capturing) st = il_prepare(ne, jobs, fp32);
+    if (!st && (!ctx().ws[WS_IL] || ctx().wsz[WS_IL] < sizeof(double) * il_ws_doubles(ig) ||
+                !ctx().ws[WS_ILMU] || ctx().wsz[WS_ILMU] < sizeof(double) * il_mu_doubles(ig)))
+      st = PEVSL_ERR_ARG; /* il_prepare not run before the capture */
+    if (st) return st;
+  }
+  auto clusters = [&]() -> int {
+    if (cj.empty()) return 0;
+    const int r = cluster_filter((int)cj.size(), cj.data(), fp32);
+    if (r) return r;
     int dmax = 0;
     for (size_t i = 0; i < cj.size(); i++) {
       const pevsl_devcsr *A = cj[i].A;
@@ -469,28 +584,44 @@ static int cheb_filter_batch(int ne, const FilterJob *jobs, bool fp32) {
                           matrix_bytes(A, fp32);
     }
     g_filter_launches += (uint64_t)dmax;
-  }
-  std::vector<std::array<const double *, 3>> ilv(ig.size()); /* vk, vkm1 per group */
-  std::vector<int> ilw(ig.size(), 0);                          /* last degree added to y */
-  const int defer = il_defer_setting();
-  if (!ig.empty()) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    cudaStreamIsCapturing(ctx().stream, &cs);
-    /* inside a capture the caller prepared the workspace and coefficients */
-    if (cs == cudaStreamCaptureStatusNone) st = il_prepare(ne, jobs, fp32);
-    if (!st && (!ctx().ws[WS_IL] || ctx().wsz[WS_IL] < sizeof(double) * il_ws_doubles(ig) ||
-                !ctx().ws[WS_ILMU] || ctx().wsz[WS_ILMU] < sizeof(double) * il_mu_doubles(ig)))
-      st = PEVSL_ERR_ARG; /* il_prepare not run before the capture */
-    for (size_t gi = 0; gi < ig.size() && !st; gi++) {
-      const IlGroup &G = ig[gi];
-      const double *xs[kMaxBatch];
-      for (int c = 0; c < G.S; c++) xs[c] = jobs[G.idx[c < G.cnt ? c : 0]].x; /* padding: mu 0 */
-      double *X0, *B0, *B1, *Y;
-      il_buffers(G, &X0, &B0, &B1, &Y);
-      st = il_pack(G.A->nrows, G.S, xs, X0);
-      ilv[gi] = {X0, nullptr, nullptr};
+    return 0;
+  };
+  /* a group through all its degrees, so that its working set stays in L2
+   * between them (il_group_cap); the groups are independent, so every
+   * slice's bits are those of the degree-major order */
+  auto group = [&](const IlGroup &G) -> int {
+    int r = packed ? 0 : il_pack_group(G, jobs);
+    double *X0, *B0, *B1, *Y;
+    il_buffers(G, &X0, &B0, &B1, &Y);
+    const double *dmu = (const double *)ctx().ws[WS_ILMU] + G.mu_off;
+    const double *gk = X0, *gkm1 = nullptr;
+    for (int k = 1, lastw = 0; k <= G.maxdeg && !r; k++) {
+      double *gkp1 = k == 1 ? B0 : k == 2 ? B1 : const_cast<double *>(gkm1);
+      const int ny = deferred_terms(k, lastw, G.maxdeg, defer), fresh = ny > 0 && lastw == 0;
+      r = cheb_step_il_y(G.A, G.S, gk, gk, gkm1, gkp1, Y, G.cc, (k == 1 ? 1.0 : 2.0) / G.dd, dmu,
+                         dmu + (size_t)k * G.S, ny, fresh);
+      if (ny > 0) lastw = k;
+      /* read v_k, v_{k-1} (from degree 2), write v_{k+1}; y read unless
+       * fresh and written when updated */
+      const double vec = (k == 1 ? 16.0 : 24.0) + (ny > 0 ? (fresh ? 8.0 : 16.0) : 0.0);
+      g_filter_bytes += il_matrix_bytes(G.A) + vec * (double)G.A->nrows * G.S;
+      g_filter_launches++;
+      gkm1 = gk;
+      gk = gkp1;
     }
-    if (st) return st;
+    if (!r && !packed) r = il_unpack_group(G, jobs);
+    return r;
+  };
+  st = clusters();
+  if (st) return st;
+  /* in a capture the groups become parallel branches of the graph */
+  std::vector<int> branch(ig.size(), 0);
+  const int nb = capturing ? filter_branches(ig, &branch) : 1;
+  if (nb > 1 && (st = fork_branches(nb))) return st;
+  for (int b = nb - 1; b >= 0 && !st; b--) {
+    BranchScope on(b);
+    for (size_t gi = 0; gi < ig.size() && !st; gi++)
+      if (branch[gi] == b) st = group(ig[gi]);
   }
   std::vector<const void *> vk(nlive), vkm1(nlive);
   std::vector<void *> b0(nlive), b1(nlive), acc(nlive);
@@ -510,31 +641,6 @@ static int cheb_filter_batch(int ne, const FilterJob *jobs, bool fp32) {
       acc[i] = J.y;
     }
     vkm1[i] = nullptr;
-  }
-  /* the interleaved groups one after another, each through all its
-   * degrees, so that a group's working set stays in L2 between degrees
-   * (il_group_cap); the groups are independent, so every slice's bits are
-   * those of the degree-major order */
-  for (size_t gi = 0; gi < ig.size() && !st; gi++) {
-    const IlGroup &G = ig[gi];
-    double *X0, *B0, *B1, *Y;
-    il_buffers(G, &X0, &B0, &B1, &Y);
-    const double *dmu = (const double *)ctx().ws[WS_ILMU] + G.mu_off;
-    for (int k = 1; k <= G.maxdeg && !st; k++) {
-      const double *gk = ilv[gi][0], *gkm1 = ilv[gi][1];
-      double *gkp1 = k == 1 ? B0 : k == 2 ? B1 : const_cast<double *>(gkm1);
-      const int ny = deferred_terms(k, ilw[gi], G.maxdeg, defer), fresh = ny > 0 && ilw[gi] == 0;
-      st = cheb_step_il_y(G.A, G.S, gk, gk, gkm1, gkp1, Y, G.cc, (k == 1 ? 1.0 : 2.0) / G.dd, dmu,
-                          dmu + (size_t)k * G.S, ny, fresh);
-      if (ny > 0) ilw[gi] = k;
-      /* read v_k, v_{k-1} (from degree 2), write v_{k+1}; y read unless
-       * fresh and written when updated */
-      const double vec = (k == 1 ? 16.0 : 24.0) + (ny > 0 ? (fresh ? 8.0 : 16.0) : 0.0);
-      g_filter_bytes += il_matrix_bytes(G.A) + vec * (double)G.A->nrows * G.S;
-      g_filter_launches++;
-      ilv[gi][1] = gk;
-      ilv[gi][0] = gkp1;
-    }
   }
   int nother = 0, other = -1;
   maxdeg = 0;
@@ -593,13 +699,9 @@ static int cheb_filter_batch(int ne, const FilterJob *jobs, bool fp32) {
     g_filter_launches++;
     g_filter_bytes += bytes;
   }
-  for (size_t gi = 0; gi < ig.size() && !st; gi++) {
-    const IlGroup &G = ig[gi];
-    double *ys[kMaxBatch];
-    for (int c = 0; c < G.cnt; c++) ys[c] = jobs[G.idx[c]].y;
-    double *X0, *B0, *B1, *Y;
-    il_buffers(G, &X0, &B0, &B1, &Y);
-    st = il_unpack(G.A->nrows, G.S, G.cnt, Y, ys);
+  if (nb > 1) {
+    const int r = join_branches(nb);
+    if (!st) st = r;
   }
   return st;
 }
@@ -622,6 +724,8 @@ static bool all_cluster(const std::vector<FilterJob> &jobs, bool fp32) {
 struct FilterGraph {
   cudaGraphExec_t exec = nullptr;
   std::vector<char> key; /* live slices of the captured sequence */
+  std::vector<IlGroup> groups;
+  std::vector<char> grouped; /* the jobs in them */
   bool mixed = false;
   uint64_t launches = 0, kernel_launches = 0;
   double bytes = 0.0;
@@ -635,25 +739,34 @@ static int filter_graphed(FilterGraph &fg, const std::vector<char> &sel, std::ve
   const int ne = (int)jobs.size();
   std::vector<FilterJob> staged(jobs);
   int st = 0;
+  const bool renew = !fg.exec || fg.key != sel;
+  if (renew) {
+    fg.groups.clear();
+    fg.grouped.assign((size_t)ne, 0);
+    if (filter_form() == 0) {
+      if ((st = il_prepare(ne, jobs.data(), fg.mixed)) || (st = branch_streams())) return st;
+      il_partition(ne, jobs.data(), fg.mixed, fg.groups, fg.grouped);
+    }
+  }
+  /* the groups are packed and unpacked around the graph, the others staged */
+  for (const IlGroup &G : fg.groups)
+    if ((st = il_pack_group(G, jobs.data()))) return st;
   for (int e = 0; e < ne && !st; e++) {
+    if (fg.grouped[(size_t)e]) continue;
     double *xs = (double *)((char *)jobs[e].work + 16 * (size_t)jobs[e].ld);
     st = memcpy_async(xs, jobs[e].x, sizeof(double) * (size_t)jobs[e].A->nrows);
     staged[e].x = xs;
     staged[e].y = xs + jobs[e].ld;
   }
   if (st) return st;
-  if (!fg.exec || fg.key != sel) {
+  if (renew) {
     if (fg.exec) cudaGraphExecDestroy(fg.exec);
     fg.exec = nullptr;
-    if (filter_form() == 0) {
-      st = il_prepare(ne, staged.data(), fg.mixed);
-      if (st) return st;
-    }
     const uint64_t l0 = g_filter_launches, k0 = c.launches;
     const double b0 = g_filter_bytes;
     if (fail(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal), "BeginCapture"))
       return PEVSL_ERR_CUDA;
-    st = cheb_filter_batch(ne, staged.data(), fg.mixed);
+    st = cheb_filter_batch(ne, staged.data(), fg.mixed, true);
     cudaGraph_t gr = nullptr;
     const cudaError_t ec = cudaStreamEndCapture(c.stream, &gr);
     if (st || fail(ec, "EndCapture")) {
@@ -681,8 +794,11 @@ static int filter_graphed(FilterGraph &fg, const std::vector<char> &sel, std::ve
     c.launches += fg.kernel_launches;
   }
   if (fail(cudaGraphLaunch(fg.exec, c.stream), "cudaGraphLaunch")) return PEVSL_ERR_CUDA;
+  for (const IlGroup &G : fg.groups)
+    if ((st = il_unpack_group(G, jobs.data()))) return st;
   for (int e = 0; e < ne && !st; e++)
-    st = memcpy_async(jobs[e].y, staged[e].y, sizeof(double) * (size_t)jobs[e].A->nrows);
+    if (!fg.grouped[(size_t)e])
+      st = memcpy_async(jobs[e].y, staged[e].y, sizeof(double) * (size_t)jobs[e].A->nrows);
   return st;
 }
 
@@ -1895,11 +2011,12 @@ static int cheblannr_group(SliceState *SL, int ns, double tol, FILE *fstats,
    * the one-slice filter and breakdown restarts; 16 ld bytes of batched
    * filter work per slice; the filter coefficients on the device */
   double *Vall = (double *)ws(WS_BASIS, sizeof(double) * basis_elems);
-  double *w3 = (double *)ws(WS_CHEB, sizeof(double) * 3 * (size_t)nmax + (batched ? work_bytes : 0));
+  const size_t w3len = (size_t)round_ld(3 * nmax);
+  double *w3 = (double *)ws(WS_CHEB, sizeof(double) * w3len + (batched ? work_bytes : 0));
   double *vrand = (double *)ws(all_builtin ? WS_VEC : WS_RITZ2, sizeof(double) * (size_t)nmax);
   double *dmu_all = batched ? (double *)ws(WS_MU, sizeof(double) * mu_elems) : nullptr;
   if (!Vall || !w3 || !vrand || (batched && !dmu_all)) return PEVSL_ERR_NOMEM;
-  char *bwork = (char *)(w3 + 3 * (size_t)nmax);
+  char *bwork = (char *)(w3 + w3len);
   std::vector<char *> work(ns, nullptr);
   std::vector<const double *> dmu(ns, nullptr);
   int st = 0;
