@@ -249,7 +249,8 @@ int b_axpy(const BLen &len, int S, CPtrs x, VPtrs y, BScal a, unsigned mask);
 int b_scal(const BLen &len, int S, VPtrs x, BScal a, unsigned mask);
 /* y_s += sign coef[s] x_s and x_s *= 1 / nrm[s] for all S entries, the
  * scalars in device memory */
-int b_axpy_dev(const BLen &len, int S, const double *coef, double sign, CPtrs x, VPtrs y);
+int b_axpy_dev_dot(const BLen &len, int S, const double *coef, double sign, CPtrs x, VPtrs y,
+                   CPtrs z, double *out);
 int b_scal_inv_dev(const BLen &len, int S, const double *nrm, VPtrs x);
 int b_dot(const BLen &len, int S, CPtrs x, CPtrs y, double *out, int fin, unsigned mask);
 int b_axpy_dev_nrm2(const BLen &len, int S, const double *coef, CPtrs x, VPtrs y, double *nrm,

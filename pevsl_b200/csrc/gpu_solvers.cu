@@ -1184,8 +1184,9 @@ static int lan_step(LanRuns &R, int k, bool prev) {
   } else {
     for (int s = 0; s < S && !st; s++) st = apply_A(R.pevsl, v.p[s], vn.p[s]);
   }
-  if (!st && prev) st = b_axpy_dev(len, S, R.beta(k - 1), -1.0, vm, vn);
-  if (!st) st = b_dot(len, S, v, vc, R.alpha(k), FIN_ID, all);
+  if (!st)
+    st = prev ? b_axpy_dev_dot(len, S, R.beta(k - 1), -1.0, vm, vn, v, R.alpha(k))
+              : b_dot(len, S, v, vc, R.alpha(k), FIN_ID, all);
   if (!st) st = b_axpy_dev_nrm2(len, S, R.alpha(k), v, vn, R.nrm0, all);
   const long ldw = R.maxk + 1;
   if (!st) st = b_gemvT(len, S, k + 1, base, vc, R.w, ldw, nullptr, all);

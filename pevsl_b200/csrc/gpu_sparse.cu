@@ -660,8 +660,9 @@ __global__ void __launch_bounds__(kThreads)
     k_spmv_stencil_batch(int n, const __grid_constant__ Stencil S, const __grid_constant__ CPtrs x,
                          const __grid_constant__ VPtrs y) {
   const int row = (int)(blockIdx.x * (unsigned)kThreads + threadIdx.x);
+  const unsigned m = row < n ? stencil_mask<M>(S, row) : 0u;
+  pdl_wait_then_release();
   if (row >= n) return;
-  const unsigned m = stencil_mask<M>(S, row);
   y.p[blockIdx.y][row] = stencil_dot<K, false>(S, m, x.p[blockIdx.y] + row, 0.0);
 }
 
@@ -1541,7 +1542,7 @@ int spmv_batch(const pevsl_devcsr *A, int S, CPtrs x, VPtrs y) {
            : A->sbytes == 1 ? k_spmv_stencil_batch<0, unsigned char>
            : A->sbytes == 2 ? k_spmv_stencil_batch<0, unsigned short>
                             : k_spmv_stencil_batch<0, unsigned>;
-  k<<<g, kThreads, 0, ctx().stream>>>(A->nrows, stencil_of(A), x, y);
+  launch_pdl_block(k, g, kThreads, 0, ctx().stream, A->nrows, stencil_of(A), x, y);
   return launched("spmv_stencil_batch");
 }
 
