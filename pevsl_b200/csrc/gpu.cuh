@@ -79,6 +79,7 @@ enum Ws {
   WS_LAN,       /* Lanczos runs: alpha and beta of every step, CGS coefficients */
   WS_TUNE,      /* scratch vectors of the autotuner (its own: a tuning may come
                    between other uses)                        */
+  WS_JAC,       /* projected matrix of a thick restart       */
   WS_LANV,      /* Lanczos DOS: the start vectors of a group */
   WS_COUNT
 };
@@ -369,6 +370,12 @@ int cvt_f64_f32(long n, const double *x, float *y);
 int gemm_tn(long n, int k, int m, const double *V, long ldv, const double *W, long ldw, double *C,
             long ldc);
 /* U = V(:, 0:k) Y  (n x m, V column-major ldv, Y k x m column-major ldy) */
+/* the ends of the spectrum of a symmetric n x n host matrix (column major):
+ * val[0..3] = lam_1, lam_2, lam_{n-1}, lam_n, val[4..5] the last elements of
+ * the eigenvectors of lam_1 and lam_n, which go to Y (device, 2n); waits.
+ * ritz_ends_ok: the n it takes */
+bool ritz_ends_ok(int n);
+int ritz_ends(int n, const double *T, int ldt, double *Y, double *val);
 int gemm_nn(long n, int k, int m, const double *V, long ldv, const double *Y, long ldy,
             double *U, long ldu);
 

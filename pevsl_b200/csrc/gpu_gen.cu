@@ -740,34 +740,46 @@ int pevsl_gen_lantrbounds(pevsl_Data *pevsl, int lanm, int maxit, double tol, pe
       T[(k - 1) * L + k] = beta;
     }
     if (st) break;
-    if (pevsl_dense_symeig(k, T, lanm1, EvecT, lanm1, Rval)) {
-      st = PEVSL_ERR_EIG;
-      break;
+    double end[6];
+    if (ritz_ends_ok(k)) {
+      if ((st = ritz_ends(k, T, lanm1, dY, end))) break;
+    } else {
+      if (pevsl_dense_symeig(k, T, lanm1, EvecT, lanm1, Rval)) {
+        st = PEVSL_ERR_EIG;
+        break;
+      }
+      end[0] = Rval[0];
+      end[1] = Rval[1];
+      end[2] = k > 1 ? Rval[k - 2] : 0.0;
+      end[3] = Rval[k - 1];
+      end[4] = EvecT[k - 1];
+      end[5] = EvecT[(size_t)(k - 1) * L + (k - 1)];
+      memcpy(hY, EvecT, sizeof(double) * (size_t)k);
+      memcpy(hY + k, EvecT + (size_t)(k - 1) * L, sizeof(double) * (size_t)k);
+      if ((st = memcpy_async(dY, hY, sizeof(double) * 2 * (size_t)k))) break;
     }
-    s[0] = beta * EvecT[k - 1];
-    s[1] = beta * EvecT[(size_t)(k - 1) * L + (k - 1)];
+    s[0] = beta * end[4];
+    s[1] = beta * end[5];
     double t1, t2;
     if (bndtype <= 1) {
       t1 = fabs(s[0]);
       t2 = fabs(s[1]);
     } else {
-      t1 = 2.0 * s[0] * s[0] / (Rval[1] - Rval[0]);
-      t2 = 2.0 * s[1] * s[1] / (Rval[k - 1] - Rval[k - 2]);
+      t1 = 2.0 * s[0] * s[0] / (end[1] - end[0]);
+      t2 = 2.0 * s[1] * s[1] / (end[3] - end[2]);
     }
-    lmin = Rval[0] - t1;
-    lmax = Rval[k - 1] + t2;
+    lmin = end[0] - t1;
+    lmax = end[3] + t2;
     /* the extreme Ritz vectors and their B images become V, Z (:, 0:2) */
-    memcpy(hY, EvecT, sizeof(double) * (size_t)k);
-    memcpy(hY + k, EvecT + (size_t)(k - 1) * L, sizeof(double) * (size_t)k);
-    st = memcpy_async(dY, hY, sizeof(double) * 2 * (size_t)k);
-    if (!st) st = gemm_nn(n, k, 2, V, ld, dY, k, R, ld);
+    st = gemm_nn(n, k, 2, V, ld, dY, k, R, ld);
     if (!st) st = gemm_nn(n, k, 2, Z, ld, dY, k, R + 2 * ld, ld);
     if (!st) st = vcopy(R, VC(0), n);
     if (!st) st = vcopy(R + ld, VC(1), n);
     if (!st) st = vcopy(R + 2 * ld, ZC(0), n);
     if (!st) st = vcopy(R + 3 * ld, ZC(1), n);
     trlen = 2;
-    Rval[1] = Rval[k - 1];
+    Rval[0] = end[0];
+    Rval[1] = end[3];
     if (fstats)
       fprintf(fstats, "it %4d, k %3d: ritz %.15e %.15e, t1,t2 %e %e, res %.15e %.15e\n", it, k,
               Rval[0], Rval[1], t1, t2, fabs(s[0]), fabs(s[1]));

@@ -1531,31 +1531,43 @@ int pEVSL_LanTrbounds(pevsl_Data *pevsl, int lanm, int maxit, double tol, pevsl_
       prev = true;
     }
     if (st) break;
-    if (pevsl_dense_symeig(k, T, lanm1, EvecT, lanm1, Rval)) {
-      st = PEVSL_ERR_EIG;
-      break;
+    double end[6];
+    if (ritz_ends_ok(k)) {
+      if ((st = ritz_ends(k, T, lanm1, dY, end))) break;
+    } else {
+      if (pevsl_dense_symeig(k, T, lanm1, EvecT, lanm1, Rval)) {
+        st = PEVSL_ERR_EIG;
+        break;
+      }
+      end[0] = Rval[0];
+      end[1] = Rval[1];
+      end[2] = k > 1 ? Rval[k - 2] : 0.0;
+      end[3] = Rval[k - 1];
+      end[4] = EvecT[k - 1];
+      end[5] = EvecT[(size_t)(k - 1) * L + (k - 1)];
+      memcpy(hY, EvecT, sizeof(double) * (size_t)k);
+      memcpy(hY + k, EvecT + (size_t)(k - 1) * L, sizeof(double) * (size_t)k);
+      if ((st = memcpy_async(dY, hY, sizeof(double) * 2 * (size_t)k))) break;
     }
-    s[0] = beta * EvecT[k - 1];
-    s[1] = beta * EvecT[(size_t)(k - 1) * L + (k - 1)];
+    s[0] = beta * end[4];
+    s[1] = beta * end[5];
     double t1, t2;
     if (bndtype <= 1) {
       t1 = fabs(s[0]);
       t2 = fabs(s[1]);
     } else {
-      t1 = 2.0 * s[0] * s[0] / (Rval[1] - Rval[0]);
-      t2 = 2.0 * s[1] * s[1] / (Rval[k - 1] - Rval[k - 2]);
+      t1 = 2.0 * s[0] * s[0] / (end[1] - end[0]);
+      t2 = 2.0 * s[1] * s[1] / (end[3] - end[2]);
     }
-    lmin = Rval[0] - t1;
-    lmax = Rval[k - 1] + t2;
+    lmin = end[0] - t1;
+    lmax = end[3] + t2;
     /* the two extreme Ritz vectors become V(:,0:2) */
-    memcpy(hY, EvecT, sizeof(double) * (size_t)k);
-    memcpy(hY + k, EvecT + (size_t)(k - 1) * L, sizeof(double) * (size_t)k);
-    st = memcpy_async(dY, hY, sizeof(double) * 2 * (size_t)k);
-    if (!st) st = gemm_nn(n, k, 2, V, ld, dY, k, R2, ld);
+    st = gemm_nn(n, k, 2, V, ld, dY, k, R2, ld);
     if (!st) st = vcopy(R2, VC(0), n);
     if (!st) st = vcopy(R2 + ld, VC(1), n);
     trlen = 2;
-    Rval[1] = Rval[k - 1];
+    Rval[0] = end[0];
+    Rval[1] = end[3];
     if (fstats)
       fprintf(fstats, "it %4d, k %3d: ritz %.15e %.15e, t1,t2 %e %e, res %.15e %.15e\n", it, k,
               Rval[0], Rval[1], t1, t2, fabs(s[0]), fabs(s[1]));
