@@ -419,11 +419,11 @@ def run_b200(args, dist):
                        "fused with the recurrence), CUDA-graph replays; one launch = one degree"
                        if gen else
                        "cheb_step_il (fused SpMV + Chebyshev recurrence, all slices per launch with "
-                       "row-interleaved vectors in groups of two that stay in L2, filter sum updated "
-                       "every third degree: k_cheb_il2_e on the ELL copy of the packed entries; one "
-                       "live slice: k_cheb_il_e<1>), all filter launches of the timed steps"
-                       if batched else "cheb_step (fused SpMV + Chebyshev recurrence, CSR-stream, "
-                       "packed entries)"),
+                       "row-interleaved vectors in groups that stay in L2, filter sum updated every "
+                       "third degree: k_cheb_il_mid on the stencil form; one live slice: "
+                       "k_cheb_stencil; small problems: k_filter_cluster, counted per degree), all "
+                       "filter launches of the timed steps"
+                       if batched else "cheb_step (fused SpMV + Chebyshev recurrence, stencil form)"),
             "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak if achieved else None, "peak_source": peak_kind,
             "bytes_per_launch": per_launch_bytes, "launches": f_launch,

@@ -144,9 +144,7 @@ int vcopy(const double *x, double *y, long n);
 int vscal(double *x, long n, double a);
 int vaxpy(long n, double a, const double *x, double *y);
 /* y += sign * (*coef) * x, coef in device memory */
-int vaxpy_dev(long n, const double *coef, double sign, const double *x, double *y);
 /* x *= 1 / (*s), s in device memory */
-int vscal_inv_dev(long n, const double *s, double *x);
 /* *out = <x, y> (deterministic); out in device memory */
 int vdot(long n, const double *x, const double *y, double *out);
 /* *out = ||x|| */

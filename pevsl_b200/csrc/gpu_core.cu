@@ -226,17 +226,6 @@ __global__ void k_axpy(long n, double a, const double *__restrict__ x, double *_
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
     y[i] += a * x[i];
 }
-__global__ void k_axpy_dev(long n, const double *coef, double sign, const double *__restrict__ x,
-                           double *__restrict__ y) {
-  const double a = sign * *coef;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-    y[i] += a * x[i];
-}
-__global__ void k_scal_inv_dev(long n, const double *s, double *x) {
-  const double a = 1.0 / *s;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-    x[i] *= a;
-}
 __global__ void k_sum(long n, const double *__restrict__ x, double *partials, unsigned *counter,
                       double *out) {
   double s = 0.0;
@@ -312,16 +301,6 @@ int vaxpy(long n, double a, const double *x, double *y) {
   if (n <= 0) return 0;
   k_axpy<<<grid_for(n, 4), kThreads, 0, g_ctx.stream>>>(n, a, x, y);
   return launched("axpy");
-}
-int vaxpy_dev(long n, const double *coef, double sign, const double *x, double *y) {
-  if (n <= 0) return 0;
-  k_axpy_dev<<<grid_for(n, 4), kThreads, 0, g_ctx.stream>>>(n, coef, sign, x, y);
-  return launched("axpy_dev");
-}
-int vscal_inv_dev(long n, const double *s, double *x) {
-  if (n <= 0) return 0;
-  k_scal_inv_dev<<<grid_for(n, 4), kThreads, 0, g_ctx.stream>>>(n, s, x);
-  return launched("scal_inv_dev");
 }
 int vsum(long n, const double *x, double *out) {
   k_sum<<<grid_for(n, 4), kThreads, 0, g_ctx.stream>>>(n, x, g_ctx.red, g_ctx.cnt, out);

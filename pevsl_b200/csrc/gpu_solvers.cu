@@ -9,8 +9,9 @@
  *   filtered Lanczos     pEVSL_ChebLanNr  SRC/cheblanNr.c:54-448
  *
  * The control flow (step counts, tests, breakdown restarts, acceptance) is
- * the reference's.  The host reads two scalars per Lanczos step (alpha,
- * beta); everything else stays on the device.  The DGKS second
+ * the reference's.  ChebLanNr's host side reads two scalars per Lanczos step
+ * (alpha, beta), the bounds' and the Lanczos DOS's those of a whole cycle or
+ * run at once (lan_step); everything else stays on the device.  The DGKS second
  * Gram-Schmidt pass is decided on the device.  When A is the built-in
  * parcsr, the SpMV is fused into the recurrence kernels; a user matvec
  * (pEVSL_SetAMatvec) is called with device pointers instead.
@@ -207,15 +208,16 @@ static int interleave_setting() {
 
 static int il_width(int nlive) { return nlive <= 2 ? 2 : nlive <= 4 ? 4 : nlive <= 8 ? 8 : 16; }
 
-/* Slices per interleaved group.  A group's whole filter application runs
- * before the next group's, and its working set from one degree to the next
- * -- three row-interleaved vector blocks (24 n bytes per slice) and the
- * matrix -- stays in the 126 MB L2 when it is at most half of it; wider
- * groups stream it from HBM at every degree.  So a group holds the most
- * slices (2, 4, 8 or 16) that fit in 64 MB, at least 2.  Measured per
- * degree at 100^3 (n = 1e6, packed matrix 25 MB): 2 slices 20.1 us (0.64 of
- * the HBM peak in algorithmic bytes, L2-resident), 4 slices 44.0-46.7 us.
- * PEVSL_B200_IL_MAXS caps it by hand (2..16). */
+/* Slices per interleaved group.  A group runs all its degrees, and its
+ * working set from one degree to the next -- three row-interleaved vector
+ * blocks (24 n bytes per slice) and the matrix -- stays in the 126 MB L2 when
+ * it is at most half of it; wider groups stream it from HBM at every degree.
+ * So a group holds the most slices (2, 4, 8 or 16) that fit in 64 MB (stencil
+ * matrices, whose mask is nearly nothing: 70), at least 2.  Stencil matrices
+ * per degree, four slices as one group / as two: 80 x 81 x 79 (48 MB) 8.4 /
+ * 10.2 us, 90 x 91 x 89 (70 MB) 12.0 / 13.3, 99 x 100 x 101 (96 MB) 19.0 /
+ * 17.0; eight as one / as two of four: 72 x 71 x 73 (72 MB) 11.9 / 13.4, 80 x
+ * 81 x 79 (97 MB) 18.8 / 16.8.  PEVSL_B200_IL_MAXS caps it by hand (2..16). */
 static int il_group_cap(const pevsl_devcsr *A) {
   const char *e = getenv("PEVSL_B200_IL_MAXS"); /* read per call: tests change it */
   const int env = e ? atoi(e) : 0;

@@ -10,15 +10,25 @@
  *    (SRC/kpmdos.c:129-156) for a group of random vectors at once, with the
  *    dot products of two moments fused in.
  *
- * Layout: CSR with int32 row pointers / column indices and fp64 values; a
- * row is handled by a group of L lanes (L = 1..32, a power of two picked from
- * the mean row length) that read the row's entries contiguously and reduce
- * with warp shuffles.  KPM blocks are row-interleaved (row i of all s vectors
- * contiguous), so the gather of x[col] is one coalesced 8*s-byte segment.
+ * Layout: CSR with int32 row pointers / column indices and fp64 values.  What
+ * a matrix's kernels read is decided once, at set-up or at its first filter:
+ *   stencil form   at most 32 (column offset, value) pairs in all: a mask per
+ *                  row, the pairs as a kernel parameter (k_rows_stencil,
+ *                  k_cheb_stencil, k_cheb_il_stencil, k_cheb_il_mid)
+ *   packed, ELL    at most 256 distinct values: 3 bytes per entry
+ *   windowed       any values, the gathered vector's band in shared memory
+ *                  where it was measured faster (k_csr_window)
+ *   CSR-stream     short rows, one row per lane (k_csr_stream)
+ *   row groups     long rows: L lanes (2..32, from the mean length) read a
+ *                  row's entries contiguously and reduce with warp shuffles
+ * Small matrices run whole filter applications in a cluster (gpu_cluster.cu).
+ * KPM blocks are row-interleaved (row i of all s vectors contiguous), so the
+ * gather of x[col] is one coalesced 8*s-byte segment.
  */
 #include <ctype.h>
 #include <cuda_runtime.h>
 #include <algorithm>
+#include <cmath>
 #include <vector>
 #include <stdio.h>
 #include <stdlib.h>
@@ -581,8 +591,8 @@ __global__ void __launch_bounds__(kThreads, 4)
  * three to four waves of blocks, each the length of the chain mask, gather,
  * sum, store; larger ones stream from HBM.  Per degree of one vector with the
  * sum deferred, against the ELL and packed kernels: 41 x 40 x 42 2.2 / 2.5
- * us, 64 x 65 x 63 2.7 / 4.1 us, 99 x 100 x 101 6.6 / 10.6 us (30 MB: 4.6
- * TB/s), 159 x 160 x 161 24.4 / 54 us.  (The same rows described by a table
+ * us, 64 x 65 x 63 2.4 / 4.1 us, 99 x 100 x 101 5.9 / 10.6 us (30 MB: 5.1
+ * TB/s), 159 x 160 x 161 22.4 / 54 us.  (The same rows described by a table
  * of row patterns in shared memory took 8.1 us at 99 x 100 x 101, with the
  * value and the offset in one 16-byte entry 11.6 us: the table's broadcast
  * loads use as many L1 cycles as the gathers, which ran at 78%.) */
@@ -608,9 +618,12 @@ __device__ __forceinline__ unsigned stencil_mask(const Stencil &S, int row) {
 }
 
 /* sum over the row's pairs.  K: their number fixed at compile time, with the
- * diagonal in the middle (every gather of a row in flight at once), 0: any
- * number, eight at a time.  OWN: x0 is the row's element, so the diagonal
- * needs no load. */
+ * diagonal in the middle and finite values (stencil_width), 0: any number,
+ * eight at a time.  With K every gather of a row is in flight at once, and a
+ * pair that the row lacks adds its value times zero: the sum, which starts at
+ * +0 and is never -0, keeps its bits, and the additions need no predicates (64
+ * x 65 x 63 2.57 -> 2.26 us per filter degree, 99 x 100 x 101 6.36 -> 5.70).
+ * OWN: x0 is the row's element, so the diagonal needs no load. */
 template <int K, bool OWN>
 __device__ __forceinline__ double stencil_dot(const Stencil &S, unsigned m,
                                               const double *__restrict__ x, double x0) {
@@ -621,14 +634,11 @@ __device__ __forceinline__ double stencil_dot(const Stencil &S, unsigned m,
 #pragma unroll
     for (int u = 0; u < B; u++) {
       xv[u] = 0.0;
-      if (K > 0 && OWN && u == K / 2)
-        xv[u] = x0;
-      else if ((m >> (j0 + u)) & 1u)
-        xv[u] = __ldg(x + S.off[j0 + u]);
+      if ((m >> (j0 + u)) & 1u) xv[u] = K > 0 && OWN && u == K / 2 ? x0 : __ldg(x + S.off[j0 + u]);
     }
 #pragma unroll
     for (int u = 0; u < B; u++)
-      if ((m >> (j0 + u)) & 1u) r = add_rn(r, mul_rn(S.val[j0 + u], xv[u]));
+      if (K > 0 || ((m >> (j0 + u)) & 1u)) r = add_rn(r, mul_rn(S.val[j0 + u], xv[u]));
   }
   return r;
 }
@@ -697,9 +707,9 @@ struct EpiChebY {
  * v_{k-1} there, and no terms or three of them): nearly all of them, in a
  * kernel of their own without the cases that do not occur.  The branches of
  * the general one keep loads apart that can be in flight together.  Per
- * degree, general / this one: 45 x 44 x 43 1.67 / 1.63 us, 64 x 65 x 63 2.71 /
- * 2.48, 80 x 81 x 79 4.2 / 3.85, 99 x 100 x 101 6.75 / 6.25 (4.8 TB/s out of
- * L2), 1000 x 1001 5.56 / 5.30.  One row per thread, which leaves after the
+ * degree, general / this one: 45 x 44 x 43 1.67 / 1.58 us, 64 x 65 x 63 2.71 /
+ * 2.26, 80 x 81 x 79 4.2 / 3.5, 99 x 100 x 101 6.75 / 5.7 (5.3 TB/s out of
+ * L2), 1000 x 1001 5.56 / 5.10.  One row per thread, which leaves after the
  * wait where there is no row: the guarded form needs 37 registers and took
  * 2.88 us at 64 x 65 x 63. */
 template <int K>
@@ -708,7 +718,9 @@ __global__ void __launch_bounds__(kThreads)
                    const double *vkm1, double *vkp1, double *y, double cc, double t, double mua,
                    double mub, double muk, int upd) {
   const int row = (int)(blockIdx.x * (unsigned)kThreads + threadIdx.x);
-  const unsigned m = row < n ? stencil_mask<unsigned char>(S, row) : 0u;
+  /* a plain load stays ahead of the wait; one through the read-only path took
+   * 2.57 us at 64 x 65 x 63 against 2.47 */
+  const unsigned m = row < n ? ((const unsigned char *)S.mask)[row] : 0u;
   pdl_wait_then_release();
   if (row >= n) return;
   const double x = vk[row], xm1 = vkm1[row], yold = upd ? y[row] : 0.0;
@@ -718,9 +730,8 @@ __global__ void __launch_bounds__(kThreads)
   if (upd) y[row] = __fma_rn(muk, w, __fma_rn(mub, x, __fma_rn(mua, xm1, yold)));
 }
 
-/* two rows per thread, 32 registers: 126 x 125 x 127 10.7 us against 11.3
- * with one, 160 x 161 x 159 23 against 25-26, 1500 x 1501 9.9 against 10.4;
- * 99 x 100 x 101 6.3 against 6.25 */
+/* two rows per thread, 32 registers: 160 x 161 x 159 22.4 us against 24.4
+ * with one, 1500 x 1501 9.9 against 10.4; 126 x 127 x 125 10.6 against 10.2 */
 template <int K>
 __global__ void __launch_bounds__(kThreads, 8)
     k_cheb_stencil2(int n, const __grid_constant__ Stencil S, const double *__restrict__ vk,
@@ -1409,10 +1420,13 @@ static const T *packed_table(const pevsl_devcsr *A) {
   return sizeof(T) == 4 ? (const T *)(const void *)A->pvtab32 : (const T *)(const void *)A->pvtab;
 }
 
-/* the width the kernels are built for (5 and 7, the diagonal in the middle)
- * or 0 */
+/* the width the kernels are built for (5 and 7, the diagonal in the middle,
+ * finite values) or 0 */
 static int stencil_width(const pevsl_devcsr *A) {
-  return (A->sk == 5 || A->sk == 7) && A->sdiag == A->sk / 2 ? A->sk : 0;
+  if ((A->sk != 5 && A->sk != 7) || A->sdiag != A->sk / 2) return 0;
+  for (int j = 0; j < A->sk; j++)
+    if (!std::isfinite(A->sval[j])) return 0;
+  return A->sk;
 }
 
 template <class Epi>
@@ -1586,8 +1600,8 @@ int cheb_step_y(const pevsl_devcsr *A, const double *vk, const double *vkm1, dou
   if (!cheb_defers(A) || ny < 0 || ny > 3 || ny > k || (ny > 1 && !vkm1)) return PEVSL_ERR_ARG;
   const int w = stencil_width(A);
   if (w && vkm1 && (ny == 0 || (ny == 3 && !fresh))) {
-    /* two rows per thread from four waves of blocks on */
-    const int rpt = (long)A->nrows > 4L * 8 * kThreads * ctx().sms ? 2 : 1;
+    /* two rows per thread from eight waves of blocks on */
+    const int rpt = (long)A->nrows > 7L * 8 * kThreads * ctx().sms ? 2 : 1;
     const unsigned g = (unsigned)((A->nrows + kThreads * rpt - 1) / (kThreads * rpt));
     launch_pdl(rpt == 1 ? (w == 7 ? k_cheb_stencil<7> : k_cheb_stencil<5>)
                         : (w == 7 ? k_cheb_stencil2<7> : k_cheb_stencil2<5>),
@@ -2104,7 +2118,8 @@ static Il2Kernel il2_kernel(int ew) {
   return k_cheb_il2_e<0>;
 }
 
-/* Which filter-degree form runs, where the matrix has the ELL copy.  One
+/* Which filter-degree form runs, where the matrix has the ELL copy (packed,
+ * not a stencil).  One
  * vector: k_cheb_il_e<1> or the CSR-stream kernel; groups of two:
  * k_cheb_il2_e or k_cheb_il_p<2> -- each chosen per matrix by timing both
  * on this GPU at set-up (filter_tune; measured at 100^3 with the any-width

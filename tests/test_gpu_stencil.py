@@ -103,9 +103,9 @@ def test_generalized_lockstep_equals_one_by_one(gpu):
         x.free()
 
 
-@pytest.mark.parametrize("grid", [(107, 108, 106), (1103, 1101, 1)])
+@pytest.mark.parametrize("grid", [(107, 108, 106), (1103, 1101, 1), (129, 130, 128), (1461, 1463, 1)])
 def test_two_rows_per_thread(gpu, grid):
-    """Past four waves of blocks the degrees between the sum's first and last update take two rows per thread."""
+    """Past seven waves of blocks the degrees between the sum's first and last update take two rows per thread."""
     n, ia, ja, a = laplacian(*grid)
     M, G = pv.Matrix.from_csr(n, ia, ja, a), pv.Matrix.from_csr(*with_extra_rows(n, ia, ja, a))
     v = np.random.default_rng(9).standard_normal(n + 40)
@@ -133,3 +133,34 @@ def test_lockstep_past_one_wave(gpu, grid, slices):
             one = ev.cheblannr(ivs[s], 30, 1e3, v, fl[s])
             assert one["nev"] == outs[s]["nev"] and np.array_equal(one["lam"], outs[s]["lam"])
     M.free()
+
+
+def without(n, ia, ja, a, drop):
+    rows = np.repeat(np.arange(n), np.diff(ia))
+    keep = ~drop(rows, ja)
+    return n, np.concatenate([[0], np.cumsum(np.bincount(rows[keep], minlength=n))]).astype(np.int32), ja[keep], a[keep]
+
+
+@pytest.mark.parametrize("name", ["no_diagonal_in_some_rows", "empty_rows", "infinite_value"])
+def test_rows_that_lack_pairs(gpu, name):
+    """A pair that a row lacks adds nothing: not where it is the diagonal, not
+    in an empty row, and not where its value is infinite."""
+    n, ia, ja, a = laplacian(41, 43, 42)
+    if name == "no_diagonal_in_some_rows":
+        n, ia, ja, a = without(n, ia, ja, a, lambda r, c: (r == c) & (r % 7 == 0))
+    elif name == "empty_rows":
+        n, ia, ja, a = without(n, ia, ja, a, lambda r, c: r % 11 == 3)
+    else:
+        rows = np.repeat(np.arange(n), np.diff(ia))
+        a = np.where(ja == rows + 41, np.inf, a)
+    M, G = pv.Matrix.from_csr(n, ia, ja, a), pv.Matrix.from_csr(*with_extra_rows(n, ia, ja, a))
+    v = np.random.default_rng(10).standard_normal(n + 40)
+    v[5] = -0.0
+    got, want = M.matvec(v[:n]), G.matvec(v)[:n]
+    assert np.array_equal(got, want, equal_nan=True) and np.array_equal(np.signbit(got), np.signbit(want))
+    with pv.Instance(M) as e, pv.Instance(G) as f:
+        k = np.arange(12)
+        p = pv.Filter(1, 11, 0.0, 0.5, 6.0, 7.5, np.cos(0.7 * k) / (1.0 + 0.1 * k))
+        assert np.array_equal(e.chebav(p, v[:n]), f.chebav(p, v)[:n], equal_nan=True)
+    M.free()
+    G.free()
