@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(kThreads, R == 1 ? 5 : 1)
  * and HBM in about equal parts.  Per degree with 17 entries per row against
  * the CSR-stream kernel: 10^6 rows within +-5000 63 / 84 us (214 MB, 3.4
  * TB/s), within +-9000 (two blocks per SM in turn) 70 / 85, within +-500 55 /
- * 66; 5 10^5 rows 30 / 45, 10^5 8.4 / 12.7, 4 10^4 5.6 / 7.8. */
+ * 66; 5 10^5 rows 30 / 45, 10^5 8.4 / 12.7. */
 constexpr int kWinThreads = 1024;
 constexpr size_t kWinSmem = 232000; /* dynamic shared memory of a block, of 232448 bytes */
 
@@ -1324,7 +1324,10 @@ int stream_tune(pevsl_devcsr *A) {
   A->stream_r = force == 2 ? 2 : 1;
   const long n = A->nrows;
   if (force == 1 || force == 2 || n < 4096 || A->smask) return 0; /* the stencil form: other kernels */
-  if (window_prepare(A)) return PEVSL_ERR_CUDA;
+  /* the window is tried from 2^16 rows on: below, it gains 0-5% of a degree
+   * (7.2 -> 6.4 us at best, 22751 rows) and its preparation and timing cost
+   * the first filter 70-100 us; at 80323 rows 9.0 -> 7.4 us, at 61368 7.2 */
+  if ((force == 3 || n >= 65536) && window_prepare(A)) return PEVSL_ERR_CUDA;
   if (force == 3) {
     if (A->wdj) A->stream_r = 3;
     return 0;
