@@ -377,6 +377,64 @@ __global__ void __launch_bounds__(kThreads, R == 1 ? 5 : 1)
   stream_rows<R>(n, ia, ja, a, x, epi, blockIdx.x, prod);
 }
 
+/* ---------------------------------------------------------------- entries ahead
+ * Small matrices of rows that are not short: a degree is one wave, and its
+ * time the chain row pointer, entry, gather, sum.  The first two links do not
+ * depend on the degree before, so a warp has the entries of its 32 rows (up
+ * to 640 at a time) in registers before it waits for that one; blocks of four
+ * warps reach more SMs.  The products are those of k_csr_stream, added in the
+ * same order.  The loads before the wait are plain ones: the compiler may move
+ * those of the read-only path behind it.  Per filter degree, k_csr_stream /
+ * this one: 20000 rows of 19 entries 6.1 / 4.9 us, 30000 of 17 5.8 / 4.05, 40000
+ * of 9 4.8 / 3.7 and of 17 6.9 / 5.2, 50000 of 13 5.0 / 4.7. */
+constexpr int kAheadThreads = 128, kAheadLoads = 20;
+constexpr long kAheadRows = 65536, kAheadEntries = 800000;
+
+template <class Epi>
+__global__ void __launch_bounds__(kAheadThreads)
+    k_csr_ahead(int n, const int *ia, const int *ja, const double *a,
+                const double *__restrict__ x, Epi epi) {
+  constexpr int CH = 32 * kAheadLoads;
+  __shared__ double prod[kAheadThreads / 32][CH];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int r0 = (int)(blockIdx.x * (unsigned)kAheadThreads) + 32 * w, row = r0 + lane;
+  const int nr = n - r0 < 32 ? n - r0 : 32; /* <= 0: no rows */
+  int rs = 0, re = 0, col[kAheadLoads];
+  double val[kAheadLoads];
+  if (lane < nr) {
+    rs = ia[row];
+    re = ia[row + 1];
+  }
+  const int base = nr > 0 ? ia[r0] : 0, len = nr > 0 ? ia[r0 + nr] - base : 0;
+  auto fetch = [&](int c0) {
+#pragma unroll
+    for (int q = 0; q < kAheadLoads; q++) {
+      const int t = c0 + q * 32 + lane;
+      col[q] = t < len ? ja[base + t] : -1;
+      val[q] = t < len ? a[base + t] : 0.0;
+    }
+  };
+  fetch(0);
+  rs -= base;
+  re -= base;
+  pdl_wait_then_release();
+  if (nr <= 0) return; /* the whole warp */
+  typename Epi::Pre pre;
+  if (lane < nr) pre = epi.pre(row);
+  double acc = 0.0, *pw = prod[w];
+  for (int c0 = 0; c0 < len; c0 += CH) {
+    if (c0) fetch(c0);
+#pragma unroll
+    for (int q = 0; q < kAheadLoads; q++)
+      pw[q * 32 + lane] = mul_rn(val[q], col[q] >= 0 ? __ldg(x + col[q]) : 0.0);
+    __syncwarp();
+    const int lo = rs > c0 ? rs : c0, hi = re < c0 + CH ? re : c0 + CH;
+    for (int t = lo; t < hi; t++) acc = add_rn(acc, pw[t - c0]);
+    __syncwarp();
+  }
+  if (lane < nr) epi(row, acc, pre);
+}
+
 /* ---------------------------------------------------------------- windowed CSR
  * Scattered columns within a band: a gather that touches 32 lines takes 32
  * cycles of the L1 pipeline (the CSR-stream kernel ran at 90% of it on a
@@ -1320,10 +1378,18 @@ static int window_prepare(pevsl_devcsr *A) {
 int stream_tune(pevsl_devcsr *A) {
   if (!A || A->stream_r) return 0;
   const char *e = getenv("PEVSL_B200_STREAM_R");
-  const int force = e && atoi(e) >= 1 && atoi(e) <= 3 ? atoi(e) : 0;
+  const int force = e && atoi(e) >= 1 && atoi(e) <= 4 ? atoi(e) : 0;
   A->stream_r = force == 2 ? 2 : 1;
   const long n = A->nrows;
   if (force == 1 || force == 2 || n < 4096 || A->smask) return 0; /* the stencil form: other kernels */
+  /* entries ahead: one wave of warps, whose registers hold their rows' entries.
+   * 64000 rows of 11 entries (704000) 6.1 -> 5.7 us, of 19 (1.2 10^6) 7.9 ->
+   * 8.8.  No timing: the first filter of a matrix is 80 us shorter. */
+  if (force == 4 ||
+      (!force && n < kAheadRows && A->nnz >= 8 * n && A->nnz <= kAheadEntries)) {
+    A->stream_r = 4;
+    return 0;
+  }
   /* the window is tried from 2^16 rows on: below, it gains 0-5% of a degree
    * (7.2 -> 6.4 us at best, 22751 rows) and its preparation and timing cost
    * the first filter 70-100 us; at 80323 rows 9.0 -> 7.4 us, at 61368 7.2 */
@@ -1473,6 +1539,11 @@ static void launch_stream(const pevsl_devcsr *A, const T *a, const T *x, const E
   if constexpr (sizeof(T) == 8) {
     if (use_window(A)) {
       launch_window(A, x, epi);
+      return;
+    }
+    if (A->stream_r == 4) {
+      launch_pdl_block(k_csr_ahead<Epi>, dim3((unsigned)((A->nrows + kAheadThreads - 1) / kAheadThreads)),
+                       kAheadThreads, 0, ctx().stream, A->nrows, A->ia, A->ja, a, x, epi);
       return;
     }
   }

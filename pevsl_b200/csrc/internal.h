@@ -54,7 +54,8 @@ typedef struct pevsl_devcsr {
   /* form of the CSR-stream kernels, 0 until tuned: 1 or 2 rows per lane, or
    * 3, the gathered vector's window in shared memory (with wdj = column -
    * 32 * (row / 32) as int16 and the rows of each block, wsplit[0..wblocks],
-   * on the device; wlen: the largest window) */
+   * on the device; wlen: the largest window); 4, its warps' entries loaded
+   * before they wait for the degree before */
   int stream_r;
   short *wdj;
   int *wsplit;
