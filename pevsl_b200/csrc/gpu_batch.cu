@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(kThreads, 4)
   for (int j = threadIdx.x; j < k; j += blockDim.x) wsh[j] = w[(size_t)s * ldw + j];
   __syncthreads();
   const long n = g.n[s], ldv = g.ld[s], stride = (long)g.nb[s] * blockDim.x;
-  const double *__restrict__ Vs = V.p[s];
+  const double *Vs = V.p[s];
   double *vs = v.p[s];
   double ss = 0.0;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += kSubRows * stride) {
@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(kThreads, 4)
 #pragma unroll
       for (int q = 0; q < kSubRows; q++)
 #pragma unroll
-        for (int u = 0; u < 8; u++) x[q][u] = __ldg(p[q] + (size_t)(j + u) * ldv);
+        for (int u = 0; u < 8; u++) x[q][u] = p[q][(size_t)(j + u) * ldv];
 #pragma unroll
       for (int q = 0; q < kSubRows; q++)
 #pragma unroll
@@ -333,8 +333,8 @@ __global__ void __launch_bounds__(kThreads, 4)
     for (; j + 3 < k; j += 4) {
 #pragma unroll
       for (int q = 0; q < kSubRows; q++) {
-        const double x0 = __ldg(p[q] + (size_t)j * ldv), x1 = __ldg(p[q] + (size_t)(j + 1) * ldv);
-        const double x2 = __ldg(p[q] + (size_t)(j + 2) * ldv), x3 = __ldg(p[q] + (size_t)(j + 3) * ldv);
+        const double x0 = p[q][(size_t)j * ldv], x1 = p[q][(size_t)(j + 1) * ldv];
+        const double x2 = p[q][(size_t)(j + 2) * ldv], x3 = p[q][(size_t)(j + 3) * ldv];
         acc[q].a0 = fma(x0, wsh[j], acc[q].a0);
         acc[q].a1 = fma(x1, wsh[j + 1], acc[q].a1);
         acc[q].a2 = fma(x2, wsh[j + 2], acc[q].a2);
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(kThreads, 4)
     }
     for (; j < k; j++)
 #pragma unroll
-      for (int q = 0; q < kSubRows; q++) acc[q].a0 = fma(__ldg(p[q] + (size_t)j * ldv), wsh[j], acc[q].a0);
+      for (int q = 0; q < kSubRows; q++) acc[q].a0 = fma(p[q][(size_t)j * ldv], wsh[j], acc[q].a0);
 #pragma unroll
     for (int q = 0; q < kSubRows; q++) {
       const long r = i + q * stride;

@@ -28,7 +28,14 @@ namespace pv {
  * synchronisation, and never again while the matrix lives.  Without the
  * attribute the wait returns at once.  (Loading the first entries of a row
  * before the wait as well took the one-vector kernel from 32 to 48
- * registers and measured slower.) */
+ * registers and measured slower.)
+ *
+ * Such a grid is resident while the one before it still writes, so what an
+ * earlier launch wrote is not read-only for its lifetime: vectors, partial
+ * sums and scalars are read after the wait, through plain pointers without
+ * __restrict__, never through the read-only path (__ldg, const __restrict__),
+ * whose loads the compiler may move across the wait.  That path is for what
+ * was written at set-up: matrix entries, masks, tables, weights. */
 __device__ __forceinline__ void pdl_wait_then_release() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

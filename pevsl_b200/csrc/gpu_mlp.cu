@@ -77,7 +77,7 @@ __device__ __forceinline__ void ldm4t(uint32_t r[4], uint32_t addr) {
 
 /* db[n] = sum_m dZ[m][n], rows in order, for the 32 columns from n0 on: the
  * block's warps stage 64 rows at a time and warp 0 adds them */
-__device__ __forceinline__ void colsum(int Bn, int N, int n0, const float *__restrict__ dZ, int ld,
+__device__ __forceinline__ void colsum(int Bn, int N, int n0, const float *dZ, int ld,
                                        float *__restrict__ db, float *sh) {
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, n = n0 + lane;
   float s = 0.f, next[16];
@@ -85,7 +85,7 @@ __device__ __forceinline__ void colsum(int Bn, int N, int n0, const float *__res
 #pragma unroll
     for (int q = 0; q < 16; q++) {
       const int m = t + wib * 16 + q;
-      next[q] = m < Bn && n < N ? __ldg(dZ + (size_t)m * ld + n) : 0.f;
+      next[q] = m < Bn && n < N ? dZ[(size_t)m * ld + n] : 0.f;
     }
   };
   fetch(0);
@@ -122,10 +122,10 @@ __device__ __forceinline__ void colsum(int Bn, int N, int n0, const float *__res
  * round trip per k step).  The k steps come in the same order: the same bits. */
 template <bool TA, bool TB, int EPI>
 __global__ void __launch_bounds__(128)
-    k_gemm_bf16(int M, int N, int K, const bf16 *__restrict__ A, int lda,
+    k_gemm_bf16(int M, int N, int K, const bf16 *A, int lda,
                 const bf16 *__restrict__ B, int ldb, float *__restrict__ C, int ldc,
                 const float *__restrict__ bias, bf16 *__restrict__ act, int ldact,
-                const float *__restrict__ zp, int ldzp, float *__restrict__ db) {
+                const float *zp, int ldzp, float *__restrict__ db) {
   /* a tile's rows: k along them (32 rows of kGKC + 8) or across (kGKC rows of
    * 32 + 8); the padding makes the eight rows of an ldmatrix hit eight banks */
   constexpr int LDK = kGKC + 8, LDT = kGT + 8;
@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(128)
 /* dY = 2 (Y - T) / (B * nout) on columns < nout (0 elsewhere), bf16 copy,
  * and the mean squared error: per-block sums, the last block adds them in
  * block order */
-__global__ void k_mse(int Bn, int ld, int nout, const float *__restrict__ Y,
+__global__ void k_mse(int Bn, int ld, int nout, const float *Y,
                       const float *__restrict__ T, int ldt, float *__restrict__ dY,
                       bf16 *__restrict__ dYh, double *partials, unsigned *counter, float *loss) {
   __shared__ double sh[256];
@@ -264,7 +264,7 @@ __global__ void k_mse(int Bn, int ld, int nout, const float *__restrict__ Y,
 
 /* Adam (Kingma & Ba, 2015) with bias correction on FP32 master weights;
  * entries with mask 0 (padding) stay 0 */
-__global__ void k_adam(long np, float *__restrict__ p, const float *__restrict__ g,
+__global__ void k_adam(long np, float *__restrict__ p, const float *g,
                        float *__restrict__ m1, float *__restrict__ m2, const uint8_t *__restrict__ mask,
                        bf16 *__restrict__ ph, float lr, float b1, float b2, float eps, float c1,
                        float c2) {
@@ -292,7 +292,7 @@ __global__ void k_to_bf16(long n, const float *__restrict__ x, bf16 *__restrict_
 }
 
 /* X [B][ld] (bf16, zero padding) from a row-major FP32 block [B][nin] */
-__global__ void k_pack_input(int Bn, int nin, int ld, const float *__restrict__ x, bf16 *__restrict__ xh) {
+__global__ void k_pack_input(int Bn, int nin, int ld, const float *x, bf16 *__restrict__ xh) {
   pdl_wait_then_release();
   const long tot = (long)Bn * ld;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < tot; i += (long)gridDim.x * blockDim.x) {

@@ -283,7 +283,7 @@ struct EntriesPacked {
 
 /* R == 1 for the packed accessor: the column offsets are relative to the
  * warp's one 32-row group */
-template <int R, class T, class Epi, bool NC, class Ent>
+template <int R, class T, class Epi, class Ent>
 __device__ __forceinline__ void stream_rows_e(int n, const int *__restrict__ ia, const Ent &ent,
                                               const T *x, const Epi &epi, long rblk,
                                               T (*prod)[kStreamChunk * R]) {
@@ -295,7 +295,9 @@ __device__ __forceinline__ void stream_rows_e(int n, const int *__restrict__ ia,
   const int nr = n - r0 < 32 * R ? n - r0 : 32 * R;
   typename Epi::Pre pre[R];
   int rs[R], re[R];
-  /* the matrix is read-only for every launch: the non-coherent path */
+  /* the matrix is read-only while it lives: the non-coherent path.  x is not:
+   * the launch before this one, or other blocks of this one (the persistent
+   * filter), wrote it */
 #pragma unroll
   for (int j = 0; j < R; j++) {
     const int row = r0 + lane + 32 * j;
@@ -326,9 +328,7 @@ __device__ __forceinline__ void stream_rows_e(int n, const int *__restrict__ ia,
     }
 #pragma unroll
     for (int q = 0; q < PL; q++) {
-      /* NC: x is read-only for the launch (non-coherent path); otherwise it
-       * was written earlier in the same launch by other blocks */
-      const T xv = col[q] >= 0 ? (NC ? __ldg(x + col[q]) : x[col[q]]) : T(0);
+      const T xv = col[q] >= 0 ? x[col[q]] : T(0);
       pw[q * 32 + lane] = mul_rn(val[q], xv);
     }
     __syncwarp();
@@ -345,12 +345,12 @@ __device__ __forceinline__ void stream_rows_e(int n, const int *__restrict__ ia,
     if (lane + 32 * j < nr) epi(r0 + lane + 32 * j, acc[j], pre[j]);
 }
 
-template <int R, class T, class Epi, bool NC = true>
+template <int R, class T, class Epi>
 __device__ __forceinline__ void stream_rows(int n, const int *__restrict__ ia,
                                             const int *__restrict__ ja, const T *__restrict__ a,
                                             const T *x, const Epi &epi, long rblk,
                                             T (*prod)[kStreamChunk * R]) {
-  stream_rows_e<R, T, Epi, NC>(n, ia, EntriesCSR<T>{ja, a}, x, epi, rblk, prod);
+  stream_rows_e<R, T, Epi>(n, ia, EntriesCSR<T>{ja, a}, x, epi, rblk, prod);
 }
 
 /* the packed form: the block stages the value table in shared memory */
@@ -358,20 +358,20 @@ template <class T, class Epi>
 __global__ void __launch_bounds__(kThreads, 5)
     k_csr_stream_packed(int n, const int *__restrict__ ia, const short *__restrict__ dj,
                         const unsigned char *__restrict__ vi, const T *__restrict__ vtab, int nv,
-                        const T *__restrict__ x, Epi epi) {
+                        const T *x, Epi epi) {
   __shared__ T prod[kThreads / 32][kStreamChunk];
   __shared__ T vt[256];
   for (int i = threadIdx.x; i < nv; i += blockDim.x) vt[i] = vtab[i];
   __syncthreads();
   pdl_wait_then_release();
-  stream_rows_e<1, T, Epi, true>(n, ia, EntriesPacked<T>{dj, vi, vt}, x, epi, blockIdx.x, prod);
+  stream_rows_e<1, T, Epi>(n, ia, EntriesPacked<T>{dj, vi, vt}, x, epi, blockIdx.x, prod);
 }
 
 /* R = 1 fits 48 registers (5 blocks per SM) without spilling */
 template <int R, class T, class Epi>
 __global__ void __launch_bounds__(kThreads, R == 1 ? 5 : 1)
     k_csr_stream(int n, const int *__restrict__ ia, const int *__restrict__ ja,
-                 const T *__restrict__ a, const T *__restrict__ x, Epi epi) {
+                 const T *__restrict__ a, const T *x, Epi epi) {
   __shared__ T prod[kThreads / 32][kStreamChunk * R];
   pdl_wait_then_release();
   stream_rows<R>(n, ia, ja, a, x, epi, blockIdx.x, prod);
@@ -393,7 +393,7 @@ constexpr long kAheadRows = 65536, kAheadEntries = 800000;
 template <class Epi>
 __global__ void __launch_bounds__(kAheadThreads)
     k_csr_ahead(int n, const int *ia, const int *ja, const double *a,
-                const double *__restrict__ x, Epi epi) {
+                const double *x, Epi epi) {
   constexpr int CH = 32 * kAheadLoads;
   __shared__ double prod[kAheadThreads / 32][CH];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(kAheadThreads)
     if (c0) fetch(c0);
 #pragma unroll
     for (int q = 0; q < kAheadLoads; q++)
-      pw[q * 32 + lane] = mul_rn(val[q], col[q] >= 0 ? __ldg(x + col[q]) : 0.0);
+      pw[q * 32 + lane] = mul_rn(val[q], col[q] >= 0 ? x[col[q]] : 0.0);
     __syncwarp();
     const int lo = rs > c0 ? rs : c0, hi = re < c0 + CH ? re : c0 + CH;
     for (int t = lo; t < hi; t++) acc = add_rn(acc, pw[t - c0]);
@@ -459,7 +459,7 @@ template <int CH, class Epi>
 __global__ void __launch_bounds__(kWinThreads, 1)
     k_csr_window(int n, int kl, int ku, const int *__restrict__ split, const int *__restrict__ ia,
                  const short *__restrict__ dj, const double *__restrict__ a,
-                 const double *__restrict__ x, Epi epi) {
+                 const double *x, Epi epi) {
   constexpr int PL = CH / 32;
   extern __shared__ __align__(16) double wsm[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -472,7 +472,7 @@ __global__ void __launch_bounds__(kWinThreads, 1)
   double *win = wsm + (kWinThreads / 32) * CH + odd;
   pdl_wait_then_release();
   if (r0 >= r1) return;
-  if (threadIdx.x == 0 && odd) win[0] = __ldg(x + lo);
+  if (threadIdx.x == 0 && odd) win[0] = x[lo];
   for (int i = odd + 2 * (int)threadIdx.x; i < hi - lo; i += 2 * kWinThreads) {
     if (i + 1 < hi - lo)
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
@@ -480,7 +480,7 @@ __global__ void __launch_bounds__(kWinThreads, 1)
                    "l"(x + lo + i)
                    : "memory");
     else
-      win[i] = __ldg(x + lo + i);
+      win[i] = x[lo + i];
   }
   asm volatile("cp.async.commit_group;\n" ::: "memory");
   int col[PL];
@@ -632,8 +632,8 @@ __global__ void __launch_bounds__(kThreads, 4)
   __syncthreads();
   pdl_wait_then_release();
   const int e = (int)(blockIdx.x % (unsigned)b.nb);
-  stream_rows_e<1, T, Epi, true>(n0, ia0, EntriesPacked<T>{dj, vi, vt}, (const T *)b.epi[e].vk,
-                                 b.epi[e], (long)(blockIdx.x / (unsigned)b.nb), prod);
+  stream_rows_e<1, T, Epi>(n0, ia0, EntriesPacked<T>{dj, vi, vt}, (const T *)b.epi[e].vk,
+                           b.epi[e], (long)(blockIdx.x / (unsigned)b.nb), prod);
 }
 
 /* ---------------------------------------------------------------- stencil form
@@ -684,7 +684,7 @@ __device__ __forceinline__ unsigned stencil_mask(const Stencil &S, int row) {
  * OWN: x0 is the row's element, so the diagonal needs no load. */
 template <int K, bool OWN>
 __device__ __forceinline__ double stencil_dot(const Stencil &S, unsigned m,
-                                              const double *__restrict__ x, double x0) {
+                                              const double *x, double x0) {
   constexpr int B = K > 0 ? K : 8;
   double r = 0.0;
   for (int j0 = 0; j0 < (K > 0 ? 1 : S.k); j0 += B) {
@@ -692,7 +692,7 @@ __device__ __forceinline__ double stencil_dot(const Stencil &S, unsigned m,
 #pragma unroll
     for (int u = 0; u < B; u++) {
       xv[u] = 0.0;
-      if ((m >> (j0 + u)) & 1u) xv[u] = K > 0 && OWN && u == K / 2 ? x0 : __ldg(x + S.off[j0 + u]);
+      if ((m >> (j0 + u)) & 1u) xv[u] = K > 0 && OWN && u == K / 2 ? x0 : x[S.off[j0 + u]];
     }
 #pragma unroll
     for (int u = 0; u < B; u++)
@@ -704,7 +704,7 @@ __device__ __forceinline__ double stencil_dot(const Stencil &S, unsigned m,
 /* RPT rows per thread, kThreads apart */
 template <int RPT, int K, class M, class Epi>
 __global__ void __launch_bounds__(kThreads)
-    k_rows_stencil(int n, const __grid_constant__ Stencil S, const double *__restrict__ x, Epi epi) {
+    k_rows_stencil(int n, const __grid_constant__ Stencil S, const double *x, Epi epi) {
   const int r0 = (int)(blockIdx.x * (unsigned)(kThreads * RPT) + threadIdx.x);
   unsigned m[RPT];
 #pragma unroll
@@ -714,12 +714,15 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
   for (int q = 0; q < RPT; q++)
     if (r0 + q * kThreads < n) pre[q] = epi.pre(r0 + q * kThreads);
+  double r[RPT]; /* every row's loads before the first store, which may alias them */
 #pragma unroll
   for (int q = 0; q < RPT; q++) {
     const int row = r0 + q * kThreads;
-    if (row < n)
-      epi(row, stencil_dot<K, Epi::kOwn>(S, m[q], x + row, Epi::own(pre[q])), pre[q]);
+    if (row < n) r[q] = stencil_dot<K, Epi::kOwn>(S, m[q], x + row, Epi::own(pre[q]));
   }
+#pragma unroll
+  for (int q = 0; q < RPT; q++)
+    if (r0 + q * kThreads < n) epi(r0 + q * kThreads, r[q], pre[q]);
 }
 
 /* y_s = A x_s, vector s = blockIdx.y */
@@ -772,7 +775,7 @@ struct EpiChebY {
  * 2.88 us at 64 x 65 x 63. */
 template <int K>
 __global__ void __launch_bounds__(kThreads)
-    k_cheb_stencil(int n, const __grid_constant__ Stencil S, const double *__restrict__ vk,
+    k_cheb_stencil(int n, const __grid_constant__ Stencil S, const double *vk,
                    const double *vkm1, double *vkp1, double *y, double cc, double t, double mua,
                    double mub, double muk, int upd) {
   const int row = (int)(blockIdx.x * (unsigned)kThreads + threadIdx.x);
@@ -792,7 +795,7 @@ __global__ void __launch_bounds__(kThreads)
  * with one, 1500 x 1501 9.9 against 10.4; 126 x 127 x 125 10.6 against 10.2 */
 template <int K>
 __global__ void __launch_bounds__(kThreads, 8)
-    k_cheb_stencil2(int n, const __grid_constant__ Stencil S, const double *__restrict__ vk,
+    k_cheb_stencil2(int n, const __grid_constant__ Stencil S, const double *vk,
                     const double *vkm1, double *vkp1, double *y, double cc, double t, double mua,
                     double mub, double muk, int upd) {
   const int r0 = (int)(blockIdx.x * (unsigned)(2 * kThreads) + threadIdx.x);
@@ -811,12 +814,17 @@ __global__ void __launch_bounds__(kThreads, 8)
       yold[q] = upd ? y[row] : 0.0;
     }
   }
+  double r[2]; /* both rows' loads before the first store, which may alias them */
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    const int row = r0 + q * kThreads;
+    if (row < n) r[q] = stencil_dot<K, true>(S, m[q], vk + row, x[q]);
+  }
 #pragma unroll
   for (int q = 0; q < 2; q++) {
     const int row = r0 + q * kThreads;
     if (row < n) {
-      const double r = stencil_dot<K, true>(S, m[q], vk + row, x[q]);
-      const double w = __dsub_rn(__dmul_rn(__fma_rn(-cc, x[q], r), t), xm1[q]);
+      const double w = __dsub_rn(__dmul_rn(__fma_rn(-cc, x[q], r[q]), t), xm1[q]);
       vkp1[row] = w;
       if (upd) y[row] = __fma_rn(muk, w, __fma_rn(mub, x[q], __fma_rn(mua, xm1[q], yold[q])));
     }
@@ -935,13 +943,11 @@ __global__ void __launch_bounds__(kThreads, MINB)
       rotation<T>(E, j, &vk, &vkm1, &vkp1);
       if constexpr (sizeof(T) == 8) {
         EpiCheb epi{vk, vkm1, vkp1, (double *)E.acc, E.cc, t, mu0, muj, j == 1};
-        stream_rows<1, double, EpiCheb, false>(E.n, E.ia, E.ja, (const double *)E.a, vk, epi, rblk,
-                                               prod);
+        stream_rows<1>(E.n, E.ia, E.ja, (const double *)E.a, vk, epi, rblk, prod);
       } else {
         EpiCheb32 epi{vk, vkm1, vkp1, (float *)E.acc, j == E.deg ? E.y : nullptr, (float)E.cc,
                       (float)t, (float)mu0, (float)muj, j == 1};
-        stream_rows<1, float, EpiCheb32, false>(E.n, E.ia, E.ja, (const float *)E.a, vk, epi, rblk,
-                                                prod);
+        stream_rows<1>(E.n, E.ia, E.ja, (const float *)E.a, vk, epi, rblk, prod);
       }
     }
     if (j < maxdeg) {
@@ -1141,7 +1147,7 @@ __device__ __forceinline__ void kpm_finish(KpmAcc t, int L, int RB, double *part
 
 template <int K, class M>
 __global__ void __launch_bounds__(kThreads, kKpmPerSm)
-    k_kpm_stencil(int n, int L, const __grid_constant__ Stencil S, const double2 *__restrict__ Xk,
+    k_kpm_stencil(int n, int L, const __grid_constant__ Stencil S, const double2 *Xk,
                   const double2 *Xkm1, double2 *Xkp1, double ctr, double sc, double *part) {
   pdl_wait_then_release();
   const int RB = kThreads / L, rl = (int)threadIdx.x / L, l = (int)threadIdx.x % L;
@@ -1150,7 +1156,7 @@ __global__ void __launch_bounds__(kThreads, kKpmPerSm)
   for (int row = on ? (int)blockIdx.x * RB + rl : n; row < n; row += (int)gridDim.x * RB) {
     const size_t me = (size_t)row * L + l;
     const unsigned m = stencil_mask<M>(S, row);
-    const double2 x = __ldg(Xk + me);
+    const double2 x = Xk[me];
     const double2 xm1 = Xkm1 ? Xkm1[me] : make_double2(0.0, 0.0);
     double2 r = make_double2(0.0, 0.0);
     constexpr int B = K > 0 ? K : 4;
@@ -1161,7 +1167,7 @@ __global__ void __launch_bounds__(kThreads, kKpmPerSm)
       for (int u = 0; u < B; u++) {
         xv[u] = x;
         if (!(K > 0 && j0 + u == K / 2) && ((m >> (j0 + u)) & 1u))
-          xv[u] = __ldg(Xk + me + (long)S.off[j0 + u] * L);
+          xv[u] = Xk[me + (long)S.off[j0 + u] * L];
       }
 #pragma unroll
       for (int u = 0; u < B; u++)
@@ -1177,7 +1183,7 @@ __global__ void __launch_bounds__(kThreads, kKpmPerSm)
 
 __global__ void __launch_bounds__(kThreads, kKpmPerSm)
     k_kpm_csr(int n, int L, const int *__restrict__ ia, const int *__restrict__ ja,
-              const double *__restrict__ a, const double2 *__restrict__ Xk,
+              const double *__restrict__ a, const double2 *Xk,
               const double2 *Xkm1, double2 *Xkp1, double ctr, double sc, double *part) {
   pdl_wait_then_release();
   const int RB = kThreads / L, rl = (int)threadIdx.x / L, l = (int)threadIdx.x % L;
@@ -1187,7 +1193,7 @@ __global__ void __launch_bounds__(kThreads, kKpmPerSm)
     const size_t me = (size_t)row * L + l;
     const int e = __ldg(ia + row + 1);
     int j = __ldg(ia + row);
-    const double2 x = __ldg(Xk + me);
+    const double2 x = Xk[me];
     const double2 xm1 = Xkm1 ? Xkm1[me] : make_double2(0.0, 0.0);
     double2 r = make_double2(0.0, 0.0);
     for (; j < e; j += 4) {
@@ -1199,7 +1205,7 @@ __global__ void __launch_bounds__(kThreads, kKpmPerSm)
         xv[u] = x;
         if (j + u < e) {
           av[u] = __ldg(a + j + u);
-          xv[u] = __ldg(Xk + (size_t)__ldg(ja + j + u) * L + l);
+          xv[u] = Xk[(size_t)__ldg(ja + j + u) * L + l];
         }
       }
 #pragma unroll
@@ -1639,7 +1645,7 @@ template <int S, int EW = 0>
 __global__ void k_cheb_il_e(int n, const short *__restrict__ edj,
                             const unsigned char *__restrict__ evi, int ew_arg,
                             const double *__restrict__ vtab, int nv,
-                            const double *__restrict__ Xk, const double *Xkm1, double *Xkp1,
+                            const double *Xk, const double *Xkm1, double *Xkp1,
                             double *Y, double cc, double t, const double *__restrict__ mu0,
                             const double *__restrict__ muk, double mu0s, double muks, int ny,
                             int fresh);
@@ -1819,7 +1825,7 @@ template <int S>
 __global__ void __launch_bounds__(kThreads)
     k_cheb_il_p(int n, const int *__restrict__ ia, const short *__restrict__ dj,
                 const unsigned char *__restrict__ vi, const double *__restrict__ vtab, int nv,
-                const double *__restrict__ Xg, const double *__restrict__ Xk, const double *Xkm1,
+                const double *Xg, const double *Xk, const double *Xkm1,
                 double *Xkp1, double *Y, double cc, double t, const double *__restrict__ mu0,
                 const double *__restrict__ muk, int ny, int fresh) {
   __shared__ double vt[256];
@@ -1844,15 +1850,15 @@ __global__ void __launch_bounds__(kThreads)
     const int c2 = g0 + __ldg(dj + j + 2), c3 = g0 + __ldg(dj + j + 3);
     const double a0 = vt[__ldg(vi + j)], a1 = vt[__ldg(vi + j + 1)];
     const double a2 = vt[__ldg(vi + j + 2)], a3 = vt[__ldg(vi + j + 3)];
-    const double x0 = __ldg(Xg + (size_t)c0 * S + s), x1 = __ldg(Xg + (size_t)c1 * S + s);
-    const double x2 = __ldg(Xg + (size_t)c2 * S + s), x3 = __ldg(Xg + (size_t)c3 * S + s);
+    const double x0 = Xg[(size_t)c0 * S + s], x1 = Xg[(size_t)c1 * S + s];
+    const double x2 = Xg[(size_t)c2 * S + s], x3 = Xg[(size_t)c3 * S + s];
     r = __dadd_rn(r, __dmul_rn(a0, x0));
     r = __dadd_rn(r, __dmul_rn(a1, x1));
     r = __dadd_rn(r, __dmul_rn(a2, x2));
     r = __dadd_rn(r, __dmul_rn(a3, x3));
   }
   for (; j < e; j++)
-    r = __dadd_rn(r, __dmul_rn(vt[__ldg(vi + j)], __ldg(Xg + (size_t)(g0 + __ldg(dj + j)) * S + s)));
+    r = __dadd_rn(r, __dmul_rn(vt[__ldg(vi + j)], Xg[(size_t)(g0 + __ldg(dj + j)) * S + s]));
   double w = __dmul_rn(__fma_rn(-cc, x, r), t);
   if (Xkm1) w = __dsub_rn(w, xm1);
   Xkp1[me] = w;
@@ -1875,7 +1881,7 @@ __global__ void __launch_bounds__(kThreads)
 template <int B, int S, class Idx>
 __device__ __forceinline__ void il_entries(int j0, int ew, const short *__restrict__ edj,
                                            const unsigned char *__restrict__ evi, Idx b,
-                                           const double *__restrict__ Xk, int g0, int s,
+                                           const double *Xk, int g0, int s,
                                            const double *vt, double &r) {
   int dv[B];
   unsigned iv[B];
@@ -1891,7 +1897,7 @@ __device__ __forceinline__ void il_entries(int j0, int ew, const short *__restri
   }
 #pragma unroll
   for (int u = 0; u < B; u++)
-    xv[u] = dv[u] != INT16_MIN ? __ldg(Xk + ((size_t)(g0 + dv[u]) * S + s)) : 0.0;
+    xv[u] = dv[u] != INT16_MIN ? Xk[(size_t)(g0 + dv[u]) * S + s] : 0.0;
 #pragma unroll
   for (int u = 0; u < B; u++)
     if (dv[u] != INT16_MIN) r = __dadd_rn(r, __dmul_rn(vt[iv[u]], xv[u]));
@@ -1902,7 +1908,7 @@ __device__ __forceinline__ void il_entries(int j0, int ew, const short *__restri
 template <int S, int EW>
 __global__ void __launch_bounds__(kThreads, S == 1 ? 8 : 1)
     k_cheb_il_e(int n, const short *__restrict__ edj, const unsigned char *__restrict__ evi,
-                int ew_arg, const double *__restrict__ vtab, int nv, const double *__restrict__ Xk,
+                int ew_arg, const double *__restrict__ vtab, int nv, const double *Xk,
                 const double *Xkm1, double *Xkp1, double *Y, double cc, double t,
                 const double *__restrict__ mu0, const double *__restrict__ muk, double mu0s,
                 double muks, int ny, int fresh) {
@@ -1952,7 +1958,7 @@ __global__ void __launch_bounds__(kThreads, S == 1 ? 8 : 1)
 template <int B>
 __device__ __forceinline__ void il2_entries(int j0, int ew, const short *__restrict__ edj,
                                             const unsigned char *__restrict__ evi, unsigned b,
-                                            const double2 *__restrict__ Xk, int g0,
+                                            const double2 *Xk, int g0,
                                             const double *vt, double &r0, double &r1) {
   int dv[B];
   unsigned iv[B];
@@ -1968,7 +1974,7 @@ __device__ __forceinline__ void il2_entries(int j0, int ew, const short *__restr
   }
 #pragma unroll
   for (int u = 0; u < B; u++)
-    xv[u] = dv[u] != INT16_MIN ? __ldg(Xk + (g0 + dv[u])) : make_double2(0.0, 0.0);
+    xv[u] = dv[u] != INT16_MIN ? Xk[g0 + dv[u]] : make_double2(0.0, 0.0);
 #pragma unroll
   for (int u = 0; u < B; u++)
     if (dv[u] != INT16_MIN) {
@@ -1989,7 +1995,7 @@ template <int EW>
 __global__ void __launch_bounds__(kThreads, 5)
     k_cheb_il2_e(int n, const short *__restrict__ edj, const unsigned char *__restrict__ evi,
                  int ew_arg, const double *__restrict__ vtab, int nv,
-                 const double2 *__restrict__ Xk, const double2 *Xkm1, double2 *Xkp1, double2 *Y,
+                 const double2 *Xk, const double2 *Xkm1, double2 *Xkp1, double2 *Y,
                  double cc, double t, const double *__restrict__ mu0,
                  const double *__restrict__ muk, int ny, int fresh) {
   const int ew = EW > 0 ? EW : ew_arg;
@@ -2033,8 +2039,8 @@ __global__ void __launch_bounds__(kThreads, 5)
  * k_cheb_il_mid. */
 template <int L, int K, class M, bool GEN>
 __global__ void __launch_bounds__(kThreads)
-    k_cheb_il_stencil(int n, const __grid_constant__ Stencil S, const double2 *__restrict__ Xg,
-                      const double2 *__restrict__ Xk, const double2 *Xkm1, double2 *Xkp1,
+    k_cheb_il_stencil(int n, const __grid_constant__ Stencil S, const double2 *Xg,
+                      const double2 *Xk, const double2 *Xkm1, double2 *Xkp1,
                       double2 *Y, double cc, double t, const double *__restrict__ mu0,
                       const double *__restrict__ muk, int ny, int fresh) {
   const unsigned me = blockIdx.x * (unsigned)kThreads + threadIdx.x;
@@ -2056,7 +2062,7 @@ __global__ void __launch_bounds__(kThreads)
       if (K > 0 && !GEN && j0 + u == K / 2)
         xv[u] = x;
       else if ((m >> (j0 + u)) & 1u)
-        xv[u] = __ldg(xr + (long)S.off[j0 + u] * L);
+        xv[u] = xr[(long)S.off[j0 + u] * L];
     }
 #pragma unroll
     for (int u = 0; u < B; u++)
@@ -2099,7 +2105,7 @@ __global__ void __launch_bounds__(kThreads)
  * against 2.5). */
 template <int L, int K, int B, int MB>
 __global__ void __launch_bounds__(kThreads, MB)
-    k_cheb_il_mid(int n, const __grid_constant__ Stencil S, const double2 *__restrict__ Xk,
+    k_cheb_il_mid(int n, const __grid_constant__ Stencil S, const double2 *Xk,
                   const double2 *Xkm1, double2 *Xkp1, double2 *Y, double cc, double t,
                   const double *__restrict__ muk, int upd) {
   const unsigned me = blockIdx.x * (unsigned)kThreads + threadIdx.x;
@@ -2121,7 +2127,7 @@ __global__ void __launch_bounds__(kThreads, MB)
       if (j0 + u == K / 2)
         xv[u] = x;
       else if (j0 + u < K && ((m >> (j0 + u)) & 1u))
-        xv[u] = __ldg(xr + (long)S.off[j0 + u] * L);
+        xv[u] = xr[(long)S.off[j0 + u] * L];
     }
 #pragma unroll
     for (int u = 0; u < B; u++)
