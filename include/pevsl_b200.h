@@ -72,6 +72,13 @@ int pEVSL_B200_SetBarrierSpins(unsigned spins);
  * report clears the counter again. */
 int pEVSL_B200_SeedBarrierArrivals(unsigned count);
 
+/* Wait limit of the cluster launches of small problems, in microseconds: how
+ * long a block waits for its neighbours' values of one degree.  < 0 restores
+ * the default (2 s); with 0 every wait runs out at once (for tests).  When a
+ * wait runs out the launch ends with NaN in its result, and the call that
+ * launched it returns PEVSL_ERR_CUDA; the context stays usable. */
+int pEVSL_B200_SetClusterWait(long microseconds);
+
 /* The cross-group sum of a split KPM: pEVSL_Kpmdos with ngroups > 1 computes
  * the moments of its group's share of the random vectors (pEVSL_Part1d)
  * and then, in place of MPI_Allreduce on gl_comm (SRC/kpmdos.c:160-176),

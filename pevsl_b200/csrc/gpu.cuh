@@ -357,6 +357,9 @@ constexpr int kClusterMaxRows = 32768;
 bool cluster_filter_ok(const pevsl_devcsr *A, const pevsl_devcsr *B, bool fp32);
 /* the applications of ne jobs, all with B or all without */
 int cluster_filter(int ne, const ClusterJob *jobs, bool fp32);
+/* microseconds after which a block of a cluster launch stops waiting for its
+ * neighbours and the call fails: < 0 the default, 0 at once (for tests) */
+void set_cluster_wait(long us);
 
 /* ---------------------------------------------------------------- FP32 (mixed) */
 int csr_make_fp32(pevsl_devcsr *A); /* FP32 copy of the values, once */

@@ -22,8 +22,9 @@
  * so the degrees do not meet there: the values are sent with st.async, which
  * counts their bytes on the receiving block's mbarrier, and a block goes on
  * when its own have arrived (three windows instead of two keep a faster
- * neighbour from overwriting what is still read).  The waits are bounded; one
- * that runs out makes the call return PEVSL_ERR_CUDA.  Where some block would
+ * neighbour from overwriting what is still read).  A wait lasts at most a
+ * given time (set_cluster_wait); when one runs out its cluster gives up and
+ * the call returns PEVSL_ERR_CUDA.  Where some block would
  * send to one that it does not hear from (windows of a matrix without
  * symmetric structure), the cluster barrier ends each degree.
  *
@@ -112,20 +113,61 @@ __device__ __forceinline__ void cl_send(unsigned addr, float v, unsigned mbar) {
                : "memory");
 }
 
-/* wait for the phase of this parity, at most kClPolls polls */
-constexpr int kClPolls = 1 << 22;
-__device__ __forceinline__ bool cl_wait(unsigned mbar, unsigned parity) {
-  for (int i = 0; i < kClPolls; i++) {
-    unsigned ok;
+__device__ __forceinline__ unsigned long long cl_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)::"memory");
+  return t;
+}
+
+/* a poll for the phase of this parity; HINT: suspended for that many ns at
+ * most, 0: for a time that the hardware chooses */
+template <int HINT>
+__device__ __forceinline__ bool cl_poll(unsigned mbar, unsigned parity) {
+  unsigned ok;
+  if constexpr (HINT == 0)
     asm volatile(
         "{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
         "selp.u32 %0, 1, 0, p;\n}"
         : "=r"(ok)
         : "r"(mbar), "r"(parity)
         : "memory");
-    if (ok) return true;
-  }
+  else
+    asm volatile(
+        "{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n"
+        "selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(mbar), "r"(parity), "n"(HINT)
+        : "memory");
+  return ok != 0;
+}
+
+/* the word of this block that a block of the cluster sets when it gives up */
+__device__ __forceinline__ bool cl_gave_up(unsigned addr) {
+  unsigned v;
+  asm volatile("ld.relaxed.cluster.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v != 0;
+}
+
+/* the rest of a long wait, by the clock */
+__device__ __noinline__ bool cl_wait_long(unsigned mbar, unsigned parity, unsigned long long limit,
+                                          unsigned gave_up) {
+  const unsigned long long t0 = cl_ns();
+  while (!cl_gave_up(gave_up) && cl_ns() - t0 < limit)
+    if (cl_poll<10000>(mbar, parity)) return true;
   return false;
+}
+
+/* wait for the phase of this parity: false when `limit` ns have passed (at
+ * once when it is 0) or another block gave up.  A few polls come before the
+ * clock is looked at, and the rest is out of the way: in the loop it costs
+ * the products 3%. */
+constexpr int kClPolls = 16;
+__device__ __forceinline__ bool cl_wait(unsigned mbar, unsigned parity, unsigned long long limit,
+                                        unsigned gave_up) {
+#pragma unroll 1
+  for (int i = limit ? kClPolls : 0; i > 0; i--)
+    if (cl_poll<0>(mbar, parity)) return true;
+  return cl_wait_long(mbar, parity, limit, gave_up);
 }
 
 /* one matrix of a job, as the kernel reads it */
@@ -217,10 +259,12 @@ __device__ __forceinline__ void cl_load(ClRow<T, CW> &row, const ClEnt<T> &e, co
  * slot; Rp: at least R, a multiple of 32. */
 template <class T, int RPT, int CW, bool GEN>
 __global__ void __launch_bounds__(kClThreads, 1)
-    k_filter_cluster(const __grid_constant__ ClTable tab, int Z, int Rp, int nwin, unsigned *err) {
+    k_filter_cluster(const __grid_constant__ ClTable tab, int Z, int Rp, int nwin, unsigned *err,
+                     unsigned long long limit) {
   extern __shared__ __align__(16) unsigned char cl_smem[];
   __shared__ int s_lo, s_hi, s_tlo[kClMaxBlocks], s_thi[kClMaxBlocks], s_async;
   __shared__ __align__(8) unsigned long long s_mbar[3];
+  __shared__ unsigned s_gave_up;
   const unsigned nc = cl_size(), rank = cl_rank();
   const ClJob &J = tab.job[blockIdx.x / nc];
   const int n = J.n, R = (n + (int)nc - 1) / (int)nc, r0 = (int)rank * R;
@@ -254,6 +298,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
                    : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     s_async = nwin == 3;
+    s_gave_up = 0;
   }
   __syncthreads();
   /* the window: every column the block's rows touch, and the rows */
@@ -348,6 +393,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
    * reads.  False when a wait ran out. */
   const unsigned rx = (unsigned)(hi - lo - nloc) * (unsigned)sizeof(T);
   unsigned parity = 0; /* bit i: of window i's mbarrier */
+  const unsigned gave_up = (unsigned)__cvta_generic_to_shared(&s_gave_up);
   auto arm = [&]() {
     if (async && rx && threadIdx.x == 0)
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
@@ -363,7 +409,8 @@ __global__ void __launch_bounds__(kClThreads, 1)
     }
     bool ok = true;
     if (rx) {
-      ok = cl_wait((unsigned)__cvta_generic_to_shared(&s_mbar[cur]), (parity >> cur) & 1u);
+      ok = cl_wait((unsigned)__cvta_generic_to_shared(&s_mbar[cur]), (parity >> cur) & 1u, limit,
+                   gave_up);
       parity ^= 1u << cur;
     }
     return !__syncthreads_or(!ok);
@@ -440,11 +487,21 @@ __global__ void __launch_bounds__(kClThreads, 1)
   if (async) {
     /* no block ends while another may still write its windows, nor writes a
      * result over an input that another has yet to read */
-    if (!ok) {
-      if (threadIdx.x == 0) atomicExch_system(err, 1u);
-      __nanosleep(200000); /* stores still under way */
-    }
+    if (!ok && threadIdx.x < nc)
+      asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(cl_map(gave_up, threadIdx.x)),
+                   "r"(1)
+                   : "memory");
     cl_barrier();
+    if (cl_gave_up(gave_up)) {
+      /* the same in every block.  Nobody sends any more; values sent before
+       * take a microsecond or two, and nobody waits for them: give them 100 */
+      if (threadIdx.x == 0) {
+        if (rank == 0) atomicExch_system(err, 1u);
+        for (const unsigned long long t0 = cl_ns(); cl_ns() - t0 < 100000;) __nanosleep(1000);
+      }
+      ok = false;
+      cl_barrier();
+    }
   }
 #pragma unroll
   for (int q = 0; q < RPT; q++) {
@@ -589,6 +646,14 @@ bool cluster_filter_ok(const pevsl_devcsr *A, const pevsl_devcsr *B, bool fp32) 
   return B || fp32 || !A->smask || s.rpt <= 2;
 }
 
+/* two seconds: a step's wait is for neighbours that run at the same time */
+constexpr unsigned long long kClWaitNs = 2000000000ull;
+static unsigned long long g_cluster_wait = kClWaitNs;
+
+void set_cluster_wait(long us) {
+  g_cluster_wait = us < 0 ? kClWaitNs : 1000ull * (unsigned long long)us;
+}
+
 int cluster_filter(int ne, const ClusterJob *jobs, bool fp32) {
   if (ne <= 0) return 0;
   const bool gen = jobs[0].B != nullptr;
@@ -619,7 +684,8 @@ int cluster_filter(int ne, const ClusterJob *jobs, bool fp32) {
     cudaLaunchConfig_t cfg;
     cl_config(s, nb, &cfg, &at);
     unsigned *err = ctx().cl_err;
-    void *args[] = {(void *)&tab, (void *)&s.Z, (void *)&s.Rp, (void *)&s.nwin, (void *)&err};
+    void *args[] = {(void *)&tab,    (void *)&s.Z, (void *)&s.Rp,
+                    (void *)&s.nwin, (void *)&err, (void *)&g_cluster_wait};
     if (fail(cudaLaunchKernelExC(&cfg, k, args), "filter_cluster")) return PEVSL_ERR_CUDA;
     if (launched("filter_cluster")) return PEVSL_ERR_CUDA;
   }

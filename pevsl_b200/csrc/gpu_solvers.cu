@@ -1952,6 +1952,11 @@ int pEVSL_B200_SetBarrierSpins(unsigned spins) {
 
 int pEVSL_B200_SeedBarrierArrivals(unsigned count) { return seed_barrier_arrivals(count); }
 
+int pEVSL_B200_SetClusterWait(long microseconds) {
+  set_cluster_wait(microseconds);
+  return 0;
+}
+
 /* Filtered Lanczos in lockstep (pEVSL_ChebLanNr, SRC/cheblanNr.c:54-448) for
  * ns <= kMaxEntries slices, which may belong to different problems (each
  * entry carries its instance, matrix, length and start vector).  Every
