@@ -1132,7 +1132,11 @@ static void host_parallel(size_t m, bool worth, F f) {
 /* Lanczos steps of S <= kMaxBatch independent runs in lockstep, queued
  * without a host synchronisation: alpha and beta stay on the device, where
  * the next step reads them, and the host reads all steps at once.  (A
- * breakdown therefore shows only then; what was queued past it is dropped.)
+ * breakdown therefore shows only then; what was queued past it is dropped.
+ * A user operator, whose call waits for the GPU anyway, must not see such
+ * steps' vectors, which were divided by nearly nothing: with one, a step is
+ * queued only when the one before has been looked at.)  The callers count
+ * the products of the built-in operator, those of the dropped steps apart.
  * Run s has its basis at V[s] (leading dimension ld).  Per run the kernels
  * and their decompositions are those of a single run, so each run's values
  * are the bits it has alone. */
@@ -1181,7 +1185,6 @@ static int lan_step(LanRuns &R, int k, bool prev) {
   int *flag = ctx().gflag;
   int st = 0;
   if (pevsl_devcsr *A = pevsl_builtin_A(R.pevsl)) {
-    R.pevsl->stats->n_mvA += (size_t)S;
     st = spmv_batch(A, S, v, vn);
   } else {
     for (int s = 0; s < S && !st; s++) st = apply_A(R.pevsl, v.p[s], vn.p[s]);
@@ -1283,6 +1286,7 @@ static int landos_lockstep(pevsl_Data *pevsl, int S, int maxit, double *V, long 
       if (beta * nwn < orthTol * wn) *broke = true;
     }
   }
+  if (!st && !*broke) pevsl->stats->n_mvA += (size_t)maxit * (size_t)S;
   return st;
 }
 
@@ -1296,10 +1300,11 @@ int pEVSL_LanDosG(pevsl_Data *pevsl, const int nvec, int msteps, int npts, doubl
   int vec_start = 0, vec_end = nvec;
   if (ngroups > 1) pEVSL_Part1d(nvec, ngroups, &groupid, &vec_start, &vec_end, 1);
   /* runs in lockstep: up to kMaxBatch, their bases within 4 GB, the groups
-   * about equal; one at a time with B-solves */
+   * about equal; one at a time with B-solves or a user operator */
   const double basis = 8.0 * (double)ld * (maxit + 1);
   const int nrun = PEVSL_MAX(vec_end - vec_start, 0);
-  int lock = pevsl->ifGenEv ? 1 : (int)PEVSL_MIN((double)kMaxBatch, PEVSL_MAX(1.0, 4e9 / basis));
+  const bool ahead = !pevsl->ifGenEv && pevsl_builtin_A(pevsl);
+  int lock = !ahead ? 1 : (int)PEVSL_MIN((double)kMaxBatch, PEVSL_MAX(1.0, 4e9 / basis));
   const int ngr = PEVSL_MAX(1, (nrun + lock - 1) / lock);
   lock = PEVSL_MAX(1, (nrun + ngr - 1) / ngr);
   double *V = (double *)ws(WS_BASIS, sizeof(double) * (size_t)ld * (size_t)(maxit + 1) * (size_t)lock);
@@ -1329,7 +1334,7 @@ int pEVSL_LanDosG(pevsl_Data *pevsl, const int nvec, int msteps, int npts, doubl
       return next < drawn ? vcopy(vinit + (size_t)next++ * ld, v, n) : pevsl_rand_vector_dev(v, (int)n);
     };
     bool broke = true;
-    if (!st && !pevsl->ifGenEv) st = landos_lockstep(pevsl, S, maxit, V, ld, vinit, n, dT, eT, &broke);
+    if (!st && ahead) st = landos_lockstep(pevsl, S, maxit, V, ld, vinit, n, dT, eT, &broke);
     double *one = vinit + (size_t)lock * ld;
     for (int s = 0; s < S && broke && !st; s++) {
       st = draw(one);
@@ -1495,12 +1500,12 @@ int pEVSL_LanTrbounds(pevsl_Data *pevsl, int lanm, int maxit, double tol, pevsl_
     /* the steps of this cycle, queued at once; then their alpha and beta are
      * read, and after a breakdown the steps past it are queued again */
     bool prev = k > 0;
+    const bool ahead = pevsl_builtin_A(pevsl) != nullptr;
     const int kend = PEVSL_MIN(lanm, k + maxit - it);
     while (k < kend && !st) {
-      const int k0 = k;
+      const int k0 = k, m = ahead ? kend - k0 : 1;
       if (prev) st = memcpy_async(R.beta(k0 - 1), &beta, sizeof(double));
-      for (int j = k0; j < kend && !st; j++) st = lan_step(R, j, j > k0 || prev);
-      const int m = kend - k0;
+      for (int j = k0; j < k0 + m && !st; j++) st = lan_step(R, j, j > k0 || prev);
       if (!st) st = memcpy_async(hist.data(), R.alpha(k0), sizeof(double) * 2 * (size_t)m);
       if (!st) st = sync();
       bool broke = false;
@@ -1509,6 +1514,7 @@ int pEVSL_LanTrbounds(pevsl_Data *pevsl, int lanm, int maxit, double tol, pevsl_
         beta = hist[2 * (size_t)j + 1];
         k++;
         it++;
+        if (ahead) pevsl->stats->n_mvA++;
         T[(k - 1) * L + (k - 1)] = alpha;
         wn += fabs(alpha) + 2.0 * beta;
         nwn += 3;
