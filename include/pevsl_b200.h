@@ -72,6 +72,13 @@ int pEVSL_B200_SetBarrierSpins(unsigned spins);
  * report clears the counter again. */
 int pEVSL_B200_SeedBarrierArrivals(unsigned count);
 
+/* The largest workspace that the library allocates, in bytes (0: no limit,
+ * the default): a larger one is refused as if there were no memory for it.
+ * Calls that can do with less then take less, the others return
+ * PEVSL_ERR_NOMEM.  Workspaces already held are not looked at
+ * (pEVSL_B200_ReleaseWorkspace gives them back). */
+int pEVSL_B200_SetWorkspaceLimit(size_t bytes);
+
 /* Wait limit of the cluster launches of small problems, in microseconds: how
  * long a block waits for its neighbours' values of one degree.  < 0 restores
  * the default (2 s); with 0 every wait runs out at once (for tests).  When a

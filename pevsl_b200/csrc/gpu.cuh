@@ -121,6 +121,10 @@ int launched(const char *what); /* count a launch and check for errors */
 void l2_window(const void *base, size_t bytes);
 int sync();
 void *ws(int slot, size_t bytes);
+/* the same without a report when there is no memory (what the slot held is
+ * gone then); ws_free gives a slot back */
+void *ws_try(int slot, size_t bytes);
+void ws_free(int slot);
 /* device memory of matrices, in order on the context stream, from a pool that
  * keeps up to 64 MB of freed memory (pEVSL_B200_ReleaseWorkspace gives it
  * back); NULL when there is none */

@@ -11,6 +11,7 @@
  */
 #include <cuda_runtime.h>
 #include <math.h>
+#include <stdint.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
@@ -151,7 +152,9 @@ int sync() {
   return 0;
 }
 
-void *ws(int slot, size_t bytes) {
+static size_t g_ws_limit = SIZE_MAX;
+
+void *ws_try(int slot, size_t bytes) {
   if (ensure()) return nullptr;
   if (bytes == 0) bytes = 256;
   if (g_ctx.wsz[slot] >= bytes) return g_ctx.ws[slot];
@@ -161,17 +164,35 @@ void *ws(int slot, size_t bytes) {
     g_ctx.ws[slot] = nullptr;
     g_ctx.wsz[slot] = 0;
   }
+  if (bytes > g_ws_limit) return nullptr;
   void *p = nullptr;
   if (cudaMalloc(&p, bytes) != cudaSuccess) {
     /* once more without the memory that the pool keeps */
     cudaGetLastError();
     cudaStreamSynchronize(g_ctx.stream);
     if (g_ctx.pool) cudaMemPoolTrimTo(g_ctx.pool, 0);
-    if (fail(cudaMalloc(&p, bytes), "cudaMalloc workspace")) return nullptr;
+    if (cudaMalloc(&p, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
   }
   g_ctx.ws[slot] = p;
   g_ctx.wsz[slot] = bytes;
   return p;
+}
+
+void *ws(int slot, size_t bytes) {
+  void *p = ws_try(slot, bytes);
+  if (!p && g_ctx.ready) fail(cudaErrorMemoryAllocation, "workspace");
+  return p;
+}
+
+void ws_free(int slot) {
+  if (!g_ctx.ws[slot]) return;
+  cudaStreamSynchronize(g_ctx.stream);
+  cudaFree(g_ctx.ws[slot]);
+  g_ctx.ws[slot] = nullptr;
+  g_ctx.wsz[slot] = 0;
 }
 
 /* The blocks of a matrix.  cudaMalloc and cudaFree of the 660 KB of an 8000-row
@@ -582,6 +603,11 @@ void pEVSL_B200_ReleaseWorkspace(void) {
     g_ctx.wsz[i] = 0;
   }
   if (g_ctx.pool) cudaMemPoolTrimTo(g_ctx.pool, 0);
+}
+
+int pEVSL_B200_SetWorkspaceLimit(size_t bytes) {
+  g_ws_limit = bytes ? bytes : SIZE_MAX;
+  return 0;
 }
 
 int pEVSL_B200_Info(char *buf, int len) {

@@ -1290,6 +1290,8 @@ static int landos_lockstep(pevsl_Data *pevsl, int S, int maxit, double *V, long 
   return st;
 }
 
+static constexpr size_t kKeepBasis = (size_t)1 << 30;
+
 int pEVSL_LanDosG(pevsl_Data *pevsl, const int nvec, int msteps, int npts, double *xdos,
                   double *ydos, double *neig, double *intv, int ngroups, int groupid,
                   MPI_Comm gl_comm) {
@@ -1299,16 +1301,25 @@ int pEVSL_LanDosG(pevsl_Data *pevsl, const int nvec, int msteps, int npts, doubl
   const int maxit = msteps < pevsl->N ? msteps : pevsl->N;
   int vec_start = 0, vec_end = nvec;
   if (ngroups > 1) pEVSL_Part1d(nvec, ngroups, &groupid, &vec_start, &vec_end, 1);
-  /* runs in lockstep: up to kMaxBatch, their bases within 4 GB, the groups
-   * about equal; one at a time with B-solves or a user operator */
-  const double basis = 8.0 * (double)ld * (maxit + 1);
+  /* runs in lockstep: up to kMaxBatch, their bases within 4 GB and their
+   * eigenvectors of T within 256 MB of host memory, the groups about equal;
+   * fewer where there is no memory for as many; one at a time with B-solves
+   * or a user operator */
+  const double basis = 8.0 * (double)ld * (maxit + 1), evec = 8.0 * maxit * (double)maxit;
   const int nrun = PEVSL_MAX(vec_end - vec_start, 0);
   const bool ahead = !pevsl->ifGenEv && pevsl_builtin_A(pevsl);
-  int lock = !ahead ? 1 : (int)PEVSL_MIN((double)kMaxBatch, PEVSL_MAX(1.0, 4e9 / basis));
-  const int ngr = PEVSL_MAX(1, (nrun + lock - 1) / lock);
-  lock = PEVSL_MAX(1, (nrun + ngr - 1) / ngr);
-  double *V = (double *)ws(WS_BASIS, sizeof(double) * (size_t)ld * (size_t)(maxit + 1) * (size_t)lock);
-  double *vinit = (double *)ws(WS_LANV, sizeof(double) * (size_t)ld * (size_t)(lock + 1));
+  int lock = !ahead ? 1 : (int)PEVSL_MIN((double)kMaxBatch, PEVSL_MAX(1.0, PEVSL_MIN(4e9 / basis, 256e6 / evec)));
+  const size_t held = ctx().wsz[WS_BASIS];
+  double *V = nullptr, *vinit = nullptr;
+  for (;; lock /= 2) {
+    const int ngr = PEVSL_MAX(1, (nrun + lock - 1) / lock);
+    lock = PEVSL_MAX(1, (nrun + ngr - 1) / ngr);
+    const size_t vb = sizeof(double) * (size_t)ld * (size_t)(maxit + 1) * (size_t)lock;
+    const size_t ib = sizeof(double) * (size_t)ld * (size_t)(lock + 1);
+    V = (double *)(lock > 1 ? ws_try(WS_BASIS, vb) : ws(WS_BASIS, vb));
+    vinit = !V ? nullptr : (double *)(lock > 1 ? ws_try(WS_LANV, ib) : ws(WS_LANV, ib));
+    if (vinit || lock == 1) break;
+  }
   double *y = (double *)calloc((size_t)npts, sizeof(double));
   int *ind = (int *)malloc(sizeof(int) * (size_t)npts);
   double *dT = (double *)malloc(sizeof(double) * (size_t)maxit * (size_t)lock);
@@ -1386,6 +1397,9 @@ int pEVSL_LanDosG(pevsl_Data *pevsl, const int nvec, int msteps, int npts, doubl
   free(eT);
   free(EvalT);
   free(EvecT);
+  /* bases of several runs beyond 1 GB go back, unless the workspace was as
+   * large before */
+  if (lock > 1 && held < kKeepBasis && ctx().wsz[WS_BASIS] > kKeepBasis) ws_free(WS_BASIS);
   pevsl->stats->t_dos = pevsl_now() - t0;
   return st;
 }

@@ -1,0 +1,44 @@
+"""Calls with less workspace than they would like.
+
+The limit of pEVSL_B200_SetWorkspaceLimit refuses larger workspaces as a full
+GPU would, without filling one.
+"""
+import numpy as np
+import pytest
+
+import pevsl_b200 as pv
+from pevsl_b200.problems import laplacian
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def limit():
+    lib = pv.load()
+    lib.pEVSL_B200_ReleaseWorkspace()
+    yield lib.pEVSL_B200_SetWorkspaceLimit
+    lib.pEVSL_B200_SetWorkspaceLimit(0)
+    lib.pEVSL_B200_ReleaseWorkspace()
+    lib.pEVSL_B200_LastError()
+
+
+@pytest.mark.parametrize("bases", [1, 2, 5])
+def test_lanczos_dos_takes_fewer_runs_at_a_time(gpu, limit, bases):
+    """The same bits with memory for one, two or five bases, and an error
+    with less than one."""
+    M = pv.Matrix.from_csr(*laplacian(30, 31, 29))
+    nvec, msteps = 11, 25
+    one = 8 * ((M.n + 31) // 32 * 32) * (msteps + 1)
+    outs = []
+    with pv.Instance(M) as ev:
+        for bytes_ in (0, int((bases + 0.5) * one)):
+            ev.lib.pEVSL_B200_ReleaseWorkspace()
+            limit(bytes_)
+            pv.set_rng(pv.RNG_GAUSS, 11)
+            outs.append(ev.landos(nvec, msteps, 61, [0.5, 6.0, 0.0, 12.0]))
+        ev.lib.pEVSL_B200_ReleaseWorkspace()
+        limit(one // 2)
+        assert ev.landos(nvec, msteps, 61, [0.5, 6.0, 0.0, 12.0])[0] == pv.ERR_NOMEM
+    M.free()
+    assert outs[0][0] == outs[1][0] == 0
+    assert np.array_equal(outs[0][2], outs[1][2]) and outs[0][3] == outs[1][3]
