@@ -859,6 +859,8 @@ int pEVSL_B200_ChebAv(pevsl_Data *pevsl, pevsl_Polparams *pol, const double *v, 
 
 /* ================================================================ KPM DOS */
 
+static constexpr int kKpmChunk = 64;
+
 int pEVSL_Kpmdos(pevsl_Data *pevsl, int Mdeg, int damping, int nvec, double *intv, int ngroups,
                  int groupid, MPI_Comm gl_comm, double *mu, double *ecnt) {
   const double t0 = pevsl_now();
@@ -957,7 +959,10 @@ int pEVSL_Kpmdos(pevsl_Data *pevsl, int Mdeg, int damping, int nvec, double *int
       const int s = PEVSL_MIN(smax, vec_end - m0), ld = (s + 1) / 2 * 2;
       const size_t blk = (size_t)n * (size_t)ld, np = (size_t)kpm_blocks(A, s) * 2 * (size_t)ld;
       double *X = (double *)ws(WS_KPM, sizeof(double) * 2 * blk);
-      double *part = (double *)ws(WS_PART, sizeof(double) * np * (size_t)PEVSL_MAX(steps, 1));
+      /* the blocks' sums of up to kKpmChunk steps, then added up: 39 MB for 64
+       * vectors, however many moments */
+      const int chunk = PEVSL_MIN(PEVSL_MAX(steps, 1), kKpmChunk);
+      double *part = (double *)ws(WS_PART, sizeof(double) * np * (size_t)chunk);
       double *mom = (double *)ws(WS_MOM, sizeof(double) * 4 * (size_t)ld * (size_t)PEVSL_MAX(steps, 1));
       double *nrm2 = (double *)ws(WS_SMALL, sizeof(double) * 64);
       if (!X || !part || !mom || !nrm2) {
@@ -973,10 +978,13 @@ int pEVSL_Kpmdos(pevsl_Data *pevsl, int Mdeg, int damping, int nvec, double *int
       if (!st) st = pevsl_rand_block_dev(X, (int)n, s, ld);
       if (!st) st = block_colnorm2(n, s, ld, X, nrm2);
       if (!st) st = block_normalize(n, s, ld, X, nrm2);
-      for (int k = 0; k < steps && !st; k++)
+      for (int k = 0; k < steps && !st; k++) {
+        const int at = k % chunk;
         st = kpm_step(A, s, B[k % 2], k > 0 ? B[(k + 1) % 2] : nullptr, B[(k + 1) % 2], ctr,
-                      (k == 0 ? 1.0 : 2.0) / wid, part + np * (size_t)k);
-      if (!st) st = kpm_reduce(A, s, steps, part, mom);
+                      (k == 0 ? 1.0 : 2.0) / wid, part + np * (size_t)at);
+        if (!st && (at == chunk - 1 || k == steps - 1))
+          st = kpm_reduce(A, s, at + 1, part, mom + 4 * (size_t)ld * (size_t)(k - at));
+      }
       if (!st) st = memcpy_async(hmom.data(), mom, sizeof(double) * hmom.size());
       if (!st) st = memcpy_async(hn, nrm2, sizeof(double) * (size_t)s);
       if (!st) st = sync();

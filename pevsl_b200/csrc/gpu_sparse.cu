@@ -1086,7 +1086,7 @@ static unsigned stream_grid(int n, int R) {
  * the degrees and three block transfers instead of four in each.  Each
  * thread keeps its columns over all its rows; per block the sums go to
  * part[block][4 L] = (d0, d1 of column 0, of column 1, ...), added over the
- * blocks in order by k_kpm_reduce for all degrees at the end.
+ * blocks in order by k_kpm_reduce, for many degrees at a time.
  *
  * Bound by L2 and HBM bandwidth (48 bytes per row and pair of vectors, 16 of
  * them written).  With more blocks than are resident, each wave of blocks
@@ -1095,7 +1095,7 @@ static unsigned stream_grid(int n, int R) {
  * 99.  Five or six blocks per SM with four gathers in flight: 23.1 and 25.2
  * against 22.0 ms for the 300 moments. */
 constexpr int kKpmPerSm = 4; /* 64 registers, every gather of a row in flight */
-constexpr int kKpmBlocks = kKpmPerSm * 148; /* all resident: the blocks sweep the rows together */
+static int kpm_resident() { return kKpmPerSm * ctx().sms; } /* the blocks sweep the rows together */
 
 struct KpmAcc {
   double a0, a1, b0, b1; /* d0, d1 of the first column, of the second */
@@ -2512,7 +2512,7 @@ static unsigned warp_row_grid(long n) {
 
 int kpm_blocks(const pevsl_devcsr *A, int s) {
   const int RB = kThreads / ((s + 1) / 2);
-  return (int)std::min<long>(((long)A->nrows + RB - 1) / RB, kKpmBlocks);
+  return (int)std::min<long>(((long)A->nrows + RB - 1) / RB, kpm_resident());
 }
 
 int kpm_step(const pevsl_devcsr *A, int s, const double *Xk, const double *Xkm1, double *Xkp1,

@@ -42,3 +42,20 @@ def test_lanczos_dos_takes_fewer_runs_at_a_time(gpu, limit, bases):
     M.free()
     assert outs[0][0] == outs[1][0] == 0
     assert np.array_equal(outs[0][2], outs[1][2]) and outs[0][3] == outs[1][3]
+
+
+@pytest.mark.parametrize("mdeg", [1, 127, 128, 129, 4000])
+def test_kpm_workspace_does_not_grow_with_the_moments(gpu, limit, mdeg):
+    """64 vectors at 205 blocks: 210 KB of partial sums per step, 420 MB for
+    all steps of 4000 moments; 32 MB do for any number."""
+    M = pv.Matrix.from_csr(*laplacian(41, 40, 1))
+    outs = []
+    with pv.Instance(M) as ev:
+        for bytes_ in (0, 32 << 20):
+            ev.lib.pEVSL_B200_ReleaseWorkspace()
+            limit(bytes_)
+            pv.set_rng(pv.RNG_GAUSS, 5)
+            outs.append(ev.kpmdos(mdeg, 1, 64, [0.5, 6.0, 0.0, 8.0]))
+    M.free()
+    assert outs[0][0] == outs[1][0] == 0
+    assert np.array_equal(outs[0][1], outs[1][1]) and outs[0][2] == outs[1][2]
