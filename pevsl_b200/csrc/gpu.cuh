@@ -221,6 +221,8 @@ int cheb_combine(long n, const double *ax, const double *vk, const double *vkm1,
 int kpm_blocks(const pevsl_devcsr *A, int s);
 int kpm_step(const pevsl_devcsr *A, int s, const double *Xk, const double *Xkm1, double *Xkp1,
              double ctr, double sc, double *part);
+/* the same sums part for <x_0, x_0> of the start vectors (and 0) */
+int kpm_start(const pevsl_devcsr *A, int s, const double *X, double *part);
 int kpm_reduce(const pevsl_devcsr *A, int s, int steps, const double *part, double *out);
 /* vectors that share a group (at most 64) */
 int kpm_group(const pevsl_devcsr *A, int nvec);

@@ -954,7 +954,6 @@ int pEVSL_Kpmdos(pevsl_Data *pevsl, int Mdeg, int damping, int nvec, double *int
      * c_1, so half the degrees do. */
     const int smax = kpm_group(A, vec_end - vec_start), steps = (Mdeg + 1) / 2;
     std::vector<double> hmom;
-    double hn[64];
     for (int m0 = vec_start; m0 < vec_end && !st; m0 += smax) {
       const int s = PEVSL_MIN(smax, vec_end - m0), ld = (s + 1) / 2 * 2;
       const size_t blk = (size_t)n * (size_t)ld, np = (size_t)kpm_blocks(A, s) * 2 * (size_t)ld;
@@ -963,13 +962,14 @@ int pEVSL_Kpmdos(pevsl_Data *pevsl, int Mdeg, int damping, int nvec, double *int
        * vectors, however many moments */
       const int chunk = PEVSL_MIN(PEVSL_MAX(steps, 1), kKpmChunk);
       double *part = (double *)ws(WS_PART, sizeof(double) * np * (size_t)chunk);
-      double *mom = (double *)ws(WS_MOM, sizeof(double) * 4 * (size_t)ld * (size_t)PEVSL_MAX(steps, 1));
+      /* per step, and first for the start vectors */
+      double *mom = (double *)ws(WS_MOM, sizeof(double) * 4 * (size_t)ld * (size_t)(steps + 1));
       double *nrm2 = (double *)ws(WS_SMALL, sizeof(double) * 64);
       if (!X || !part || !mom || !nrm2) {
         st = PEVSL_ERR_NOMEM;
         break;
       }
-      hmom.resize(4 * (size_t)ld * (size_t)steps);
+      hmom.resize(4 * (size_t)ld * (size_t)(steps + 1));
       double *B[2] = {X, X + blk};
       if (s < ld)
         st = fail(cudaMemset2DAsync(X + s, sizeof(double) * (size_t)ld, 0, sizeof(double), (size_t)n,
@@ -978,27 +978,30 @@ int pEVSL_Kpmdos(pevsl_Data *pevsl, int Mdeg, int damping, int nvec, double *int
       if (!st) st = pevsl_rand_block_dev(X, (int)n, s, ld);
       if (!st) st = block_colnorm2(n, s, ld, X, nrm2);
       if (!st) st = block_normalize(n, s, ld, X, nrm2);
+      if (!st) st = kpm_start(A, s, X, part);
+      if (!st) st = kpm_reduce(A, s, 1, part, mom);
       for (int k = 0; k < steps && !st; k++) {
         const int at = k % chunk;
         st = kpm_step(A, s, B[k % 2], k > 0 ? B[(k + 1) % 2] : nullptr, B[(k + 1) % 2], ctr,
                       (k == 0 ? 1.0 : 2.0) / wid, part + np * (size_t)at);
         if (!st && (at == chunk - 1 || k == steps - 1))
-          st = kpm_reduce(A, s, at + 1, part, mom + 4 * (size_t)ld * (size_t)(k - at));
+          st = kpm_reduce(A, s, at + 1, part, mom + 4 * (size_t)ld * (size_t)(k - at + 1));
       }
       if (!st) st = memcpy_async(hmom.data(), mom, sizeof(double) * hmom.size());
-      if (!st) st = memcpy_async(hn, nrm2, sizeof(double) * (size_t)s);
       if (!st) st = sync();
       pevsl->stats->n_mvA += (size_t)steps * (size_t)s;
       /* accumulate exactly as the reference: vector by vector, degree by degree */
       for (int c = 0; c < s && !st; c++) {
         mu[0] += jac[0];
         tcnt -= jac[0] * (beta2 - beta1);
-        /* c_0 of the start vector as block_normalize left it: one up to rounding */
-        const long double q = 1.0 / sqrt(hn[c]), c0 = (long double)hn[c] * q * q;
-        const long double c1 = steps > 0 ? (long double)hmom[4 * (size_t)c + 2] + hmom[4 * (size_t)c + 3] : 0;
+        /* c_0 of the start vector as block_normalize left it, one up to
+         * rounding, and known as well as the products it is subtracted from */
+        const double *h1 = hmom.data() + 4 * (size_t)ld; /* the first step's */
+        const long double c0 = (long double)hmom[4 * (size_t)c] + hmom[4 * (size_t)c + 1];
+        const long double c1 = steps > 0 ? (long double)h1[4 * (size_t)c + 2] + h1[4 * (size_t)c + 3] : 0;
         for (int k = 0; k < Mdeg; k++) {
           const int k1 = k + 1;
-          const double *d = &hmom[4 * ((size_t)(k / 2) * ld + c)];
+          const double *d = h1 + 4 * ((size_t)(k / 2) * ld + c);
           const double ck = (double)(k == 0       ? c1
                                      : k1 % 2 ? 2.0L * ((long double)d[2] + d[3]) - c1
                                               : 2.0L * ((long double)d[0] + d[1]) - c0);

@@ -1088,12 +1088,13 @@ static unsigned stream_grid(int n, int R) {
  * part[block][4 L] = (d0, d1 of column 0, of column 1, ...), added over the
  * blocks in order by k_kpm_reduce, for many degrees at a time.
  *
- * Bound by L2 and HBM bandwidth (48 bytes per row and pair of vectors, 16 of
- * them written).  With more blocks than are resident, each wave of blocks
- * sweeps every other stripe of rows and reads its neighbours again: 985
- * instead of 720 MB of DRAM traffic per degree of 30 vectors at 101 x 100 x
- * 99.  Five or six blocks per SM with four gathers in flight: 23.1 and 25.2
- * against 22.0 ms for the 300 moments. */
+ * Bound by the operations of the row sums (KpmSum) and the latency of the
+ * gathers together: four vectors at 101 x 100 x 99 23.5 us per degree, of
+ * which the FP64 pipes work 11.  With more blocks than are resident, each
+ * wave of blocks sweeps every other stripe of rows and reads its neighbours
+ * again.  Four blocks per SM with every gather of a row in flight 28.2 ms for
+ * 300 moments of 30 vectors; three 28.0, two 35.0, five and six (spills) 38.5
+ * and 69.8, four with half a row's gathers in flight 30.8. */
 constexpr int kKpmPerSm = 4; /* 64 registers, every gather of a row in flight */
 static int kpm_resident() { return kKpmPerSm * ctx().sms; } /* the blocks sweep the rows together */
 
@@ -1101,9 +1102,41 @@ struct KpmAcc {
   double a0, a1, b0, b1; /* d0, d1 of the first column, of the second */
 };
 
-__device__ __forceinline__ void kpm_row(double2 r, double2 x, double2 xm1, double2 *Xkp1, size_t me,
-                                        double ctr, double sc, KpmAcc &t) {
-  const double2 w = make_double2((r.x - ctr * x.x) * sc - xm1.x, (r.y - ctr * x.y) * sc - xm1.y);
+/* The doubled moments hold the rounding errors of v_k twice, and along v_k
+ * itself, where those of a constant-coefficient row do not average out: with
+ * the row's sum in plain arithmetic they are 1.5 to 7 times as far off as
+ * moments against the start vector.  So an element of v_{k+1} is rounded
+ * once.  A sum starts at a power of two above all partial sums (|v_k| <= 1,
+ * and a row of A is at most as long as A's norm, so 8 (|ctr| + wid) is), which
+ * makes its increments exact differences and the rounding of each product a
+ * second sum; where the spectrum is not inside the interval and v_k grows,
+ * the correction is only less exact.  Four operations per entry instead of
+ * one.  Errors of the moments past the tenth, 33 x 32 x 31 and 100 x 101, 300
+ * moments, against those of the plain recurrence: 0.6 to 1.0 times. */
+struct KpmSum {
+  double s, lo;
+  __device__ __forceinline__ void add(double a, double x) {
+    const double n = fma(a, x, s), q = n - s; /* q: exact */
+    lo += fma(a, x, -q);
+    s = n;
+  }
+};
+constexpr double kKpmAnchor = 8.0; /* the same for sc r - x_{k-1} */
+
+/* (r - ctr x) sc - xm1, r's terms added */
+__device__ __forceinline__ double kpm_element(KpmSum r, double anchor, double x, double xm1,
+                                              double ctr, double sc) {
+  r.add(-ctr, x);
+  KpmSum w{kKpmAnchor - xm1, 0.0};
+  w.lo = -xm1 - (w.s - kKpmAnchor);
+  w.add(sc, r.s - anchor);
+  return (w.s - kKpmAnchor) + fma(sc, r.lo, w.lo);
+}
+
+__device__ __forceinline__ void kpm_row(KpmSum r0, KpmSum r1, double anchor, double2 x, double2 xm1,
+                                        double2 *Xkp1, size_t me, double ctr, double sc, KpmAcc &t) {
+  const double2 w = make_double2(kpm_element(r0, anchor, x.x, xm1.x, ctr, sc),
+                                 kpm_element(r1, anchor, x.y, xm1.y, ctr, sc));
   Xkp1[me] = w;
   t.a0 = fma(w.x, w.x, t.a0);
   t.a1 = fma(w.x, x.x, t.a1);
@@ -1148,7 +1181,8 @@ __device__ __forceinline__ void kpm_finish(KpmAcc t, int L, int RB, double *part
 template <int K, class M>
 __global__ void __launch_bounds__(kThreads, kKpmPerSm)
     k_kpm_stencil(int n, int L, const __grid_constant__ Stencil S, const double2 *Xk,
-                  const double2 *Xkm1, double2 *Xkp1, double ctr, double sc, double *part) {
+                  const double2 *Xkm1, double2 *Xkp1, double ctr, double sc, double anchor,
+                  double *part) {
   pdl_wait_then_release();
   const int RB = kThreads / L, rl = (int)threadIdx.x / L, l = (int)threadIdx.x % L;
   const bool on = rl < RB;
@@ -1158,7 +1192,7 @@ __global__ void __launch_bounds__(kThreads, kKpmPerSm)
     const unsigned m = stencil_mask<M>(S, row);
     const double2 x = Xk[me];
     const double2 xm1 = Xkm1 ? Xkm1[me] : make_double2(0.0, 0.0);
-    double2 r = make_double2(0.0, 0.0);
+    KpmSum r0{anchor, 0.0}, r1{anchor, 0.0};
     constexpr int B = K > 0 ? K : 4;
 #pragma unroll
     for (int j0 = 0; j0 < (K > 0 ? K : S.k); j0 += B) {
@@ -1172,11 +1206,11 @@ __global__ void __launch_bounds__(kThreads, kKpmPerSm)
 #pragma unroll
       for (int u = 0; u < B; u++)
         if ((m >> (j0 + u)) & 1u) {
-          r.x = fma(S.val[j0 + u], xv[u].x, r.x);
-          r.y = fma(S.val[j0 + u], xv[u].y, r.y);
+          r0.add(S.val[j0 + u], xv[u].x);
+          r1.add(S.val[j0 + u], xv[u].y);
         }
     }
-    kpm_row(r, x, xm1, Xkp1, me, ctr, sc, t);
+    kpm_row(r0, r1, anchor, x, xm1, Xkp1, me, ctr, sc, t);
   }
   kpm_finish(t, L, RB, part);
 }
@@ -1184,7 +1218,8 @@ __global__ void __launch_bounds__(kThreads, kKpmPerSm)
 __global__ void __launch_bounds__(kThreads, kKpmPerSm)
     k_kpm_csr(int n, int L, const int *__restrict__ ia, const int *__restrict__ ja,
               const double *__restrict__ a, const double2 *Xk,
-              const double2 *Xkm1, double2 *Xkp1, double ctr, double sc, double *part) {
+              const double2 *Xkm1, double2 *Xkp1, double ctr, double sc, double anchor,
+              double *part) {
   pdl_wait_then_release();
   const int RB = kThreads / L, rl = (int)threadIdx.x / L, l = (int)threadIdx.x % L;
   const bool on = rl < RB;
@@ -1195,7 +1230,7 @@ __global__ void __launch_bounds__(kThreads, kKpmPerSm)
     int j = __ldg(ia + row);
     const double2 x = Xk[me];
     const double2 xm1 = Xkm1 ? Xkm1[me] : make_double2(0.0, 0.0);
-    double2 r = make_double2(0.0, 0.0);
+    KpmSum r0{anchor, 0.0}, r1{anchor, 0.0};
     for (; j < e; j += 4) {
       double2 xv[4];
       double av[4];
@@ -1211,11 +1246,25 @@ __global__ void __launch_bounds__(kThreads, kKpmPerSm)
 #pragma unroll
       for (int u = 0; u < 4; u++)
         if (j + u < e) {
-          r.x = fma(av[u], xv[u].x, r.x);
-          r.y = fma(av[u], xv[u].y, r.y);
+          r0.add(av[u], xv[u].x);
+          r1.add(av[u], xv[u].y);
         }
     }
-    kpm_row(r, x, xm1, Xkp1, me, ctr, sc, t);
+    kpm_row(r0, r1, anchor, x, xm1, Xkp1, me, ctr, sc, t);
+  }
+  kpm_finish(t, L, RB, part);
+}
+
+/* <x_0, x_0> in the place of d0, summed as the steps' products are */
+__global__ void __launch_bounds__(kThreads)
+    k_kpm_start(int n, int L, const double2 *X, double *part) {
+  pdl_wait_then_release();
+  const int RB = kThreads / L, rl = (int)threadIdx.x / L, l = (int)threadIdx.x % L;
+  KpmAcc t{0.0, 0.0, 0.0, 0.0};
+  for (int row = rl < RB ? (int)blockIdx.x * RB + rl : n; row < n; row += (int)gridDim.x * RB) {
+    const double2 x = X[(size_t)row * L + l];
+    t.a0 = fma(x.x, x.x, t.a0);
+    t.b0 = fma(x.y, x.y, t.b0);
   }
   kpm_finish(t, L, RB, part);
 }
@@ -2523,9 +2572,13 @@ int kpm_step(const pevsl_devcsr *A, int s, const double *Xk, const double *Xkm1,
   cudaStream_t st = ctx().stream;
   const double2 *xk = (const double2 *)Xk, *xm = (const double2 *)Xkm1;
   double2 *xp = (double2 *)Xkp1;
+  /* sc = 2 / wid, in the first step 1 / wid */
+  const double anchor = ldexp(1.0, std::min(ilogb(8.0 * (fabs(ctr) + 2.0 / sc)) + 1, 1000));
   if (A->smask) {
     const int w = stencil_width(A);
-    auto go = [&](auto k) { launch_pdl(k, g, st, A->nrows, L, stencil_of(A), xk, xm, xp, ctr, sc, part); };
+    auto go = [&](auto k) {
+      launch_pdl(k, g, st, A->nrows, L, stencil_of(A), xk, xm, xp, ctr, sc, anchor, part);
+    };
     if (w == 7) go(k_kpm_stencil<7, unsigned char>);
     else if (w == 5) go(k_kpm_stencil<5, unsigned char>);
     else if (A->sbytes == 1) go(k_kpm_stencil<0, unsigned char>);
@@ -2533,8 +2586,14 @@ int kpm_step(const pevsl_devcsr *A, int s, const double *Xk, const double *Xkm1,
     else go(k_kpm_stencil<0, unsigned>);
     return launched("kpm_stencil");
   }
-  launch_pdl(k_kpm_csr, g, st, A->nrows, L, A->ia, A->ja, A->a, xk, xm, xp, ctr, sc, part);
+  launch_pdl(k_kpm_csr, g, st, A->nrows, L, A->ia, A->ja, A->a, xk, xm, xp, ctr, sc, anchor, part);
   return launched("kpm_csr");
+}
+
+int kpm_start(const pevsl_devcsr *A, int s, const double *X, double *part) {
+  launch_pdl(k_kpm_start, (unsigned)kpm_blocks(A, s), ctx().stream, A->nrows, (s + 1) / 2,
+             (const double2 *)X, part);
+  return launched("kpm_start");
 }
 
 int kpm_reduce(const pevsl_devcsr *A, int s, int steps, const double *part, double *out) {
@@ -2548,9 +2607,10 @@ int kpm_reduce(const pevsl_devcsr *A, int s, int steps, const double *part, doub
  * 16 bytes per row and vector.  In the stencil form the matrix costs nothing,
  * so a group holds what stays in L2 from one degree to the next (72 MB of
  * 126), the groups about equal: 101 x 100 x 99, 300 moments of 30 vectors, in
- * groups of 4 22.0 ms, of 8 27.8, of 2 29.6, all 30 25.4; 64 x 65 x 63 of 16
- * 5.5, all 30 7.2.  Where not even two fit, and for a matrix whose entries
- * each group would read again, as many as a launch takes (64). */
+ * groups of 4 28.2 ms, of 8 28.8, of 2 31.7, all 30 26.8 at first and 30.0 in
+ * a loop; 64 x 65 x 63 of 16 7.6, all 30 7.65.  Where not even two fit, and
+ * for a matrix whose entries each group would read again, as many as a launch
+ * takes (64). */
 int kpm_group(const pevsl_devcsr *A, int nvec) {
   long g = A->smask ? (long)(72e6 / (16.0 * std::max(A->nrows, 1))) / 2 * 2 : 0;
   g = g < 2 ? 64 : std::min(g, 64L);
