@@ -1391,15 +1391,19 @@ static int window_prepare(pevsl_devcsr *A) {
   const long ng = (n - 1) / 32 + 1;
   const unsigned gg = (unsigned)((ng * 32 + kThreads - 1) / kThreads); /* a warp per 32 rows */
   std::vector<int> ia((size_t)ng), split;
-  int *dband = (int *)ws(WS_TUNE, 2 * sizeof(int)), band[2];
-  if (!dband) return PEVSL_ERR_NOMEM;
-  if (fail(cudaMemsetAsync(dband, 0, 2 * sizeof(int), ctx().stream), "cudaMemsetAsync")) return PEVSL_ERR_CUDA;
-  k_csr_band<<<gg, kThreads, 0, ctx().stream>>>(A->nrows, A->ia, A->ja, dband);
-  if (launched("csr_band") || memcpy_async(band, dband, sizeof band) || fail(cudaMemcpy2DAsync(ia.data(), sizeof(int), A->ia, 32 * sizeof(int), sizeof(int), (size_t)ng,
-                             cudaMemcpyDeviceToHost, ctx().stream),
-           "cudaMemcpy2DAsync") ||
-      sync())
-    return PEVSL_ERR_CUDA;
+  int *dband = (int *)ws_try(WS_TUNE, 2 * sizeof(int)), band[2];
+  if (!dband) return 0;
+  int st = fail(cudaMemsetAsync(dband, 0, 2 * sizeof(int), ctx().stream), "cudaMemsetAsync");
+  if (!st) {
+    k_csr_band<<<gg, kThreads, 0, ctx().stream>>>(A->nrows, A->ia, A->ja, dband);
+    st = launched("csr_band");
+  }
+  if (!st) st = memcpy_async(band, dband, sizeof band);
+  if (!st)
+    st = fail(cudaMemcpy2DAsync(ia.data(), sizeof(int), A->ia, 32 * sizeof(int), sizeof(int),
+                                (size_t)ng, cudaMemcpyDeviceToHost, ctx().stream),
+              "cudaMemcpy2DAsync");
+  if (sync() || st) return PEVSL_ERR_CUDA;
   A->band_lo = band[0];
   A->band_hi = band[1];
   if (band[0] > 32000 || band[1] > 32000) return 0;
@@ -1430,6 +1434,8 @@ static int window_prepare(pevsl_devcsr *A) {
   return launched("window_offsets");
 }
 
+constexpr size_t kTuneKeep = (size_t)64 << 20;
+
 int stream_tune(pevsl_devcsr *A) {
   if (!A || A->stream_r) return 0;
   const char *e = getenv("PEVSL_B200_STREAM_R");
@@ -1453,9 +1459,10 @@ int stream_tune(pevsl_devcsr *A) {
     if (A->wdj) A->stream_r = 3;
     return 0;
   }
-  /* scratch vectors, kept in a workspace: no allocation per matrix */
+  /* scratch vectors, kept up to 64 MB (10^6 rows need 32; taken from the
+   * matrices' pool they made the first filter there 6 ms longer) */
   const long ld = (n + 31) / 32 * 32;
-  double *buf = (double *)ws(WS_TUNE, sizeof(double) * 4 * (size_t)ld);
+  double *buf = (double *)ws_try(WS_TUNE, sizeof(double) * 4 * (size_t)ld);
   if (!buf) return 0;
   cudaStream_t st = ctx().stream;
   cudaMemsetAsync(buf, 0, sizeof(double) * 4 * (size_t)ld, st);
@@ -1485,6 +1492,7 @@ int stream_tune(pevsl_devcsr *A) {
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  if (ctx().wsz[WS_TUNE] > kTuneKeep) ws_free(WS_TUNE);
   if (fail(cudaGetLastError(), "stream_tune")) return PEVSL_ERR_CUDA;
   if (ms[2] > 0.f && ms[2] < 0.97f * ms[1]) A->stream_r = 2;
   if (ms[3] > 0.f && ms[3] < 0.97f * ms[A->stream_r]) A->stream_r = 3;

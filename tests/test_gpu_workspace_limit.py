@@ -59,3 +59,25 @@ def test_kpm_workspace_does_not_grow_with_the_moments(gpu, limit, mdeg):
     M.free()
     assert outs[0][0] == outs[1][0] == 0
     assert np.array_equal(outs[0][1], outs[1][1]) and outs[0][2] == outs[1][2]
+
+
+def test_the_tuner_gives_its_scratch_back(gpu):
+    """The first product with a general matrix times the kernels' forms on
+    scratch vectors of 256 MB here; afterwards the device has them back, but
+    for at most 64 MB and the matrix's own offsets (80 MB)."""
+    import torch
+    n = 8_000_000
+    rng = np.random.default_rng(0)
+    cols = np.arange(n, dtype=np.int64)[:, None] + np.array([-40, -3, 0, 3, 40])
+    ok = (cols >= 0) & (cols < n)
+    ia = np.concatenate([[0], np.cumsum(ok.sum(1))]).astype(np.int32)
+    M = pv.Matrix.from_csr(n, ia, cols[ok].astype(np.int32), rng.standard_normal(int(ia[-1])))
+    x, y = pv.Vector(n, np.ones(n)), pv.Vector(n)
+    lib = pv.load()
+    assert lib.pEVSL_B200_Sync() == 0
+    before = torch.cuda.mem_get_info()[0]
+    lib.pEVSL_ParcsrMatvec(M.A, x.pv, y.pv)
+    assert lib.pEVSL_B200_Sync() == 0
+    after = torch.cuda.mem_get_info()[0]
+    M.free()
+    assert before - after < 200 << 20
