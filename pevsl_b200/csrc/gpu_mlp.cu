@@ -132,12 +132,13 @@ __global__ void __launch_bounds__(128)
   constexpr int SZ = kGT * LDK > kGKC * LDT ? kGT * LDK : kGKC * LDT;
   extern __shared__ __align__(16) bf16 gsm[];
   bf16 *As = gsm, *Bs = gsm + SZ;
-  if (EPI == EPI_STORE && (int)blockIdx.x * kGT >= N) {
+  /* the rows, which are the batch in a forward layer, along x: y ends at 65535 */
+  if (EPI == EPI_STORE && (int)blockIdx.y * kGT >= N) {
     pdl_wait_then_release();
-    colsum(K, M, (int)blockIdx.y * kGT, zp, ldzp, db, (float *)gsm);
+    colsum(K, M, (int)blockIdx.x * kGT, zp, ldzp, db, (float *)gsm);
     return;
   }
-  const int m0 = blockIdx.y * kGT, n0 = blockIdx.x * kGT;
+  const int m0 = blockIdx.x * kGT, n0 = blockIdx.y * kGT;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gid = lane >> 2, tig = lane & 3;
   const int wm = (warp >> 1) * 16, wn = (warp & 1) * 16;
@@ -306,7 +307,7 @@ static int gemm(int M, int N, int K, const bf16 *A, int lda, const bf16 *B, int 
                 const float *bias, bf16 *act, int ldact, const float *zp, int ldzp,
                 float *db = nullptr) {
   if (M <= 0 || N <= 0) return 0;
-  dim3 g((unsigned)((N + kGT - 1) / kGT + (EPI == EPI_STORE)), (unsigned)((M + kGT - 1) / kGT));
+  dim3 g((unsigned)((M + kGT - 1) / kGT), (unsigned)((N + kGT - 1) / kGT + (EPI == EPI_STORE)));
   /* two operands of at most kGKC x (kGT + 8) or kGT x (kGKC + 8) elements */
   constexpr size_t sm = 2 * sizeof(bf16) * (kGT * (kGKC + 8) > kGKC * (kGT + 8) ? kGT * (kGKC + 8) : kGKC * (kGT + 8));
   static_assert(sm >= 2 * 64 * 32 * sizeof(float), "the column sums stage two tiles");
