@@ -859,6 +859,20 @@ int pEVSL_B200_ChebAv(pevsl_Data *pevsl, pevsl_Polparams *pol, const double *v, 
 
 /* ================================================================ KPM DOS */
 
+/* host doubles without exceptions, which must not leave a C entry */
+struct HostBuf {
+  double *p = nullptr;
+  size_t n = 0;
+  bool reserve(size_t want) {
+    if (want <= n && p) return true;
+    free(p);
+    p = (double *)malloc(sizeof(double) * (want ? want : 1));
+    n = p ? want : 0;
+    return p != nullptr;
+  }
+  ~HostBuf() { free(p); }
+};
+
 static constexpr int kKpmChunk = 64;
 
 int pEVSL_Kpmdos(pevsl_Data *pevsl, int Mdeg, int damping, int nvec, double *intv, int ngroups,
@@ -953,9 +967,10 @@ int pEVSL_Kpmdos(pevsl_Data *pevsl, int Mdeg, int damping, int nvec, double *int
      * T_1 give c_{2k} = 2 <v_k, v_k> - c_0 and c_{2k+1} = 2 <v_{k+1}, v_k> -
      * c_1, so half the degrees do. */
     const int smax = kpm_group(A, vec_end - vec_start), steps = (Mdeg + 1) / 2;
-    std::vector<double> hmom;
+    HostBuf hmom;
     for (int m0 = vec_start; m0 < vec_end && !st; m0 += smax) {
       const int s = PEVSL_MIN(smax, vec_end - m0), ld = (s + 1) / 2 * 2;
+      const size_t nmom = 4 * (size_t)ld * (size_t)(steps + 1);
       const size_t blk = (size_t)n * (size_t)ld, np = (size_t)kpm_blocks(A, s) * 2 * (size_t)ld;
       double *X = (double *)ws(WS_KPM, sizeof(double) * 2 * blk);
       /* the blocks' sums of up to kKpmChunk steps, then added up: 39 MB for 64
@@ -963,13 +978,12 @@ int pEVSL_Kpmdos(pevsl_Data *pevsl, int Mdeg, int damping, int nvec, double *int
       const int chunk = PEVSL_MIN(PEVSL_MAX(steps, 1), kKpmChunk);
       double *part = (double *)ws(WS_PART, sizeof(double) * np * (size_t)chunk);
       /* per step, and first for the start vectors */
-      double *mom = (double *)ws(WS_MOM, sizeof(double) * 4 * (size_t)ld * (size_t)(steps + 1));
+      double *mom = (double *)ws(WS_MOM, sizeof(double) * nmom);
       double *nrm2 = (double *)ws(WS_SMALL, sizeof(double) * 64);
-      if (!X || !part || !mom || !nrm2) {
+      if (!X || !part || !mom || !nrm2 || !hmom.reserve(nmom)) {
         st = PEVSL_ERR_NOMEM;
         break;
       }
-      hmom.resize(4 * (size_t)ld * (size_t)(steps + 1));
       double *B[2] = {X, X + blk};
       if (s < ld)
         st = fail(cudaMemset2DAsync(X + s, sizeof(double) * (size_t)ld, 0, sizeof(double), (size_t)n,
@@ -987,7 +1001,7 @@ int pEVSL_Kpmdos(pevsl_Data *pevsl, int Mdeg, int damping, int nvec, double *int
         if (!st && (at == chunk - 1 || k == steps - 1))
           st = kpm_reduce(A, s, at + 1, part, mom + 4 * (size_t)ld * (size_t)(k - at + 1));
       }
-      if (!st) st = memcpy_async(hmom.data(), mom, sizeof(double) * hmom.size());
+      if (!st) st = memcpy_async(hmom.p, mom, sizeof(double) * nmom);
       if (!st) st = sync();
       pevsl->stats->n_mvA += (size_t)steps * (size_t)s;
       /* accumulate exactly as the reference: vector by vector, degree by degree */
@@ -996,8 +1010,8 @@ int pEVSL_Kpmdos(pevsl_Data *pevsl, int Mdeg, int damping, int nvec, double *int
         tcnt -= jac[0] * (beta2 - beta1);
         /* c_0 of the start vector as block_normalize left it, one up to
          * rounding, and known as well as the products it is subtracted from */
-        const double *h1 = hmom.data() + 4 * (size_t)ld; /* the first step's */
-        const long double c0 = (long double)hmom[4 * (size_t)c] + hmom[4 * (size_t)c + 1];
+        const double *h1 = hmom.p + 4 * (size_t)ld; /* the first step's */
+        const long double c0 = (long double)hmom.p[4 * (size_t)c] + hmom.p[4 * (size_t)c + 1];
         const long double c1 = steps > 0 ? (long double)h1[4 * (size_t)c + 2] + h1[4 * (size_t)c + 3] : 0;
         for (int k = 0; k < Mdeg; k++) {
           const int k1 = k + 1;
@@ -1282,8 +1296,10 @@ static int landos_lockstep(pevsl_Data *pevsl, int S, int maxit, double *V, long 
   if (!st) st = b_dot(len, S, x, x, R.nrm0, FIN_SQRT, (1u << S) - 1u);
   if (!st) st = b_scal_inv_dev(len, S, R.nrm0, v0);
   for (int k = 0; k < maxit && !st; k++) st = lan_step(R, k, k > 0);
-  std::vector<double> h(2 * (size_t)maxit * S);
-  if (!st) st = memcpy_async(h.data(), R.hist, sizeof(double) * h.size());
+  HostBuf hist;
+  if (!st && !hist.reserve(2 * (size_t)maxit * S)) st = PEVSL_ERR_NOMEM;
+  const double *h = hist.p;
+  if (!st) st = memcpy_async(hist.p, R.hist, sizeof(double) * 2 * (size_t)maxit * S);
   if (!st) st = sync();
   for (int s = 0; s < S && !st; s++) {
     double wn = 0.0;
@@ -1367,7 +1383,7 @@ int pEVSL_LanDosG(pevsl_Data *pevsl, const int nvec, int msteps, int npts, doubl
                                   eT + (size_t)s * maxit, draw);
     }
     if (st) break;
-    std::vector<int> es((size_t)S, 0);
+    int es[kMaxBatch] = {0};
     host_parallel((size_t)S, maxit >= 30, [&](size_t s) {
       es[s] = pevsl_tridiag_eig(maxit, dT + s * maxit, eT + s * maxit, EvalT + s * maxit,
                                 EvecT + s * (size_t)maxit * maxit);
@@ -1453,7 +1469,8 @@ int pEVSL_LanTrbounds(pevsl_Data *pevsl, int lanm, int maxit, double tol, pevsl_
   int st = 0, it = 0, trlen = 0;
   LanRuns R;
   st = lan_init(R, pevsl, 1, V, 0, n, ld, lanm1);
-  std::vector<double> hist(2 * L);
+  HostBuf hist;
+  if (!st && !hist.reserve(2 * L)) st = PEVSL_ERR_NOMEM;
   double lmin = 0.0, lmax = 0.0, s[3] = {0, 0, 0};
   if (fstats) fprintf(fstats, " LanTR for bounds: dim %d, maxits %d\n", lanm, maxit);
   if (!st) st = vcopy(vinit->data, V, n);
@@ -1531,12 +1548,12 @@ int pEVSL_LanTrbounds(pevsl_Data *pevsl, int lanm, int maxit, double tol, pevsl_
       const int k0 = k, m = ahead ? kend - k0 : 1;
       if (prev) st = memcpy_async(R.beta(k0 - 1), &beta, sizeof(double));
       for (int j = k0; j < k0 + m && !st; j++) st = lan_step(R, j, j > k0 || prev);
-      if (!st) st = memcpy_async(hist.data(), R.alpha(k0), sizeof(double) * 2 * (size_t)m);
+      if (!st) st = memcpy_async(hist.p, R.alpha(k0), sizeof(double) * 2 * (size_t)m);
       if (!st) st = sync();
       bool broke = false;
       for (int j = 0; j < m && !st && !broke; j++) {
-        const double alpha = hist[2 * (size_t)j];
-        beta = hist[2 * (size_t)j + 1];
+        const double alpha = hist.p[2 * (size_t)j];
+        beta = hist.p[2 * (size_t)j + 1];
         k++;
         it++;
         if (ahead) pevsl->stats->n_mvA++;

@@ -29,6 +29,8 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cmath>
+#include <memory>
+#include <new>
 #include <vector>
 #include <stdio.h>
 #include <stdlib.h>
@@ -1390,7 +1392,10 @@ static int window_prepare(pevsl_devcsr *A) {
   if (A->lanes != 0 || A->smask || A->ncols != n || A->nnz <= 0 || n < 64L * sms) return 0;
   const long ng = (n - 1) / 32 + 1;
   const unsigned gg = (unsigned)((ng * 32 + kThreads - 1) / kThreads); /* a warp per 32 rows */
-  std::vector<int> ia((size_t)ng), split;
+  /* the row pointer of every 32nd row; without memory for it no windows */
+  const std::unique_ptr<int[]> ia(new (std::nothrow) int[(size_t)ng]);
+  int split[3 * 512 + 1];
+  if (!ia || sms > 512) return 0;
   int *dband = (int *)ws_try(WS_TUNE, 2 * sizeof(int)), band[2];
   if (!dband) return 0;
   int st = fail(cudaMemsetAsync(dband, 0, 2 * sizeof(int), ctx().stream), "cudaMemsetAsync");
@@ -1400,7 +1405,7 @@ static int window_prepare(pevsl_devcsr *A) {
   }
   if (!st) st = memcpy_async(band, dband, sizeof band);
   if (!st)
-    st = fail(cudaMemcpy2DAsync(ia.data(), sizeof(int), A->ia, 32 * sizeof(int), sizeof(int),
+    st = fail(cudaMemcpy2DAsync(ia.get(), sizeof(int), A->ia, 32 * sizeof(int), sizeof(int),
                                 (size_t)ng, cudaMemcpyDeviceToHost, ctx().stream),
               "cudaMemcpy2DAsync");
   if (sync() || st) return PEVSL_ERR_CUDA;
@@ -1410,14 +1415,14 @@ static int window_prepare(pevsl_devcsr *A) {
   int nb = 0;
   for (int m = 1; m <= 3; m++) {
     nb = m * sms;
-    split.assign((size_t)nb + 1, (int)n);
     split[0] = 0;
+    split[nb] = (int)n;
     int rows = 0;
     for (int b = 1; b < nb; b++) {
       const int want = (int)((double)A->nnz * b / nb);
-      split[(size_t)b] = (int)std::min<long>(n, 32 * (std::lower_bound(ia.begin(), ia.end(), want) - ia.begin()));
+      split[b] = (int)std::min<long>(n, 32 * (std::lower_bound(ia.get(), ia.get() + ng, want) - ia.get()));
     }
-    for (int b = 0; b < nb; b++) rows = std::max(rows, split[(size_t)b + 1] - split[(size_t)b]);
+    for (int b = 0; b < nb; b++) rows = std::max(rows, split[b + 1] - split[b]);
     A->wlen = (int)std::min<long>(n, (long)rows + A->band_lo + A->band_hi);
     if (window_smem(A) <= kWinSmem) break;
     nb = 0;
@@ -1429,7 +1434,7 @@ static int window_prepare(pevsl_devcsr *A) {
   A->wdj = (short *)p;
   A->wsplit = (int *)(p + bo);
   A->wblocks = nb;
-  if (memcpy_async(A->wsplit, split.data(), sizeof(int) * (size_t)(nb + 1))) return PEVSL_ERR_CUDA;
+  if (memcpy_async(A->wsplit, split, sizeof(int) * (size_t)(nb + 1))) return PEVSL_ERR_CUDA;
   k_window_offsets<<<gg, kThreads, 0, ctx().stream>>>(A->nrows, A->ia, A->ja, A->wdj);
   return launched("window_offsets");
 }
@@ -2788,7 +2793,7 @@ static int pack_entries(pevsl_devcsr *d, const pevsl_Csr *Ai) {
 /* The stencil form of a matrix: at most 32 (offset, value) pairs in all,
  * values compared bit for bit, and every row's entries in ascending column
  * order.  True, with the rows' masks in out, when the matrix has it. */
-static bool build_stencil(pevsl_devcsr *d, const pevsl_Csr *Ai, std::vector<unsigned char> &out) {
+static bool build_stencil(pevsl_devcsr *d, const pevsl_Csr *Ai, std::unique_ptr<unsigned char[]> &out) {
   const int nr = d->nrows;
   if (nr <= 0 || d->nnz <= 0 || d->max_row_nnz > 32 || d->lanes != 0) return false;
   struct Pair {
@@ -2797,7 +2802,9 @@ static bool build_stencil(pevsl_devcsr *d, const pevsl_Csr *Ai, std::vector<unsi
   };
   Pair pair[32];
   int np = 0; /* in order of first appearance */
-  std::vector<unsigned> mask((size_t)nr);
+  const std::unique_ptr<unsigned[]> mask(new (std::nothrow) unsigned[(size_t)nr]);
+  out.reset(new (std::nothrow) unsigned char[(size_t)nr * 4]);
+  if (!mask || !out) return false;
   for (int i = 0; i < nr; i++) {
     /* most rows repeat the one before, one column further */
     const int s = Ai->ia[i], len = Ai->ia[i + 1] - s;
@@ -2844,7 +2851,6 @@ static bool build_stencil(pevsl_devcsr *d, const pevsl_Csr *Ai, std::vector<unsi
   }
   d->sk = np;
   d->sbytes = np <= 8 ? 1 : np <= 16 ? 2 : 4;
-  out.resize((size_t)nr * (size_t)d->sbytes);
   unsigned last_in = 0, last_out = 0; /* masks repeat along a grid line */
   for (int i = 0; i < nr; i++) {
     const unsigned m = mask[(size_t)i];
@@ -2854,7 +2860,7 @@ static bool build_stencil(pevsl_devcsr *d, const pevsl_Csr *Ai, std::vector<unsi
       for (int j = 0; j < np; j++)
         if ((m >> j) & 1u) last_out |= 1u << at[j];
     }
-    memcpy(out.data() + (size_t)i * d->sbytes, &last_out, (size_t)d->sbytes); /* little endian */
+    memcpy(out.get() + (size_t)i * d->sbytes, &last_out, (size_t)d->sbytes); /* little endian */
   }
   return true;
 }
@@ -2889,10 +2895,11 @@ int pEVSL_ParcsrSetup(pevsl_Csr *Ai, pevsl_Parcsr *A) {
   const size_t bytes_a = ((sizeof(double) * (size_t)nnz + 255) / 256) * 256;
   const size_t bytes_ja = ((sizeof(int) * (size_t)nnz + 255) / 256) * 256;
   const size_t bytes_ia = sizeof(int) * (size_t)(nr + 1);
-  std::vector<unsigned char> smask;
+  std::unique_ptr<unsigned char[]> smask;
   const bool stencil = build_stencil(d, Ai, smask);
+  const size_t bytes_mask = stencil ? (size_t)nr * (size_t)d->sbytes : 0;
   const size_t off_mask = (bytes_a + bytes_ja + bytes_ia + 255) / 256 * 256;
-  char *base = (char *)alloc_dev(off_mask + smask.size());
+  char *base = (char *)alloc_dev(off_mask + bytes_mask);
   if (!base) {
     free(d);
     return PEVSL_ERR_NOMEM;
@@ -2906,7 +2913,7 @@ int pEVSL_ParcsrSetup(pevsl_Csr *Ai, pevsl_Parcsr *A) {
   if (!st) st = memcpy_async(d->a, Ai->a, sizeof(double) * (size_t)nnz);
   if (stencil) {
     d->smask = base + off_mask;
-    if (!st) st = memcpy_async(d->smask, smask.data(), smask.size());
+    if (!st) st = memcpy_async(d->smask, smask.get(), bytes_mask);
   }
   if (!st) st = sync();
   if (st) return st;
