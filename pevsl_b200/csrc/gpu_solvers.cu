@@ -1279,10 +1279,12 @@ static int landos_lanczos(pevsl_Data *pevsl, int maxit, double *V, long ld, cons
 }  // extern "C++"
 
 /* the S runs of a group in lockstep from the start vectors vinit(:, 0:S)
- * (unchanged); *broke: a run broke down, the group is to be run one by one */
+ * (unchanged); *good: how many of them, from the first on, did not break down.
+ * (The next one draws another start vector, so it and those after it are to
+ * be run one by one.) */
 static int landos_lockstep(pevsl_Data *pevsl, int S, int maxit, double *V, long ld,
-                           const double *vinit, long n, double *dT, double *eT, bool *broke) {
-  *broke = false;
+                           const double *vinit, long n, double *dT, double *eT, int *good) {
+  *good = S;
   LanRuns R;
   int st = lan_init(R, pevsl, S, V, ld * (maxit + 1), n, ld, maxit + 1);
   CPtrs x{};
@@ -1301,7 +1303,7 @@ static int landos_lockstep(pevsl_Data *pevsl, int S, int maxit, double *V, long 
   const double *h = hist.p;
   if (!st) st = memcpy_async(hist.p, R.hist, sizeof(double) * 2 * (size_t)maxit * S);
   if (!st) st = sync();
-  for (int s = 0; s < S && !st; s++) {
+  for (int s = 0; s < *good && !st; s++) {
     double wn = 0.0;
     int nwn = 0;
     for (int k = 0; k < maxit; k++) {
@@ -1310,10 +1312,10 @@ static int landos_lockstep(pevsl_Data *pevsl, int S, int maxit, double *V, long 
       eT[(size_t)s * maxit + k] = beta;
       wn += fabs(alpha) + 2.0 * beta;
       nwn += 3;
-      if (beta * nwn < orthTol * wn) *broke = true;
+      if (beta * nwn < orthTol * wn) *good = s;
     }
   }
-  if (!st && !*broke) pevsl->stats->n_mvA += (size_t)maxit * (size_t)S;
+  if (!st) pevsl->stats->n_mvA += (size_t)maxit * (size_t)*good;
   return st;
 }
 
@@ -1331,10 +1333,10 @@ int pEVSL_LanDosG(pevsl_Data *pevsl, const int nvec, int msteps, int npts, doubl
   /* runs in lockstep: up to kMaxBatch, their bases within 4 GB and their
    * eigenvectors of T within 256 MB of host memory, the groups about equal;
    * fewer where there is no memory for as many; one at a time with B-solves
-   * or a user operator */
+   * or a user operator, and where every run breaks down at its N-th step */
   const double basis = 8.0 * (double)ld * (maxit + 1), evec = 8.0 * maxit * (double)maxit;
   const int nrun = PEVSL_MAX(vec_end - vec_start, 0);
-  const bool ahead = !pevsl->ifGenEv && pevsl_builtin_A(pevsl);
+  const bool ahead = !pevsl->ifGenEv && pevsl_builtin_A(pevsl) && maxit < pevsl->N;
   int lock = !ahead ? 1 : (int)PEVSL_MIN((double)kMaxBatch, PEVSL_MAX(1.0, PEVSL_MIN(4e9 / basis, 256e6 / evec)));
   const size_t held = ctx().wsz[WS_BASIS];
   double *V = nullptr, *vinit = nullptr;
@@ -1366,15 +1368,15 @@ int pEVSL_LanDosG(pevsl_Data *pevsl, const int nvec, int msteps, int npts, doubl
     const int S = PEVSL_MIN(lock, vec_end - m0);
     /* the group's start vectors in draw order; a breakdown restart takes the
      * next one, as in runs one after the other */
-    int drawn = 0, next = 0;
+    int drawn = 0, next = 0, good = 0;
     for (; drawn < S && !st; drawn++) st = pevsl_rand_vector_dev(vinit + (size_t)drawn * ld, (int)n);
     auto draw = [&](double *v) -> int {
       return next < drawn ? vcopy(vinit + (size_t)next++ * ld, v, n) : pevsl_rand_vector_dev(v, (int)n);
     };
-    bool broke = true;
-    if (!st && ahead) st = landos_lockstep(pevsl, S, maxit, V, ld, vinit, n, dT, eT, &broke);
+    if (!st && ahead) st = landos_lockstep(pevsl, S, maxit, V, ld, vinit, n, dT, eT, &good);
+    next = good;
     double *one = vinit + (size_t)lock * ld;
-    for (int s = 0; s < S && broke && !st; s++) {
+    for (int s = good; s < S && !st; s++) {
       st = draw(one);
       if (!st)
         st = pevsl->ifGenEv

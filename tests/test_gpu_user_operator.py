@@ -69,6 +69,24 @@ def test_lanczos_dos(gpu, n, distinct, msteps, nvec):
     assert np.array_equal(outs[0][2], outs[1][2]) and outs[0][3] == outs[1][3]
 
 
+def test_lanczos_dos_of_a_tiny_problem_runs_once(gpu):
+    """As many steps as rows: every run breaks down at the last, so none is
+    queued ahead only to be repeated."""
+    M = pv.Matrix.from_csr(*diagonal(30, 30))
+    op, launches = Operator(M), []
+    lib = pv.load()
+    for user in (False, True):
+        with pv.Instance(M) as ev:
+            if user:
+                op.install(ev)
+            pv.set_rng(pv.RNG_GAUSS, 7)
+            first = lib.pEVSL_B200_LaunchCount()
+            assert ev.landos(18, 40, 51, [0.5, 30.5, 0.0, 31.0])[0] == 0
+            launches.append(lib.pEVSL_B200_LaunchCount() - first)
+    M.free()
+    assert launches[0] <= launches[1]
+
+
 @pytest.mark.parametrize("n,distinct,lanm,maxit", [(600, 3, 20, 40), (30, 30, 30, 60), (500, 5, 4, 30)])
 def test_bounds(gpu, n, distinct, lanm, maxit):
     M = pv.Matrix.from_csr(*diagonal(n, distinct))
