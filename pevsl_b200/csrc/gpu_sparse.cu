@@ -2115,7 +2115,14 @@ __global__ void __launch_bounds__(kThreads)
   const double2 yold = (ny > 0 && !fresh) ? Y[me] : make_double2(0.0, 0.0);
   const double2 *xr = Xg + me;
   double r0 = 0.0, r1 = 0.0;
-  constexpr int B = K > 0 ? (K + 1) / 2 : 4;
+  /* any number of pairs: four gathers at a time, five with one lane per row,
+   * where all a row has to wait for is its own.  Two vectors per degree, four /
+   * five / the ELL kernel, which such matrices ran on before: nine-point rows
+   * at 400 x 401 5.2 / 4.2 / 4.7 us, 1000 x 1001 12.8 / 12.4 / 20.0, thirteen at
+   * 400 x 401 6.2 / 5.0 / 5.8; eight 4.7 and 14.9, 4.9 */
+  constexpr int B = K > 0 ? (K + 1) / 2 : L == 1 ? 5 : 4;
+  /* the last batch of five reaches past the mask's 32 bits */
+  auto has = [&](int j) { return (32 % B == 0 || K > 0 || j < 32) && ((m >> j) & 1u); };
   auto batch = [&](int j0) {
     double2 xv[B];
 #pragma unroll
@@ -2123,12 +2130,12 @@ __global__ void __launch_bounds__(kThreads)
       xv[u] = make_double2(0.0, 0.0);
       if (K > 0 && !GEN && j0 + u == K / 2)
         xv[u] = x;
-      else if ((m >> (j0 + u)) & 1u)
+      else if (has(j0 + u))
         xv[u] = xr[(long)S.off[j0 + u] * L];
     }
 #pragma unroll
     for (int u = 0; u < B; u++)
-      if ((m >> (j0 + u)) & 1u) {
+      if (has(j0 + u)) {
         r0 = __dadd_rn(r0, __dmul_rn(S.val[j0 + u], xv[u].x));
         r1 = __dadd_rn(r1, __dmul_rn(S.val[j0 + u], xv[u].y));
       }
