@@ -72,6 +72,12 @@ int pEVSL_B200_SetBarrierSpins(unsigned spins);
  * report clears the counter again. */
 int pEVSL_B200_SeedBarrierArrivals(unsigned count);
 
+/* The form that one product y = A x runs in (chosen at set-up, or at the first
+ * product of a matrix): 0 several threads per row; 1, 2 CSR-stream with so
+ * many rows per lane; 3 the vector's window in shared memory; 4 entries loaded
+ * ahead; 5 packed entries; 6 stencil masks; negative: an error code. */
+int pEVSL_B200_ProductForm(pevsl_Parcsr *A);
+
 /* The largest workspace that the library allocates, in bytes (0: no limit,
  * the default): a larger one is refused as if there were no memory for it.
  * Calls that can do with less then take less, the others return

@@ -2872,6 +2872,13 @@ static bool build_stencil(pevsl_devcsr *d, const pevsl_Csr *Ai, std::unique_ptr<
   return true;
 }
 
+int pEVSL_B200_ProductForm(pevsl_Parcsr *A) {
+  const pevsl_devcsr *d = A ? pevsl_devcsr_of(A) : nullptr;
+  if (!d) return PEVSL_ERR_ARG;
+  if (d->lanes != 0) return 0;
+  return d->smask ? 6 : use_packed(d) ? 5 : use_window(d) ? 3 : d->stream_r == 4 ? 4 : stream_r(d);
+}
+
 int pEVSL_ParcsrSetup(pevsl_Csr *Ai, pevsl_Parcsr *A) {
   if (ensure()) return PEVSL_ERR_CUDA;
   const int nr = A->nrow_local;
