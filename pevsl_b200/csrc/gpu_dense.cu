@@ -247,11 +247,23 @@ __global__ void __launch_bounds__(kJacThreads)
   __shared__ int rp[2][kJacMax / 2], rq[2][kJacMax / 2], rank[kJacMax];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int NW = kJacThreads / 32;
+  double big = 0.0;
   for (int i = warp; i < m; i += NW)
     for (int j = lane; j < m; j += 32) {
-      S[i * ld + j] = i < n && j < n ? A[(size_t)j * lda + i] : 0.0;
+      const double x = i < n && j < n ? A[(size_t)j * lda + i] : 0.0;
+      big = fmax(big, fabs(x));
+      S[i * ld + j] = x;
       V[i * ld + j] = i == j ? 1.0 : 0.0;
     }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) big = fmax(big, __shfl_xor_sync(0xffffffffu, big, o));
+  if (lane == 0) red[0][warp] = big;
+  __syncthreads();
+  for (int w = 0; w < NW; w++) big = fmax(big, red[0][w]);
+  /* by a power of two, so that the squares neither overflow nor vanish */
+  const int e = big > 0.0 && big <= DBL_MAX ? max(ilogb(big), -1000) : 0;
+  for (int i = warp; i < m; i += NW)
+    for (int j = lane; j < m; j += 32) S[i * ld + j] = scalbn(S[i * ld + j], -e);
   __syncthreads();
   /* the rotations of round r, by warp 0, into buffer w */
   auto rotations = [&](int r, int w) {
@@ -352,7 +364,7 @@ __global__ void __launch_bounds__(kJacThreads)
       __syncthreads();
     }
   }
-  if (tid < n) lam[tid] = S[tid * ld + tid];
+  if (tid < n) lam[tid] = scalbn(S[tid * ld + tid], e);
   if (tid < 6) val[tid] = nan(""); /* stays where a NaN has no rank */
   if (tid < 2 * n) Y[tid] = nan("");
   __syncthreads();

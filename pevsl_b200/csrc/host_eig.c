@@ -217,9 +217,15 @@ int pevsl_dense_symeig(int n, const double *A, int lda, double *Q, int ldq, doub
     free(V);
     return PEVSL_ERR_NOMEM;
   }
+  /* by a power of two, so that the squares neither overflow nor vanish */
+  double big = 0.0;
+  for (int j = 0; j < n; j++)
+    for (int i = 0; i < n; i++) big = fmax(big, fabs(A[(size_t)j * lda + i]));
+  int ex = big > 0.0 && big <= DBL_MAX ? ilogb(big) : 0;
+  if (ex < -1000) ex = -1000;
   for (int j = 0; j < n; j++)
     for (int i = 0; i < n; i++) {
-      S[(size_t)j * n + i] = A[(size_t)j * lda + i];
+      S[(size_t)j * n + i] = scalbn(A[(size_t)j * lda + i], -ex);
       V[(size_t)j * n + i] = i == j ? 1.0 : 0.0;
     }
   for (int sweep = 0; sweep < 100; sweep++) {
@@ -257,7 +263,7 @@ int pevsl_dense_symeig(int n, const double *A, int lda, double *Q, int ldq, doub
     }
   }
   double *diag = (double *)malloc((size_t)n * sizeof(double));
-  for (int i = 0; i < n; i++) diag[i] = S[(size_t)i * n + i];
+  for (int i = 0; i < n; i++) diag[i] = scalbn(S[(size_t)i * n + i], ex);
   int *ord = ascending_order(n, diag);
   for (int i = 0; i < n; i++) {
     lam[i] = diag[ord[i]];
