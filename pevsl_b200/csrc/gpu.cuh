@@ -359,6 +359,13 @@ struct ClusterJob {
 };
 /* largest matrix of a cluster launch */
 constexpr int kClusterMaxRows = 32768;
+/* A cluster launch costs about 10 us more than the first of the launches per
+ * degree (it loads the entries and meets its neighbours twice first) and gains 1
+ * to 1.3 us per degree: one vector, 7980 rows, launches / cluster, degree 2 12.4
+ * / 20.3 us, 6 20.9 / 23.2, 8 24.8 / 24.5, 24 56.5 / 37.7; 15600 rows 8 25.4 /
+ * 28.3, 12 33.5 / 32.5; 6007 rows of 11 scattered entries 8 32.5 / 34.4, 12 45.2
+ * / 41.3.  So single applications of lower degree are launched per degree. */
+constexpr int kClusterMinDeg = 8;
 /* whether the matrices fit the shared memory of a cluster */
 bool cluster_filter_ok(const pevsl_devcsr *A, const pevsl_devcsr *B, bool fp32);
 /* the applications of ne jobs, all with B or all without */

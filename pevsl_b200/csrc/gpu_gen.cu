@@ -70,7 +70,7 @@ namespace {
 int cheb_series(const pevsl_devcsr *M, const double *mu, const double *dmu, int m, double cc,
                 double dd, const double *v, double *y, double *w) {
   const long n = M->nrows;
-  if (m > 0 && cluster_filter_ok(M, nullptr, false)) {
+  if (m >= kClusterMinDeg && cluster_filter_ok(M, nullptr, false)) {
     const ClusterJob J{M, nullptr, v, y, dmu, nullptr, cc, dd, 0.0, 0.0, m, 0};
     return cluster_filter(1, &J, false);
   }

@@ -119,7 +119,7 @@ int cheb_apply(pevsl_Data *pevsl, const pevsl_Polparams *pol, const double *v, d
     return vscal(y, n, mu[0]);
   }
   if (!A && (!pevsl->Amv || !pevsl->Amv->func)) return PEVSL_ERR_NOMATVEC;
-  if (A && cluster_filter_ok(A, nullptr, false)) {
+  if (A && m >= kClusterMinDeg && cluster_filter_ok(A, nullptr, false)) {
     /* a small problem: every degree in one launch, the same bits */
     double *dmu = (double *)ws(WS_CLMU, sizeof(double) * (size_t)(m + 1));
     if (!dmu) return PEVSL_ERR_NOMEM;

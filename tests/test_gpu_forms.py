@@ -52,3 +52,19 @@ def test_other_forms(gpu):
     n, ia, ja, a = laplacian(30, 29, 28)
     assert form_of(test_gpu_stencil.with_extra_rows(n, ia, ja, a)) == 5
     assert form_of(random_sparse_symmetric(5003, 60, 300, 1)) == 0
+
+
+@pytest.mark.parametrize("deg", [1, 2, 7, 8, 30])
+def test_small_problems_by_degree(gpu, deg):
+    """One cluster launch from degree 8 on, a launch per degree below."""
+    import numpy as np
+    lib = pv.load()
+    M = pv.Matrix.from_csr(*laplacian(19, 20, 21))
+    k = np.arange(deg + 1)
+    p = pv.Filter(1, deg, 0.0, 0.5, 6.0, 7.5, np.cos(0.7 * k) / (1.0 + 0.1 * k))
+    with pv.Instance(M) as ev:
+        ev.chebav(p, np.ones(M.n))
+        first = lib.pEVSL_B200_LaunchCount()
+        ev.chebav(p, np.ones(M.n))
+        assert lib.pEVSL_B200_LaunchCount() - first == (1 if deg >= 8 else deg)
+    M.free()
