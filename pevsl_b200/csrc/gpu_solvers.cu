@@ -106,7 +106,7 @@ int apply_A(pevsl_Data *pevsl, const double *x, double *y) {
   return fail(cudaDeviceSynchronize(), "user matvec");
 }
 
-/* y = p((A - cc)/dd) v with mu[0..deg]; w3 holds 3n doubles. */
+/* y = p((A - cc)/dd) v with mu[0..deg]; w3 holds 3n doubles; y may be v. */
 int cheb_apply(pevsl_Data *pevsl, const pevsl_Polparams *pol, const double *v, double *y,
                double *w3, long n) {
   pevsl_devcsr *A = pevsl_builtin_A(pevsl);
@@ -131,6 +131,10 @@ int cheb_apply(pevsl_Data *pevsl, const pevsl_Polparams *pol, const double *v, d
     return cluster_filter(1, &J, false);
   }
   double *buf[2] = {w3, w3 + n};
+  if (y == v) { /* the first degree's rows read their neighbours' v */
+    if (vcopy(v, w3 + 2 * n, n)) return PEVSL_ERR_CUDA;
+    v = w3 + 2 * n;
+  }
   if (A) {
     g_filter_launches += (uint64_t)m;
     pevsl->stats->n_mvA += (size_t)m;
