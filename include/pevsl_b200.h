@@ -87,10 +87,14 @@ int pEVSL_B200_SetWorkspaceLimit(size_t bytes);
 
 /* Wait limit of the cluster launches of small problems, in microseconds: how
  * long a block waits for its neighbours' values of one degree.  < 0 restores
- * the default (2 s); with 0 every wait runs out at once (for tests).  When a
- * wait runs out the launch ends with NaN in its result, and the call that
- * launched it returns PEVSL_ERR_CUDA; the context stays usable. */
+ * the default (2 s).  When a wait runs out the launch ends with NaN in its
+ * result, and the call that launched it returns PEVSL_ERR_CUDA; the context
+ * stays usable. */
 int pEVSL_B200_SetClusterWait(long microseconds);
+
+/* Fault injection for tests: with `on`, the blocks of a cluster launch wait for
+ * a value more than their neighbours send, so that every wait runs out. */
+int pEVSL_B200_WithholdClusterValues(int on);
 
 /* The cross-group sum of a split KPM: pEVSL_Kpmdos with ngroups > 1 computes
  * the moments of its group's share of the random vectors (pEVSL_Part1d)

@@ -201,6 +201,7 @@ SIGNATURES = [
     ("pEVSL_B200_ProductForm", _I, [C.POINTER(Parcsr)]),
     ("pEVSL_B200_SetWorkspaceLimit", _I, [C.c_size_t]),
     ("pEVSL_B200_SetClusterWait", _I, [C.c_long]),
+    ("pEVSL_B200_WithholdClusterValues", _I, [_I]),
     ("pEVSL_B200_CopyEigenvectors", _I, [C.POINTER(Parvecs), _I, _dp, C.c_long]),
     ("pEVSL_B200_SetGroupReduce", _I, [C.POINTER(PevslData), _vp, _vp]),
     ("pEVSL_B200_ChebLanNrBatch", _I, [C.POINTER(PevslData), _I, _dp, _ip, _D,

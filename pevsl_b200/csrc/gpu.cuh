@@ -371,8 +371,10 @@ bool cluster_filter_ok(const pevsl_devcsr *A, const pevsl_devcsr *B, bool fp32);
 /* the applications of ne jobs, all with B or all without */
 int cluster_filter(int ne, const ClusterJob *jobs, bool fp32);
 /* microseconds after which a block of a cluster launch stops waiting for its
- * neighbours and the call fails: < 0 the default, 0 at once (for tests) */
+ * neighbours and the call fails; < 0 the default */
 void set_cluster_wait(long us);
+/* for tests: every block waits for eight bytes that nobody sends */
+void withhold_cluster_values(bool on);
 
 /* ---------------------------------------------------------------- FP32 (mixed) */
 int csr_make_fp32(pevsl_devcsr *A); /* FP32 copy of the values, once */

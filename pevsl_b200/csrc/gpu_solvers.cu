@@ -2011,6 +2011,11 @@ int pEVSL_B200_SetClusterWait(long microseconds) {
   return 0;
 }
 
+int pEVSL_B200_WithholdClusterValues(int on) {
+  withhold_cluster_values(on != 0);
+  return 0;
+}
+
 /* Filtered Lanczos in lockstep (pEVSL_ChebLanNr, SRC/cheblanNr.c:54-448) for
  * ns <= kMaxEntries slices, which may belong to different problems (each
  * entry carries its instance, matrix, length and start vector).  Every

@@ -1,8 +1,8 @@
 """The bounded wait between the blocks of a cluster launch.
 
-With a limit of zero every wait runs out before the first poll: the launch
-ends by itself, the call returns PEVSL_ERR_CUDA, and the next call with the
-default limit gives the bits of the launch-per-degree recurrence.
+With a value withheld and a limit of 200 microseconds every wait runs out: the
+launch ends by itself, the call returns PEVSL_ERR_CUDA, and the next call
+without the fault gives the bits of the launch-per-degree recurrence.
 """
 import ctypes as C
 
@@ -30,8 +30,13 @@ def poly(deg):
 @pytest.fixture
 def wait():
     lib = pv.load()
-    yield lib.pEVSL_B200_SetClusterWait
-    lib.pEVSL_B200_SetClusterWait(-1)
+
+    def fault(on):
+        lib.pEVSL_B200_SetClusterWait(200 if on else -1)
+        lib.pEVSL_B200_WithholdClusterValues(on)
+
+    yield fault
+    fault(0)
     lib.pEVSL_B200_LastError()
 
 
@@ -44,10 +49,10 @@ def test_filter_wait_runs_out(gpu, wait, name):
     with pv.Instance(M) as ev:
         want = ev.chebav(poly(37), v)
         x, y = pv.Vector(n, v), pv.Vector(n)
-        wait(0)
+        wait(1)
         assert ev.lib.pEVSL_B200_ChebAv(ev.p, C.byref(pol), x.pv.data, y.pv.data) == pv.ERR_CUDA
         assert np.all(np.isnan(y.get()))
-        wait(-1)
+        wait(0)
         assert ev.lib.pEVSL_B200_ChebAv(ev.p, C.byref(pol), x.pv.data, y.pv.data) == 0
         assert np.array_equal(y.get(), want)
     M.free()
@@ -60,8 +65,8 @@ def test_lockstep_solve_reports_it(gpu, wait):
     fl = [pv.findpol(iv)[1] for iv in intvs]
     v = np.cos(np.arange(n) * 0.37)
     outs = []
-    for limit in (-1, 0, -1):
-        wait(limit)
+    for on in (0, 1, 0):
+        wait(on)
         with pv.Instance(M) as ev:
             outs.append(pv.cheblannr_batch(ev, intvs, [150] * 4, 1e-8, v, fl))
     M.free()
