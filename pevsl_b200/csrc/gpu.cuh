@@ -147,8 +147,6 @@ int vfill(double *x, long n, double v);
 int vcopy(const double *x, double *y, long n);
 int vscal(double *x, long n, double a);
 int vaxpy(long n, double a, const double *x, double *y);
-/* y += sign * (*coef) * x, coef in device memory */
-/* x *= 1 / (*s), s in device memory */
 /* *out = <x, y> (deterministic); out in device memory */
 int vdot(long n, const double *x, const double *y, double *out);
 /* *out = ||x|| */
@@ -252,10 +250,11 @@ struct BLen {
 BLen blen_uniform(long n, long ld, int S);
 int b_axpy(const BLen &len, int S, CPtrs x, VPtrs y, BScal a, unsigned mask);
 int b_scal(const BLen &len, int S, VPtrs x, BScal a, unsigned mask);
-/* y_s += sign coef[s] x_s and x_s *= 1 / nrm[s] for all S entries, the
+/* y_s += sign coef[s] x_s, then out[s] = <z_s, y_s>, for all S entries; the
  * scalars in device memory */
 int b_axpy_dev_dot(const BLen &len, int S, const double *coef, double sign, CPtrs x, VPtrs y,
                    CPtrs z, double *out);
+/* x_s *= 1 / nrm[s] for all S entries, nrm in device memory */
 int b_scal_inv_dev(const BLen &len, int S, const double *nrm, VPtrs x);
 int b_dot(const BLen &len, int S, CPtrs x, CPtrs y, double *out, int fin, unsigned mask);
 int b_axpy_dev_nrm2(const BLen &len, int S, const double *coef, CPtrs x, VPtrs y, double *nrm,
@@ -385,13 +384,13 @@ int cvt_f64_f32(long n, const double *x, float *y);
 /* C = V(:, 0:k)' W(:, 0:m)  (k x m, column-major ldc); deterministic */
 int gemm_tn(long n, int k, int m, const double *V, long ldv, const double *W, long ldw, double *C,
             long ldc);
-/* U = V(:, 0:k) Y  (n x m, V column-major ldv, Y k x m column-major ldy) */
 /* the ends of the spectrum of a symmetric n x n host matrix (column major):
  * val[0..3] = lam_1, lam_2, lam_{n-1}, lam_n, val[4..5] the last elements of
  * the eigenvectors of lam_1 and lam_n, which go to Y (device, 2n); waits.
  * ritz_ends_ok: the n it takes */
 bool ritz_ends_ok(int n);
 int ritz_ends(int n, const double *T, int ldt, double *Y, double *val);
+/* U = V(:, 0:k) Y  (n x m, V column-major ldv, Y k x m column-major ldy) */
 int gemm_nn(long n, int k, int m, const double *V, long ldv, const double *Y, long ldy,
             double *U, long ldu);
 

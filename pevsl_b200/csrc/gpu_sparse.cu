@@ -651,7 +651,7 @@ __global__ void __launch_bounds__(kThreads, 4)
  * three to four waves of blocks, each the length of the chain mask, gather,
  * sum, store; larger ones stream from HBM.  Per degree of one vector with the
  * sum deferred, against the ELL and packed kernels: 41 x 40 x 42 2.2 / 2.5
- * us, 64 x 65 x 63 2.4 / 4.1 us, 99 x 100 x 101 5.9 / 10.6 us (30 MB: 5.1
+ * us, 64 x 65 x 63 2.3 / 4.1 us, 99 x 100 x 101 5.5 / 10.6 us (30 MB: 5.5
  * TB/s), 159 x 160 x 161 22.4 / 54 us.  (The same rows described by a table
  * of row patterns in shared memory took 8.1 us at 99 x 100 x 101, with the
  * value and the offset in one 16-byte entry 11.6 us: the table's broadcast
@@ -1351,13 +1351,6 @@ __global__ void k_block_normalize(long n, int s, int ld, double *X, const double
     }                                                                                            \
   } while (0)
 
-/* Autotuner of the CSR-stream kernels: on a matrix's first use, time one
- * Chebyshev degree with one and with two rows per lane and, where the windows
- * fit, the windowed form (1 warm-up + 5 timed launches each, CUDA events,
- * scratch vectors of the matrix's size) and keep the fastest; a later one must
- * win by 3%.  All give the same bits (the per-row summation order is the
- * same), so the choice never changes a result.  PEVSL_B200_STREAM_R=1|2|3
- * fixes it; matrices under 4096 rows keep one.  Must not run while the stream is being captured. */
 /* 256 entries per pass where the staging leaves room for the window */
 static int window_chunk(const pevsl_devcsr *A) {
   const size_t win = sizeof(double) * (size_t)(A->wlen + 2);
@@ -1439,6 +1432,14 @@ static int window_prepare(pevsl_devcsr *A) {
   return launched("window_offsets");
 }
 
+/* Autotuner of the products of general matrices: on a matrix's first use, the
+ * entries-ahead form by rule, else time one Chebyshev degree with one and with
+ * two rows per lane and, where the windows fit, the windowed form (1 warm-up +
+ * 5 timed launches each, CUDA events, scratch vectors of the matrix's size) and
+ * keep the fastest; a later one must win by 3%.  All give the same bits (the
+ * per-row summation order is the same), so the choice never changes a result.
+ * PEVSL_B200_STREAM_R=1|2|3|4 fixes it; matrices under 4096 rows keep one row
+ * per lane.  Must not run while the stream is being captured. */
 constexpr size_t kTuneKeep = (size_t)64 << 20;
 
 int stream_tune(pevsl_devcsr *A) {
@@ -1511,8 +1512,6 @@ int stream_tune(pevsl_devcsr *A) {
   return 0;
 }
 
-/* one CSR-stream launch with the matrix's rows per lane (tuned on first use
- * when the stream is not being captured) */
 /* Which kernels read the packed entries (PEVSL_B200_PACKED): 0 none, 1 the
  * one-vector kernels (default), 2 also the shared-matrix batch.  Measured
  * per filter degree at 100^3: one vector 22.3 vs 28.1 us, but 4 slices
@@ -1586,6 +1585,8 @@ static void launch_rows_stencil(const pevsl_devcsr *A, const double *x, const Ep
 #undef PV_RS
 }
 
+/* one product launch in the matrix's form (tuned on first use when the stream
+ * is not being captured) */
 template <class T, class Epi>
 static void launch_stream(const pevsl_devcsr *A, const T *a, const T *x, const Epi &epi) {
   if constexpr (sizeof(T) == 8) {
@@ -1742,7 +1743,7 @@ int cheb_step_y(const pevsl_devcsr *A, const double *vk, const double *vkm1, dou
   if (!cheb_defers(A) || ny < 0 || ny > 3 || ny > k || (ny > 1 && !vkm1)) return PEVSL_ERR_ARG;
   const int w = stencil_width(A);
   if (w && vkm1 && (ny == 0 || (ny == 3 && !fresh))) {
-    /* two rows per thread from eight waves of blocks on */
+    /* two rows per thread past seven waves of blocks */
     const int rpt = (long)A->nrows > 7L * 8 * kThreads * ctx().sms ? 2 : 1;
     const unsigned g = (unsigned)((A->nrows + kThreads * rpt - 1) / (kThreads * rpt));
     launch_pdl(rpt == 1 ? (w == 7 ? k_cheb_stencil<7> : k_cheb_stencil<5>)
