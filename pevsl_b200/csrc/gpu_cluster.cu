@@ -639,8 +639,12 @@ bool cluster_filter_ok(const pevsl_devcsr *A, const pevsl_devcsr *B, bool fp32) 
   J.B = B;
   ClShape s;
   if (!cl_choose(1, &J, fp32, &s)) return false;
-  /* a matrix in the stencil form takes 2.1 us per launched degree, less than
-   * a cluster with more than two rows per thread */
+  /* A matrix in the stencil form takes 2.1 us per launched degree, less than a
+   * cluster with more than two rows per thread.  A general one is not slower
+   * here where its entries fit, k_csr_ahead included (us per degree, cluster /
+   * launched, one vector and four in lockstep): 16000 rows of 9 entries 2.81 /
+   * 2.94 and 2.90 / 4.78, 24000 of 5 2.96 / 3.12 and 2.93 / 4.54, 32000 of 3 2.86
+   * / 2.74 and 2.82 / 3.89, 12000 of 13 2.89 / 3.11 and 2.85 / 5.01. */
   return B || fp32 || !A->smask || s.rpt <= 2;
 }
 

@@ -1091,12 +1091,12 @@ static unsigned stream_grid(int n, int R) {
  * blocks in order by k_kpm_reduce, for many degrees at a time.
  *
  * Bound by the operations of the row sums (KpmSum) and the latency of the
- * gathers together: four vectors at 101 x 100 x 99 23.5 us per degree, of
+ * gathers together: four vectors at 101 x 100 x 99 20.8 us per degree, of
  * which the FP64 pipes work 11.  With more blocks than are resident, each
  * wave of blocks sweeps every other stripe of rows and reads its neighbours
- * again.  Four blocks per SM with every gather of a row in flight 28.2 ms for
- * 300 moments of 30 vectors; three 28.0, two 35.0, five and six (spills) 38.5
- * and 69.8, four with half a row's gathers in flight 30.8. */
+ * again.  Four blocks per SM with every gather of a row in flight 25.0 ms for
+ * 300 moments of 30 vectors (28.2 with predicated additions); three 24.7, two
+ * 30.6, five 25.9, four with half a row's gathers in flight 26.7. */
 constexpr int kKpmPerSm = 4; /* 64 registers, every gather of a row in flight */
 static int kpm_resident() { return kKpmPerSm * ctx().sms; } /* the blocks sweep the rows together */
 
@@ -1201,13 +1201,13 @@ __global__ void __launch_bounds__(kThreads, kKpmPerSm)
       double2 xv[B];
 #pragma unroll
       for (int u = 0; u < B; u++) {
-        xv[u] = x;
-        if (!(K > 0 && j0 + u == K / 2) && ((m >> (j0 + u)) & 1u))
-          xv[u] = Xk[me + (long)S.off[j0 + u] * L];
+        xv[u] = make_double2(0.0, 0.0); /* what a row lacks changes no sum (K: finite values) */
+        if ((m >> (j0 + u)) & 1u)
+          xv[u] = K > 0 && j0 + u == K / 2 ? x : Xk[me + (long)S.off[j0 + u] * L];
       }
 #pragma unroll
       for (int u = 0; u < B; u++)
-        if ((m >> (j0 + u)) & 1u) {
+        if (K > 0 || ((m >> (j0 + u)) & 1u)) {
           r0.add(S.val[j0 + u], xv[u].x);
           r1.add(S.val[j0 + u], xv[u].y);
         }
@@ -2628,8 +2628,8 @@ int kpm_reduce(const pevsl_devcsr *A, int s, int steps, const double *part, doub
  * 16 bytes per row and vector.  In the stencil form the matrix costs nothing,
  * so a group holds what stays in L2 from one degree to the next (72 MB of
  * 126), the groups about equal: 101 x 100 x 99, 300 moments of 30 vectors, in
- * groups of 4 28.2 ms, of 8 28.8, of 2 31.7, all 30 26.8 at first and 30.0 in
- * a loop; 64 x 65 x 63 of 16 7.6, all 30 7.65.  Where not even two fit, and
+ * groups of 4 25.0 ms, of 8 28.4, of 2 28.3, all 30 27.0; 64 x 65 x 63 of 16
+ * 6.8, all 30 7.3.  Where not even two fit, and
  * for a matrix whose entries each group would read again, as many as a launch
  * takes (64). */
 int kpm_group(const pevsl_devcsr *A, int nvec) {
